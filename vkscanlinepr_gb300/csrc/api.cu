@@ -106,11 +106,10 @@ enum Ctl : int {
     CTL_CHAINS = 4,    // chain counter
     CTL_LONG = 8,      // long-piece counter
     CTL_QUEUE = 9,     // chain work-queue counter
-    CTL_WIDE = 10,     // chains solved by a whole warp
-    CTL_WIDE_QUEUE = 11,    // their work-queue counter
-    CTL_WIDE_CURVES = 12,   // curves with such a chain
     CTL_ROW_SCAN = 13,      // row-start scan's tile counter
-    CTL_WORDS = 16,
+    CTL_CLASSES = 16,       // chains of each class
+    CTL_CLASS_NEXT = CTL_CLASSES + sr::kChainClassWords,
+    CTL_WORDS = CTL_CLASS_NEXT + sr::kChainClassWords,
 };
 
 std::atomic<uint64_t> g_launches{0};
@@ -292,8 +291,7 @@ struct Pipeline {
     DevBuf pos, pos_path, curve_pos, curve_type, curve_path, fill_rule, fill_info, path_scene, scenes_d, cta_base_d;
     DevBuf cta_narrow_d;
     // frame
-    DevBuf tpos, path_visible, cut, count, offs, ctl, scan_status, pieces, chain_lists, chain_sort_scratch, long_list;
-    DevBuf curve_wide, wide_curves;
+    DevBuf tpos, path_visible, cut, count, offs, ctl, scan_status, pieces, chain_lists, long_list;
     DevBuf cbuf, rec, keys, keys_alt, wnp, skeys, svals, vals_alt, sort_scratch, wind_status, draw, draw_row, totals;
     DevBuf rkeys, rvals, rkeys_alt, rvals_alt, row_sort_scratch, row_start, seg_cut, row_count, row_px, row_scan, image;
     DevBuf d_fkey, d_fwn, d_fleft, d_wscan, d_fflag, d_sflag, d_skey;
@@ -327,25 +325,16 @@ struct Pipeline {
     cudaEvent_t ev[2 * ST_COUNT_ALL] = {};
     bool ev_pending = false, capturing = false;
     cudaStream_t cur = nullptr;
-    // second stream of a frame (lowest priority): the chains other than the
-    // wide ones, and their curves' merge and fragments, run on it beside the
-    // wide chains on the frame's stream (forked and joined by events)
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_merged = nullptr, ev_join = nullptr;
 
     ~Pipeline() {
         DevBuf* all[] = {&pos, &pos_path, &curve_pos, &curve_type, &curve_path, &fill_rule, &fill_info, &path_scene,
                          &scenes_d, &cta_base_d, &tpos, &path_visible, &cut, &count, &offs, &ctl, &scan_status,
-                         &pieces, &chain_lists, &chain_sort_scratch, &long_list, &cbuf, &rec, &keys, &keys_alt,
+                         &pieces, &chain_lists, &long_list, &cbuf, &rec, &keys, &keys_alt,
                          &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_status, &draw, &draw_row, &totals,
                          &rkeys, &rvals, &rkeys_alt, &rvals_alt, &row_sort_scratch, &row_start, &seg_cut, &row_count, &row_px,
                          &row_scan, &image, &d_fkey, &d_fwn, &d_fleft, &d_wscan, &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw,
-                         &feats, &preds, &allot, &plan_tot, &judge_out, &seg_scratch, &seg_tiles, &curve_wide,
-                         &wide_curves, &cta_narrow_d, &paints_d, &aa_acc};
+                         &feats, &preds, &allot, &plan_tot, &judge_out, &seg_scratch, &seg_tiles, &cta_narrow_d, &paints_d, &aa_acc};
         for (DevBuf* b : all) release(*b);
-        for (cudaEvent_t e : {ev_fork, ev_merged, ev_join})
-            if (e) cudaEventDestroy(e);
-        if (side) cudaStreamDestroy(side);
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
         if (h_u32) cudaFreeHost(h_u32);
@@ -398,23 +387,14 @@ struct Pipeline {
         CUDA_TRY(cudaMallocHost(&h_u64, sizeof(uint64_t) * 4));
         CUDA_TRY(ensure(ctl, sizeof(uint32_t) * CTL_WORDS));
         CUDA_TRY(sr::geom_init());
-        // the side stream takes the lowest priority: when both streams'
-        // chain kernels become ready at once, the caller's stream, which
-        // carries the wide chains (the frame's longest dependency), is
-        // placed first
-        int lo_prio = 0, hi_prio = 0;
-        CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio));
-        CUDA_TRY(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, lo_prio));
-        for (cudaEvent_t* e : {&ev_fork, &ev_merged, &ev_join})
-            CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         return SR_OK;
     }
 
-    void mark(int stage, bool end, cudaStream_t on = nullptr) {
+    void mark(int stage, bool end) {
         if (!(flags & SR_FLAG_PROFILE) || capturing) return;
         cudaEvent_t& e = ev[2 * stage + (end ? 1 : 0)];
         if (!e) cudaEventCreate(&e);
-        cudaEventRecord(e, on ? on : cur);
+        cudaEventRecord(e, cur);
     }
 
     sr::KeyLayout layout() const {
@@ -603,17 +583,13 @@ struct Pipeline {
         const uint32_t lc = list_cap();
         cw.pieces = pieces.as<uint4>();
         cw.chain_items = cl;
-        cw.chain_keys = cl + lc;
-        cw.sorted_items = cl + 2 * (size_t)lc;
-        cw.sorted_keys = cl + 3 * (size_t)lc;
+        cw.sorted_items = cl + lc;
+        cw.chain_keys = reinterpret_cast<uint8_t*>(cl + 2 * (size_t)lc);
         cw.list_cap = lc;
         cw.chain_count = ctlp + CTL_CHAINS;
+        cw.class_count = ctlp + CTL_CLASSES;
+        cw.class_next = ctlp + CTL_CLASS_NEXT;
         cw.chain_queue = ctlp + CTL_QUEUE;
-        cw.wide_count = ctlp + CTL_WIDE;
-        cw.wide_queue = ctlp + CTL_WIDE_QUEUE;
-        cw.curve_wide = curve_wide.as<uint8_t>();
-        cw.wide_curves = wide_curves.as<uint32_t>();
-        cw.wide_curve_count = ctlp + CTL_WIDE_CURVES;
         cw.long_list = long_list.as<uint32_t>();
         cw.long_count = ctlp + CTL_LONG;
         return cw;
@@ -629,12 +605,8 @@ struct Pipeline {
         CUDA_TRY(ensure(scan_status, sizeof(uint64_t) * sr::scan_status_words(C)));
         CUDA_TRY(ensure(pieces, sr::piece_table_bytes(std::max<uint32_t>(C, 1))));
         const uint32_t lc = list_cap();
-        CUDA_TRY(ensure(chain_lists, sizeof(uint32_t) * 6 * (size_t)lc));
+        CUDA_TRY(ensure(chain_lists, 9 * (size_t)lc));
         CUDA_TRY(ensure(long_list, sizeof(uint32_t) * (size_t)lc));
-        CUDA_TRY(ensure(curve_wide, std::max<size_t>(C, 1)));
-        CUDA_TRY(ensure(wide_curves, sizeof(uint32_t) * std::max<size_t>(C, 1)));
-        sr::SortPlan cp = sr::sort_plan(lc, sr::chain_key_bits(), ctl.as<uint32_t>() + CTL_CHAINS);
-        CUDA_TRY(ensure(chain_sort_scratch, sr::sort_scratch_bytes(cp)));
         CUDA_TRY(ensure(totals, sizeof(uint64_t) * 4));
         CUDA_TRY(ensure(row_start, sizeof(int32_t) * ((size_t)total_rows + 1)));
         CUDA_TRY(ensure(seg_cut, sizeof(uint32_t) * std::max<size_t>(cut_words(), 1)));
@@ -713,8 +685,7 @@ struct Pipeline {
         add(8 * v1); add(4 * p1); add(20 * c1); add(4 * (c1 + 1)); add(4 * (c1 + 1));
         add(8 * sr::scan_status_words(C)); add(sr::piece_table_bytes((uint32_t)c1));
         const size_t lc = list_cap();
-        add(4 * 6 * lc); add(4 * lc);
-        add(sr::sort_scratch_bytes(sr::sort_plan((int64_t)lc, sr::chain_key_bits(), nullptr)));
+        add(9 * lc); add(4 * lc);
         add(32); add(4 * ((size_t)total_rows + 1));
         post_count_buffers(cap, dcap, [&](DevBuf&, size_t b) { add(b); });
         return total;
@@ -738,7 +709,7 @@ struct Pipeline {
             &Pipeline::curve_path, &Pipeline::fill_rule, &Pipeline::fill_info, &Pipeline::path_scene,
             &Pipeline::scenes_d, &Pipeline::cta_base_d, &Pipeline::tpos, &Pipeline::path_visible, &Pipeline::cut,
             &Pipeline::count, &Pipeline::offs, &Pipeline::ctl, &Pipeline::scan_status, &Pipeline::pieces,
-            &Pipeline::chain_lists, &Pipeline::chain_sort_scratch, &Pipeline::long_list, &Pipeline::cbuf,
+            &Pipeline::chain_lists, &Pipeline::long_list, &Pipeline::cbuf,
             &Pipeline::rec, &Pipeline::keys, &Pipeline::keys_alt, &Pipeline::wnp, &Pipeline::skeys,
             &Pipeline::svals, &Pipeline::vals_alt, &Pipeline::sort_scratch, &Pipeline::wind_status,
             &Pipeline::draw, &Pipeline::draw_row, &Pipeline::totals, &Pipeline::rkeys, &Pipeline::rvals,
@@ -746,7 +717,7 @@ struct Pipeline {
             &Pipeline::seg_cut, &Pipeline::row_count, &Pipeline::row_px, &Pipeline::row_scan, &Pipeline::image,
             &Pipeline::path_first, &Pipeline::path_draw, &Pipeline::feats, &Pipeline::preds, &Pipeline::allot,
             &Pipeline::plan_tot, &Pipeline::judge_out, &Pipeline::seg_scratch, &Pipeline::seg_tiles,
-            &Pipeline::curve_wide, &Pipeline::wide_curves, &Pipeline::cta_narrow_d};
+            &Pipeline::cta_narrow_d};
         *moved = false;
         CUDA_TRY(cudaSetDevice(device));
         for (DevBuf Pipeline::* b : bufs) {
@@ -772,15 +743,14 @@ struct Pipeline {
     uint64_t held_bytes() const {
         const DevBuf* all[] = {&pos, &pos_path, &curve_pos, &curve_type, &curve_path, &fill_rule, &fill_info,
                                &path_scene, &scenes_d, &cta_base_d, &tpos, &path_visible, &cut, &count, &offs,
-                               &ctl, &scan_status, &pieces, &chain_lists, &chain_sort_scratch, &long_list, &cbuf,
+                               &ctl, &scan_status, &pieces, &chain_lists, &long_list, &cbuf,
                                &rec, &keys, &keys_alt, &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_status,
                                &draw, &draw_row, &totals, &rkeys, &rvals, &rkeys_alt, &rvals_alt,
                                &row_sort_scratch, &row_start, &seg_cut, &row_count, &row_px, &row_scan, &image, &d_fkey,
                                &d_fwn, &d_fleft,
                                &d_wscan,
                                &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw, &feats, &preds, &allot,
-                               &plan_tot, &judge_out, &seg_scratch, &seg_tiles, &curve_wide, &wide_curves,
-                               &cta_narrow_d};
+                               &plan_tot, &judge_out, &seg_scratch, &seg_tiles, &cta_narrow_d};
         uint64_t t = 0;
         for (const DevBuf* b : all) t += b->cap;
         return t;
@@ -826,13 +796,8 @@ struct Pipeline {
         mark(ST_TRANSFORM, true);
         const GeomArgs g = geom(0);
         const ChainWork cw = chain_work();
-        const uint32_t lc = list_cap();
-        SortPlan cp = sort_plan(lc, chain_key_bits(), ctlp + CTL_CHAINS);
-        uint32_t* cl = chain_lists.as<uint32_t>();
         mark(ST_COUNT, false);
         launch_count(g, cut.as<float>(), count.as<int32_t>(), cw, status, st);
-        launch_sort_u32(cp, cw.chain_keys, cw.chain_items, cw.sorted_keys, cw.sorted_items, cl + 4 * (size_t)lc,
-                        cl + 5 * (size_t)lc, chain_sort_scratch.p, status, st);
         mark(ST_COUNT, true);
         mark(ST_SCAN, false);
         launch_exclusive_scan_i32(count.as<int32_t>(), offs.as<int32_t>(), C, scan_status.as<uint64_t>(),
@@ -862,35 +827,16 @@ struct Pipeline {
             dbg.fleft = d_fleft.as<int32_t>();
             CUDA_TRY(cudaMemsetAsync(d_wscan.p, 0, sizeof(int32_t) * ((size_t)std::max<int64_t>(cap, 1) + 1), st));
         }
-        // The wide chains -- the frame's longest dependency -- and their
-        // curves' merge and fragments stay on st, right behind the count
-        // pass, so that they start first; the other chains, merge and
-        // fragments run on the side stream beside them.  st's merge waits for
-        // the side stream's (which marks the wide curves' records pending and
-        // covers the short chains of the wide curves), and st waits for the
-        // side stream before the sort.
-        CUDA_TRY(cudaEventRecord(ev_fork, st));
-        CUDA_TRY(cudaStreamWaitEvent(side, ev_fork, 0));
-        mark(ST_WIDE, false, st);
-        launch_chains(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), sm_count, 0, st);
-        mark(ST_CHAINS, false, side);
-        launch_chains(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), sm_count, 1, side);
-        mark(ST_CHAINS, true, side);
-        mark(ST_MERGE, false, side);
-        launch_merge(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), rec.as<int2>(), status, 0, side);
-        mark(ST_MERGE, true, side);
-        CUDA_TRY(cudaEventRecord(ev_merged, side));
-        CUDA_TRY(cudaStreamWaitEvent(st, ev_merged, 0));
-        launch_merge(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), rec.as<int2>(), status, 1, st);
-        mark(ST_FRAGMENT, false, side);
+        mark(ST_CHAINS, false);
+        launch_chains(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), sm_count, st);
+        mark(ST_CHAINS, true);
+        mark(ST_MERGE, false);
+        launch_merge(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), rec.as<int2>(), status, st);
+        mark(ST_MERGE, true);
+        mark(ST_FRAGMENT, false);
         launch_fragment(g, rec.as<int2>(), offs.as<int32_t>(), cap, n_dev, keys.as<uint64_t>(),
-                        keep ? wnp.as<uint8_t>() : nullptr, dbg, cw, 0, side);
-        mark(ST_FRAGMENT, true, side);
-        launch_fragment(g, rec.as<int2>(), offs.as<int32_t>(), cap, n_dev, keys.as<uint64_t>(),
-                        keep ? wnp.as<uint8_t>() : nullptr, dbg, cw, 1, st);
-        mark(ST_WIDE, true, st);
-        CUDA_TRY(cudaEventRecord(ev_join, side));
-        CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
+                        keep ? wnp.as<uint8_t>() : nullptr, dbg, st);
+        mark(ST_FRAGMENT, true);
         const KeyLayout L = g.L;
         SortPlan sp = sort_plan(cap, L.pbits + L.rbits + L.xbits, n_dev, tune.sort_items);
         mark(ST_SORT, false);

@@ -6,6 +6,8 @@
 // gen_fragment.comp           -> k_intersect_fragment (one pass: each
 //                                intersection record's fragment is built as
 //                                soon as the next record's t is known)
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -155,6 +157,9 @@ SR_DEV int32_t cut_range(int32_t size, int32_t F, int32_t& b, int32_t& e) {
 constexpr int kMaxPieces = 5;
 // Pieces with at least this many records are merged by a whole CTA.
 constexpr int32_t kLongPiece = 64;
+// A lane of a split chain takes at least 1 << kSegLog bisected roots.
+constexpr int32_t kSegLog = 4;
+constexpr int kChainCtas = 8;   // of four warps, an SM
 
 // Piece record layout in the output: [t0][x crossings][y crossings], the
 // crossing values of each side solved by one chain (k_chains), then merged
@@ -165,12 +170,12 @@ SR_DEV uint32_t pack_n(int32_t nx, bool xneg, int32_t ny, bool yneg) {
 SR_DEV int32_t piece_nx(uint32_t n) { return (int32_t)(n & 0x7FFFu); }
 SR_DEV int32_t piece_ny(uint32_t n) { return (int32_t)((n >> 16) & 0x7FFFu); }
 
-// Sort key of a chain: longest length class first (so the longest dependency
-// chains start in the first wave of k_chains), then cubic, quadric, line, so
-// that a warp runs one curve type with lengths within a factor of 2.  A line
-// root is a closed form, far cheaper than a 24-step bisection, so a line
-// chain is classed 7 length classes lower (at most class 7, below every
-// wide chain).
+// Class of a chain: longest length class first (so the longest chains start
+// in the first wave of k_chains), then cubic, quadric, line, arc, so that a
+// warp runs one curve type with lengths within a factor of 2.  A line root is
+// a closed form, far cheaper than a 24-step bisection, so a line chain is
+// classed 7 length classes lower.
+constexpr uint32_t kChainClasses = 64;
 SR_DEV uint32_t chain_key(int32_t len, uint32_t type) {
     uint32_t lg = 31u - (uint32_t)__clz(len);
     if (lg > 14u) lg = 14u;
@@ -178,10 +183,13 @@ SR_DEV uint32_t chain_key(int32_t len, uint32_t type) {
     uint32_t cls = type == 4u ? 0u : (type == 3u ? 1u : (type == kArc ? 3u : 2u));
     return ((14u - lg) << 2) | cls;
 }
-// Cubic, quadric and arc chains of >= 512 bisected roots (class >= 9) are solved
-// by a whole warp each (run_chain_warp); they sort before every other chain.
-SR_DEV bool chain_key_wide(uint32_t key) { return (key >> 2) <= 14u - 9u && (key & 3u) != 2u; }
-constexpr uint32_t kChainKeyBits = 6;
+// log2 of the lanes that share a chain of this class (run_segments): a lane
+// takes 16 to 31 bisected roots, or 512 to 1,023 line roots, as far as 32
+// lanes go.
+SR_DEV uint32_t chain_lanes_log(uint32_t key) {
+    const int32_t lg = 14 - (int32_t)(key >> 2);
+    return (uint32_t)imin(imax((key & 3u) == 2u ? lg - 2 : lg - kSegLog, 0), 5);
+}
 
 // get_xy_begin_end_delta + udpate_cut_range for one axis
 // (make_intersection_1.comp:150-213): number of grid crossings, first
@@ -210,15 +218,17 @@ SR_DEV int32_t axis_range_rd(float a0, float a1, int32_t size, int32_t F, float&
 // x and y crossing chains, which are appended with their sort keys.
 __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restrict__ cut_cache,
                                                int32_t* __restrict__ count, uint4* __restrict__ pieces,
-                                               uint32_t* __restrict__ chain_items, uint32_t* __restrict__ chain_keys,
+                                               uint32_t* __restrict__ chain_items, uint8_t* __restrict__ chain_keys,
                                                uint32_t list_cap, uint32_t* __restrict__ chain_count,
-                                               uint32_t* __restrict__ wide_count,
-                                               uint8_t* __restrict__ curve_wide, uint32_t* __restrict__ wide_curves,
-                                               uint32_t* __restrict__ wide_curve_count,
+                                               uint32_t* __restrict__ class_count,
                                                uint32_t* __restrict__ long_list, uint32_t* __restrict__ long_count,
                                                uint32_t* __restrict__ status) {
+    __shared__ uint32_t s_hist[kChainClasses], s_total, s_base;
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = c < g.n_curves;
+    if (threadIdx.x < kChainClasses) s_hist[threadIdx.x] = 0;
+    if (threadIdx.x == kChainClasses) s_total = 0;
+    __syncthreads();
     uint32_t my_chains[2 * kMaxPieces];
     uint32_t my_key[2 * kMaxPieces];
     int n_chains = 0;
@@ -354,10 +364,6 @@ __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restri
         }
         count[c] = pc;
         if (walk != pc) set_error(status, ERR_RECORD_RANGE);
-        bool wide = false;
-        for (int k = 0; k < n_chains; ++k) wide |= chain_key_wide(my_key[k]);
-        curve_wide[c] = wide ? 1 : 0;
-        if (wide) wide_curves[atomicAdd(wide_curve_count, 1u)] = c;
     }
     // append long pieces (warp-aggregated)
     const uint32_t lane = lane_id();
@@ -375,27 +381,73 @@ __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restri
             else set_error(status, ERR_CAPACITY);
         }
     }
-    // append the chains with their sort keys (warp-aggregated)
-    for (int k = 0; k < 2 * kMaxPieces; ++k) {
-        bool has = k < n_chains;
-        uint32_t m = __ballot_sync(0xFFFFFFFFu, has);
-        if (!m) break;
-        uint32_t leader = (uint32_t)(__ffs(m) - 1);
-        uint32_t base = 0;
-        const uint32_t wm = __ballot_sync(0xFFFFFFFFu, has && chain_key_wide(my_key[k]));
-        if (lane == leader) {
-            base = atomicAdd(chain_count, (uint32_t)__popc(m));
-            if (wm) atomicAdd(wide_count, (uint32_t)__popc(wm));
+    // append the chains with their classes, and count the classes (one
+    // append and at most one add per class for the CTA)
+    uint32_t at = 0;
+    if (n_chains) at = atomicAdd(&s_total, (uint32_t)n_chains);
+    for (int k = 0; k < n_chains; ++k) atomicAdd(&s_hist[my_key[k]], 1u);
+    __syncthreads();
+    if (threadIdx.x < kChainClasses && s_hist[threadIdx.x]) atomicAdd(&class_count[threadIdx.x], s_hist[threadIdx.x]);
+    if (threadIdx.x == kChainClasses && s_total) s_base = atomicAdd(chain_count, s_total);
+    __syncthreads();
+    for (int k = 0; k < n_chains; ++k) {
+        const uint32_t slot = s_base + at + (uint32_t)k;
+        if (slot < list_cap) {
+            chain_items[slot] = my_chains[k];
+            chain_keys[slot] = (uint8_t)my_key[k];
+        } else {
+            set_error(status, ERR_CAPACITY);
         }
-        base = __shfl_sync(0xFFFFFFFFu, base, leader);
-        if (has) {
-            uint32_t slot = base + (uint32_t)__popc(m & lanemask_lt());
-            if (slot < list_cap) {
-                chain_items[slot] = my_chains[k];
-                chain_keys[slot] = my_key[k];
-            } else {
-                set_error(status, ERR_CAPACITY);
-            }
+    }
+}
+
+// First list position of each class: an exclusive scan of the class counts
+// by one warp (two classes a lane).
+SR_DEV void class_starts(const uint32_t* __restrict__ class_count, uint32_t& s0, uint32_t& s1) {
+    const uint32_t lane = lane_id();
+    const uint32_t a = class_count[2 * lane], b = class_count[2 * lane + 1];
+    uint32_t x = a + b;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+        if ((int)lane >= d) x += y;
+    }
+    s0 = x - a - b;
+    s1 = s0 + a;
+}
+
+// Orders the chains by class (in no order within one): a counting sort whose
+// counts the count pass made, so one launch.  The radix sort that it
+// replaced took five (two clears, histogram, scan, pass).
+__global__ void __launch_bounds__(256) k_order_chains(const uint32_t* __restrict__ items,
+                                                      const uint8_t* __restrict__ keys, uint32_t list_cap,
+                                                      const uint32_t* __restrict__ chain_count,
+                                                      const uint32_t* __restrict__ class_count,
+                                                      uint32_t* __restrict__ class_next, uint32_t* __restrict__ sorted) {
+    __shared__ uint32_t s_start[kChainClasses], s_hist[kChainClasses], s_at[kChainClasses];
+    const uint32_t n = imin((int32_t)*chain_count, (int32_t)list_cap);
+    if (threadIdx.x < 32) {
+        uint32_t a, b;
+        class_starts(class_count, a, b);
+        s_start[2 * threadIdx.x] = a;
+        s_start[2 * threadIdx.x + 1] = b;
+    }
+    for (uint32_t i0 = blockIdx.x * 256u; i0 < n; i0 += gridDim.x * 256u) {
+        if (threadIdx.x < kChainClasses) s_hist[threadIdx.x] = 0;
+        __syncthreads();
+        const uint32_t i = i0 + threadIdx.x;
+        uint32_t key = 0, rank = 0;
+        if (i < n) {
+            key = keys[i];
+            rank = atomicAdd(&s_hist[key], 1u);
+        }
+        __syncthreads();
+        if (threadIdx.x < kChainClasses && s_hist[threadIdx.x])
+            s_at[threadIdx.x] = s_start[threadIdx.x] + atomicAdd(&class_next[threadIdx.x], s_hist[threadIdx.x]);
+        __syncthreads();
+        if (i < n) {
+            const uint32_t o = s_at[key] + rank;
+            if (o < list_cap) sorted[o] = items[i];
         }
     }
 }
@@ -465,25 +517,21 @@ SR_DEV float bisect(const AxisPoly& a, float c, float t_min, float t_max) {
     return t_solve;
 }
 
-template <int kType>
-SR_DEV void run_chain(const AxisPoly& a, int32_t len, float x, float dx, float t_lo, float t_hi, int side,
-                      int32_t* __restrict__ out) {
-    float lo = t_lo;
-    float inv = 0.0f;
-    if (kType == 2) {
-        float d = __fsub_rn(a.p1, a.p0);
-        inv = (d != 0.0f) ? __fdiv_rn(1.0f, d) : 0.0f;
-    }
-    for (int32_t k = 0; k < len; ++k) {
-        float c = x;
-        x = __fadd_rn(x, dx);
-        float t;
-        if (kType == 2) t = gmin(gmax(__fmul_rn(__fsub_rn(c, a.p0), inv), lo), t_hi);
-        else t = bisect<kType>(a, c, lo, t_hi);
-        int32_t ob = (fbits(t) & ~3) | side;
-        out[k] = ob;
-        lo = bitsf(ob);
-    }
+// The state after root k of a chain whose state before it is lo: its t with
+// the side bit in the flag bits.
+struct ChainSide {
+    AxisPoly a;
+    float inv;            // 1 / (p1 - p0) of a line
+    float x, dx, t_hi;    // first grid line, step, end of the piece
+    int side;
+};
+template <int kType> SR_DEV int32_t next_root(const ChainSide& s, int32_t k, int32_t lo) {
+    // x + k dx: whole numbers below 2^15, exact like the repeated sum
+    const float c = __fadd_rn(s.x, __fmul_rn((float)k, s.dx));
+    float t;
+    if (kType == 2) t = gmin(gmax(__fmul_rn(__fsub_rn(c, s.a.p0), s.inv), bitsf(lo)), s.t_hi);
+    else t = bisect<kType>(s.a, c, bitsf(lo), s.t_hi);
+    return (fbits(t) & ~3) | s.side;
 }
 
 // Warp-cooperative solve of one long chain.  By the invariant above, the 31
@@ -582,34 +630,96 @@ SR_DEV float bisect_warp(const AxisPoly& a, float c, float t_min, float t_max, c
     return eq0 ? t_min : t;
 }
 
-// A chain solved by the whole warp; lane k%32 keeps root k until 32 roots
-// are stored at once.
+// The rest of run_segments for a chain of 32 lanes some of which disagree:
+// the first stretch whose entry state is not its neighbour's end is solved
+// root by root by the whole warp, until the state meets a root that is there
+// already, and so on to the next.
 template <int kType>
-SR_DEV void run_chain_warp(const AxisPoly& a, int32_t len, float x, float dx, float t_lo, float t_hi, int side,
-                           int32_t* __restrict__ out, const TreeLane& tl) {
-    const uint32_t lane = lane_id();
-    float lo = t_lo;
-    int32_t keep = 0;
-    for (int32_t k = 0; k < len; ++k) {
-        const float c = x;
-        x = __fadd_rn(x, dx);
-        const float t = bisect_warp<kType>(a, c, lo, t_hi, tl);
-        const int32_t ob = (fbits(t) & ~3) | side;
-        if ((uint32_t)(k & 31) == lane) keep = ob;
-        if ((k & 31) == 31 || k + 1 == len) {
-            const int32_t k0 = k & ~31;
-            if ((int32_t)lane <= (k - k0)) out[k0 + (int32_t)lane] = keep;
+SR_DEV void finish_chain_warp(const ChainSide& s, int32_t len, int32_t seg, int32_t* __restrict__ out, int32_t entry,
+                              int32_t end) {
+    const int32_t lane = (int32_t)lane_id();
+    const TreeLane tl = tree_lane((uint32_t)lane);
+    for (;;) {
+        const int32_t prev = __shfl_up_sync(0xFFFFFFFFu, end, 1);
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, lane > 0 && lane * seg < len && prev != entry);
+        if (!m) return;
+        const int32_t f = __ffs(m) - 1;
+        int32_t st = __shfl_sync(0xFFFFFFFFu, prev, f);
+        if (lane == f) entry = st;
+        const int32_t k1 = imin((f + 1) * seg, len);
+        bool met = false;
+        for (int32_t k = f * seg; k < k1 && !met; ++k) {
+            const float c = __fadd_rn(s.x, __fmul_rn((float)k, s.dx));
+            const float t = bisect_warp<kType>(s.a, c, bitsf(st), s.t_hi, tl);
+            st = (fbits(t) & ~3) | s.side;
+            met = out[k] == st;
+            __syncwarp();
+            if (lane == 0) out[k] = st;
         }
-        lo = bitsf(ob);
+        if (lane == f && !met) end = st;
+        __syncwarp();
+    }
+}
+
+// One chain by `lanes` lanes, lane l of them taking the roots [ks, ke) of
+// its stretch.  A root depends on the one before it only through the low end
+// of its interval, and by little: the 24 steps end within 2^-24 of the
+// interval from the crossing wherever they start, and the state keeps t to
+// 4 ulp.  So two chains started from different low ends soon hold the same
+// state (on the generated scenes, after two roots in 95% of the cases; later
+// for t under an eighth of the piece, where 4 ulp is finer than the steps'
+// end).  Each lane starts two roots before its stretch from the piece's own
+// start and solves on from there; then every lane whose state at its
+// stretch's start is not the one its left neighbour ended with solves again
+// from that one, until it meets a root it already has.  Rounds of this end
+// when all neighbours agree, which makes every root the one that the
+// sequential chain gives.  A chain of 32 lanes that has not settled after
+// two rounds (its t small all along) is finished root by root by the warp.
+template <int kType>
+SR_DEV void run_segments(const ChainSide& s, int32_t len, float t_lo, int32_t* __restrict__ out, int32_t lanes,
+                         int32_t l) {
+    const int32_t seg = (len + lanes - 1) / lanes;
+    const int32_t ks = imin(l * seg, len), ke = imin(ks + seg, len);
+    int32_t st = fbits(t_lo);
+    if (ks < ke)
+        for (int32_t k = imax(ks - 2, 0); k < ks; ++k) st = next_root<kType>(s, k, st);
+    int32_t entry = st;
+    for (int32_t k = ks; k < ke; ++k) {
+        st = next_root<kType>(s, k, st);
+        out[k] = st;
+    }
+    int32_t end = st;
+    __syncwarp();
+    for (int round = 0;; ++round) {
+        const int32_t prev = __shfl_up_sync(0xFFFFFFFFu, end, 1);
+        const bool need = l > 0 && ks < ke && prev != entry;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, need);
+        if (!m) return;
+        if (kType != 2 && lanes == 32 && round >= 2) {
+            finish_chain_warp<kType>(s, len, seg, out, entry, end);
+            return;
+        }
+        if (need) {
+            entry = prev;
+            st = prev;
+            bool met = false;
+            for (int32_t k = ks; k < ke; ++k) {
+                st = next_root<kType>(s, k, st);
+                met = out[k] == st;
+                if (met) break;
+                out[k] = st;
+            }
+            if (!met) end = st;
+        }
+        __syncwarp();
     }
 }
 
 struct ChainSetup {
-    AxisPoly a;
+    ChainSide side;
     uint32_t type;
     int32_t len;
-    float x, dx, t_lo, t_hi;
-    int side;
+    float t_lo;
     int64_t base;
 };
 
@@ -619,80 +729,89 @@ SR_DEV ChainSetup chain_setup(const GeomArgs& g, const int32_t* __restrict__ off
                               uint32_t item) {
     ChainSetup s;
     const uint32_t c = item >> 4, piece = (item >> 1) & 7u;
-    s.side = (int)(item & 1u);
+    const int side = (int)(item & 1u);
+    s.side.side = side;
     s.type = g.curve_type[c];
     const uint4* pt = pieces + (size_t)c * kMaxPieces;
     int64_t base = offs[c];
     for (uint32_t j = 0; j < piece; ++j) base += 1 + piece_nx(pt[j].x) + piece_ny(pt[j].x);
     const uint4 me = pt[piece];
     const int32_t nx = piece_nx(me.x), ny = piece_ny(me.x);
-    s.base = base + 1 + (s.side ? nx : 0);
-    s.len = s.side ? ny : nx;
-    const bool neg = s.side ? (me.x & 0x80000000u) != 0 : (me.x & 0x8000u) != 0;
-    s.x = __uint_as_float(s.side ? me.w : me.z);
-    s.dx = neg ? -(float)g.F : (float)g.F;
+    s.base = base + 1 + (side ? nx : 0);
+    s.len = side ? ny : nx;
+    const bool neg = side ? (me.x & 0x80000000u) != 0 : (me.x & 0x8000u) != 0;
+    s.side.x = __uint_as_float(side ? me.w : me.z);
+    s.side.dx = neg ? -(float)g.F : (float)g.F;
     s.t_lo = piece == 0 ? 0.0f : __uint_as_float(pt[piece - 1].y);
-    s.t_hi = __uint_as_float(me.y);
+    s.side.t_hi = __uint_as_float(me.y);
     const float2* cp = g.tpos + g.curve_pos[c];
     const uint32_t np = curve_slots(s.type);
     float p[4];
 #pragma unroll
     for (uint32_t k = 0; k < 4; ++k) {
         float2 v = k < np ? cp[k] : make_float2(0.0f, 0.0f);
-        p[k] = s.side ? v.y : v.x;
+        p[k] = side ? v.y : v.x;
     }
-    s.a.p0 = p[0]; s.a.p1 = p[1]; s.a.p2 = p[2]; s.a.p3 = p[3];
-    s.a.d01 = __fsub_rn(p[1], p[0]);
-    s.a.d12 = __fsub_rn(p[2], p[1]);
-    s.a.d23 = __fsub_rn(p[3], p[2]);
+    AxisPoly& a = s.side.a;
+    a.p0 = p[0]; a.p1 = p[1]; a.p2 = p[2]; a.p3 = p[3];
+    a.d01 = __fsub_rn(p[1], p[0]);
+    a.d12 = __fsub_rn(p[2], p[1]);
+    a.d23 = __fsub_rn(p[3], p[2]);
+    s.side.inv = s.type == 2u && a.d01 != 0.0f ? __fdiv_rn(1.0f, a.d01) : 0.0f;
     return s;
 }
 
-// Part 0 solves the wide chains (first in the list), one per warp; part 1
-// the others in groups of 32 in list order, so the longest groups go to the
-// first warp of every SM rather than to one block.  The two parts run on two
-// streams at once.
+// Every warp takes tickets, longest class first: a ticket is 32 / lanes
+// chains of one class (chain_lanes_log).
 __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t* __restrict__ offs,
                                                 const uint4* __restrict__ pieces,
-                                                const uint32_t* __restrict__ items, const uint32_t* __restrict__ keys,
-                                                uint32_t list_cap, const uint32_t* __restrict__ chain_count,
-                                                const uint32_t* __restrict__ wide_count,
-                                                uint32_t* __restrict__ queue, int32_t* __restrict__ cbuf, int part) {
-    const uint32_t total = imin((int32_t)*chain_count, (int32_t)list_cap);
-    const uint32_t n_wide = imin((int32_t)*wide_count, (int32_t)total);
+                                                const uint32_t* __restrict__ items, uint32_t list_cap,
+                                                const uint32_t* __restrict__ class_count,
+                                                uint32_t* __restrict__ queue, int32_t* __restrict__ cbuf) {
     const uint32_t lane = lane_id();
-    if (part == 0) {
-        const TreeLane tl = tree_lane(lane);
-        for (;;) {
-            uint32_t ticket = 0;
-            if (lane == 0) ticket = atomicAdd(queue, 1u);
-            ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
-            if (ticket >= n_wide) break;
-            const ChainSetup s = chain_setup(g, offs, pieces, items[ticket]);
-            if (s.base + s.len > g.rec_cap) continue;   // overflow: k_merge reports it
-            int32_t* out = cbuf + s.base;
-            if (s.type == 4u) run_chain_warp<4>(s.a, s.len, s.x, s.dx, s.t_lo, s.t_hi, s.side, out, tl);
-            else if (s.type == 3u) run_chain_warp<3>(s.a, s.len, s.x, s.dx, s.t_lo, s.t_hi, s.side, out, tl);
-            else if (s.type == kArc)
-                run_chain_warp<(int)kArc>(s.a, s.len, s.x, s.dx, s.t_lo, s.t_hi, s.side, out, tl);
-        }
-        return;
+    // first ticket and list position of each class, two classes a lane
+    uint32_t start0, start1;
+    class_starts(class_count, start0, start1);
+    const uint32_t n0 = class_count[2 * lane], n1 = class_count[2 * lane + 1];
+    const uint32_t t0 = (n0 * (1u << chain_lanes_log(2 * lane)) + 31u) / 32u;
+    const uint32_t t1 = (n1 * (1u << chain_lanes_log(2 * lane + 1)) + 31u) / 32u;
+    uint32_t x = t0 + t1;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+        if ((int)lane >= d) x += y;
     }
+    const uint32_t tickets = __shfl_sync(0xFFFFFFFFu, x, 31);
+    const uint32_t first0 = x - t0 - t1, first1 = first0 + t0;
     for (;;) {
         uint32_t ticket = 0;
         if (lane == 0) ticket = atomicAdd(queue, 1u);
         ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
-        const uint32_t first = n_wide + ticket * 32u;
-        if (first >= total) break;
-        const uint32_t it = first + lane;
-        if (it >= total) continue;
-        const ChainSetup s = chain_setup(g, offs, pieces, items[it]);
-        if (s.base + s.len > g.rec_cap) continue;   // overflow: k_merge reports it
+        if (ticket >= tickets) break;
+        // the class whose tickets hold it: the last that starts at or before
+        // it (empty classes start where the next one does)
+        const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, first0 <= ticket), m1 = __ballot_sync(0xFFFFFFFFu, first1 <= ticket);
+        const uint32_t at = 31u - (uint32_t)__clz((int)m0);
+        const bool odd = (m1 >> at) & 1u;
+        const uint32_t key = 2 * at + (odd ? 1u : 0u);
+        const uint32_t tfirst = __shfl_sync(0xFFFFFFFFu, odd ? first1 : first0, at);
+        const uint32_t cfirst = __shfl_sync(0xFFFFFFFFu, odd ? start1 : start0, at);
+        const uint32_t ccount = __shfl_sync(0xFFFFFFFFu, odd ? n1 : n0, at);
+        const uint32_t gl = chain_lanes_log(key);
+        const uint32_t i = ((ticket - tfirst) * 32u + lane) >> gl;
+        ChainSetup s;
+        const bool listed = i < ccount && cfirst + i < list_cap;
+        s = chain_setup(g, offs, pieces, items[listed ? cfirst + i : cfirst]);
+        // a lane without a chain, or whose chain overflows (k_merge reports
+        // it), has no roots
+        const int32_t len = listed && s.base + s.len <= g.rec_cap ? s.len : 0;
         int32_t* out = cbuf + s.base;
-        if (s.type == 2u) run_chain<2>(s.a, s.len, s.x, s.dx, s.t_lo, s.t_hi, s.side, out);
-        else if (s.type == 3u) run_chain<3>(s.a, s.len, s.x, s.dx, s.t_lo, s.t_hi, s.side, out);
-        else if (s.type == kArc) run_chain<(int)kArc>(s.a, s.len, s.x, s.dx, s.t_lo, s.t_hi, s.side, out);
-        else run_chain<4>(s.a, s.len, s.x, s.dx, s.t_lo, s.t_hi, s.side, out);
+        const int32_t lanes = 1 << gl, l = (int32_t)(lane & ((1u << gl) - 1u));
+        const uint32_t cls = key & 3u;
+        if (cls == 0u) run_segments<4>(s.side, len, s.t_lo, out, lanes, l);
+        else if (cls == 1u) run_segments<3>(s.side, len, s.t_lo, out, lanes, l);
+        else if (cls == 2u) run_segments<2>(s.side, len, s.t_lo, out, lanes, l);
+        else run_segments<(int)kArc>(s.side, len, s.t_lo, out, lanes, l);
     }
 }
 
@@ -702,16 +821,13 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
 // side counting as 2.0 (with its side bit); a record whose t (flag bits
 // masked) equals the previous one ORs the flags into both
 // (make_intersection_1.comp:361-375).
-// Records of a wide curve hold this until its merge, which runs on the other
-// stream, writes them; the record-parallel fragment pass skips them.
-constexpr int32_t kPendingCurve = -1;
 
 // Piece j of curve c, a thread each (pieces are merged independently: each
 // starts from its own t0 and flag state).  The piece-0 thread also checks
 // that the pieces cover the curve's records exactly.
 SR_DEV void merge_piece(const GeomArgs& g, const int32_t* __restrict__ offs, const uint4* __restrict__ pieces,
                         const int32_t* __restrict__ cbuf, int2* __restrict__ rec, uint32_t* __restrict__ status,
-                        uint32_t c, int j, bool pending_only) {
+                        uint32_t c, int j) {
     const int64_t start = offs[c], end = offs[c + 1];
     if (start >= end) return;
     if (end > g.rec_cap) {
@@ -732,10 +848,6 @@ SR_DEV void merge_piece(const GeomArgs& g, const int32_t* __restrict__ offs, con
     const int32_t n_loop = nx + ny + 1;
     if (pc + n_loop > end) return;   // reported by the piece-0 thread
     if (n_loop >= kLongPiece) return;   // k_merge_long
-    if (pending_only) {
-        for (int32_t k = 0; k < n_loop; ++k) rec[pc + k] = make_int2(kPendingCurve, 0);
-        return;
-    }
     const int32_t t0 = j == 0 ? 0 : (int32_t)pt[j - 1].y;   // bits of 0.0f for the first piece
     const int32_t minus_one = fbits(-1.0f);
     const int32_t ex_x = fbits(2.0f), ex_y = fbits(2.0f) | 1;
@@ -771,25 +883,13 @@ SR_DEV void merge_piece(const GeomArgs& g, const int32_t* __restrict__ offs, con
     }
 }
 
-// Part 0 merges every curve but the wide ones, whose records it marks
-// pending; part 1 merges the wide curves once their chains are done.  A
-// thread per (curve, piece).
+// A thread per (curve, piece).
 __global__ void __launch_bounds__(128) k_merge(const GeomArgs g, const int32_t* __restrict__ offs,
                                                const uint4* __restrict__ pieces, const int32_t* __restrict__ cbuf,
-                                               int2* __restrict__ rec, uint32_t* __restrict__ status,
-                                               const uint8_t* __restrict__ curve_wide,
-                                               const uint32_t* __restrict__ wide_curves,
-                                               const uint32_t* __restrict__ wide_curve_count, int part) {
+                                               int2* __restrict__ rec, uint32_t* __restrict__ status) {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (part == 0) {
-        const uint32_t c = tid / kMaxPieces;
-        if (c < g.n_curves)
-            merge_piece(g, offs, pieces, cbuf, rec, status, c, (int)(tid % kMaxPieces), curve_wide[c] != 0);
-        return;
-    }
-    const uint32_t nw = imin((int32_t)*wide_curve_count, (int32_t)g.n_curves);
-    for (uint32_t k = tid; k < nw * kMaxPieces; k += gridDim.x * blockDim.x)
-        merge_piece(g, offs, pieces, cbuf, rec, status, wide_curves[k / kMaxPieces], (int)(k % kMaxPieces), false);
+    const uint32_t c = tid / kMaxPieces;
+    if (c < g.n_curves) merge_piece(g, offs, pieces, cbuf, rec, status, c, (int)(tid % kMaxPieces));
 }
 
 // Merge of one long piece by a CTA.  The chains are non-decreasing (each
@@ -920,56 +1020,23 @@ SR_DEV void merge_long_piece(uint32_t c, int32_t t0, int64_t base, int32_t nx, i
     __syncthreads();
 }
 
-// Part 0: the long pieces of the list, a CTA each; those of wide curves are
-// marked pending.  Part 1: the wide curves, a CTA each, merging their long
-// pieces.
+// The long pieces of the list, a CTA each.
 __global__ void __launch_bounds__(256) k_merge_long(const GeomArgs g, const int32_t* __restrict__ offs,
                                                     const uint4* __restrict__ pieces,
                                                     const uint32_t* __restrict__ long_list, uint32_t list_cap,
                                                     const uint32_t* __restrict__ long_count,
-                                                    int32_t* __restrict__ cbuf, int2* __restrict__ rec,
-                                                    const uint8_t* __restrict__ curve_wide,
-                                                    const uint32_t* __restrict__ wide_curves,
-                                                    const uint32_t* __restrict__ wide_curve_count, int part,
-                                                    int32_t cap) {
+                                                    int32_t* __restrict__ cbuf, int2* __restrict__ rec, int32_t cap) {
     extern __shared__ int32_t sm_long[];   // [cap] chains in, [cap + 1] records out
     __shared__ int32_t s_i0;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    if (part == 0) {
-        const uint32_t n_long = imin((int32_t)*long_count, (int32_t)list_cap);
-        for (uint32_t item = blockIdx.x; item < n_long; item += gridDim.x) {
-            const uint32_t c = long_list[item] >> 3, piece = long_list[item] & 7u;
-            const uint4* pt = pieces + (size_t)c * kMaxPieces;
-            int64_t base = offs[c];
-            for (uint32_t j = 0; j < piece; ++j) base += 1 + piece_nx(pt[j].x) + piece_ny(pt[j].x);
-            const int32_t nx = piece_nx(pt[piece].x), ny = piece_ny(pt[piece].x);
-            const int32_t L = 1 + nx + ny;
-            if (base + L > g.rec_cap) continue;   // overflow: k_merge reports it
-            if (curve_wide[c]) {   // merged by part 1: mark pending
-                for (int32_t k = tid; k < L; k += nt) rec[base + k] = make_int2(kPendingCurve, 0);
-                continue;
-            }
-            merge_long_piece(c, piece == 0 ? 0 : (int32_t)pt[piece - 1].y, base, nx, ny, cbuf, rec, sm_long, cap,
-                             &s_i0);
-        }
-        return;
-    }
-    const uint32_t nw = imin((int32_t)*wide_curve_count, (int32_t)g.n_curves);
-    for (uint32_t k = blockIdx.x; k < nw; k += gridDim.x) {
-        const uint32_t c = wide_curves[k];
+    const uint32_t n_long = imin((int32_t)*long_count, (int32_t)list_cap);
+    for (uint32_t item = blockIdx.x; item < n_long; item += gridDim.x) {
+        const uint32_t c = long_list[item] >> 3, piece = long_list[item] & 7u;
         const uint4* pt = pieces + (size_t)c * kMaxPieces;
         int64_t base = offs[c];
-        const int64_t end = offs[c + 1];
-        if (end > g.rec_cap) continue;   // overflow: k_merge reports it
-        for (int j = 0; j < kMaxPieces && base < end; ++j) {
-            const int32_t nx = piece_nx(pt[j].x), ny = piece_ny(pt[j].x);
-            const int32_t L = 1 + nx + ny;
-            if (base + L > end) break;   // k_merge reports the range error
-            if (L >= kLongPiece)
-                merge_long_piece(c, j == 0 ? 0 : (int32_t)pt[j - 1].y, base, nx, ny, cbuf, rec, sm_long, cap,
-                                 &s_i0);
-            base += L;
-        }
+        for (uint32_t j = 0; j < piece; ++j) base += 1 + piece_nx(pt[j].x) + piece_ny(pt[j].x);
+        const int32_t nx = piece_nx(pt[piece].x), ny = piece_ny(pt[piece].x);
+        if (base + 1 + nx + ny > g.rec_cap) continue;   // overflow: k_merge reports it
+        merge_long_piece(c, piece == 0 ? 0 : (int32_t)pt[piece - 1].y, base, nx, ny, cbuf, rec, sm_long, cap, &s_i0);
     }
 }
 
@@ -1042,32 +1109,14 @@ SR_DEV void fragment_record(const GeomArgs& g, const int2* __restrict__ rec, con
     }
 }
 
-// Part 0: every record but those of wide curves (pending, or already
-// merged by part 1); part 1: the wide curves' records, a CTA per curve.
 __global__ void __launch_bounds__(256) k_fragment(const GeomArgs g, const int2* __restrict__ rec,
                                                   const int32_t* __restrict__ offs, int64_t n_cap,
                                                   const uint32_t* __restrict__ n_dev, uint64_t* __restrict__ keys,
-                                                  uint8_t* __restrict__ wnp, DebugOut dbg,
-                                                  const uint8_t* __restrict__ curve_wide,
-                                                  const uint32_t* __restrict__ wide_curves,
-                                                  const uint32_t* __restrict__ wide_curve_count, int part) {
+                                                  uint8_t* __restrict__ wnp, DebugOut dbg) {
     const int64_t n = n_dev ? (int64_t)min((uint64_t)*n_dev, (uint64_t)n_cap) : n_cap;
-    if (part == 0) {
-        const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-        if (i >= n) return;
-        const int2 r0 = rec[i];
-        if (r0.x == kPendingCurve) return;
-        if ((uint32_t)r0.x < g.n_curves && curve_wide[r0.x]) return;
-        fragment_record(g, rec, offs, n, i, r0, keys, wnp, dbg);
-        return;
-    }
-    const uint32_t nw = imin((int32_t)*wide_curve_count, (int32_t)g.n_curves);
-    for (uint32_t k = blockIdx.x; k < nw; k += gridDim.x) {
-        const uint32_t c = wide_curves[k];
-        const int64_t end = min((int64_t)offs[c + 1], n);
-        for (int64_t i = (int64_t)offs[c] + threadIdx.x; i < end; i += blockDim.x)
-            fragment_record(g, rec, offs, n, i, rec[i], keys, wnp, dbg);
-    }
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    fragment_record(g, rec, offs, n, i, rec[i], keys, wnp, dbg);
 }
 
 // -------------------------------------------------------------- launches --
@@ -1104,65 +1153,48 @@ uint32_t chain_list_capacity(uint32_t n_curves) { return 2u * kMaxPieces * n_cur
 void launch_count(const GeomArgs& g, float* cut_cache, int32_t* count, const ChainWork& w, uint32_t* status,
                   cudaStream_t st) {
     if (g.n_curves == 0) return;
-    count_launches(1);
+    count_launches(2);
     k_count<<<(g.n_curves + 255) / 256, 256, 0, st>>>(g, cut_cache, count, w.pieces, w.chain_items, w.chain_keys,
-                                                      w.list_cap, w.chain_count, w.wide_count, w.curve_wide,
-                                                      w.wide_curves, w.wide_curve_count, w.long_list, w.long_count,
-                                                      status);
+                                                      w.list_cap, w.chain_count, w.class_count, w.long_list,
+                                                      w.long_count, status);
+    const unsigned most = (unsigned)sm_count_hint() / 2;
+    const unsigned grid = (unsigned)std::min<size_t>(((size_t)w.list_cap + 255) / 256, most);
+    k_order_chains<<<grid, 256, 0, st>>>(w.chain_items, w.chain_keys, w.list_cap, w.chain_count, w.class_count,
+                                         w.class_next, w.sorted_items);
 }
 
-uint32_t chain_key_bits() { return kChainKeyBits; }
-
-void launch_chains(const GeomArgs& g, const int32_t* offs, const ChainWork& w, int32_t* cbuf, int sm_count, int part,
+void launch_chains(const GeomArgs& g, const int32_t* offs, const ChainWork& w, int32_t* cbuf, int sm_count,
                    cudaStream_t st) {
     if (g.n_curves == 0) return;
     count_launches(1);
-    // Part 1 runs two CTAs (8 warps) an SM.  Fewer warps share each SM's
-    // issue slots, so each group of chains, the longest first, finishes
-    // sooner, and the wide chains beside them and the merge waiting on them
-    // start earlier: on the 4096^2 frame its stage took 0.83 / 0.61 / 0.73 /
-    // 0.75 / 0.78 ms at 1 / 2 / 4 / 8 / 16 CTAs an SM.
-    if (part == 0)
-        k_chains<<<sm_count * 4, 128, 0, st>>>(g, offs, w.pieces, w.sorted_items, w.sorted_keys, w.list_cap,
-                                               w.chain_count, w.wide_count, w.wide_queue, cbuf, 0);
-    else
-        k_chains<<<sm_count * 2, 128, 0, st>>>(g, offs, w.pieces, w.sorted_items, w.sorted_keys, w.list_cap,
-                                                w.chain_count, w.wide_count, w.chain_queue, cbuf, 1);
+    k_chains<<<sm_count * kChainCtas, 128, 0, st>>>(g, offs, w.pieces, w.sorted_items, w.list_cap, w.class_count,
+                                                    w.chain_queue, cbuf);
 }
 
-constexpr int32_t kLongCapMain = 3072, kLongCapSide = 12288;
+constexpr int32_t kLongCap = 3072;
 
 cudaError_t geom_init() {
     return cudaFuncSetAttribute(k_merge_long, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(int32_t) * (2 * (size_t)kLongCapSide + 1)));
+                                (int)(sizeof(int32_t) * (2 * (size_t)kLongCap + 1)));
 }
 
 void launch_merge(const GeomArgs& g, const int32_t* offs, const ChainWork& w, int32_t* cbuf, int2* rec,
-                  uint32_t* status, int part, cudaStream_t st) {
+                  uint32_t* status, cudaStream_t st) {
     if (g.n_curves == 0) return;
     count_launches(2);
-    const unsigned grid = part == 0 ? (unsigned)(((size_t)g.n_curves * kMaxPieces + 127) / 128)
-                                    : (unsigned)sm_count_hint() / 8;
-    k_merge<<<grid, 128, 0, st>>>(g, offs, w.pieces, cbuf, rec, status, w.curve_wide, w.wide_curves,
-                                  w.wide_curve_count, part);
-    // chains of up to 3 K elements in 25 KB of shared memory (eight CTAs an
-    // SM) on the main stream; up to 12 K on the second stream, whose few
-    // pieces are the longest
-    const int32_t cap = part == 0 ? kLongCapMain : kLongCapSide;
-    const size_t smem = sizeof(int32_t) * (2 * (size_t)cap + 1);
-    k_merge_long<<<part == 0 ? sm_count_hint() : sm_count_hint() / 4, 256, smem, st>>>(
-        g, offs, w.pieces, w.long_list, w.list_cap, w.long_count, cbuf, rec, w.curve_wide, w.wide_curves,
-        w.wide_curve_count, part, cap);
+    k_merge<<<(unsigned)(((size_t)g.n_curves * kMaxPieces + 127) / 128), 128, 0, st>>>(g, offs, w.pieces, cbuf, rec,
+                                                                                       status);
+    // chains of up to 3 K elements in 25 KB of shared memory (eight CTAs an SM)
+    const size_t smem = sizeof(int32_t) * (2 * (size_t)kLongCap + 1);
+    k_merge_long<<<sm_count_hint(), 256, smem, st>>>(g, offs, w.pieces, w.long_list, w.list_cap, w.long_count, cbuf,
+                                                     rec, kLongCap);
 }
 
 void launch_fragment(const GeomArgs& g, const int2* rec, const int32_t* offs, int64_t n_cap, const uint32_t* n_dev,
-                     uint64_t* keys, uint8_t* wnp, const DebugOut& dbg, const ChainWork& w, int part,
-                     cudaStream_t st) {
+                     uint64_t* keys, uint8_t* wnp, const DebugOut& dbg, cudaStream_t st) {
     if (n_cap <= 0 || g.n_curves == 0) return;
     count_launches(1);
-    const unsigned grid = part == 0 ? (unsigned)((n_cap + 255) / 256) : (unsigned)sm_count_hint() / 4;
-    k_fragment<<<grid, 256, 0, st>>>(g, rec, offs, n_cap, n_dev, keys, wnp, dbg, w.curve_wide, w.wide_curves,
-                                     w.wide_curve_count, part);
+    k_fragment<<<(unsigned)((n_cap + 255) / 256), 256, 0, st>>>(g, rec, offs, n_cap, n_dev, keys, wnp, dbg);
 }
 
 }  // namespace sr
