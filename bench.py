@@ -53,8 +53,7 @@ ORACLE_SAMPLE = 64
 # the HBM fraction is the roofline only for the stages that move bytes.
 LIMITS = {
     "resolve": "latency of each segment's walk back to its collapse cut and of the record gathers",
-    "chains": "the dependent bisection steps of the longest crossing chains",
-    "wide": "the longest chain's bisection rounds (lane exchange latency), beside the rest of the frame",
+    "chains": "instruction issue: 24 bisection steps a root, and the stretches solved again",
     "sort": "shared-memory ranking latency of the tile sort and merge rounds",
     "winding_emit": "latency of each tile's flag, look-back and emission phases at 4-5 CTAs per SM, DRAM ~14%",
 }
@@ -200,9 +199,7 @@ def stage_bytes(st, n_curves, n_points, W, H):
         # records it reads depend on where the cuts fall: no byte count
         # comparable with the streaming stages (its time is reported)
         "resolve": 0,
-        # the wide chains and their curves' merge and fragments, on a second
-        # stream beside chains, merge and fragment (their bytes are counted there)
-        "wide": 0,
+        "wide": 0,   # not used
     }
 
 

@@ -215,9 +215,8 @@ typedef struct sr_stats {
                                 * sizing (cumulative; 0 for batches)        */
     /* with SR_FLAG_PROFILE: device time of each stage (CUDA events):
      * transform, count, offset scan, crossing chains, record merge,
-     * fragments (these three on the context's second stream), sort,
-     * winding+emit, row sort, resolve; then the wide chains with their
-     * curves' merge and fragments, on the render stream beside them */
+     * fragments, sort, winding+emit, row sort, resolve; the eleventh is not
+     * used (0) */
     float stage_ms[12];
 } sr_stats;
 sr_status sr_get_stats(const sr_ctx* ctx, sr_stats* out);

@@ -2,10 +2,8 @@
 //
 // transform_pos.comp          -> k_transform
 // make_intersection_0.comp    -> k_count
-// make_intersection_1.comp +
-// gen_fragment.comp           -> k_intersect_fragment (one pass: each
-//                                intersection record's fragment is built as
-//                                soon as the next record's t is known)
+// make_intersection_1.comp    -> k_chains, k_merge, k_merge_long
+// gen_fragment.comp           -> k_fragment
 #include <algorithm>
 
 #include "common.cuh"
@@ -157,9 +155,15 @@ SR_DEV int32_t cut_range(int32_t size, int32_t F, int32_t& b, int32_t& e) {
 constexpr int kMaxPieces = 5;
 // Pieces with at least this many records are merged by a whole CTA.
 constexpr int32_t kLongPiece = 64;
-// A lane of a split chain takes at least 1 << kSegLog bisected roots.
+// A lane of a split chain takes at least 1 << kSegLog bisected roots.  With
+// 8 / 16 / 32 the chain stage of the 4096^2 frame of 20,000 paths took 0.379 /
+// 0.311 / 0.281 ms (longer stretches waste fewer run-up and repeated roots),
+// that of the 1024^2 frame of 500 paths 0.054 / 0.057 / 0.072 ms (a lane's
+// stretch is its latency) and that of a 2048^2 frame of 5,000 paths 0.142 /
+// 0.140 / 0.177 ms.  (One chain a lane, and the longest a warp each beside
+// them, took 1.35, 0.33 and 0.82 ms.)
 constexpr int32_t kSegLog = 4;
-constexpr int kChainCtas = 8;   // of four warps, an SM
+constexpr int kChainCtas = 8;   // of four warps, an SM; 4 and 16 took the same
 
 // Piece record layout in the output: [t0][x crossings][y crossings], the
 // crossing values of each side solved by one chain (k_chains), then merged
