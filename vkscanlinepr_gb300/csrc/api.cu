@@ -104,7 +104,6 @@ enum Ctl : int {
     CTL_WIND_COUNTER = 2,
     CTL_NDRAW = 3,     // merged fragments + spans of the frame
     CTL_CHAINS = 4,    // chain counter
-    CTL_LONG = 8,      // long-piece counter
     CTL_QUEUE = 9,     // chain work-queue counter
     CTL_ROW_SCAN = 13,      // row-start scan's tile counter
     CTL_CLASSES = 16,       // chains of each class
@@ -291,7 +290,7 @@ struct Pipeline {
     DevBuf pos, pos_path, curve_pos, curve_type, curve_path, fill_rule, fill_info, path_scene, scenes_d, cta_base_d;
     DevBuf cta_narrow_d;
     // frame
-    DevBuf tpos, path_visible, cut, count, offs, ctl, scan_status, pieces, chain_lists, long_list;
+    DevBuf tpos, curve_end, path_visible, cut, count, offs, ctl, scan_status, pieces, chain_lists;
     DevBuf cbuf, rec, keys, keys_alt, wnp, skeys, svals, vals_alt, sort_scratch, wind_status, draw, draw_row, totals;
     DevBuf rkeys, rvals, rkeys_alt, rvals_alt, row_sort_scratch, row_start, seg_cut, row_count, row_px, row_scan, image;
     DevBuf d_fkey, d_fwn, d_fleft, d_wscan, d_fflag, d_sflag, d_skey;
@@ -320,6 +319,10 @@ struct Pipeline {
     int64_t last_N = 0, last_O = 0, last_cap = 0, last_dcap = 0;
     uint32_t last_largest = 0;   // records of the frame's largest sort segment
     bool stages_valid = false;
+    // a frame's records carry no flag bits: they are merged again with them
+    // when they are dumped, with the arguments of the frame
+    bool rec_flags = false;
+    sr::GeomArgs frame_geom{};
     bool last_segsort = false;   // the last frame sorted its records per path (segsort.cu)
     // profiling
     cudaEvent_t ev[2 * ST_COUNT_ALL] = {};
@@ -328,8 +331,8 @@ struct Pipeline {
 
     ~Pipeline() {
         DevBuf* all[] = {&pos, &pos_path, &curve_pos, &curve_type, &curve_path, &fill_rule, &fill_info, &path_scene,
-                         &scenes_d, &cta_base_d, &tpos, &path_visible, &cut, &count, &offs, &ctl, &scan_status,
-                         &pieces, &chain_lists, &long_list, &cbuf, &rec, &keys, &keys_alt,
+                         &scenes_d, &cta_base_d, &tpos, &curve_end, &path_visible, &cut, &count, &offs, &ctl, &scan_status,
+                         &pieces, &chain_lists, &cbuf, &rec, &keys, &keys_alt,
                          &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_status, &draw, &draw_row, &totals,
                          &rkeys, &rvals, &rkeys_alt, &rvals_alt, &row_sort_scratch, &row_start, &seg_cut, &row_count, &row_px,
                          &row_scan, &image, &d_fkey, &d_fwn, &d_fleft, &d_wscan, &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw,
@@ -386,7 +389,6 @@ struct Pipeline {
         CUDA_TRY(cudaMallocHost(&h_u32, sizeof(uint32_t) * 8));
         CUDA_TRY(cudaMallocHost(&h_u64, sizeof(uint64_t) * 4));
         CUDA_TRY(ensure(ctl, sizeof(uint32_t) * CTL_WORDS));
-        CUDA_TRY(sr::geom_init());
         return SR_OK;
     }
 
@@ -563,6 +565,7 @@ struct Pipeline {
         g.curve_pos = curve_pos.as<uint32_t>();
         g.curve_path = curve_path.as<uint32_t>();
         g.tpos = tpos.as<float2>();
+        g.curve_end = curve_end.as<float2>();
         g.path_visible = path_visible.as<int32_t>();
         g.W = Wmax;
         g.H = Hmax;
@@ -590,14 +593,13 @@ struct Pipeline {
         cw.class_count = ctlp + CTL_CLASSES;
         cw.class_next = ctlp + CTL_CLASS_NEXT;
         cw.chain_queue = ctlp + CTL_QUEUE;
-        cw.long_list = long_list.as<uint32_t>();
-        cw.long_count = ctlp + CTL_LONG;
         return cw;
     }
 
     // Buffers of the stages before the record count is known.
     sr_status prepare_front() {
         CUDA_TRY(ensure(tpos, sizeof(float2) * std::max<uint32_t>(V, 1)));
+        CUDA_TRY(ensure(curve_end, sizeof(float2) * std::max<uint32_t>(C, 1)));
         CUDA_TRY(ensure(path_visible, sizeof(int32_t) * std::max<uint32_t>(P, 1)));
         CUDA_TRY(ensure(cut, sizeof(float) * 5 * (size_t)std::max<uint32_t>(C, 1)));
         CUDA_TRY(ensure(count, sizeof(int32_t) * ((size_t)C + 1)));
@@ -606,7 +608,6 @@ struct Pipeline {
         CUDA_TRY(ensure(pieces, sr::piece_table_bytes(std::max<uint32_t>(C, 1))));
         const uint32_t lc = list_cap();
         CUDA_TRY(ensure(chain_lists, 9 * (size_t)lc));
-        CUDA_TRY(ensure(long_list, sizeof(uint32_t) * (size_t)lc));
         CUDA_TRY(ensure(totals, sizeof(uint64_t) * 4));
         CUDA_TRY(ensure(row_start, sizeof(int32_t) * ((size_t)total_rows + 1)));
         CUDA_TRY(ensure(seg_cut, sizeof(uint32_t) * std::max<size_t>(cut_words(), 1)));
@@ -682,10 +683,10 @@ struct Pipeline {
         add(4 * p1); add(4 * p1); add(4 * p1);                      // fill rule/info, path scene
         add(sizeof(sr::SceneInfo) * std::max<uint32_t>(S, 1)); add(4 * ((size_t)S + 1));
         add(4 * std::max<uint64_t>(total_pixels, 1));               // images
-        add(8 * v1); add(4 * p1); add(20 * c1); add(4 * (c1 + 1)); add(4 * (c1 + 1));
+        add(8 * v1); add(8 * c1); add(4 * p1); add(20 * c1); add(4 * (c1 + 1)); add(4 * (c1 + 1));
         add(8 * sr::scan_status_words(C)); add(sr::piece_table_bytes((uint32_t)c1));
         const size_t lc = list_cap();
-        add(9 * lc); add(4 * lc);
+        add(9 * lc);
         add(32); add(4 * ((size_t)total_rows + 1));
         post_count_buffers(cap, dcap, [&](DevBuf&, size_t b) { add(b); });
         return total;
@@ -707,9 +708,9 @@ struct Pipeline {
         static DevBuf Pipeline::* const bufs[] = {
             &Pipeline::pos, &Pipeline::pos_path, &Pipeline::curve_pos, &Pipeline::curve_type,
             &Pipeline::curve_path, &Pipeline::fill_rule, &Pipeline::fill_info, &Pipeline::path_scene,
-            &Pipeline::scenes_d, &Pipeline::cta_base_d, &Pipeline::tpos, &Pipeline::path_visible, &Pipeline::cut,
+            &Pipeline::scenes_d, &Pipeline::cta_base_d, &Pipeline::tpos, &Pipeline::curve_end, &Pipeline::path_visible, &Pipeline::cut,
             &Pipeline::count, &Pipeline::offs, &Pipeline::ctl, &Pipeline::scan_status, &Pipeline::pieces,
-            &Pipeline::chain_lists, &Pipeline::long_list, &Pipeline::cbuf,
+            &Pipeline::chain_lists, &Pipeline::cbuf,
             &Pipeline::rec, &Pipeline::keys, &Pipeline::keys_alt, &Pipeline::wnp, &Pipeline::skeys,
             &Pipeline::svals, &Pipeline::vals_alt, &Pipeline::sort_scratch, &Pipeline::wind_status,
             &Pipeline::draw, &Pipeline::draw_row, &Pipeline::totals, &Pipeline::rkeys, &Pipeline::rvals,
@@ -742,8 +743,8 @@ struct Pipeline {
     // Device bytes currently held by this pipeline.
     uint64_t held_bytes() const {
         const DevBuf* all[] = {&pos, &pos_path, &curve_pos, &curve_type, &curve_path, &fill_rule, &fill_info,
-                               &path_scene, &scenes_d, &cta_base_d, &tpos, &path_visible, &cut, &count, &offs,
-                               &ctl, &scan_status, &pieces, &chain_lists, &long_list, &cbuf,
+                               &path_scene, &scenes_d, &cta_base_d, &tpos, &curve_end, &path_visible, &cut, &count, &offs,
+                               &ctl, &scan_status, &pieces, &chain_lists, &cbuf,
                                &rec, &keys, &keys_alt, &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_status,
                                &draw, &draw_row, &totals, &rkeys, &rvals, &rkeys_alt, &rvals_alt,
                                &row_sort_scratch, &row_start, &seg_cut, &row_count, &row_px, &row_scan, &image, &d_fkey,
@@ -830,12 +831,14 @@ struct Pipeline {
         mark(ST_CHAINS, false);
         launch_chains(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), sm_count, st);
         mark(ST_CHAINS, true);
+        rec_flags = false;   // sr_debug_dump adds them when asked
+        frame_geom = g;
         mark(ST_MERGE, false);
-        launch_merge(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), rec.as<int2>(), status, st);
+        launch_order_records(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), rec.as<int2>(), status, sm_count, st);
         mark(ST_MERGE, true);
         mark(ST_FRAGMENT, false);
-        launch_fragment(g, rec.as<int2>(), offs.as<int32_t>(), cap, n_dev, keys.as<uint64_t>(),
-                        keep ? wnp.as<uint8_t>() : nullptr, dbg, st);
+        launch_fragment(g, rec.as<int2>(), cap, n_dev, keys.as<uint64_t>(), keep ? wnp.as<uint8_t>() : nullptr, dbg,
+                        st);
         mark(ST_FRAGMENT, true);
         const KeyLayout L = g.L;
         SortPlan sp = sort_plan(cap, L.pbits + L.rbits + L.xbits, n_dev, tune.sort_items);
@@ -921,6 +924,17 @@ struct Pipeline {
         launch_resolve(ra, res_ctas, st);
         mark(ST_RESOLVE, true);
         CUDA_TRY(cudaGetLastError());
+        return SR_OK;
+    }
+
+    // The last frame's intersection records with their flags, from its chains
+    // (which stay as they are until the next frame's).
+    sr_status merge_records() {
+        if (rec_flags) return SR_OK;
+        sr::launch_merge(frame_geom, offs.as<int32_t>(), chain_work(), cbuf.as<int32_t>(), rec.as<int2>(),
+                         ctl.as<uint32_t>() + CTL_STATUS, nullptr);
+        CUDA_TRY(cudaGetLastError());
+        rec_flags = true;
         return SR_OK;
     }
 
@@ -1396,6 +1410,9 @@ sr_status sr_debug_dump(sr_ctx* c, int stage, void* dst, size_t* bytes) {
     if (*bytes < need) return fail(SR_ERR_INVALID_ARG, "buffer of %zu bytes, need %zu", *bytes, need);
     if (need && !src) return fail(SR_ERR_INVALID_ARG, "stage %d not available", stage);
     CUDA_TRY(cudaSetDevice(p.device));
+    if (stage == SR_STAGE_INTERSECTION && need) {
+        SR_TRY(p.merge_records());
+    }
     if (need) CUDA_TRY(cudaMemcpy(dst, src, need, cudaMemcpyDeviceToHost));
     *bytes = need;
     return SR_OK;

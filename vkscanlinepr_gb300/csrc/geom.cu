@@ -2,7 +2,8 @@
 //
 // transform_pos.comp          -> k_transform
 // make_intersection_0.comp    -> k_count
-// make_intersection_1.comp    -> k_chains, k_merge, k_merge_long
+// make_intersection_1.comp    -> k_chains (the crossings), k_order_records
+//                                (their order), k_merge (for a read-back)
 // gen_fragment.comp           -> k_fragment
 #include <algorithm>
 
@@ -114,6 +115,16 @@ SR_DEV void load_curve(const float2* __restrict__ tpos, uint32_t first, uint32_t
     }
 }
 
+// interp() without a branch per curve type (but arcs): every level's lerps,
+// and the level that the type ends at.  Warps hold mixed types.
+SR_DEV float curve_coord(uint32_t type, float t, const float* p) {
+    if (type == kArc) return interp(type, t, p);
+    const float q0 = lerp_rn(p[0], p[1], t), q1 = lerp_rn(p[1], p[2], t), q2 = lerp_rn(p[2], p[3], t);
+    const float l0 = lerp_rn(q0, q1, t), l1 = lerp_rn(q1, q2, t);
+    const float b = lerp_rn(l0, l1, t);
+    return type == 2u ? q0 : (type == 3u ? l0 : b);
+}
+
 // solveQuadEquation (make_intersection_0.comp:76-129)
 SR_DEV void solve_quad(float a, float b, float c, float& r0, float& r1) {
     if (a == 0.0f) {
@@ -153,8 +164,6 @@ SR_DEV int32_t cut_range(int32_t size, int32_t F, int32_t& b, int32_t& e) {
 
 // Pieces of a curve: at most 4 monotonic cuts + the end at t = 1.
 constexpr int kMaxPieces = 5;
-// Pieces with at least this many records are merged by a whole CTA.
-constexpr int32_t kLongPiece = 64;
 // A lane of a split chain takes at least 1 << kSegLog bisected roots.  With
 // 8 / 16 / 32 the chain stage of the 4096^2 frame of 20,000 paths took 0.379 /
 // 0.311 / 0.281 ms (longer stretches waste fewer run-up and repeated roots),
@@ -176,23 +185,29 @@ SR_DEV int32_t piece_ny(uint32_t n) { return (int32_t)((n >> 16) & 0x7FFFu); }
 
 // Class of a chain: longest length class first (so the longest chains start
 // in the first wave of k_chains), then cubic, quadric, line, arc, so that a
-// warp runs one curve type with lengths within a factor of 2.  A line root is
-// a closed form, far cheaper than a 24-step bisection, so a line chain is
-// classed 7 length classes lower.
+// warp runs one curve type with lengths within a factor of 2.
 constexpr uint32_t kChainClasses = 64;
+constexpr uint32_t kEmptyPiece = 63;   // a piece without crossings: nothing to solve, one record
 SR_DEV uint32_t chain_key(int32_t len, uint32_t type) {
     uint32_t lg = 31u - (uint32_t)__clz(len);
     if (lg > 14u) lg = 14u;
-    if (type == 2u) lg = lg > 7u ? lg - 7u : 0u;
     uint32_t cls = type == 4u ? 0u : (type == 3u ? 1u : (type == kArc ? 3u : 2u));
     return ((14u - lg) << 2) | cls;
 }
-// log2 of the lanes that share a chain of this class (run_segments): a lane
-// takes 16 to 31 bisected roots, or 512 to 1,023 line roots, as far as 32
-// lanes go.
-SR_DEV uint32_t chain_lanes_log(uint32_t key) {
+// How the chains of a class are shared out: 2^lanes lanes a chain and 2^warps
+// warps (warps only with 32 lanes).  Solving, a lane takes 16 to 31 bisected
+// roots or, a line's root being a closed form, 512 to 1,023 of a line, as far
+// as 32 lanes go (run_segments).  Ordering, a lane takes every 32nd root, up
+// to 256 a warp, so that a warp's roots are neighbours in memory.
+struct ChainShare {
+    uint32_t lanes, warps;
+};
+template <bool kSolve> SR_DEV ChainShare chain_share(uint32_t key) {
     const int32_t lg = 14 - (int32_t)(key >> 2);
-    return (uint32_t)imin(imax((key & 3u) == 2u ? lg - 2 : lg - kSegLog, 0), 5);
+    ChainShare s;
+    s.lanes = (uint32_t)imin(imax(kSolve ? lg - ((key & 3u) == 2u ? kSegLog + 5 : kSegLog) : lg + 1, 0), 5);
+    s.warps = kSolve ? 0u : (uint32_t)imax(lg + 1 - 8, 0);
+    return s;
 }
 
 // get_xy_begin_end_delta + udpate_cut_range for one axis
@@ -224,9 +239,7 @@ __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restri
                                                int32_t* __restrict__ count, uint4* __restrict__ pieces,
                                                uint32_t* __restrict__ chain_items, uint8_t* __restrict__ chain_keys,
                                                uint32_t list_cap, uint32_t* __restrict__ chain_count,
-                                               uint32_t* __restrict__ class_count,
-                                               uint32_t* __restrict__ long_list, uint32_t* __restrict__ long_count,
-                                               uint32_t* __restrict__ status) {
+                                               uint32_t* __restrict__ class_count, uint32_t* __restrict__ status) {
     __shared__ uint32_t s_hist[kChainClasses], s_total, s_base;
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = c < g.n_curves;
@@ -236,7 +249,6 @@ __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restri
     uint32_t my_chains[2 * kMaxPieces];
     uint32_t my_key[2 * kMaxPieces];
     int n_chains = 0;
-    uint32_t long_mask = 0;   // pieces merged by k_merge_long
     if (active) {
         uint32_t type = g.curve_type[c];
         CurvePts P;
@@ -325,7 +337,7 @@ __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restri
         for (uint32_t i = 0; i < (uint32_t)kMaxPieces; ++i) {
             if (i >= n) break;
             float t1 = q[i];
-            float x1 = interp(type, t1, P.x), y1 = interp(type, t1, P.y);
+            float x1 = curve_coord(type, t1, P.x), y1 = curve_coord(type, t1, P.y);
             // count: get_xy_begin_end (make_intersection_0.comp:167-183)
             int32_t xb, xe, yb, ye;
             if (x0 <= x1) {
@@ -361,29 +373,17 @@ __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restri
                 my_chains[n_chains] = (c << 4) | (i << 1) | 1u;
                 my_key[n_chains++] = chain_key(ny, type);
             }
+            if (nx <= 0 && ny <= 0) {   // a record of its own start only
+                my_chains[n_chains] = (c << 4) | (i << 1);
+                my_key[n_chains++] = kEmptyPiece;
+            }
             walk += 1 + nx + ny;
-            if (1 + nx + ny >= kLongPiece) long_mask |= 1u << i;
             x0 = x1;
             y0 = y1;
         }
         count[c] = pc;
+        g.curve_end[c] = make_float2(x0, y0);   // at t = 1
         if (walk != pc) set_error(status, ERR_RECORD_RANGE);
-    }
-    // append long pieces (warp-aggregated)
-    const uint32_t lane = lane_id();
-    for (int i = 0; i < kMaxPieces; ++i) {
-        bool has = (long_mask >> i) & 1u;
-        uint32_t m = __ballot_sync(0xFFFFFFFFu, has);
-        if (!m) continue;
-        uint32_t leader = (uint32_t)(__ffs(m) - 1);
-        uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(long_count, (uint32_t)__popc(m));
-        base = __shfl_sync(0xFFFFFFFFu, base, leader);
-        if (has) {
-            uint32_t slot = base + (uint32_t)__popc(m & lanemask_lt());
-            if (slot < list_cap) long_list[slot] = (c << 3) | (uint32_t)i;
-            else set_error(status, ERR_CAPACITY);
-        }
     }
     // append the chains with their classes, and count the classes (one
     // append and at most one add per class for the CTA)
@@ -765,53 +765,76 @@ SR_DEV ChainSetup chain_setup(const GeomArgs& g, const int32_t* __restrict__ off
     return s;
 }
 
-// Every warp takes tickets, longest class first: a ticket is 32 / lanes
-// chains of one class (chain_lanes_log).
+// Work of the chains by tickets, longest class first: a ticket is a warp's
+// share of a class (chain_share).  Built by every warp.
+template <bool kSolve> struct ChainTickets {
+    uint32_t start0, start1, n0, n1, first0, first1;   // two classes a lane
+    uint32_t total;
+    SR_DEV static uint32_t tickets_of(uint32_t n, uint32_t key) {
+        const ChainShare s = chain_share<kSolve>(key);
+        return s.lanes == 5 ? n << s.warps : ((n << s.lanes) + 31u) / 32u;
+    }
+    SR_DEV void build(const uint32_t* __restrict__ class_count) {
+        const uint32_t lane = lane_id();
+        class_starts(class_count, start0, start1);
+        n0 = class_count[2 * lane];
+        n1 = class_count[2 * lane + 1];
+        if (2 * lane + 1 == kEmptyPiece && kSolve) n1 = 0;
+        const uint32_t t0 = tickets_of(n0, 2 * lane), t1 = tickets_of(n1, 2 * lane + 1);
+        uint32_t x = t0 + t1;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+            if ((int)lane >= d) x += y;
+        }
+        total = __shfl_sync(0xFFFFFFFFu, x, 31);
+        first0 = x - t0 - t1;
+        first1 = first0 + t0;
+    }
+    // The class of a ticket, this lane's chain of it (its list position; that
+    // of the class's first chain, and false, for a lane without one) and which
+    // of the chain's warps this is.
+    SR_DEV bool find(uint32_t ticket, uint32_t list_cap, uint32_t& key, uint32_t& pos, uint32_t& warp) const {
+        // the last class that starts at or before it (an empty class starts
+        // where the next one does)
+        const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, first0 <= ticket);
+        const uint32_t m1 = __ballot_sync(0xFFFFFFFFu, first1 <= ticket);
+        const uint32_t at = 31u - (uint32_t)__clz((int)m0);
+        const bool odd = (m1 >> at) & 1u;
+        key = 2 * at + (odd ? 1u : 0u);
+        const uint32_t tfirst = __shfl_sync(0xFFFFFFFFu, odd ? first1 : first0, at);
+        const uint32_t cfirst = __shfl_sync(0xFFFFFFFFu, odd ? start1 : start0, at);
+        const uint32_t ccount = __shfl_sync(0xFFFFFFFFu, odd ? n1 : n0, at);
+        const ChainShare s = chain_share<kSolve>(key);
+        const uint32_t i = s.lanes == 5 ? (ticket - tfirst) >> s.warps : ((ticket - tfirst) * 32u + lane_id()) >> s.lanes;
+        warp = (ticket - tfirst) & ((1u << s.warps) - 1u);
+        const bool listed = i < ccount && cfirst + i < list_cap;
+        pos = cfirst + (listed ? i : 0u);
+        return listed;
+    }
+};
+
 __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t* __restrict__ offs,
                                                 const uint4* __restrict__ pieces,
                                                 const uint32_t* __restrict__ items, uint32_t list_cap,
                                                 const uint32_t* __restrict__ class_count,
                                                 uint32_t* __restrict__ queue, int32_t* __restrict__ cbuf) {
-    const uint32_t lane = lane_id();
-    // first ticket and list position of each class, two classes a lane
-    uint32_t start0, start1;
-    class_starts(class_count, start0, start1);
-    const uint32_t n0 = class_count[2 * lane], n1 = class_count[2 * lane + 1];
-    const uint32_t t0 = (n0 * (1u << chain_lanes_log(2 * lane)) + 31u) / 32u;
-    const uint32_t t1 = (n1 * (1u << chain_lanes_log(2 * lane + 1)) + 31u) / 32u;
-    uint32_t x = t0 + t1;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-        if ((int)lane >= d) x += y;
-    }
-    const uint32_t tickets = __shfl_sync(0xFFFFFFFFu, x, 31);
-    const uint32_t first0 = x - t0 - t1, first1 = first0 + t0;
+    ChainTickets<true> T;
+    T.build(class_count);
     for (;;) {
         uint32_t ticket = 0;
-        if (lane == 0) ticket = atomicAdd(queue, 1u);
+        if (lane_id() == 0) ticket = atomicAdd(queue, 1u);
         ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
-        if (ticket >= tickets) break;
-        // the class whose tickets hold it: the last that starts at or before
-        // it (empty classes start where the next one does)
-        const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, first0 <= ticket), m1 = __ballot_sync(0xFFFFFFFFu, first1 <= ticket);
-        const uint32_t at = 31u - (uint32_t)__clz((int)m0);
-        const bool odd = (m1 >> at) & 1u;
-        const uint32_t key = 2 * at + (odd ? 1u : 0u);
-        const uint32_t tfirst = __shfl_sync(0xFFFFFFFFu, odd ? first1 : first0, at);
-        const uint32_t cfirst = __shfl_sync(0xFFFFFFFFu, odd ? start1 : start0, at);
-        const uint32_t ccount = __shfl_sync(0xFFFFFFFFu, odd ? n1 : n0, at);
-        const uint32_t gl = chain_lanes_log(key);
-        const uint32_t i = ((ticket - tfirst) * 32u + lane) >> gl;
-        ChainSetup s;
-        const bool listed = i < ccount && cfirst + i < list_cap;
-        s = chain_setup(g, offs, pieces, items[listed ? cfirst + i : cfirst]);
-        // a lane without a chain, or whose chain overflows (k_merge reports
-        // it), has no roots
+        if (ticket >= T.total) break;
+        uint32_t key, pos, warp;
+        const bool listed = T.find(ticket, list_cap, key, pos, warp);
+        const ChainSetup s = chain_setup(g, offs, pieces, items[pos]);
+        // a lane without a chain, or whose chain overflows (k_order_records
+        // reports it), has no roots
         const int32_t len = listed && s.base + s.len <= g.rec_cap ? s.len : 0;
         int32_t* out = cbuf + s.base;
-        const int32_t lanes = 1 << gl, l = (int32_t)(lane & ((1u << gl) - 1u));
-        const uint32_t cls = key & 3u;
+        const uint32_t gl = chain_share<true>(key).lanes, cls = key & 3u;
+        const int32_t lanes = 1 << gl, l = (int32_t)(lane_id() & ((1u << gl) - 1u));
         if (cls == 0u) run_segments<4>(s.side, len, s.t_lo, out, lanes, l);
         else if (cls == 1u) run_segments<3>(s.side, len, s.t_lo, out, lanes, l);
         else if (cls == 2u) run_segments<2>(s.side, len, s.t_lo, out, lanes, l);
@@ -819,13 +842,102 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
     }
 }
 
-// ------------------------------------------------------------- merge -----
+// ------------------------------------------------------------- order -----
 // The record order of make_intersection_1.comp:310-441: per piece, the
 // start t0 and the two chains merged by `next_tx <= next_ty`, an exhausted
-// side counting as 2.0 (with its side bit); a record whose t (flag bits
-// masked) equals the previous one ORs the flags into both
-// (make_intersection_1.comp:361-375).
+// side counting as 2.0 (with its side bit).  Roots never decrease along a
+// chain (each is solved from the one before; only t0's flag bits may put it
+// above the first ones), so a piece's records are the i0 x roots <= t0, then
+// t0, then the stable merge (x first on ties) of the other x roots with the
+// y roots, and a root's place is its index plus its rank in the other chain.
+// A piece may run backwards: the fourth cut of a curve may lie before the
+// third (make_intersection_0.comp:340).  Its roots never increase and stay
+// below t0, and the sequential merge, which takes the lower head, takes all x
+// roots, then t0, then all y roots: i0 is all of them.
+//
+// A lane finds the place of a root by a binary search; a warp's roots are
+// neighbours, so its loads and stores are too.  Those dependent loads bound
+// it: 0.183 ms on the 4096^2 frame of 21 M records (0.014 ms on the 1024^2
+// frame of 0.37 M), where a thread per short and a CTA per long piece took
+// 0.295 (0.027); a lane walking a stretch of 16 consecutive roots took 0.52,
+// its 4-byte accesses being scattered.
+SR_DEV int32_t count_le(const int32_t* a, int32_t lo, int32_t hi, float v) {   // elements <= v, of a[lo, hi) sorted, + lo
+    while (lo < hi) {
+        const int32_t mid = (lo + hi) >> 1;
+        if (bitsf(a[mid]) <= v) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+SR_DEV int32_t count_lt(const int32_t* a, int32_t lo, int32_t hi, float v) {   // elements < v, likewise
+    while (lo < hi) {
+        const int32_t mid = (lo + hi) >> 1;
+        if (bitsf(a[mid]) < v) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
 
+__global__ void __launch_bounds__(128) k_order_records(const GeomArgs g, const int32_t* __restrict__ offs,
+                                                       const uint4* __restrict__ pieces,
+                                                       const uint32_t* __restrict__ items, uint32_t list_cap,
+                                                       const uint32_t* __restrict__ class_count,
+                                                       const int32_t* __restrict__ cbuf, int2* __restrict__ rec,
+                                                       uint32_t* __restrict__ status) {
+    ChainTickets<false> T;
+    T.build(class_count);
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    for (uint32_t ticket = blockIdx.x * (blockDim.x / 32u) + (threadIdx.x >> 5); ticket < T.total; ticket += warps) {
+        uint32_t key, pos, warp;
+        if (!T.find(ticket, list_cap, key, pos, warp)) continue;
+        const uint32_t item = items[pos], c = item >> 4, piece = (item >> 1) & 7u;
+        const uint4* pt = pieces + (size_t)c * kMaxPieces;
+        int64_t base = offs[c];
+        for (uint32_t j = 0; j < piece; ++j) base += 1 + piece_nx(pt[j].x) + piece_ny(pt[j].x);
+        const uint4 me = pt[piece];
+        const int32_t nx = piece_nx(me.x), ny = piece_ny(me.x);
+        if (base + 1 + nx + ny > g.rec_cap) {
+            set_error(status, ERR_CAPACITY);
+            continue;
+        }
+        const int32_t t0 = piece == 0 ? 0 : (int32_t)pt[piece - 1].y;   // bits of 0.0f for the first piece
+        const int32_t *X = cbuf + base + 1, *Y = X + nx;
+        int2* R = rec + base;
+        int32_t i0 = 0;
+        const bool back = __uint_as_float(me.y) < bitsf(t0);
+        if (nx > 0 && ny > 0) {
+            if (back) i0 = nx;
+            else if (bitsf(X[0]) <= bitsf(t0)) i0 = count_le(X, 0, nx, bitsf(t0));
+        }
+        const uint32_t gl = chain_share<false>(key).lanes;
+        const int32_t l = (int32_t)(lane_id() & ((1u << gl) - 1u));
+        const bool y_side = (item & 1u) != 0;
+        if (l == 0 && warp == 0 && (y_side || ny == 0)) R[i0] = make_int2((int32_t)c, t0);
+        const int32_t len = y_side ? ny : nx, m = y_side ? nx : ny;
+        const int32_t *A = y_side ? Y : X, *B = y_side ? X : Y;
+        const int32_t k0 = (int32_t)warp * 256, k1 = imin(k0 + 256, len);
+        int32_t r = 0;   // roots of the other chain before this one (x roots equal to a y root come before it)
+        for (int32_t k = k0 + l; k < k1; k += 32) {
+            const int32_t t = A[k];
+            int32_t o;
+            if (m == 0 || back) {
+                o = k + (m == 0 ? 1 : (y_side ? 1 + nx : 0));
+            } else if (y_side) {
+                r = count_le(B, r, m, bitsf(t));
+                o = 1 + k + imax(r, i0);
+            } else {
+                r = count_lt(B, r, m, bitsf(t));
+                o = k < i0 ? k : 1 + k + r;
+            }
+            R[o] = make_int2((int32_t)c, t);
+        }
+    }
+}
+
+// The reference's records for a read-back: the same order, found by the
+// sequential merge itself, and the flags: a record whose t (flag bits masked)
+// equals the previous one ORs the flags into both
+// (make_intersection_1.comp:361-375).  A frame does not need them.
 // Piece j of curve c, a thread each (pieces are merged independently: each
 // starts from its own t0 and flag state).  The piece-0 thread also checks
 // that the pieces cover the curve's records exactly.
@@ -851,7 +963,6 @@ SR_DEV void merge_piece(const GeomArgs& g, const int32_t* __restrict__ offs, con
     const int32_t nx = piece_nx(me.x), ny = piece_ny(me.x);
     const int32_t n_loop = nx + ny + 1;
     if (pc + n_loop > end) return;   // reported by the piece-0 thread
-    if (n_loop >= kLongPiece) return;   // k_merge_long
     const int32_t t0 = j == 0 ? 0 : (int32_t)pt[j - 1].y;   // bits of 0.0f for the first piece
     const int32_t minus_one = fbits(-1.0f);
     const int32_t ex_x = fbits(2.0f), ex_y = fbits(2.0f) | 1;
@@ -896,205 +1007,84 @@ __global__ void __launch_bounds__(128) k_merge(const GeomArgs g, const int32_t* 
     if (c < g.n_curves) merge_piece(g, offs, pieces, cbuf, rec, status, c, (int)(tid % kMaxPieces));
 }
 
-// Merge of one long piece by a CTA.  The chains are non-decreasing (each
-// root is solved from the previous one, flag bits included); only the
-// piece start t0 may exceed the first roots by less than 4 ulp, so the
-// sequential merge is: the x roots <= t0, then t0, then the stable merge
-// (x first on ties) of the remaining x roots with the y roots.  Each
-// element's slot is its index plus its rank in the other chain.  The
-// flag-OR of equal t values is then applied per element: record k of a
-// run [s, e] of equal masked t ends as OR(v_s .. v_min(k+1,e)).
-SR_DEV int32_t count_le(const int32_t* a, int32_t n, float v) {   // elements <= v
-    int32_t lo = 0, hi = n;
-    while (lo < hi) {
-        int32_t mid = (lo + hi) >> 1;
-        if (bitsf(a[mid]) <= v) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-SR_DEV int32_t count_lt(const int32_t* a, int32_t n, float v) {   // elements < v
-    int32_t lo = 0, hi = n;
-    while (lo < hi) {
-        int32_t mid = (lo + hi) >> 1;
-        if (bitsf(a[mid]) < v) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// A long piece merged by the CTA.  When its two chains fit in shared memory
-// (cap elements) they are merged there: each thread writes one stretch of
-// the output, its start found by a merge-path search (x first on ties), and
-// the flag-OR reads shared memory.  Larger pieces use binary-search ranks in
-// global memory.  Every thread of the CTA calls it with the same piece.
-SR_DEV void merge_long_piece(uint32_t c, int32_t t0, int64_t base, int32_t nx, int32_t ny,
-                             int32_t* __restrict__ cbuf, int2* __restrict__ rec, int32_t* sm, int32_t cap,
-                             int32_t* s_i0) {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int32_t L = 1 + nx + ny;
-    const int32_t* X = cbuf + base + 1;
-    const int32_t* Y = X + nx;
-    int2* R = rec + base;
-    if (nx + ny <= cap) {
-        int32_t* sin = sm;
-        int32_t* sout = sm + cap;
-        for (int32_t k = tid; k < nx + ny; k += nt) sin[k] = X[k];
-        __syncthreads();
-        const int32_t* sx = sin;
-        const int32_t* sy = sin + nx;
-        if (nx == 0 || ny == 0) {
-            for (int32_t k = tid; k < L; k += nt) sout[k] = k == 0 ? t0 : sin[k - 1];
-        } else {
-            const int32_t i0 = count_le(sx, nx, bitsf(t0));
-            for (int32_t k = tid; k < i0; k += nt) sout[k] = sx[k];
-            if (tid == 0) sout[i0] = t0;
-            // the merge of sx[i0..nx) with sy: this thread's stretch [d, d_end)
-            const int32_t* xr = sx + i0;
-            const int32_t nxr = nx - i0, M = nxr + ny;
-            const int32_t per = (M + nt - 1) / nt;
-            const int32_t d = imin(tid * per, M), d_end = imin(d + per, M);
-            int32_t lo = imax(0, d - ny), hi = imin(d, nxr);
-            while (lo < hi) {
-                const int32_t mid = (lo + hi) >> 1;
-                if (bitsf(xr[mid]) <= bitsf(sy[d - mid - 1])) lo = mid + 1;
-                else hi = mid;
-            }
-            int32_t ia = lo, ib = d - lo;
-            int32_t* o = sout + i0 + 1;
-            for (int32_t k = d; k < d_end; ++k) {
-                const bool take_x = ia < nxr && (ib >= ny || bitsf(xr[ia]) <= bitsf(sy[ib]));
-                o[k] = take_x ? xr[ia++] : sy[ib++];
-            }
-        }
-        __syncthreads();
-        for (int32_t k = tid; k < L; k += nt) {
-            const int32_t v = sout[k];
-            int32_t acc = v;
-            for (int32_t s2 = k - 1; s2 >= 0; --s2) {
-                const int32_t u = sout[s2];
-                if ((u & ~3) != (v & ~3)) break;
-                acc |= u;
-            }
-            if (k + 1 < L) {
-                const int32_t u = sout[k + 1];
-                if ((u & ~3) == (v & ~3)) acc |= u;
-            }
-            R[k] = make_int2((int32_t)c, acc);
-        }
-        __syncthreads();
-        return;
-    }
-    if (nx == 0 || ny == 0) {
-        const int32_t* S = nx == 0 ? Y : X;
-        for (int32_t k = tid; k < L; k += nt) R[k] = make_int2((int32_t)c, k == 0 ? t0 : S[k - 1]);
-    } else {
-        if (tid == 0) *s_i0 = count_le(X, nx, bitsf(t0));
-        __syncthreads();
-        const int32_t i0 = *s_i0;
-        for (int32_t i = tid; i < nx; i += nt) {
-            int32_t v = X[i];
-            int32_t pos = i < i0 ? i : i0 + 1 + (i - i0) + count_lt(Y, ny, bitsf(v));
-            R[pos] = make_int2((int32_t)c, v);
-        }
-        if (tid == 0) R[i0] = make_int2((int32_t)c, t0);
-        for (int32_t j = tid; j < ny; j += nt) {
-            int32_t v = Y[j];
-            int32_t pos = i0 + 1 + j + count_le(X + i0, nx - i0, bitsf(v));
-            R[pos] = make_int2((int32_t)c, v);
-        }
-    }
-    __syncthreads();
-    int32_t* T = cbuf + base;   // the chains are consumed: reuse as scratch
-    for (int32_t k = tid; k < L; k += nt) {
-        int32_t v = R[k].y, acc = v;
-        for (int32_t s2 = k - 1; s2 >= 0; --s2) {
-            int32_t u = R[s2].y;
-            if ((u & ~3) != (v & ~3)) break;
-            acc |= u;
-        }
-        if (k + 1 < L) {
-            int32_t u = R[k + 1].y;
-            if ((u & ~3) == (v & ~3)) acc |= u;
-        }
-        T[k] = acc;
-    }
-    __syncthreads();
-    for (int32_t k = tid; k < L; k += nt) R[k].y = T[k];
-    __syncthreads();
-}
-
-// The long pieces of the list, a CTA each.
-__global__ void __launch_bounds__(256) k_merge_long(const GeomArgs g, const int32_t* __restrict__ offs,
-                                                    const uint4* __restrict__ pieces,
-                                                    const uint32_t* __restrict__ long_list, uint32_t list_cap,
-                                                    const uint32_t* __restrict__ long_count,
-                                                    int32_t* __restrict__ cbuf, int2* __restrict__ rec, int32_t cap) {
-    extern __shared__ int32_t sm_long[];   // [cap] chains in, [cap + 1] records out
-    __shared__ int32_t s_i0;
-    const uint32_t n_long = imin((int32_t)*long_count, (int32_t)list_cap);
-    for (uint32_t item = blockIdx.x; item < n_long; item += gridDim.x) {
-        const uint32_t c = long_list[item] >> 3, piece = long_list[item] & 7u;
-        const uint4* pt = pieces + (size_t)c * kMaxPieces;
-        int64_t base = offs[c];
-        for (uint32_t j = 0; j < piece; ++j) base += 1 + piece_nx(pt[j].x) + piece_ny(pt[j].x);
-        const int32_t nx = piece_nx(pt[piece].x), ny = piece_ny(pt[piece].x);
-        if (base + 1 + nx + ny > g.rec_cap) continue;   // overflow: k_merge reports it
-        merge_long_piece(c, piece == 0 ? 0 : (int32_t)pt[piece - 1].y, base, nx, ny, cbuf, rec, sm_long, cap, &s_i0);
-    }
-}
-
 // ---------------------------------------------------------- fragment -----
-// gen_fragment.comp:90-245, one thread per record: the piece between this
+// gen_fragment.comp:90-245, a lane per record: the piece between this
 // record's t and the next record's t (t = 1 when the next record belongs to
 // another curve), its cell, the 64-bit sort key, the winding change across
 // the sample row and (pixel mode) the part of it left of the cell centre.
-// Record i of curve r0.x: the piece runs to the next record's t when that
-// record belongs to the same curve (i + 1 < offs[c + 1]), else to t = 1.
-SR_DEV void fragment_record(const GeomArgs& g, const int2* __restrict__ rec, const int32_t* __restrict__ offs,
-                            int64_t n, int64_t i, int2 r0, uint64_t* __restrict__ keys, uint8_t* __restrict__ wnp,
-                            const DebugOut& dbg) {
-    float t0 = gmax(bitsf(r0.y & ~3), 0.0f);
-    uint32_t c = (uint32_t)r0.x;
-    if (c >= g.n_curves) {
-        // only in a frame whose records overflowed their capacity (the
-        // frame is reported and discarded): never index with it
+// A warp takes 32 consecutive records and writes the first 31: each lane
+// evaluates the curve at its own record, and the next lane's point (or the
+// curve's end, from the count pass) is the piece's end.  Instruction issue
+// bounds it (70%): 0.209 ms on the 4096^2 frame of 21 M records; evaluating
+// both ends in every lane took 0.225.
+constexpr int kFragWarps = 8, kFragOut = 31;
+
+__global__ void __launch_bounds__(32 * kFragWarps) k_fragment(const GeomArgs g, const int2* __restrict__ rec,
+                                                              int64_t n_cap, const uint32_t* __restrict__ n_dev,
+                                                              uint64_t* __restrict__ keys, uint8_t* __restrict__ wnp,
+                                                              DebugOut dbg) {
+    const int64_t n = (int64_t)min((uint64_t)*n_dev, (uint64_t)n_cap);
+    const int64_t b = ((int64_t)blockIdx.x * kFragWarps + (threadIdx.x >> 5)) * kFragOut;
+    if (b >= n) return;
+    const uint32_t lane = lane_id();
+    const int64_t i = b + lane;
+    const int2 r = i < n ? rec[i] : make_int2(-1, 0);
+    const uint32_t c = (uint32_t)r.x;
+    // an index out of range only in a frame whose records overflowed their
+    // capacity (it is reported and discarded)
+    const bool ok = c < g.n_curves;
+    const float t0 = gmax(bitsf(r.y & ~3), 0.0f);
+    uint32_t path = 0;
+    float2 pf = make_float2(0.0f, 0.0f);
+    if (ok) {
+        const uint32_t type = g.curve_type[c];
+        path = g.curve_path[c];
+        CurvePts P;
+        load_curve(g.tpos, g.curve_pos[c], type, P);
+        pf = make_float2(curve_coord(type, t0, P.x), curve_coord(type, t0, P.y));
+    }
+    const bool more = __shfl_down_sync(0xFFFFFFFFu, c, 1) == c;
+    float t1 = __shfl_down_sync(0xFFFFFFFFu, t0, 1);
+    float2 pl = make_float2(__shfl_down_sync(0xFFFFFFFFu, pf.x, 1), __shfl_down_sync(0xFFFFFFFFu, pf.y, 1));
+    if (lane == 31 || i >= n) return;
+    if (!ok) {
         keys[i] = ~0ull;
         if (wnp) wnp[i] = 0;
         return;
     }
-    float t1 = 1.0f;
-    if (i + 1 < n && i + 1 < (int64_t)offs[c + 1]) t1 = gmax(bitsf(rec[i + 1].y & ~3), 0.0f);
-    uint32_t path = g.curve_path[c];
+    if (!more) {
+        t1 = 1.0f;
+        pl = g.curve_end[c];
+    }
     int32_t yx = (int32_t)0xFFFEFFFE, wn = 0, left = 0;
     bool valid = false;
     int32_t pos_x = 0, pos_y = 0;
     if (t0 < t1) {
-        uint32_t type = g.curve_type[c];
-        CurvePts P;
-        load_curve(g.tpos, g.curve_pos[c], type, P);
-        float pfx = interp(type, t0, P.x), pfy = interp(type, t0, P.y);
-        float plx = interp(type, t1, P.x), ply = interp(type, t1, P.y);
         const int32_t F = g.F;
-        const SceneInfo& si = scene_of_path(g.st, path);
+        int32_t W = g.W, H = g.H;
+        if (g.st.n_scenes > 1) {
+            const SceneInfo& si = scene_of_path(g.st, path);
+            W = si.W;
+            H = si.H;
+        }
         const float invF = inv_F(F);
-        int32_t rx = wmul(float2int_rd(__fmul_rn(__fmul_rn(__fadd_rn(pfx, plx), 0.5f), invF)), F);
-        int32_t ry = wmul(float2int_rd(__fmul_rn(__fmul_rn(__fadd_rn(pfy, ply), 0.5f), invF)), F);
-        pos_x = imin(imax(rx, -F), wadd(si.W & (int32_t)0xFFFFFFFE, F));
-        pos_y = imin(imax(ry, -F), wadd(si.H & (int32_t)0xFFFFFFFE, F));
-        if ((uint32_t)ry < (uint32_t)si.H) {
+        int32_t rx = wmul(float2int_rd(__fmul_rn(__fmul_rn(__fadd_rn(pf.x, pl.x), 0.5f), invF)), F);
+        int32_t ry = wmul(float2int_rd(__fmul_rn(__fmul_rn(__fadd_rn(pf.y, pl.y), 0.5f), invF)), F);
+        pos_x = imin(imax(rx, -F), wadd(W & (int32_t)0xFFFFFFFE, F));
+        pos_y = imin(imax(ry, -F), wadd(H & (int32_t)0xFFFFFFFE, F));
+        if ((uint32_t)ry < (uint32_t)H) {
             valid = true;
             yx = (int32_t)(((uint32_t)wadd(pos_y, 0x7FFF) << 16) | ((uint32_t)wadd(pos_x, 0x7FFF) & 0xFFFFu));
         }
         // winding sample row cell_y + FRAG_SIZE/2 (gen_fragment.comp:188-199)
         float wn_y = __fadd_rn((float)pos_y, __fmul_rn(0.5f, (float)F));
-        if (pfy == ply) wn = 0;
-        else if (pfy < wn_y && wn_y <= ply) wn = -1;
-        else if (ply < wn_y && wn_y <= pfy) wn = 1;
+        if (pf.y == pl.y) wn = 0;
+        else if (pf.y < wn_y && wn_y <= pl.y) wn = -1;
+        else if (pl.y < wn_y && wn_y <= pf.y) wn = 1;
         if (g.pixel_mode && wn != 0) {
-            float dyv = __fsub_rn(ply, pfy);
-            float tc = __fdiv_rn(__fsub_rn(wn_y, pfy), dyv);
-            float xc = __fadd_rn(pfx, __fmul_rn(tc, __fsub_rn(plx, pfx)));
+            float dyv = __fsub_rn(pl.y, pf.y);
+            float tc = __fdiv_rn(__fsub_rn(wn_y, pf.y), dyv);
+            float xc = __fadd_rn(pf.x, __fmul_rn(tc, __fsub_rn(pl.x, pf.x)));
             if (xc < __fadd_rn((float)pos_x, 0.5f)) left = wn;
         }
     }
@@ -1111,16 +1101,6 @@ SR_DEV void fragment_record(const GeomArgs& g, const int2* __restrict__ rec, con
         dbg.fwn[i] = wn;
         dbg.fleft[i] = left;
     }
-}
-
-__global__ void __launch_bounds__(256) k_fragment(const GeomArgs g, const int2* __restrict__ rec,
-                                                  const int32_t* __restrict__ offs, int64_t n_cap,
-                                                  const uint32_t* __restrict__ n_dev, uint64_t* __restrict__ keys,
-                                                  uint8_t* __restrict__ wnp, DebugOut dbg) {
-    const int64_t n = n_dev ? (int64_t)min((uint64_t)*n_dev, (uint64_t)n_cap) : n_cap;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    fragment_record(g, rec, offs, n, i, rec[i], keys, wnp, dbg);
 }
 
 // -------------------------------------------------------------- launches --
@@ -1159,8 +1139,7 @@ void launch_count(const GeomArgs& g, float* cut_cache, int32_t* count, const Cha
     if (g.n_curves == 0) return;
     count_launches(2);
     k_count<<<(g.n_curves + 255) / 256, 256, 0, st>>>(g, cut_cache, count, w.pieces, w.chain_items, w.chain_keys,
-                                                      w.list_cap, w.chain_count, w.class_count, w.long_list,
-                                                      w.long_count, status);
+                                                      w.list_cap, w.chain_count, w.class_count, status);
     const unsigned most = (unsigned)sm_count_hint() / 2;
     const unsigned grid = (unsigned)std::min<size_t>(((size_t)w.list_cap + 255) / 256, most);
     k_order_chains<<<grid, 256, 0, st>>>(w.chain_items, w.chain_keys, w.list_cap, w.chain_count, w.class_count,
@@ -1175,30 +1154,28 @@ void launch_chains(const GeomArgs& g, const int32_t* offs, const ChainWork& w, i
                                                     w.chain_queue, cbuf);
 }
 
-constexpr int32_t kLongCap = 3072;
-
-cudaError_t geom_init() {
-    return cudaFuncSetAttribute(k_merge_long, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(int32_t) * (2 * (size_t)kLongCap + 1)));
-}
-
-void launch_merge(const GeomArgs& g, const int32_t* offs, const ChainWork& w, int32_t* cbuf, int2* rec,
+void launch_merge(const GeomArgs& g, const int32_t* offs, const ChainWork& w, const int32_t* cbuf, int2* rec,
                   uint32_t* status, cudaStream_t st) {
     if (g.n_curves == 0) return;
-    count_launches(2);
+    count_launches(1);
     k_merge<<<(unsigned)(((size_t)g.n_curves * kMaxPieces + 127) / 128), 128, 0, st>>>(g, offs, w.pieces, cbuf, rec,
                                                                                        status);
-    // chains of up to 3 K elements in 25 KB of shared memory (eight CTAs an SM)
-    const size_t smem = sizeof(int32_t) * (2 * (size_t)kLongCap + 1);
-    k_merge_long<<<sm_count_hint(), 256, smem, st>>>(g, offs, w.pieces, w.long_list, w.list_cap, w.long_count, cbuf,
-                                                     rec, kLongCap);
 }
 
-void launch_fragment(const GeomArgs& g, const int2* rec, const int32_t* offs, int64_t n_cap, const uint32_t* n_dev,
-                     uint64_t* keys, uint8_t* wnp, const DebugOut& dbg, cudaStream_t st) {
+void launch_order_records(const GeomArgs& g, const int32_t* offs, const ChainWork& w, const int32_t* cbuf, int2* rec,
+                          uint32_t* status, int sm_count, cudaStream_t st) {
+    if (g.n_curves == 0) return;
+    count_launches(1);
+    k_order_records<<<sm_count * 32, 128, 0, st>>>(g, offs, w.pieces, w.sorted_items, w.list_cap, w.class_count, cbuf,
+                                                   rec, status);
+}
+
+void launch_fragment(const GeomArgs& g, const int2* rec, int64_t n_cap, const uint32_t* n_dev, uint64_t* keys,
+                     uint8_t* wnp, const DebugOut& dbg, cudaStream_t st) {
     if (n_cap <= 0 || g.n_curves == 0) return;
     count_launches(1);
-    k_fragment<<<(unsigned)((n_cap + 255) / 256), 256, 0, st>>>(g, rec, offs, n_cap, n_dev, keys, wnp, dbg);
+    constexpr int64_t per = kFragWarps * kFragOut;
+    k_fragment<<<(unsigned)((n_cap + per - 1) / per), 32 * kFragWarps, 0, st>>>(g, rec, n_cap, n_dev, keys, wnp, dbg);
 }
 
 }  // namespace sr

@@ -67,6 +67,7 @@ struct GeomArgs {
     const uint32_t* curve_path;
     const float2* tpos;
     const int32_t* path_visible;
+    float2* curve_end;   // [n_curves] each curve's point at t = 1 (written by the count pass)
     int32_t W, H, F;
     int32_t pixel_mode;
     KeyLayout L;
@@ -92,8 +93,6 @@ struct ChainWork {
     uint32_t* class_count;    // [kChainClassWords] chains of each class
     uint32_t* class_next;     // [kChainClassWords] next place of each class in sorted_items
     uint32_t* chain_queue;    // [1] next ticket of the chains
-    uint32_t* long_list;      // [list_cap] (curve << 3 | piece) of long pieces
-    uint32_t* long_count;     // [1] zeroed before the count pass
 };
 constexpr int kChainClassWords = 64;
 size_t piece_table_bytes(uint32_t n_curves);
@@ -107,21 +106,22 @@ void launch_transform(const float2* pos, const uint32_t* pos_path, uint32_t n_po
                       float2* tpos, int32_t* path_visible, cudaStream_t st);
 void launch_count(const GeomArgs& g, float* cut_cache, int32_t* count, const ChainWork& w, uint32_t* status,
                   cudaStream_t st);
-// Crossing chains (longest first), then the per-curve merge into the
-// reference's intersection records rec[N] (curve, t bits | flags).
-// Kernel attributes of the geometry kernels (the long-piece merge's shared
-// memory); once per device before the first frame.
-cudaError_t geom_init();
+// Crossing chains (longest first): their t values in cbuf.
 void launch_chains(const GeomArgs& g, const int32_t* offs, const ChainWork& w, int32_t* cbuf, int sm_count,
                    cudaStream_t st);
-void launch_merge(const GeomArgs& g, const int32_t* offs, const ChainWork& w, int32_t* cbuf, int2* rec,
+// The records (curve, t bits) in the reference's order, from the chains.
+void launch_order_records(const GeomArgs& g, const int32_t* offs, const ChainWork& w, const int32_t* cbuf, int2* rec,
+                          uint32_t* status, int sm_count, cudaStream_t st);
+// The same with the reference's flag bits (make_intersection_1.comp:361-375),
+// for a read-back only.
+void launch_merge(const GeomArgs& g, const int32_t* offs, const ChainWork& w, const int32_t* cbuf, int2* rec,
                   uint32_t* status, cudaStream_t st);
 // One fragment per record: sort key + packed winding bits (4 bits: change,
 // centre part).  With wnp NULL the bits are stored above the key bits of
 // each key instead of in wnp[].
 // n_cap launches the grid; the record count is read from n_dev (offs[C]).
-void launch_fragment(const GeomArgs& g, const int2* rec, const int32_t* offs, int64_t n_cap, const uint32_t* n_dev,
-                     uint64_t* keys, uint8_t* wnp, const DebugOut& dbg, cudaStream_t st);
+void launch_fragment(const GeomArgs& g, const int2* rec, int64_t n_cap, const uint32_t* n_dev, uint64_t* keys,
+                     uint8_t* wnp, const DebugOut& dbg, cudaStream_t st);
 
 // ---- scan.cu
 // Exclusive scan of n int32 values into out[0..n] (out[n] = total), single
