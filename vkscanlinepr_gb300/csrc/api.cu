@@ -98,14 +98,21 @@ uint32_t bits_for(uint64_t v) {   // bits needed to hold values 0..v
     return b == 0 ? 1 : b;
 }
 
+// Words of a frame's control block.  The first nine are its report, read
+// back at its end (and, with exact sizing, after the count).
 enum Ctl : int {
     CTL_STATUS = 0,
-    CTL_SCAN_COUNTER = 1,
-    CTL_WIND_COUNTER = 2,
-    CTL_NDRAW = 3,     // merged fragments + spans of the frame
-    CTL_CHAINS = 4,    // chain counter
-    CTL_QUEUE = 9,     // chain work-queue counter
-    CTL_ROW_SCAN = 13,      // row-start scan's tile counter
+    CTL_N = 1,         // records
+    CTL_LARGEST = 2,   // largest sort segment of more than half a tile
+    CTL_NDRAW = 3,     // merged fragments + spans
+    CTL_TOTALS = 4,    // merged fragments, spans (two 64-bit words)
+    CTL_WIDE = 8,      // sort tiles that needed 64-bit items
+    CTL_REPORT = 9,
+    CTL_SCAN_COUNTER = 9,
+    CTL_WIND_COUNTERS = 10, // next tile, tiles summed
+    CTL_CHAINS = 12,        // chain counter
+    CTL_QUEUE = 13,         // chain work-queue counter
+    CTL_ROW_SCAN = 14,      // row-start scan's tile counter
     CTL_CLASSES = 16,       // chains of each class
     CTL_CLASS_NEXT = CTL_CLASSES + sr::kChainClassWords,
     CTL_WORDS = CTL_CLASS_NEXT + sr::kChainClassWords,
@@ -278,6 +285,7 @@ struct Pipeline {
     // the largest segment the tables accept without flagging an overflow
     int seg_levels = 0;
     uint32_t seg_check = 0;
+    bool seg_wide = true;   // tiles that need 64-bit items are expected
     // scenes
     uint32_t S = 0, V = 0, C = 0, P = 0;
     int32_t Wmax = 1, Hmax = 1;
@@ -286,17 +294,21 @@ struct Pipeline {
     std::vector<sr::SceneInfo> info;
     std::vector<uint32_t> cta_base;
     std::vector<uint8_t> cta_narrow;
-    bool any_narrow = false;
+    bool any_narrow = false, any_wide = false;
     DevBuf pos, pos_path, curve_pos, curve_type, curve_path, fill_rule, fill_info, path_scene, scenes_d, cta_base_d;
     DevBuf cta_narrow_d;
     // frame
-    DevBuf tpos, curve_end, path_visible, cut, count, offs, ctl, scan_status, pieces, chain_lists;
-    DevBuf cbuf, rec, keys, keys_alt, wnp, skeys, svals, vals_alt, sort_scratch, wind_status, draw, draw_row, totals;
-    DevBuf rkeys, rvals, rkeys_alt, rvals_alt, row_sort_scratch, row_start, seg_cut, row_count, row_px, row_scan, image;
+    DevBuf tpos, curve_end, path_begin, cut, count, offs, pieces, chain_lists;
+    // what starts a frame zeroed, cleared by one memset each: before the count
+    // pass the control block, path_visible and the offset scan's words; after
+    // it the tables sized by the capacity (back_layout)
+    DevBuf ctl, zeroed;
+    DevBuf cbuf, rec, keys, keys_alt, wnp, skeys, svals, vals_alt, sort_scratch, wind_sums, draw, draw_row;
+    DevBuf rkeys, rvals, rkeys_alt, rvals_alt, row_sort_scratch, row_start, image;
     DevBuf d_fkey, d_fwn, d_fleft, d_wscan, d_fflag, d_sflag, d_skey;
     // learned sizing: per-path curve ranges, draw counters, features,
     // predictions, allotments and their sums
-    DevBuf path_first, path_draw, feats, preds, allot, plan_tot, judge_out, seg_scratch, seg_tiles;
+    DevBuf path_first, path_draw, feats, preds, allot, plan_tot, judge_out, seg_tiles;
     bool path_first_valid = false, count_paths = false, planned = false;
     unsigned long long* h_plan_ptr = nullptr;   // pinned plan totals
     size_t h_plan_words = 0;
@@ -311,13 +323,12 @@ struct Pipeline {
         size_t off, bytes;
     };
     std::vector<StagedCopy> staged;
-    // host scalars (pinned): N, status; fragments, spans
-    uint32_t* h_u32 = nullptr;
-    uint64_t* h_u64 = nullptr;
+    uint32_t* h_report = nullptr;   // pinned copy of the control block's report
     // results
     sr_stats stats{};
     int64_t last_N = 0, last_O = 0, last_cap = 0, last_dcap = 0;
     uint32_t last_largest = 0;   // records of the frame's largest sort segment
+    uint32_t last_wide = 0;      // its sort tiles that needed 64-bit items
     bool stages_valid = false;
     // a frame's records carry no flag bits: they are merged again with them
     // when they are dumped, with the arguments of the frame
@@ -331,17 +342,15 @@ struct Pipeline {
 
     ~Pipeline() {
         DevBuf* all[] = {&pos, &pos_path, &curve_pos, &curve_type, &curve_path, &fill_rule, &fill_info, &path_scene,
-                         &scenes_d, &cta_base_d, &tpos, &curve_end, &path_visible, &cut, &count, &offs, &ctl, &scan_status,
+                         &scenes_d, &cta_base_d, &tpos, &curve_end, &path_begin, &cut, &count, &offs, &ctl, &zeroed,
                          &pieces, &chain_lists, &cbuf, &rec, &keys, &keys_alt,
-                         &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_status, &draw, &draw_row, &totals,
-                         &rkeys, &rvals, &rkeys_alt, &rvals_alt, &row_sort_scratch, &row_start, &seg_cut, &row_count, &row_px,
-                         &row_scan, &image, &d_fkey, &d_fwn, &d_fleft, &d_wscan, &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw,
-                         &feats, &preds, &allot, &plan_tot, &judge_out, &seg_scratch, &seg_tiles, &cta_narrow_d, &paints_d, &aa_acc};
+                         &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_sums, &draw, &draw_row,
+                         &rkeys, &rvals, &rkeys_alt, &rvals_alt, &row_sort_scratch, &row_start, &image, &d_fkey, &d_fwn, &d_fleft, &d_wscan, &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw,
+                         &feats, &preds, &allot, &plan_tot, &judge_out, &seg_tiles, &cta_narrow_d, &paints_d, &aa_acc};
         for (DevBuf* b : all) release(*b);
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
-        if (h_u32) cudaFreeHost(h_u32);
-        if (h_u64) cudaFreeHost(h_u64);
+        if (h_report) cudaFreeHost(h_report);
         if (h_plan_ptr) cudaFreeHost(h_plan_ptr);
         if (h_stage) cudaFreeHost(h_stage);
         if (up_stream) cudaStreamDestroy(up_stream);
@@ -386,8 +395,7 @@ struct Pipeline {
         CUDA_TRY(cudaSetDevice(dev));
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
         if (sm_count <= 0) sm_count = 148;
-        CUDA_TRY(cudaMallocHost(&h_u32, sizeof(uint32_t) * 8));
-        CUDA_TRY(cudaMallocHost(&h_u64, sizeof(uint64_t) * 4));
+        CUDA_TRY(cudaMallocHost(&h_report, sizeof(uint32_t) * CTL_REPORT));
         CUDA_TRY(ensure(ctl, sizeof(uint32_t) * CTL_WORDS));
         return SR_OK;
     }
@@ -422,7 +430,7 @@ struct Pipeline {
         Hmax = 1;
         cta_base.assign(S + 1, 0);
         cta_narrow.clear();
-        any_narrow = false;
+        any_narrow = any_wide = false;
         for (uint32_t s = 0; s < S; ++s) {
             sr::SceneInfo& si = info[s];
             si.rows = (uint32_t)((si.H + F - 1) / F);
@@ -436,7 +444,7 @@ struct Pipeline {
             uint32_t rpc = sr::resolve_rows_per_cta(si.W, tune.resolve_warps);
             res_ctas += (si.rows + rpc - 1) / rpc;
             cta_narrow.resize(res_ctas, rpc > 1 ? 1 : 0);
-            any_narrow = any_narrow || rpc > 1;
+            (rpc > 1 ? any_narrow : any_wide) = true;
         }
         cta_base[S] = res_ctas;
         CUDA_TRY(ensure(scenes_d, sizeof(sr::SceneInfo) * std::max<uint32_t>(S, 1)));
@@ -561,12 +569,14 @@ struct Pipeline {
     sr::GeomArgs geom(int64_t cap) const {
         sr::GeomArgs g;
         g.n_curves = C;
+        g.n_paths = P;
         g.curve_type = curve_type.as<uint32_t>();
         g.curve_pos = curve_pos.as<uint32_t>();
         g.curve_path = curve_path.as<uint32_t>();
         g.tpos = tpos.as<float2>();
         g.curve_end = curve_end.as<float2>();
-        g.path_visible = path_visible.as<int32_t>();
+        g.path_begin = path_begin.as<uint32_t>();
+        g.path_visible = path_visible();
         g.W = Wmax;
         g.H = Hmax;
         g.F = F;
@@ -600,22 +610,64 @@ struct Pipeline {
     sr_status prepare_front() {
         CUDA_TRY(ensure(tpos, sizeof(float2) * std::max<uint32_t>(V, 1)));
         CUDA_TRY(ensure(curve_end, sizeof(float2) * std::max<uint32_t>(C, 1)));
-        CUDA_TRY(ensure(path_visible, sizeof(int32_t) * std::max<uint32_t>(P, 1)));
+        CUDA_TRY(ensure(path_begin, sizeof(uint32_t) * ((size_t)P + 1)));
+        CUDA_TRY(ensure(ctl, front_bytes()));
         CUDA_TRY(ensure(cut, sizeof(float) * 5 * (size_t)std::max<uint32_t>(C, 1)));
         CUDA_TRY(ensure(count, sizeof(int32_t) * ((size_t)C + 1)));
         CUDA_TRY(ensure(offs, sizeof(int32_t) * ((size_t)C + 1)));
-        CUDA_TRY(ensure(scan_status, sizeof(uint64_t) * sr::scan_status_words(C)));
         CUDA_TRY(ensure(pieces, sr::piece_table_bytes(std::max<uint32_t>(C, 1))));
-        const uint32_t lc = list_cap();
-        CUDA_TRY(ensure(chain_lists, 9 * (size_t)lc));
-        CUDA_TRY(ensure(totals, sizeof(uint64_t) * 4));
+        CUDA_TRY(ensure(chain_lists, 9 * (size_t)list_cap()));
         CUDA_TRY(ensure(row_start, sizeof(int32_t) * ((size_t)total_rows + 1)));
-        CUDA_TRY(ensure(seg_cut, sizeof(uint32_t) * std::max<size_t>(cut_words(), 1)));
-        CUDA_TRY(ensure(row_count, sizeof(uint32_t) * std::max<size_t>(total_rows, 1)));
-        CUDA_TRY(ensure(row_px, sizeof(unsigned long long) * std::max<size_t>(total_rows, 1)));
-        CUDA_TRY(ensure(row_scan, sizeof(uint64_t) * sr::scan_status_words(total_rows)));
-        if (segmented()) CUDA_TRY(ensure(seg_scratch, sr::segsort_scratch_bytes(std::max<uint32_t>(C, 1))));
         return SR_OK;
+    }
+
+    // The buffers zeroed before the count pass: control block, then
+    // path_visible, then the offset scan's look-back words.
+    static size_t pad(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+    size_t visible_at() const { return pad(sizeof(uint32_t) * CTL_WORDS); }
+    size_t scan_at() const { return visible_at() + pad(sizeof(int32_t) * (size_t)std::max<uint32_t>(P, 1)); }
+    size_t front_bytes() const { return scan_at() + sizeof(uint64_t) * sr::offset_scan_words(C); }
+    int32_t* path_visible() const { return reinterpret_cast<int32_t*>(ctl.as<char>() + visible_at()); }
+    uint64_t* offset_scan() const { return reinterpret_cast<uint64_t*>(ctl.as<char>() + scan_at()); }
+
+    // Places in the buffer zeroed after it.
+    struct BackLayout {
+        size_t seg, wind, cut, row_px, row_count, row_scan, row_sort, total;
+    };
+    BackLayout back_layout(int64_t cap, int64_t dcap) const {
+        BackLayout l;
+        size_t at = 0;
+        auto place = [&](size_t bytes) {
+            const size_t here = at;
+            at += pad(bytes);
+            return here;
+        };
+        l.seg = place(segmented() ? sr::segsort_zeroed_bytes(P, std::max<int64_t>(cap, 1)) : 0);
+        l.wind = place(sizeof(uint64_t) * sr::winding_status_words(cap, tune.wind_items));
+        l.cut = place(sizeof(uint32_t) * cut_words());
+        l.row_px = place(sizeof(unsigned long long) * (size_t)total_rows);
+        l.row_count = place(sizeof(uint32_t) * (size_t)total_rows);
+        l.row_scan = place(sizeof(uint64_t) * sr::row_scan_words(total_rows));
+        l.row_sort = place(sr::sort_scratch_bytes(row_plan(draw_cap_for(cap, dcap), nullptr)));
+        l.total = at;
+        return l;
+    }
+    sr::SortPlan row_plan(int64_t draws, const uint32_t* n_dev) const {
+        return sr::sort_plan(draws, bits_for(total_rows), n_dev);
+    }
+    sr::SegArgs seg_args(int64_t cap, void* zero) const {
+        sr::SegArgs a;
+        a.path_begin = path_begin.as<uint32_t>();
+        a.offs = offs.as<int32_t>();
+        a.n_paths = P;
+        a.cap = std::max<int64_t>(cap, 1);
+        a.max_size = seg_check;
+        a.largest = ctl.as<uint32_t>() + CTL_LARGEST;
+        a.wide_count = ctl.as<uint32_t>() + CTL_WIDE;
+        a.wide = seg_wide;
+        a.tables = seg_tiles.p;
+        a.zeroed = zero;
+        return a;
     }
 
     // Resolve segments per cell row (the widest scene's) and the words of
@@ -655,7 +707,7 @@ struct Pipeline {
         const sr::KeyLayout L = layout();
         fn(sort_scratch,
            sr::sort_scratch_bytes(sr::sort_plan(cap, L.pbits + L.rbits + L.xbits, nullptr, tune.sort_items)));
-        fn(wind_status, sizeof(uint64_t) * sr::winding_status_words(cap, tune.wind_items));
+        fn(wind_sums, sizeof(uint64_t) * sr::winding_tile_words(cap, tune.wind_items));
         const size_t d1 = (size_t)draw_cap_for(cap, dcap);
         fn(draw, sizeof(int4) * d1);
         fn(draw_row, sizeof(uint32_t) * d1);
@@ -663,8 +715,8 @@ struct Pipeline {
         fn(rvals, sizeof(uint32_t) * d1);
         fn(rkeys_alt, sizeof(uint32_t) * d1);
         fn(rvals_alt, sizeof(uint32_t) * d1);
-        fn(row_sort_scratch, sr::sort_scratch_bytes(sr::sort_plan((int64_t)d1, bits_for(total_rows), nullptr)));
-        fn(seg_tiles, segmented() ? sr::segsort_tile_bytes(C, std::max<int64_t>(cap, 1)) : 0);
+        fn(zeroed, back_layout(cap, dcap).total);
+        fn(seg_tiles, segmented() ? sr::segsort_table_bytes(P, std::max<int64_t>(cap, 1)) : 0);
     }
 
     // Device bytes a frame of this scene set holds with capacities (cap,
@@ -683,11 +735,11 @@ struct Pipeline {
         add(4 * p1); add(4 * p1); add(4 * p1);                      // fill rule/info, path scene
         add(sizeof(sr::SceneInfo) * std::max<uint32_t>(S, 1)); add(4 * ((size_t)S + 1));
         add(4 * std::max<uint64_t>(total_pixels, 1));               // images
-        add(8 * v1); add(8 * c1); add(4 * p1); add(20 * c1); add(4 * (c1 + 1)); add(4 * (c1 + 1));
-        add(8 * sr::scan_status_words(C)); add(sr::piece_table_bytes((uint32_t)c1));
+        add(8 * v1); add(8 * c1); add(front_bytes()); add(4 * (p1 + 1)); add(20 * c1); add(4 * (c1 + 1)); add(4 * (c1 + 1));
+        add(sr::piece_table_bytes((uint32_t)c1));
         const size_t lc = list_cap();
         add(9 * lc);
-        add(32); add(4 * ((size_t)total_rows + 1));
+        add(4 * ((size_t)total_rows + 1));
         post_count_buffers(cap, dcap, [&](DevBuf&, size_t b) { add(b); });
         return total;
     }
@@ -708,16 +760,16 @@ struct Pipeline {
         static DevBuf Pipeline::* const bufs[] = {
             &Pipeline::pos, &Pipeline::pos_path, &Pipeline::curve_pos, &Pipeline::curve_type,
             &Pipeline::curve_path, &Pipeline::fill_rule, &Pipeline::fill_info, &Pipeline::path_scene,
-            &Pipeline::scenes_d, &Pipeline::cta_base_d, &Pipeline::tpos, &Pipeline::curve_end, &Pipeline::path_visible, &Pipeline::cut,
-            &Pipeline::count, &Pipeline::offs, &Pipeline::ctl, &Pipeline::scan_status, &Pipeline::pieces,
+            &Pipeline::scenes_d, &Pipeline::cta_base_d, &Pipeline::tpos, &Pipeline::curve_end, &Pipeline::path_begin, &Pipeline::cut,
+            &Pipeline::count, &Pipeline::offs, &Pipeline::ctl, &Pipeline::zeroed, &Pipeline::pieces,
             &Pipeline::chain_lists, &Pipeline::cbuf,
             &Pipeline::rec, &Pipeline::keys, &Pipeline::keys_alt, &Pipeline::wnp, &Pipeline::skeys,
-            &Pipeline::svals, &Pipeline::vals_alt, &Pipeline::sort_scratch, &Pipeline::wind_status,
-            &Pipeline::draw, &Pipeline::draw_row, &Pipeline::totals, &Pipeline::rkeys, &Pipeline::rvals,
+            &Pipeline::svals, &Pipeline::vals_alt, &Pipeline::sort_scratch, &Pipeline::wind_sums,
+            &Pipeline::draw, &Pipeline::draw_row, &Pipeline::rkeys, &Pipeline::rvals,
             &Pipeline::rkeys_alt, &Pipeline::rvals_alt, &Pipeline::row_sort_scratch, &Pipeline::row_start,
-            &Pipeline::seg_cut, &Pipeline::row_count, &Pipeline::row_px, &Pipeline::row_scan, &Pipeline::image,
+            &Pipeline::image,
             &Pipeline::path_first, &Pipeline::path_draw, &Pipeline::feats, &Pipeline::preds, &Pipeline::allot,
-            &Pipeline::plan_tot, &Pipeline::judge_out, &Pipeline::seg_scratch, &Pipeline::seg_tiles,
+            &Pipeline::plan_tot, &Pipeline::judge_out, &Pipeline::seg_tiles,
             &Pipeline::cta_narrow_d};
         *moved = false;
         CUDA_TRY(cudaSetDevice(device));
@@ -743,15 +795,15 @@ struct Pipeline {
     // Device bytes currently held by this pipeline.
     uint64_t held_bytes() const {
         const DevBuf* all[] = {&pos, &pos_path, &curve_pos, &curve_type, &curve_path, &fill_rule, &fill_info,
-                               &path_scene, &scenes_d, &cta_base_d, &tpos, &curve_end, &path_visible, &cut, &count, &offs,
-                               &ctl, &scan_status, &pieces, &chain_lists, &cbuf,
-                               &rec, &keys, &keys_alt, &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_status,
-                               &draw, &draw_row, &totals, &rkeys, &rvals, &rkeys_alt, &rvals_alt,
-                               &row_sort_scratch, &row_start, &seg_cut, &row_count, &row_px, &row_scan, &image, &d_fkey,
+                               &path_scene, &scenes_d, &cta_base_d, &tpos, &curve_end, &path_begin, &cut, &count, &offs,
+                               &ctl, &zeroed, &pieces, &chain_lists, &cbuf,
+                               &rec, &keys, &keys_alt, &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_sums,
+                               &draw, &draw_row, &rkeys, &rvals, &rkeys_alt, &rvals_alt,
+                               &row_sort_scratch, &row_start, &image, &d_fkey,
                                &d_fwn, &d_fleft,
                                &d_wscan,
                                &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw, &feats, &preds, &allot,
-                               &plan_tot, &judge_out, &seg_scratch, &seg_tiles, &cta_narrow_d};
+                               &plan_tot, &judge_out, &seg_tiles, &cta_narrow_d};
         uint64_t t = 0;
         for (const DevBuf* b : all) t += b->cap;
         return t;
@@ -783,17 +835,14 @@ struct Pipeline {
         using namespace sr;
         uint32_t* ctlp = ctl.as<uint32_t>();
         uint32_t* status = ctlp + CTL_STATUS;
-        CUDA_TRY(cudaMemsetAsync(ctlp, 0, sizeof(uint32_t) * CTL_WORDS, st));
-        CUDA_TRY(cudaMemsetAsync(path_visible.p, 0, sizeof(int32_t) * std::max<uint32_t>(P, 1), st));
-        CUDA_TRY(cudaMemsetAsync(scan_status.p, 0, sizeof(uint64_t) * scan_status_words(C), st));
-        CUDA_TRY(cudaMemsetAsync(totals.p, 0, sizeof(uint64_t) * 4, st));
+        CUDA_TRY(cudaMemsetAsync(ctl.p, 0, front_bytes(), st));
         if (count_paths) CUDA_TRY(cudaMemsetAsync(path_draw.p, 0, sizeof(uint32_t) * std::max<uint32_t>(P, 1), st));
         mark(ST_TRANSFORM, false);
         launch_transform(pos.as<float2>(), pos_path.as<uint32_t>(), V, table(), tpos.as<float2>(),
-                         path_visible.as<int32_t>(), st);
+                         path_visible(), st);
         if (arcs)
             launch_arc_fixup(curve_type.as<uint32_t>(), curve_pos.as<uint32_t>(), curve_path.as<uint32_t>(), C,
-                             pos.as<float2>(), table(), tpos.as<float2>(), path_visible.as<int32_t>(), st);
+                             pos.as<float2>(), table(), tpos.as<float2>(), path_visible(), st);
         mark(ST_TRANSFORM, true);
         const GeomArgs g = geom(0);
         const ChainWork cw = chain_work();
@@ -801,11 +850,8 @@ struct Pipeline {
         launch_count(g, cut.as<float>(), count.as<int32_t>(), cw, status, st);
         mark(ST_COUNT, true);
         mark(ST_SCAN, false);
-        launch_exclusive_scan_i32(count.as<int32_t>(), offs.as<int32_t>(), C, scan_status.as<uint64_t>(),
-                                  ctlp + CTL_SCAN_COUNTER, status, st);
-        if (segmented())
-            launch_segsort_tables(curve_path.as<uint32_t>(), offs.as<int32_t>(), C, seg_check, seg_scratch.p, status,
-                                  st);
+        launch_offsets_and_order(g, count.as<int32_t>(), offs.as<int32_t>(), cw, offset_scan(),
+                                 ctlp + CTL_SCAN_COUNTER, ctlp + CTL_N, status, sm_count, st);
         mark(ST_SCAN, true);
         CUDA_TRY(cudaGetLastError());
         return SR_OK;
@@ -819,6 +865,9 @@ struct Pipeline {
         uint32_t* status = ctlp + CTL_STATUS;
         const bool keep = (flags & SR_FLAG_KEEP_STAGES) != 0;
         const uint32_t* n_dev = reinterpret_cast<const uint32_t*>(offs.as<int32_t>() + C);
+        const BackLayout at = back_layout(cap, dcap_req);
+        char* zero = zeroed.as<char>();
+        CUDA_TRY(cudaMemsetAsync(zero, 0, at.total, st));
         const GeomArgs g = geom(cap);
         const ChainWork cw = chain_work();
         DebugOut dbg{nullptr, nullptr, nullptr};
@@ -845,14 +894,13 @@ struct Pipeline {
         mark(ST_SORT, false);
         last_segsort = segmented() && seg_levels >= 0;
         if (last_segsort)
-            launch_segsort(keys.as<uint64_t>(), skeys.as<uint64_t>(), keys_alt.as<uint64_t>(), cap, C, L, seg_levels,
-                           seg_scratch.p, seg_tiles.p, sm_count, status, st);
+            launch_segsort(seg_args(cap, zero + at.seg), keys.as<uint64_t>(), skeys.as<uint64_t>(),
+                           keys_alt.as<uint64_t>(), L, seg_levels, sm_count, status, st);
         else
             launch_sort_u64(sp, keys.as<uint64_t>(), nullptr, skeys.as<uint64_t>(),
                             keep ? svals.as<uint32_t>() : nullptr, keys_alt.as<uint64_t>(),
                             keep ? vals_alt.as<uint32_t>() : nullptr, sort_scratch.p, status, st);
         mark(ST_SORT, true);
-        CUDA_TRY(cudaMemsetAsync(wind_status.p, 0, sizeof(uint64_t) * winding_status_words(cap, tune.wind_items), st));
         WindArgs wa;
         wa.n = cap;
         wa.n_dev = n_dev;
@@ -872,35 +920,31 @@ struct Pipeline {
         const int64_t dcap = draw_cap_for(cap, dcap_req);
         wa.draw_capacity = dcap;
         wa.draw_row = draw_row.as<uint32_t>();
-        wa.totals = totals.as<uint64_t>();
+        wa.totals = reinterpret_cast<uint64_t*>(ctlp + CTL_TOTALS);
         wa.n_draw = ctlp + CTL_NDRAW;
         wa.path_draw = count_paths ? path_draw.as<uint32_t>() : nullptr;
         wa.dbg_wscan = keep ? d_wscan.as<int32_t>() : nullptr;
         wa.dbg_fflag = keep ? d_fflag.as<int32_t>() : nullptr;
         wa.dbg_sflag = keep ? d_sflag.as<int32_t>() : nullptr;
         wa.dbg_skey = keep ? d_skey.as<int32_t>() : nullptr;
-        wa.seg_cut = seg_cut.as<uint32_t>();
+        wa.seg_cut = reinterpret_cast<uint32_t*>(zero + at.cut);
         wa.cut_rows = total_rows;
         wa.cut_segs = cut_segs();
-        wa.row_count = row_count.as<uint32_t>();
-        wa.row_px = row_px.as<unsigned long long>();
-        CUDA_TRY(cudaMemsetAsync(seg_cut.p, 0, sizeof(uint32_t) * cut_words(), st));
-        CUDA_TRY(cudaMemsetAsync(row_count.p, 0, sizeof(uint32_t) * total_rows, st));
-        CUDA_TRY(cudaMemsetAsync(row_px.p, 0, sizeof(unsigned long long) * total_rows, st));
-        CUDA_TRY(cudaMemsetAsync(row_scan.p, 0, sizeof(uint64_t) * sr::scan_status_words(total_rows), st));
+        wa.row_count = reinterpret_cast<uint32_t*>(zero + at.row_count);
+        wa.row_px = reinterpret_cast<unsigned long long*>(zero + at.row_px);
         mark(ST_WINDING, false);
-        launch_winding_emit(wa, tune.wind_items, wind_status.as<uint64_t>(), ctlp + CTL_WIND_COUNTER, status, st);
+        launch_winding_emit(wa, tune.wind_items, reinterpret_cast<uint64_t*>(zero + at.wind), wind_sums.as<uint64_t>(),
+                            ctlp + CTL_WIND_COUNTERS, status, st);
         mark(ST_WINDING, true);
-        SortPlan rp = sort_plan(dcap, bits_for(total_rows), ctlp + CTL_NDRAW);
+        SortPlan rp = row_plan(dcap, ctlp + CTL_NDRAW);
         mark(ST_ROWSORT, false);
         // the emit counted the records of every row: their exclusive scan is
         // each row's start in the row order, and their digits the sort's
         // histogram
-        launch_exclusive_scan_i32(row_count.as<int32_t>(), row_start.as<int32_t>(), total_rows, row_scan.as<uint64_t>(),
-                                  ctlp + CTL_ROW_SCAN, status, st);
-        sort_hist_from_counts(rp, row_count.as<uint32_t>(), total_rows, row_sort_scratch.p, st);
+        launch_row_starts(rp, wa.row_count, total_rows, row_start.as<int32_t>(), zero + at.row_sort,
+                          reinterpret_cast<uint64_t*>(zero + at.row_scan), ctlp + CTL_ROW_SCAN, status, st);
         launch_sort_u32(rp, draw_row.as<uint32_t>(), nullptr, rkeys.as<uint32_t>(), rvals.as<uint32_t>(),
-                        rkeys_alt.as<uint32_t>(), rvals_alt.as<uint32_t>(), row_sort_scratch.p, status, st);
+                        rkeys_alt.as<uint32_t>(), rvals_alt.as<uint32_t>(), zero + at.row_sort, status, st);
         mark(ST_ROWSORT, true);
         ResolveArgs ra;
         ra.draw = draw.as<int4>();
@@ -913,11 +957,12 @@ struct Pipeline {
         ra.warps = tune.resolve_warps;
         ra.pixel_mode = g.pixel_mode;
         ra.image = image.as<uint32_t>();
-        ra.seg_cut = seg_cut.as<uint32_t>();
+        ra.seg_cut = wa.seg_cut;
         ra.cut_segs = cut_segs();
-        ra.row_px = row_px.as<unsigned long long>();
+        ra.row_px = wa.row_px;
         ra.cta_narrow = cta_narrow_d.as<uint8_t>();
         ra.any_narrow = any_narrow ? 1 : 0;
+        ra.any_wide = any_wide ? 1 : 0;
         ra.paints = n_paints ? paints_d.as<DevPaint>() : nullptr;
         ra.n_paints = n_paints;
         mark(ST_RESOLVE, false);
@@ -940,16 +985,12 @@ struct Pipeline {
 
     // Read N back (the reference's count read-back, scanline_rasterizer.cpp:355-356).
     sr_status read_count(cudaStream_t st, int64_t* N) {
-        CUDA_TRY(cudaMemcpyAsync(&h_u32[0], offs.as<int32_t>() + C, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaMemcpyAsync(&h_u32[1], ctl.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        h_u32[2] = 0;
-        if (segmented())
-            CUDA_TRY(cudaMemcpyAsync(&h_u32[2], sr::segsort_largest(seg_scratch.p, C), sizeof(uint32_t),
-                                     cudaMemcpyDeviceToHost, st));
+        if (segmented()) sr::launch_segsort_largest(seg_args(1, nullptr), st);
+        SR_TRY(enqueue_readback(st));
         CUDA_TRY(cudaStreamSynchronize(st));
-        SR_TRY(check_status_word(h_u32[1]));
-        seg_levels = levels_for(h_u32[2]);
-        *N = (int64_t)(int32_t)h_u32[0];
+        SR_TRY(check_status_word(h_report[CTL_STATUS]));
+        seg_levels = levels_for(h_report[CTL_LARGEST]);
+        *N = (int64_t)(int32_t)h_report[CTL_N];
         if (*N < 0 || *N >= (1ll << 30))
             return fail(SR_ERR_OVERFLOW_REFIT, "record count %lld out of range", (long long)*N);
         return SR_OK;
@@ -968,8 +1009,9 @@ struct Pipeline {
     // One frame.  cap < 0: size the record buffers exactly (one host wait
     // for N); cap >= 0: use that capacity without waiting, with `levels`
     // merge rounds of the segmented sort (a larger segment flags an
-    // overflow).  dcap <= 0 sizes the draw records at 2 x cap.
-    sr_status frame(cudaStream_t st, int64_t cap, int64_t dcap = -1, int levels = kSegLevelsMax) {
+    // overflow) and, unless `wide`, without the 64-bit sort of tiles that need
+    // it (such a tile flags one too).  dcap <= 0 sizes the draw records at 2 x cap.
+    sr_status frame(cudaStream_t st, int64_t cap, int64_t dcap = -1, int levels = kSegLevelsMax, bool wide = true) {
         CUDA_TRY(cudaSetDevice(device));
         if (!loaded) return fail(SR_ERR_NO_SCENE, "render before a scene was loaded");
         cur = st;
@@ -981,6 +1023,7 @@ struct Pipeline {
         if (levels < 0 || levels > kSegLevelsMax) levels = kSegLevelsMax;
         seg_check = cap < 0 ? 0u : (uint32_t)sr::segsort_tile() << levels;
         seg_levels = levels;
+        seg_wide = wide || cap < 0;
         SR_TRY(enqueue_front(st));
         if (cap < 0) {
             int64_t N = 0;
@@ -997,16 +1040,9 @@ struct Pipeline {
         return SR_OK;
     }
 
-    // Waits for the frame and collects its counters and status.
-    // Queues the copies of the frame's counters into pinned host memory.
+    // Queues the copy of the frame's report into pinned host memory.
     sr_status enqueue_readback(cudaStream_t st) {
-        CUDA_TRY(cudaMemcpyAsync(&h_u32[0], offs.as<int32_t>() + C, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaMemcpyAsync(&h_u32[1], ctl.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaMemcpyAsync(h_u64, totals.p, sizeof(uint64_t) * 2, cudaMemcpyDeviceToHost, st));
-        h_u32[2] = 0;
-        if (segmented())
-            CUDA_TRY(cudaMemcpyAsync(&h_u32[2], sr::segsort_largest(seg_scratch.p, C), sizeof(uint32_t),
-                                     cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaMemcpyAsync(h_report, ctl.p, sizeof(uint32_t) * CTL_REPORT, cudaMemcpyDeviceToHost, st));
         return SR_OK;
     }
 
@@ -1018,17 +1054,20 @@ struct Pipeline {
 
     // The frame's counters and status, once the read-back has landed.
     sr_status collect() {
-        last_N = (int64_t)(int32_t)h_u32[0];
-        last_O = (int64_t)(h_u64[0] + h_u64[1]);
-        last_largest = h_u32[2];
+        uint64_t totals[2];
+        std::memcpy(totals, h_report + CTL_TOTALS, sizeof totals);
+        last_N = (int64_t)(int32_t)h_report[CTL_N];
+        last_O = (int64_t)(totals[0] + totals[1]);
+        last_largest = h_report[CTL_LARGEST];
+        last_wide = h_report[CTL_WIDE];
         stats.n_intersections = (uint64_t)last_N;
         stats.n_draw_records = (uint64_t)last_O;
-        stats.n_merged_fragments = h_u64[0];
-        stats.n_spans = h_u64[1];
+        stats.n_merged_fragments = totals[0];
+        stats.n_spans = totals[1];
         const sr::KeyLayout L = layout();
         stats.key_bits = L.pbits + L.rbits + L.xbits;
         stats.sort_passes = sr::sort_plan(1, stats.key_bits).passes;
-        SR_TRY(check_status_word(h_u32[1]));
+        SR_TRY(check_status_word(h_report[CTL_STATUS]));
         if (last_N > last_cap)
             return fail(SR_ERR_OVERFLOW_REFIT, "frame needs %lld records, capacity %lld", (long long)last_N,
                         (long long)last_cap);
@@ -1062,7 +1101,7 @@ struct sr_ctx {
     bool hint_valid = false;
     uint32_t hint_C = 0, hint_P = 0;
     int64_t hint_N = 0, hint_O = 0;
-    uint32_t hint_largest = 0;
+    uint32_t hint_largest = 0, hint_wide = 0;
     uint32_t refits = 0;
 };
 
@@ -1209,7 +1248,7 @@ static sr_status render_core(sr_ctx* c, void* rgba_out, int out_is_device, cudaS
         const int64_t cap = c->hint_N + c->hint_N / 16 + 256;
         const int64_t dcap = c->hint_O + c->hint_O / 16 + 256;
         int levels = Pipeline::levels_for(c->hint_largest + c->hint_largest / 16);
-        SR_TRY(p.frame(st, cap, dcap, levels < 0 ? Pipeline::kSegLevelsMax : levels));
+        SR_TRY(p.frame(st, cap, dcap, levels < 0 ? Pipeline::kSegLevelsMax : levels, c->hint_wide != 0));
         if (rgba_out)
             CUDA_TRY(cudaMemcpyAsync(rgba_out, p.image.p, bytes,
                                      out_is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
@@ -1232,6 +1271,7 @@ static sr_status render_core(sr_ctx* c, void* rgba_out, int out_is_device, cudaS
         c->hint_N = p.last_N;
         c->hint_O = p.last_O;
         c->hint_largest = p.last_largest;
+        c->hint_wide |= p.last_wide;   // a context that met such tiles once keeps expecting them
     }
     return s;
 }
@@ -1353,6 +1393,7 @@ sr_status sr_render_draw_list(sr_ctx* c, const int32_t* records, int64_t n, void
     ra.row_px = nullptr;
     ra.cta_narrow = p.cta_narrow_d.as<uint8_t>();
     ra.any_narrow = p.any_narrow ? 1 : 0;
+    ra.any_wide = p.any_wide ? 1 : 0;
     ra.paints = p.n_paints ? p.paints_d.as<sr::DevPaint>() : nullptr;
     ra.n_paints = p.n_paints;
     sr::launch_resolve(ra, p.res_ctas, st);
@@ -1362,9 +1403,9 @@ sr_status sr_render_draw_list(sr_ctx* c, const int32_t* records, int64_t n, void
         CUDA_TRY(cudaMemcpyAsync(rgba_out, p.image.p, (size_t)c->W * c->H * 4,
                                  out_is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
     }
-    CUDA_TRY(cudaMemcpyAsync(&p.h_u32[1], status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(p.h_report, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
-    return check_status_word(p.h_u32[1]);
+    return check_status_word(p.h_report[0]);
 }
 
 sr_status sr_get_stats(const sr_ctx* cc, sr_stats* out) {
@@ -1384,7 +1425,7 @@ sr_status sr_debug_dump(sr_ctx* c, int stage, void* dst, size_t* bytes) {
     bool need_stages = true;
     switch (stage) {
         case SR_STAGE_TRANSFORMED_POS: src = p.tpos.p; need = 8 * (size_t)p.V; need_stages = false; break;
-        case SR_STAGE_PATH_VISIBLE: src = p.path_visible.p; need = 4 * (size_t)p.P; need_stages = false; break;
+        case SR_STAGE_PATH_VISIBLE: src = p.tpos.p && p.ctl.cap >= p.front_bytes() ? p.path_visible() : nullptr; need = 4 * (size_t)p.P; need_stages = false; break;
         case SR_STAGE_CUTPOINTS: src = p.cut.p; need = 20 * (size_t)p.C; need_stages = false; break;
         case SR_STAGE_CURVE_COUNT: src = p.count.p; need = 4 * (size_t)p.C; need_stages = false; break;
         case SR_STAGE_CURVE_OFFSET: src = p.offs.p; need = 4 * ((size_t)p.C + 1); need_stages = false; break;
@@ -1426,7 +1467,8 @@ sr_status sr_debug_sort_tiles(sr_ctx* c, uint32_t* tiles, uint32_t* wide_tiles) 
     CUDA_TRY(cudaSetDevice(p.device));
     CUDA_TRY(cudaDeviceSynchronize());
     uint32_t v[2] = {0, 0};
-    CUDA_TRY(sr::segsort_tile_counts(p.seg_tiles.p, p.C, p.last_cap, v));
+    CUDA_TRY(sr::segsort_tile_counts(p.seg_args(p.last_cap, p.zeroed.as<char>() + p.back_layout(p.last_cap, p.last_dcap).seg),
+                                     v));
     *tiles = v[0];
     *wide_tiles = v[1];
     return SR_OK;
@@ -1999,12 +2041,12 @@ sr_status sr_batch_path_features(sr_batch* b, float* d_feats, void* stream) {
     SR_TRY(batch_path_first(b));
     SR_TRY(p.prepare_front());
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    CUDA_TRY(cudaMemsetAsync(p.path_visible.p, 0, sizeof(int32_t) * std::max<uint32_t>(p.P, 1), st));
+    CUDA_TRY(cudaMemsetAsync(p.path_visible(), 0, sizeof(int32_t) * std::max<uint32_t>(p.P, 1), st));
     sr::launch_transform(p.pos.as<float2>(), p.pos_path.as<uint32_t>(), p.V, p.table(), p.tpos.as<float2>(),
-                         p.path_visible.as<int32_t>(), st);
+                         p.path_visible(), st);
     if (p.arcs)
         sr::launch_arc_fixup(p.curve_type.as<uint32_t>(), p.curve_pos.as<uint32_t>(), p.curve_path.as<uint32_t>(), p.C,
-                             p.pos.as<float2>(), p.table(), p.tpos.as<float2>(), p.path_visible.as<int32_t>(), st);
+                             p.pos.as<float2>(), p.table(), p.tpos.as<float2>(), p.path_visible(), st);
     sr::launch_path_features(p.geom(0), p.path_first.as<uint32_t>(), p.P, d_feats, st);
     CUDA_TRY(cudaGetLastError());
     return SR_OK;

@@ -7,8 +7,8 @@
 // gen_fragment.comp           -> k_fragment
 #include <algorithm>
 
-#include "common.cuh"
 #include "kernels.h"
+#include "scan.cuh"
 
 namespace sr {
 
@@ -383,6 +383,11 @@ __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restri
         }
         count[c] = pc;
         g.curve_end[c] = make_float2(x0, y0);   // at t = 1
+        // first curve of every path up to this curve's (curves are grouped by
+        // path, in order; a path without curves starts where the next does)
+        for (uint32_t q = c ? g.curve_path[c - 1] + 1u : 0u; q <= path; ++q) g.path_begin[q] = c;
+        if (c == g.n_curves - 1)
+            for (uint32_t q = path + 1u; q <= g.n_paths; ++q) g.path_begin[q] = g.n_curves;
         if (walk != pc) set_error(status, ERR_RECORD_RANGE);
     }
     // append the chains with their classes, and count the classes (one
@@ -420,15 +425,31 @@ SR_DEV void class_starts(const uint32_t* __restrict__ class_count, uint32_t& s0,
     s1 = s0 + a;
 }
 
-// Orders the chains by class (in no order within one): a counting sort whose
-// counts the count pass made, so one launch.  The radix sort that it
-// replaced took five (two clears, histogram, scan, pass).
-__global__ void __launch_bounds__(256) k_order_chains(const uint32_t* __restrict__ items,
-                                                      const uint8_t* __restrict__ keys, uint32_t list_cap,
-                                                      const uint32_t* __restrict__ chain_count,
-                                                      const uint32_t* __restrict__ class_count,
-                                                      uint32_t* __restrict__ class_next, uint32_t* __restrict__ sorted) {
+// Two things that follow the count pass and do not touch each other, in one
+// launch (a launch costs 2-3 us of a small frame): the first scan_tiles CTAs
+// scan the curves' counts into their record offsets; the others order the
+// chains by class (in no order within one), a counting sort whose counts the
+// count pass made (the radix sort that it replaced took five launches).  The
+// scan's last tile also leaves the record count in report_n.
+constexpr int kOffsetRows = 1;   // small tiles: 240 K curves are 234 of them
+__global__ void __launch_bounds__(256) k_offsets_and_order(
+    const int32_t* __restrict__ count, int32_t* __restrict__ offs, uint32_t n_curves, uint32_t scan_tiles,
+    uint64_t* tstat, uint32_t* counter, uint32_t* report_n, uint32_t* status, uint32_t spin_limit,
+    const uint32_t* __restrict__ items, const uint8_t* __restrict__ keys, uint32_t list_cap,
+    const uint32_t* __restrict__ chain_count, const uint32_t* __restrict__ class_count,
+    uint32_t* __restrict__ class_next, uint32_t* __restrict__ sorted) {
     __shared__ uint32_t s_start[kChainClasses], s_hist[kChainClasses], s_at[kChainClasses];
+    __shared__ uint32_t s_tile;
+    __shared__ int32_t s_warp[256 / 32 + 1];
+    if (blockIdx.x < scan_tiles) {
+        if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
+        __syncthreads();
+        int32_t total;
+        if (scan_tile_i32<kOffsetRows, 256>(count, offs, n_curves, s_tile, tstat, status, spin_limit, s_warp, &total) &&
+            threadIdx.x == 0)
+            *report_n = (uint32_t)total;
+        return;
+    }
     const uint32_t n = imin((int32_t)*chain_count, (int32_t)list_cap);
     if (threadIdx.x < 32) {
         uint32_t a, b;
@@ -436,7 +457,7 @@ __global__ void __launch_bounds__(256) k_order_chains(const uint32_t* __restrict
         s_start[2 * threadIdx.x] = a;
         s_start[2 * threadIdx.x + 1] = b;
     }
-    for (uint32_t i0 = blockIdx.x * 256u; i0 < n; i0 += gridDim.x * 256u) {
+    for (uint32_t i0 = (blockIdx.x - scan_tiles) * 256u; i0 < n; i0 += (gridDim.x - scan_tiles) * 256u) {
         if (threadIdx.x < kChainClasses) s_hist[threadIdx.x] = 0;
         __syncthreads();
         const uint32_t i = i0 + threadIdx.x;
@@ -1120,30 +1141,34 @@ void launch_transform(const float2* pos, const uint32_t* pos_path, uint32_t n_po
     k_transform<<<(n_points + 255) / 256, 256, 0, st>>>(pos, pos_path, n_points, t, tpos, path_visible);
 }
 
-static int sm_count_hint() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n * 8;
-}
-
 size_t piece_table_bytes(uint32_t n_curves) { return sizeof(uint4) * kMaxPieces * (size_t)n_curves; }
 uint32_t chain_list_capacity(uint32_t n_curves) { return 2u * kMaxPieces * n_curves; }
 
 void launch_count(const GeomArgs& g, float* cut_cache, int32_t* count, const ChainWork& w, uint32_t* status,
                   cudaStream_t st) {
     if (g.n_curves == 0) return;
-    count_launches(2);
+    count_launches(1);
     k_count<<<(g.n_curves + 255) / 256, 256, 0, st>>>(g, cut_cache, count, w.pieces, w.chain_items, w.chain_keys,
                                                       w.list_cap, w.chain_count, w.class_count, status);
-    const unsigned most = (unsigned)sm_count_hint() / 2;
-    const unsigned grid = (unsigned)std::min<size_t>(((size_t)w.list_cap + 255) / 256, most);
-    k_order_chains<<<grid, 256, 0, st>>>(w.chain_items, w.chain_keys, w.list_cap, w.chain_count, w.class_count,
-                                         w.class_next, w.sorted_items);
+}
+
+static uint32_t offset_tiles(uint32_t n_curves) { return (n_curves + 1024 * kOffsetRows - 1) / (1024 * kOffsetRows); }
+size_t offset_scan_words(uint32_t n_curves) { return (size_t)offset_tiles(n_curves) + 1; }
+
+void launch_offsets_and_order(const GeomArgs& g, const int32_t* count, int32_t* offs, const ChainWork& w,
+                              uint64_t* tile_status, uint32_t* tile_counter, uint32_t* report_n, uint32_t* status,
+                              int sm_count, cudaStream_t st) {
+    if (g.n_curves == 0) {
+        cudaMemsetAsync(offs, 0, sizeof(int32_t), st);
+        return;
+    }
+    count_launches(1);
+    const uint32_t tiles = offset_tiles(g.n_curves);
+    const unsigned order = (unsigned)std::min<size_t>(((size_t)w.list_cap + 255) / 256, (size_t)sm_count * 4);
+    k_offsets_and_order<<<tiles + order, 256, 0, st>>>(count, offs, g.n_curves, tiles, tile_status, tile_counter,
+                                                       report_n, status, spin_limit(), w.chain_items, w.chain_keys,
+                                                       w.list_cap, w.chain_count, w.class_count, w.class_next,
+                                                       w.sorted_items);
 }
 
 void launch_chains(const GeomArgs& g, const int32_t* offs, const ChainWork& w, int32_t* cbuf, int sm_count,

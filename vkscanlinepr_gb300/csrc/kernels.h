@@ -61,13 +61,14 @@ SR_DEV const SceneInfo& scene_of_path(const SceneTable& t, uint32_t path) { retu
 // largest canvas of the batch (key layout); each scene's own canvas comes
 // from the scene table.
 struct GeomArgs {
-    uint32_t n_curves;
+    uint32_t n_curves, n_paths;
     const uint32_t* curve_type;
     const uint32_t* curve_pos;
     const uint32_t* curve_path;
     const float2* tpos;
     const int32_t* path_visible;
     float2* curve_end;   // [n_curves] each curve's point at t = 1 (written by the count pass)
+    uint32_t* path_begin;   // [n_paths + 1] first curve of each path (likewise)
     int32_t W, H, F;
     int32_t pixel_mode;
     KeyLayout L;
@@ -106,6 +107,13 @@ void launch_transform(const float2* pos, const uint32_t* pos_path, uint32_t n_po
                       float2* tpos, int32_t* path_visible, cudaStream_t st);
 void launch_count(const GeomArgs& g, float* cut_cache, int32_t* count, const ChainWork& w, uint32_t* status,
                   cudaStream_t st);
+// After the count pass: the curves' record offsets offs[0..C] (exclusive scan
+// of count, look-back words and counter zeroed; the total also to report_n)
+// and the chains in class order.
+size_t offset_scan_words(uint32_t n_curves);
+void launch_offsets_and_order(const GeomArgs& g, const int32_t* count, int32_t* offs, const ChainWork& w,
+                              uint64_t* tile_status, uint32_t* tile_counter, uint32_t* report_n, uint32_t* status,
+                              int sm_count, cudaStream_t st);
 // Crossing chains (longest first): their t values in cbuf.
 void launch_chains(const GeomArgs& g, const int32_t* offs, const ChainWork& w, int32_t* cbuf, int sm_count,
                    cudaStream_t st);
@@ -139,7 +147,8 @@ struct SortPlan {
     uint32_t passes;
     uint32_t tiles;
     int items;                 // keys per thread of a tile: 8, 12 or 16
-    int hist_given = 0;        // 1: the digit counts are already in the scratch (sort_hist_from_counts)
+    int cleared = 0;           // 1: the caller has zeroed the scratch
+    int hist_given = 0;        // 1: the digit counts are in the scratch (launch_row_starts), the rest zeroed
 };
 SortPlan sort_plan(int64_t n, uint32_t key_bits, const uint32_t* n_dev = nullptr, int items = 12);
 // Device scratch needed by a plan (bytes).
@@ -151,37 +160,48 @@ size_t sort_scratch_bytes(const SortPlan& p);
 void launch_sort_u64(const SortPlan& p, const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out,
                      uint32_t* vals_out, uint64_t* keys_alt, uint32_t* vals_alt, void* scratch,
                      uint32_t* status, cudaStream_t st);
-// For keys that are bin indices 0..n_bins-1 whose counts are known: writes
-// each pass's digit counts into the plan's scratch (and sets hist_given on
-// the plan), so the sort skips its own histogram pass over the keys.
-void sort_hist_from_counts(SortPlan& p, const uint32_t* counts, uint32_t n_bins, void* scratch, cudaStream_t st);
+// For a sort by row whose records per row are known: each row's first
+// position row_start[0..rows] (exclusive scan; look-back words and counter
+// zeroed) and every pass's digit counts into the plan's zeroed scratch, so
+// that the sort needs no pass over the keys for them.
+size_t row_scan_words(uint32_t rows);
+void launch_row_starts(SortPlan& p, const uint32_t* row_count, uint32_t rows, int32_t* row_start, void* scratch,
+                       uint64_t* tile_status, uint32_t* tile_counter, uint32_t* status, cudaStream_t st);
 void launch_sort_u32(const SortPlan& p, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                      uint32_t* vals_out, uint32_t* keys_alt, uint32_t* vals_alt, void* scratch,
                      uint32_t* status, cudaStream_t st);
 
 // ---- segsort.cu  (stable sort of path-ordered keys: per-path segments)
-// Tables of the path segments from the curve offsets; max_size > 0 flags a
-// segment larger than that as a capacity overflow.
-size_t segsort_scratch_bytes(uint32_t n_curves);
-// Tile tables of a frame with capacity cap (a second buffer).
-size_t segsort_tile_bytes(uint32_t n_curves, int64_t cap);
+// Segment p is the records of path p, from the paths' first curves and the
+// curves' offsets.
+struct SegArgs {
+    const uint32_t* path_begin;   // [P + 1]
+    const int32_t* offs;          // [C + 1]
+    uint32_t n_paths;
+    int64_t cap;                  // records the tables and buffers are sized for
+    uint32_t max_size;            // > 0: a segment larger than that is flagged as a capacity overflow
+    uint32_t* largest;            // largest segment of more than half a tile (0 if none); zeroed before
+    uint32_t* wide_count;         // tiles that needed 64-bit items; zeroed before
+    bool wide;                    // those tiles are sorted (else flagged as a capacity overflow)
+    void* tables;                 // segsort_table_bytes
+    void* zeroed;                 // segsort_zeroed_bytes, zeroed before
+};
+size_t segsort_table_bytes(uint32_t n_paths, int64_t cap);
+size_t segsort_zeroed_bytes(uint32_t n_paths, int64_t cap);
 int segsort_tile();
-void launch_segsort_tables(const uint32_t* curve_path, const int32_t* offs, uint32_t n_curves, uint32_t max_size,
-                           void* scratch, uint32_t* status, cudaStream_t st);
-// Tiles of the last segmented sort with these tables, and of those the
-// ones sorted with 64-bit items (synchronous copies).
-cudaError_t segsort_tile_counts(const void* tiles, uint32_t n_curves, int64_t cap, uint32_t out[2]);
-// Device word holding the largest segment of more than half a tile (0 if none).
-const uint32_t* segsort_largest(const void* scratch, uint32_t n_curves);
+// Tiles of the sort with these tables, and of those the ones that needed
+// 64-bit items (synchronous copies).
+cudaError_t segsort_tile_counts(const SegArgs& a, uint32_t out[2]);
+// The largest segment alone (before the sort's buffers exist).
+void launch_segsort_largest(const SegArgs& a, cudaStream_t st);
 // Sorts keys_in[0, N) into keys_out by their key bits (layout L; N from the
-// tables; cap bounds the tile tables); `levels` merge rounds launched, at
+// offsets; cap bounds the tile tables); `levels` merge rounds launched, at
 // least ceil(log2(chunks of the largest segment)).  keys_alt is scratch.
 // The tile sort and the merge rounds run one wave of persistent CTAs.
 // keys_in[0, N) is left unspecified (the tiles that need 64-bit items sort
 // through it).
-void launch_segsort(uint64_t* keys_in, uint64_t* keys_out, uint64_t* keys_alt, int64_t cap, uint32_t n_curves,
-                    const KeyLayout& L, int levels, void* scratch, void* tiles, int sm_count, uint32_t* status,
-                    cudaStream_t st);
+void launch_segsort(const SegArgs& a, uint64_t* keys_in, uint64_t* keys_out, uint64_t* keys_alt, const KeyLayout& L,
+                    int levels, int sm_count, uint32_t* status, cudaStream_t st);
 
 // ---- winding.cu
 struct WindArgs {
@@ -217,9 +237,12 @@ struct WindArgs {
     int32_t* dbg_sflag;             // [N]
     int32_t* dbg_skey;              // [N]
 };
-// items: records per thread of a tile (4 or 8).
+// items: records per thread of a tile (4 or 8).  Look-back words (zeroed
+// before), and words for the tiles' sums and prefixes; counters[0] (next
+// tile) and counters[1] (tiles summed) are zeroed before.
 size_t winding_status_words(int64_t n, int items = 8);
-void launch_winding_emit(const WindArgs& a, int items, uint64_t* tile_status, uint32_t* tile_counter,
+size_t winding_tile_words(int64_t n, int items = 8);
+void launch_winding_emit(const WindArgs& a, int items, uint64_t* tile_status, uint64_t* tile_sums, uint32_t* counters,
                          uint32_t* status, cudaStream_t st);
 
 // ---- resolve.cu
@@ -261,7 +284,7 @@ struct ResolveArgs {
     const unsigned long long* row_px; // [rows] summed record widths from the emit, or NULL (every row searched)
     uint32_t cut_segs;
     const uint8_t* cta_narrow;        // [CTAs] 1 for a CTA of several rows
-    int any_narrow;                   // some CTA is (then pixel mode runs a second kernel for them)
+    int any_narrow, any_wide;         // some CTA is, some is not (pixel mode has a kernel for each)
     const DevPaint* paints;           // gradient paints of the scene (single-scene contexts), or NULL
     uint32_t n_paints;
 };

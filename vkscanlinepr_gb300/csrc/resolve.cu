@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_resolve_ref(const ResolveArgs a)
 
 template <int WARPS, bool GRAD> static void launch_resolve_t(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st) {
     if (a.pixel_mode) {
-        k_resolve_pixel<WARPS, GRAD><<<n_ctas, 32 * WARPS, 0, st>>>(a);
+        if (a.any_wide) k_resolve_pixel<WARPS, GRAD><<<n_ctas, 32 * WARPS, 0, st>>>(a);
         if (a.any_narrow) k_resolve_pixel_rows<WARPS, GRAD><<<n_ctas, 32 * WARPS, 0, st>>>(a);
     } else {
         k_resolve_ref<WARPS, GRAD><<<n_ctas, 32 * WARPS, 0, st>>>(a);
@@ -666,8 +666,7 @@ template <int WARPS, bool GRAD> static void launch_resolve_t(const ResolveArgs& 
 
 void launch_resolve(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st) {
     if (n_ctas == 0) return;
-    count_launches(1);
-    if (a.pixel_mode && a.any_narrow) count_launches(1);
+    count_launches(a.pixel_mode ? (a.any_wide ? 1 : 0) + (a.any_narrow ? 1 : 0) : 1);
     const bool grad = a.paints && a.n_paints;
     if (a.warps == 8) {
         if (grad) launch_resolve_t<8, true>(a, n_ctas, st);

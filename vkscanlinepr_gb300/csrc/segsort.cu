@@ -16,8 +16,8 @@
 // the device, one per CTA, so no CTA searches for its work.
 #include <algorithm>
 
-#include "common.cuh"
 #include "kernels.h"
+#include "scan.cuh"
 
 namespace sr {
 
@@ -37,76 +37,54 @@ constexpr uint32_t kChunkBit = 1u << 31;   // descriptor .z: a chunk of a large 
 // sorted keys, so a warp sees few distinct digits), or one ballot per bit.
 constexpr bool kMatchAny = true;
 
-// Front tables (depend on the curves only), in the segment scratch buffer.
-struct SegTables {
-    int32_t* flag;         // [C + 2] curve starts a path; then exclusive scan -> segment index
-    uint32_t* seg_start;   // [C + 2] first record of each segment, then N
-    uint64_t* scan_status;
-    uint32_t* ctl;         // [0] scan counter, [1] largest segment of more than kGroup records
-};
-
-// Back tables (depend on the record capacity), in the tile buffer.
+// The tables of a frame: descriptors, in the table buffer, and what starts
+// zeroed, in the zeroed buffer.
 struct TileTables {
-    int32_t* ntiles;       // [C + 2] tiles a segment opens; then exclusive scan -> first tile
     uint4* desc;           // [max_tiles] {start, segment size, k | rounds << 16 | chunk bit, -}
-    uint32_t* tile_end;    // [max_tiles] end of a group tile (atomic max over its segments)
     uint32_t* chunks;      // [max_tiles] the chunk tiles (of large segments), in no order
     uint32_t* fallback;    // [max_tiles] tiles left to the 64-bit tile sort, in no order
-    uint64_t* scan_status;
-    // [0] scan counter, [1] chunk tiles, [2] next tile of the tile sort,
-    // [3] tiles left to the 64-bit sort, [4] its next, [5 + l] next work
-    // item of merge round l
+    uint32_t* tile_end;    // [max_tiles] end of a group tile (atomic max over its segments); zeroed
+    uint64_t* scan_status; // look-back words of the tile scan; zeroed
+    // zeroed: [0] scan counter, [1] chunk tiles, [2] next tile of the tile
+    // sort, [3] next of the 64-bit sort, [4] tiles, [5 + l] next work item of
+    // merge round l
     uint32_t* ctl;
+    uint32_t* wide_count;  // tiles left to the 64-bit sort
 };
-constexpr int kCtlChunks = 1, kCtlSortNext = 2, kCtlFallback = 3, kCtlFallbackNext = 4, kCtlMergeNext = 5;
+constexpr int kCtlChunks = 1, kCtlSortNext = 2, kCtlFallbackNext = 3, kCtlTiles = 4, kCtlMergeNext = 5;
+constexpr int kSegThreads = 256;   // segments a CTA of the tile scan takes
 
 size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
-size_t scan_area(uint32_t C) { return round256(scan_status_words((int64_t)C + 1) * 8); }
-
-SegTables carve_front(void* base, uint32_t C) {
-    SegTables t;
-    char* b = static_cast<char*>(base);
-    const size_t ws = round256(((size_t)C + 2) * 4);
-    t.flag = reinterpret_cast<int32_t*>(b);
-    b += ws;
-    t.seg_start = reinterpret_cast<uint32_t*>(b);
-    b += ws;
-    t.scan_status = reinterpret_cast<uint64_t*>(b);
-    b += scan_area(C);
-    t.ctl = reinterpret_cast<uint32_t*>(b);
-    return t;
-}
+size_t scan_area(uint32_t P) { return round256(8 * ((size_t)P / kSegThreads + 2)); }
 
 // Tiles of a frame: at most one group tile per kGroup records (a head starts
-// its own group), plus the chunks of large segments (at most one partial
-// chunk per large segment, of which there are fewer than cap / kGroup), and
-// never more than the segments plus cap / kTile.
-size_t max_tiles(uint32_t C, int64_t cap) {
+// its own group; paths without records may make an empty one), plus the
+// chunks of large segments (at most one partial chunk per large segment, of
+// which there are fewer than cap / kGroup), and never more than the segments
+// plus cap / kTile.
+size_t max_tiles(uint32_t P, int64_t cap) {
     const size_t per_tile = (size_t)((cap + kTile - 1) / kTile);
-    return std::min<size_t>((size_t)C + 2 + per_tile, 5 * per_tile + 2);
+    return std::min<size_t>((size_t)P + 2 + per_tile, 5 * per_tile + 2);
 }
 
-TileTables carve_back(void* base, uint32_t C, int64_t cap) {
+TileTables carve(const SegArgs& a) {
     TileTables t;
-    char* b = static_cast<char*>(base);
-    const size_t mt = max_tiles(C, cap);
-    t.ntiles = reinterpret_cast<int32_t*>(b);
-    b += round256(((size_t)C + 2) * 4);
+    const size_t mt = max_tiles(a.n_paths, a.cap);
+    char* b = static_cast<char*>(a.tables);
     t.desc = reinterpret_cast<uint4*>(b);
     b += round256(mt * 16);
-    t.tile_end = reinterpret_cast<uint32_t*>(b);
-    b += round256(mt * 4);
     t.chunks = reinterpret_cast<uint32_t*>(b);
     b += round256(mt * 4);
     t.fallback = reinterpret_cast<uint32_t*>(b);
-    b += round256(mt * 4);
-    t.scan_status = reinterpret_cast<uint64_t*>(b);
-    b += scan_area(C);
-    t.ctl = reinterpret_cast<uint32_t*>(b);
+    char* z = static_cast<char*>(a.zeroed);
+    t.ctl = reinterpret_cast<uint32_t*>(z);
+    z += 256;
+    t.scan_status = reinterpret_cast<uint64_t*>(z);
+    z += scan_area(a.n_paths);
+    t.tile_end = reinterpret_cast<uint32_t*>(z);
+    t.wide_count = a.wide_count;
     return t;
 }
-
-SR_DEV uint32_t n_segments(const SegTables& t, uint32_t C) { return (uint32_t)t.flag[C]; }
 
 // Merge rounds a large segment of `chunks` sorted chunks needs.
 SR_DEV uint32_t rounds_of(uint32_t chunks) {
@@ -116,73 +94,73 @@ SR_DEV uint32_t rounds_of(uint32_t chunks) {
 }
 }  // namespace
 
-// ---------------------------------------------------------- segment tables
-__global__ void k_seg_flags(const uint32_t* __restrict__ curve_path, uint32_t C, int32_t* __restrict__ flag) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < C) flag[c] = (c == 0 || curve_path[c] != curve_path[c - 1]) ? 1 : 0;
-    else if (c == C) flag[c] = 0;
-}
-
-// seg_start[s] = record offset of the first curve of segment s; seg_start[S] = N.
-__global__ void k_seg_starts(const int32_t* __restrict__ offs, uint32_t C, SegTables t) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    const int32_t s = t.flag[c];
-    if (t.flag[c + 1] != s) t.seg_start[s] = (uint32_t)offs[c];   // curve c starts path segment s
-    if (c == C - 1) t.seg_start[n_segments(t, C)] = (uint32_t)offs[C];
+// -------------------------------------------------------------- tile tables
+// Records of path p: [a, e).
+SR_DEV void seg_span(const SegArgs& s, uint32_t p, uint32_t& a, uint32_t& e) {
+    a = (uint32_t)s.offs[s.path_begin[p]];
+    e = (uint32_t)s.offs[s.path_begin[p + 1]];
 }
 
 // The largest segment of more than kGroup records.  max_size > 0: a segment
 // larger than that is an overflow (the merge rounds of a pre-sized frame
 // cannot take it; the frame is redone with exact sizing, which chooses the
 // rounds, or the radix sort, from the largest segment).
-__global__ void k_seg_largest(uint32_t C, uint32_t max_size, SegTables t, uint32_t* status) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_segments(t, C)) return;
-    const uint32_t size = t.seg_start[s + 1] - t.seg_start[s];
-    if (size > (uint32_t)kGroup) atomicMax(&t.ctl[1], size);
-    if (max_size && size > max_size) set_error(status, ERR_CAPACITY);
+SR_DEV void seg_note_size(const SegArgs& s, uint32_t size, uint32_t* status) {
+    if (size > (uint32_t)kGroup) atomicMax(s.largest, size);
+    if (s.max_size && size > s.max_size) set_error(status, ERR_CAPACITY);
 }
 
-// Tiles each segment opens: a large one its chunks, a small one that starts
-// a group (first small segment starting in its group) one tile.
-__global__ void k_seg_ntiles(uint32_t C, SegTables t, TileTables u) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t S = n_segments(t, C);
+__global__ void k_seg_largest(const SegArgs s) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= s.n_paths) return;
+    uint32_t a, e;
+    seg_span(s, p, a, e);
+    seg_note_size(s, e - a, nullptr);
+}
+
+// One pass over the segments (a thread each) for all tables: the tiles each
+// segment opens (a large one its chunks, a small one that starts a group,
+// i.e. the first small segment starting in its group, one tile), their
+// exclusive scan, and the descriptors.  A group tile is opened by its head
+// and stretched to the end of each small segment of the group.  Tiles past mt
+// exist only in a frame whose records overflowed the capacity (it is redone);
+// they are not written.
+// (Segment starts, sizes, tiles, scan and descriptors used to be seven
+// launches, 3.6-8 us each.)
+__global__ void __launch_bounds__(kSegThreads) k_seg_tiles(const SegArgs s, uint32_t mt, TileTables u,
+                                                           uint32_t* status, uint32_t spin_limit) {
+    __shared__ uint32_t s_tile;
+    __shared__ int32_t s_warp[kSegThreads / 32 + 1];
+    if (threadIdx.x == 0) s_tile = atomicAdd(&u.ctl[0], 1u);
+    __syncthreads();
+    const uint32_t p = s_tile * kSegThreads + threadIdx.x;
+    const bool live = p < s.n_paths;
+    uint32_t a = 0, e = 0;
     int32_t n = 0;
-    if (s < S) {
-        const uint32_t a = t.seg_start[s], size = t.seg_start[s + 1] - a;
-        if (size > (uint32_t)kGroup) {
-            n = (int32_t)((size + kTile - 1) / kTile);
+    if (live) {
+        seg_span(s, p, a, e);
+        seg_note_size(s, e - a, status);
+        if (e - a > (uint32_t)kGroup) {
+            n = (int32_t)((e - a + kTile - 1) / kTile);
         } else {
-            bool head = s == 0;
+            bool head = p == 0;
             if (!head) {
-                const uint32_t pa = t.seg_start[s - 1];
+                const uint32_t pa = (uint32_t)s.offs[s.path_begin[p - 1]];
                 head = a - pa > (uint32_t)kGroup || a / (uint32_t)kGroup != pa / (uint32_t)kGroup;
             }
             n = head ? 1 : 0;
         }
     }
-    if (s <= C) u.ntiles[s] = n;
-}
-
-// Descriptors: a group tile is opened by its head and stretched to the end
-// of each small segment of the group; a large segment writes its chunks.
-// Tiles past mt exist only in a frame whose records overflowed the capacity
-// (it is redone); they are not written.
-__global__ void k_seg_desc(uint32_t C, uint32_t mt, SegTables t, TileTables u) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t S = n_segments(t, C);
-    if (s >= S) return;
-    const uint32_t a = t.seg_start[s], size = t.seg_start[s + 1] - a;
-    const int32_t first = u.ntiles[s];
-    const int32_t n = u.ntiles[s + 1] - first;
-    if (size > (uint32_t)kGroup) {
+    int32_t total;
+    const int32_t first = scan_thread_values<kSegThreads>(n, s_tile, u.scan_status, status, spin_limit, s_warp, &total);
+    if (!live) return;
+    if (p == s.n_paths - 1) u.ctl[kCtlTiles] = (uint32_t)total;
+    if (e - a > (uint32_t)kGroup) {
         const uint32_t rounds = rounds_of((uint32_t)n);
         const int32_t m = (int32_t)min((uint32_t)n, mt - min(mt, (uint32_t)first));   // chunks that fit the table
         const uint32_t at = m > 0 ? atomicAdd(&u.ctl[kCtlChunks], (uint32_t)m) : 0u;
         for (int32_t k = 0; k < m; ++k) {
-            u.desc[first + k] = make_uint4(a, size, (uint32_t)k | (rounds << 16) | kChunkBit, 0u);
+            u.desc[first + k] = make_uint4(a, e - a, (uint32_t)k | (rounds << 16) | kChunkBit, 0u);
             u.chunks[at + k] = (uint32_t)(first + k);
         }
         return;
@@ -191,7 +169,7 @@ __global__ void k_seg_desc(uint32_t C, uint32_t mt, SegTables t, TileTables u) {
     const int32_t tile = n == 1 ? first : first - 1;
     if (tile < 0 || (uint32_t)tile >= mt) return;
     if (n == 1) u.desc[tile] = make_uint4(a, 0u, 0u, 0u);
-    atomicMax(&u.tile_end[tile], a + size);
+    atomicMax(&u.tile_end[tile], e);
 }
 
 // ----------------------------------------------------------- local sort ---
@@ -595,7 +573,8 @@ struct Sort32Smem {
 // wait gave up.
 SR_DEV bool sort_tile32(Sort32Smem& S, uint32_t tile, uint32_t& phase, const uint64_t* __restrict__ keys_in,
                         uint64_t* __restrict__ keys_out, uint64_t* __restrict__ keys_alt, const KeyFields& kf,
-                        uint32_t n_cap, const TileTables& u, uint32_t* status, uint32_t spin_limit) {
+                        uint32_t n_cap, const TileTables& u, bool wide, uint32_t* status,
+                        uint32_t spin_limit) {
     const uint32_t tid = threadIdx.x;
     uint32_t a, len;
     bool to_alt;
@@ -618,7 +597,10 @@ SR_DEV bool sort_tile32(Sort32Smem& S, uint32_t tile, uint32_t& phase, const uin
     const uint32_t payb = pay_max > 0xFFFFFFFFull ? 33u : bits_of((uint32_t)pay_max);
     (void)kmask;
     if (bits + payb > 32u) {
-        if (tid == 0) u.fallback[atomicAdd(&u.ctl[kCtlFallback], 1u)] = tile;
+        if (tid == 0) {
+            u.fallback[atomicAdd(u.wide_count, 1u)] = tile;
+            if (!wide) set_error(status, ERR_CAPACITY);   // k_local_sort is not launched: the frame is redone
+        }
         return true;
     }
     if (bits == 0) {   // one key: already in order
@@ -665,13 +647,14 @@ SR_DEV bool sort_tile32(Sort32Smem& S, uint32_t tile, uint32_t& phase, const uin
 
 __global__ void __launch_bounds__(kThreads, 4) k_tile_sort32(const uint64_t* __restrict__ keys_in,
                                                              uint64_t* __restrict__ keys_out,
-                                                             uint64_t* __restrict__ keys_alt, uint32_t C,
+                                                             uint64_t* __restrict__ keys_alt,
                                                              KeyFields kf, uint32_t n_cap, uint32_t mt,
-                                                             TileTables u, uint32_t* status, uint32_t spin_limit) {
+                                                             TileTables u, bool wide, uint32_t* status,
+                                                             uint32_t spin_limit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Sort32Smem& S = *reinterpret_cast<Sort32Smem*>(smem_raw);
     // tiles past the table exist only in a frame whose records overflowed (redone)
-    const uint32_t n_tiles = min((uint32_t)u.ntiles[C], mt);
+    const uint32_t n_tiles = min(u.ctl[kCtlTiles], mt);
     if (threadIdx.x == 0) mbar_init(&S.ps.bar, 1);
     uint32_t phase = 0;
     for (;;) {
@@ -680,7 +663,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_tile_sort32(const uint64_t* __r
         const uint32_t tile = S.ps.next;
         __syncthreads();
         if (tile >= n_tiles) break;
-        if (!sort_tile32(S, tile, phase, keys_in, keys_out, keys_alt, kf, n_cap, u, status, spin_limit)) return;
+        if (!sort_tile32(S, tile, phase, keys_in, keys_out, keys_alt, kf, n_cap, u, wide, status, spin_limit)) return;
     }
 }
 
@@ -744,7 +727,7 @@ __global__ void __launch_bounds__(kThreads) k_local_sort(uint64_t* keys_in, uint
                                                          uint64_t* __restrict__ keys_alt, KeyFields kf, uint32_t n_cap,
                                                          TileTables u) {
     __shared__ PassSmem S;
-    const uint32_t n_tiles = u.ctl[kCtlFallback];
+    const uint32_t n_tiles = *u.wide_count;
     if (n_tiles == 0) return;   // the usual case: nothing handed over
     for (;;) {
         if (threadIdx.x == 0) S.next = atomicAdd(&u.ctl[kCtlFallbackNext], 1u);
@@ -876,56 +859,36 @@ __global__ void __launch_bounds__(kThreads) k_merge_level(uint64_t* __restrict__
 }
 
 // ------------------------------------------------------------- launches --
-size_t segsort_scratch_bytes(uint32_t C) { return 2 * round256(((size_t)C + 2) * 4) + scan_area(C) + 256; }
-
-size_t segsort_tile_bytes(uint32_t C, int64_t cap) {
-    const size_t mt = max_tiles(C, cap);
-    return round256(((size_t)C + 2) * 4) + round256(mt * 16) + 3 * round256(mt * 4) + scan_area(C) + 256;
+size_t segsort_table_bytes(uint32_t P, int64_t cap) {
+    const size_t mt = max_tiles(P, cap);
+    return round256(mt * 16) + 2 * round256(mt * 4);
 }
+size_t segsort_zeroed_bytes(uint32_t P, int64_t cap) { return 256 + scan_area(P) + round256(max_tiles(P, cap) * 4); }
 
 int segsort_tile() { return kTile; }
 
-void launch_segsort_tables(const uint32_t* curve_path, const int32_t* offs, uint32_t C, uint32_t max_size,
-                           void* scratch, uint32_t* status, cudaStream_t st) {
-    if (C == 0) return;
-    SegTables t = carve_front(scratch, C);
-    cudaMemsetAsync(t.scan_status, 0, scan_area(C), st);
-    cudaMemsetAsync(t.ctl, 0, 256, st);
-    const unsigned g = (C + 1 + 255) / 256;
-    count_launches(3);
-    k_seg_flags<<<g, 256, 0, st>>>(curve_path, C, t.flag);
-    launch_exclusive_scan_i32(t.flag, t.flag, C + 1, t.scan_status, t.ctl + 0, status, st);
-    k_seg_starts<<<g, 256, 0, st>>>(offs, C, t);
-    k_seg_largest<<<g, 256, 0, st>>>(C, max_size, t, status);
-}
-
-cudaError_t segsort_tile_counts(const void* tiles, uint32_t C, int64_t cap, uint32_t out[2]) {
-    TileTables u = carve_back(const_cast<void*>(tiles), C, cap);
-    cudaError_t e = cudaMemcpy(&out[0], u.ntiles + C, 4, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(&out[1], u.ctl + kCtlFallback, 4, cudaMemcpyDeviceToHost);
-    out[0] = std::min<uint32_t>(out[0], (uint32_t)max_tiles(C, cap));
+cudaError_t segsort_tile_counts(const SegArgs& a, uint32_t out[2]) {
+    TileTables u = carve(a);
+    cudaError_t e = cudaMemcpy(&out[0], u.ctl + kCtlTiles, 4, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(&out[1], a.wide_count, 4, cudaMemcpyDeviceToHost);
+    out[0] = std::min<uint32_t>(out[0], (uint32_t)max_tiles(a.n_paths, a.cap));
     return e;
 }
 
-const uint32_t* segsort_largest(const void* scratch, uint32_t C) {
-    return carve_front(const_cast<void*>(scratch), C).ctl + 1;
+void launch_segsort_largest(const SegArgs& a, cudaStream_t st) {
+    if (a.n_paths == 0) return;
+    count_launches(1);
+    k_seg_largest<<<(a.n_paths + 255) / 256, 256, 0, st>>>(a);
 }
 
-void launch_segsort(uint64_t* keys_in, uint64_t* keys_out, uint64_t* keys_alt, int64_t cap, uint32_t C,
-                    const KeyLayout& L, int levels, void* scratch, void* tiles, int sm_count, uint32_t* status,
-                    cudaStream_t st) {
-    if (cap <= 0 || C == 0) return;
-    SegTables t = carve_front(scratch, C);
-    TileTables u = carve_back(tiles, C, cap);
-    const size_t mt = max_tiles(C, cap);
-    cudaMemsetAsync(u.tile_end, 0, mt * 4, st);
-    cudaMemsetAsync(u.scan_status, 0, scan_area(C), st);
-    cudaMemsetAsync(u.ctl, 0, 256, st);
-    const unsigned g = (C + 1 + 255) / 256;
-    count_launches(2);
-    k_seg_ntiles<<<g, 256, 0, st>>>(C, t, u);
-    launch_exclusive_scan_i32(u.ntiles, u.ntiles, C + 1, u.scan_status, u.ctl + 0, status, st);
-    k_seg_desc<<<g, 256, 0, st>>>(C, (uint32_t)mt, t, u);
+void launch_segsort(const SegArgs& sa, uint64_t* keys_in, uint64_t* keys_out, uint64_t* keys_alt, const KeyLayout& L,
+                    int levels, int sm_count, uint32_t* status, cudaStream_t st) {
+    if (sa.cap <= 0 || sa.n_paths == 0) return;
+    TileTables u = carve(sa);
+    const size_t mt = max_tiles(sa.n_paths, sa.cap);
+    count_launches(1);
+    k_seg_tiles<<<(sa.n_paths + kSegThreads - 1) / kSegThreads, kSegThreads, 0, st>>>(sa, (uint32_t)mt, u, status,
+                                                                                      spin_limit());
     const uint32_t key_bits = L.pbits + L.rbits + L.xbits;
     const KeyFields kf{L.xbits, L.rbits, L.pbits, (uint32_t)(L.Hy - 1)};
     // resident CTAs per SM of the two persistent kernels (same on every
@@ -947,11 +910,11 @@ void launch_segsort(uint64_t* keys_in, uint64_t* keys_out, uint64_t* keys_alt, i
     const unsigned g_sort = (unsigned)std::min<size_t>(mt, sms);
     const unsigned g_merge =
         (unsigned)std::min<size_t>(kMergeParts * mt, sms * (size_t)std::max(occ_merge.load(), 1));
-    count_launches(2 + (uint32_t)levels);
-    const uint32_t n_cap = (uint32_t)cap;
-    k_tile_sort32<<<g_sort32, kThreads, sizeof(Sort32Smem), st>>>(keys_in, keys_out, keys_alt, C, kf, n_cap,
-                                                                  (uint32_t)mt, u, status, spin_limit());
-    k_local_sort<<<g_sort, kThreads, 0, st>>>(keys_in, keys_out, keys_alt, kf, n_cap, u);
+    count_launches(1 + (sa.wide ? 1 : 0) + (uint32_t)levels);
+    const uint32_t n_cap = (uint32_t)sa.cap;
+    k_tile_sort32<<<g_sort32, kThreads, sizeof(Sort32Smem), st>>>(keys_in, keys_out, keys_alt, kf, n_cap,
+                                                                  (uint32_t)mt, u, sa.wide, status, spin_limit());
+    if (sa.wide) k_local_sort<<<g_sort, kThreads, 0, st>>>(keys_in, keys_out, keys_alt, kf, n_cap, u);
     for (int lv = 0; lv < levels; ++lv)
         k_merge_level<<<g_merge, kThreads, sizeof(MergeSmem), st>>>(keys_out, keys_alt, (uint32_t)lv, key_bits, n_cap,
                                                                     u);

@@ -14,8 +14,8 @@
 // scattered into shared memory in digit order, then written out in runs, so
 // global stores stay mostly contiguous.  An upfront kernel histograms every
 // pass's digits in one read of the keys.
-#include "common.cuh"
 #include "kernels.h"
+#include "scan.cuh"
 
 namespace sr {
 
@@ -58,7 +58,7 @@ __host__ __device__ inline uint32_t digit_mask(uint32_t key_bits, uint32_t shift
 }
 
 struct Scratch {
-    uint32_t* hist;       // [passes][256] digit counts, then exclusive offsets
+    uint32_t* hist;       // [passes][256] digit counts
     uint32_t* lookback;   // [passes][tiles + 1][256]
     uint32_t* counters;   // [passes] tile counters
 };
@@ -124,15 +124,25 @@ __global__ void __launch_bounds__(kThreads) k_hist(const K* __restrict__ keys, i
     }
 }
 
-// Digit counts of every pass for the keys 0..n_bins-1 with the given counts.
-__global__ void __launch_bounds__(kThreads) k_hist_from_counts(const uint32_t* __restrict__ counts, uint32_t n_bins,
-                                                               uint32_t passes, uint32_t key_bits,
-                                                               uint32_t* __restrict__ hist) {
+// A tile of rows: their first positions (exclusive scan of the counts), and
+// the tile's part of every pass's digit counts (a row is the key of each of
+// its records).
+constexpr int kRowTile = kThreads * 4;
+__global__ void __launch_bounds__(kThreads) k_row_starts(const uint32_t* __restrict__ counts, uint32_t rows,
+                                                         int32_t* __restrict__ row_start, uint32_t passes,
+                                                         uint32_t key_bits, uint32_t* __restrict__ hist,
+                                                         uint64_t* tstat, uint32_t* counter, uint32_t* status,
+                                                         uint32_t spin_limit) {
     __shared__ uint32_t sh[kMaxPasses][kRadix];
-    for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kThreads) (&sh[0][0])[i] = 0;
+    __shared__ uint32_t s_tile;
+    __shared__ int32_t s_warp[kWarps + 1];
+    if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
+    for (uint32_t i = threadIdx.x; i < passes * kRadix; i += kThreads) (&sh[0][0])[i] = 0;
     __syncthreads();
-    for (uint32_t b = blockIdx.x * kThreads + threadIdx.x; b < n_bins; b += gridDim.x * kThreads) {
-        const uint32_t c = counts[b];
+    const uint32_t tile = s_tile;
+    for (uint32_t q = 0; q < 4; ++q) {
+        const uint32_t b = tile * kRowTile + q * kThreads + threadIdx.x;
+        const uint32_t c = b < rows ? counts[b] : 0u;
         if (!c) continue;
         for (uint32_t p = 0; p < passes; ++p)
             atomicAdd(&sh[p][digit_of(b, p * kRadixBits, digit_mask(key_bits, p * kRadixBits))], c);
@@ -142,41 +152,16 @@ __global__ void __launch_bounds__(kThreads) k_hist_from_counts(const uint32_t* _
         const uint32_t v = (&sh[0][0])[i];
         if (v) atomicAdd(&hist[i], v);
     }
-}
-
-// In-place exclusive scan of each pass's 256 digit counts (one CTA per pass).
-__global__ void __launch_bounds__(kRadix) k_hist_scan(uint32_t* hist) {
-    __shared__ uint32_t sw[kRadix / 32];
-    uint32_t* h = hist + blockIdx.x * kRadix;
-    uint32_t v = h[threadIdx.x];
-    uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        uint32_t t = __shfl_up_sync(0xFFFFFFFFu, x, d);
-        if ((int)lane >= d) x += t;
-    }
-    if (lane == 31) sw[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kRadix / 32 ? sw[lane] : 0;
-        uint32_t wi = w;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            uint32_t t = __shfl_up_sync(0xFFFFFFFFu, wi, d);
-            if ((int)lane >= d) wi += t;
-        }
-        if (lane < kRadix / 32) sw[lane] = wi - w;
-    }
-    __syncthreads();
-    h[threadIdx.x] = sw[warp] + x - v;
+    int32_t total;
+    scan_tile_i32<1, kThreads>(reinterpret_cast<const int32_t*>(counts), row_start, rows, tile, tstat, status,
+                               spin_limit, s_warp, &total);
 }
 
 template <typename K, bool kVals, int ITEMS> struct OnesweepSmem {
     uint32_t warp_hist[kWarps][kRadix];
     uint32_t digit_start[kRadix];   // tile-local exclusive start of each digit
     uint32_t digit_global[kRadix];  // global base minus digit_start
-    uint32_t scan_tmp[kWarps];
+    uint2 scan_tmp[kWarps];
     uint32_t tile;
     K keys[kThreads * ITEMS];
     uint32_t vals[kVals ? kThreads * ITEMS : 1];
@@ -194,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, onesweep_min_blocks(kVals, ITEMS)) k
                                                        K* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                                                        int64_t n_max, const uint32_t* __restrict__ n_dev,
                                                        uint32_t shift, uint32_t dmask,
-                                                       const uint32_t* __restrict__ global_off,
+                                                       const uint32_t* __restrict__ digit_count,
                                                        uint32_t* __restrict__ lookback, uint32_t* counter,
                                                        uint32_t* status, uint32_t spin_limit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -251,27 +236,25 @@ __global__ void __launch_bounds__(kThreads, onesweep_min_blocks(kVals, ITEMS)) k
     uint32_t* lb_mine = lookback + (size_t)tile * kRadix + d;
     st_relaxed_u32(lb_mine, (tile == 0 ? kFlagP : kFlagA) | cnt);
 
-    // tile-local digit starts: block exclusive scan over the 256 counts
-    uint32_t x = cnt;
+    // tile-local digit starts and the digits' global starts: block exclusive
+    // scans over the tile's 256 counts and over the whole input's
+    const uint32_t all = digit_count[d];
+    uint32_t x = cnt, y = all;
 #pragma unroll
     for (int dd = 1; dd < 32; dd <<= 1) {
-        uint32_t t = __shfl_up_sync(0xFFFFFFFFu, x, dd);
-        if ((int)lane >= dd) x += t;
-    }
-    if (lane == 31) S.scan_tmp[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kWarps ? S.scan_tmp[lane] : 0;
-        uint32_t wi = w;
-#pragma unroll
-        for (int dd = 1; dd < 32; dd <<= 1) {
-            uint32_t t = __shfl_up_sync(0xFFFFFFFFu, wi, dd);
-            if ((int)lane >= dd) wi += t;
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, x, dd), u = __shfl_up_sync(0xFFFFFFFFu, y, dd);
+        if ((int)lane >= dd) {
+            x += t;
+            y += u;
         }
-        if (lane < kWarps) S.scan_tmp[lane] = wi - w;
     }
+    if (lane == 31) S.scan_tmp[warp] = make_uint2(x, y);
     __syncthreads();
-    const uint32_t dstart = S.scan_tmp[warp] + x - cnt;
+    uint32_t dstart = x - cnt, gstart = y - all;
+    for (uint32_t w = 0; w < warp; ++w) {
+        dstart += S.scan_tmp[w].x;
+        gstart += S.scan_tmp[w].y;
+    }
     S.digit_start[d] = dstart;
 
     // ---- look-back for this digit: 8 preceding tiles' words per step, all
@@ -310,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, onesweep_min_blocks(kVals, ITEMS)) k
         }
         st_relaxed_u32(lb_mine, kFlagP | (excl + cnt));
     }
-    S.digit_global[d] = global_off[d] + excl - dstart;
+    S.digit_global[d] = gstart + excl - dstart;
     __syncthreads();
 
     // ---- scatter into shared memory in digit order
@@ -347,21 +330,13 @@ static void sort_impl(const SortPlan& p, const K* keys_in, const uint32_t* vals_
                       K* keys_alt, uint32_t* vals_alt, void* scratch, uint32_t* status, cudaStream_t st) {
     if (p.n <= 0) return;
     Scratch s = carve(p, scratch);
-    size_t lb_words = (size_t)p.passes * ((size_t)p.tiles + 1) * kRadix;
-    if (p.hist_given) {
-        cudaMemsetAsync(s.counters, 0, sizeof(uint32_t) * 64, st);
-    } else {
-        cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * (kMaxPasses * kRadix + 64), st);
-    }
-    cudaMemsetAsync(s.lookback, 0, sizeof(uint32_t) * lb_words, st);
+    if (!p.cleared) cudaMemsetAsync(scratch, 0, sort_scratch_bytes(p), st);
     if (!p.hist_given) {
         int hb = (int)((p.n + kThreads - 1) / kThreads);
         if (hb > kHistBlocks) hb = kHistBlocks;
         count_launches(1);
         k_hist<K><<<hb, kThreads, 0, st>>>(keys_in, p.n, p.n_dev, p.passes, p.key_bits, s.hist);
     }
-    count_launches(1);
-    k_hist_scan<<<p.passes, kRadix, 0, st>>>(s.hist);
     const size_t smem = sizeof(OnesweepSmem<K, kVals, ITEMS>);
     static std::atomic<uint32_t> attr_set{0};
     once_per_device(attr_set, [&] {
@@ -410,15 +385,20 @@ void launch_sort_u64(const SortPlan& p, const uint64_t* keys_in, const uint32_t*
     sort_dispatch<uint64_t>(p, keys_in, vals_in, keys_out, vals_out, keys_alt, vals_alt, scratch, status, st);
 }
 
-void sort_hist_from_counts(SortPlan& p, const uint32_t* counts, uint32_t n_bins, void* scratch, cudaStream_t st) {
-    Scratch s = carve(p, scratch);
-    cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * kMaxPasses * kRadix, st);
-    int blocks = (int)((n_bins + kThreads - 1) / kThreads);
-    if (blocks > kHistBlocks) blocks = kHistBlocks;
-    if (blocks < 1) blocks = 1;
-    count_launches(1);
-    k_hist_from_counts<<<blocks, kThreads, 0, st>>>(counts, n_bins, p.passes, p.key_bits, s.hist);
+size_t row_scan_words(uint32_t rows) { return (size_t)(rows + kRowTile - 1) / kRowTile + 1; }
+
+void launch_row_starts(SortPlan& p, const uint32_t* row_count, uint32_t rows, int32_t* row_start, void* scratch,
+                       uint64_t* tile_status, uint32_t* tile_counter, uint32_t* status, cudaStream_t st) {
+    p.cleared = 1;
     p.hist_given = 1;
+    if (rows == 0) {
+        cudaMemsetAsync(row_start, 0, sizeof(int32_t), st);
+        return;
+    }
+    count_launches(1);
+    k_row_starts<<<(rows + kRowTile - 1) / kRowTile, kThreads, 0, st>>>(row_count, rows, row_start, p.passes, p.key_bits,
+                                                                        carve(p, scratch).hist, tile_status,
+                                                                        tile_counter, status, spin_limit());
 }
 
 void launch_sort_u32(const SortPlan& p, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,

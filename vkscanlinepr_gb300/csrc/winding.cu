@@ -6,11 +6,11 @@
 //   naive_scan.comp over 2N flags (scanline_rasterizer.cpp:545-580)
 //   gen_merged_fragment_and_span.comp:33-103           draw-list emit
 //
-// Three launches over tiles of 2048 consecutive sorted records (ITEMS 8; 1024
+// Two launches over tiles of 2048 consecutive sorted records (ITEMS 8; 1024
 // with ITEMS 4):
 //   k_winding_reduce      each tile's (scene head seen, sum since) pair of
 //                         winding changes, a fully parallel read of the keys;
-//   k_winding_scan_tiles  one CTA scans the tile pairs into each tile's
+//                         its last CTA scans the tile pairs into each tile's
 //                         incoming winding prefix;
 //   k_winding_emit        the records' winding scan, fragment and span flags,
 //                         output slots (one decoupled look-back over packed
@@ -24,8 +24,8 @@
 // zero carries into the paths after it.  In a batch of scenes chain A is a
 // scan segmented at scene boundaries, so each scene sees exactly the global
 // scan it would see alone (with one scene the two are the same).
-#include "common.cuh"
 #include "kernels.h"
+#include "scan.cuh"
 
 namespace sr {
 
@@ -56,42 +56,33 @@ template <typename T> SR_DEV T warp_incl(T v) {
     return v;
 }
 
-// Look-back over 64-bit tile words; `add` combines values (wrapping).
-template <bool kSigned32>
+// Look-back over the tiles' packed counts: a word carries flag and value
+// together, so relaxed accesses suffice.
 SR_DEV uint64_t lookback(uint64_t* tstat, uint32_t tile, uint32_t* status, uint32_t spin_limit) {
-    uint32_t lane = lane_id();
+    const uint32_t lane = lane_id();
     uint64_t excl = 0;
     int64_t look = (int64_t)tile - 1;
     uint32_t spins = 0;
     while (look >= 0) {
-        int64_t j = look - (int64_t)lane;
-        uint64_t s = j >= 0 ? ld_acquire_u64(&tstat[j]) : kFlagP;
-        uint32_t flag = (uint32_t)(s >> 62);
-        uint32_t ready = __ballot_sync(0xFFFFFFFFu, flag != 0);
-        // a tile that holds a segment head ends the look-back like an
-        // inclusive prefix does: its value already starts at that head
-        uint32_t pm = __ballot_sync(0xFFFFFFFFu, flag == 2 || (kSigned32 && flag == 1 && (s & kHeadBit)));
-        int firstp = pm ? (__ffs(pm) - 1) : 31;
-        uint32_t need = firstp == 31 ? 0xFFFFFFFFu : ((2u << firstp) - 1u);
+        const int64_t j = look - (int64_t)lane;
+        const uint64_t s = j >= 0 ? ld_relaxed_u64(&tstat[j]) : kFlagP;
+        const uint32_t flag = (uint32_t)(s >> 62);
+        const uint32_t ready = __ballot_sync(0xFFFFFFFFu, flag != 0);
+        const uint32_t pm = __ballot_sync(0xFFFFFFFFu, flag == 2);
+        const int firstp = pm ? (__ffs(pm) - 1) : 31;
+        const uint32_t need = firstp == 31 ? 0xFFFFFFFFu : ((2u << firstp) - 1u);
         if ((ready & need) != need) {
             if (++spins > spin_limit) {
                 if (lane == 0) set_error(status, ERR_LOOKBACK_TIMEOUT);
                 break;
             }
-            __nanosleep(64);
+            __nanosleep(32);
             continue;
         }
-        uint64_t v = ((int)lane <= firstp) ? (s & (kSigned32 ? 0xFFFFFFFFull : kValMask)) : 0ull;
-        if (kSigned32) {
-            uint32_t w = (uint32_t)v;
+        uint64_t v = ((int)lane <= firstp) ? (s & kValMask) : 0ull;
 #pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) w += __shfl_xor_sync(0xFFFFFFFFu, w, d);
-            excl = (uint64_t)(uint32_t)((uint32_t)excl + w);
-        } else {
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, d);
-            excl += v;
-        }
+        for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, d);
+        excl += v;
         if (pm) break;
         look -= 32;
     }
@@ -282,13 +273,63 @@ SR_DEV void cta_seg_scan(bool tf, int32_t tv, int32_t* wv, int32_t* wf, bool& fe
 }
 }  // namespace
 
-// Per tile: the (head seen, sum since) pair of its winding changes.
+// The tiles' incoming winding prefixes: an exclusive segmented scan of the
+// tile pairs by one CTA, eight tiles a thread and round (one a thread took
+// 41 rounds, 17 us more, for the 10,290 tiles of a 21 M record frame).  Also
+// writes the scan's total (the winding scan's last entry) when the stages are
+// kept.
+template <int THREADS>
+SR_DEV void scan_tile_pairs(const uint64_t* tagg, int32_t* __restrict__ tile_in, const WindArgs& a, int64_t n,
+                            int64_t tiles, int32_t* wv, int32_t* wf) {
+    constexpr int K = 8;
+    bool cf = false;
+    int32_t cv = 0;
+    for (int64_t base = 0; base < tiles; base += THREADS * K) {
+        const int64_t t = base + (int64_t)threadIdx.x * K;
+        uint64_t w[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) w[k] = t + k < tiles ? ld_relaxed_u64(&tagg[t + k]) : 0ull;
+        bool tf = false;
+        int32_t tv = 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            bool f = (w[k] & kHeadBit) != 0;
+            int32_t v = (int32_t)(uint32_t)w[k];
+            seg_combine(tf, tv, f, v);
+            tf = f;
+            tv = v;
+        }
+        bool xf, aggf;
+        int32_t xv, agg;
+        cta_seg_scan<THREADS>(tf, tv, wv, wf, xf, xv, aggf, agg);
+        seg_combine(cf, cv, xf, xv);
+        // the value since the last head entering each tile, whatever xf says
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (t + k < tiles) tile_in[t + k] = xv;
+            bool f = (w[k] & kHeadBit) != 0;
+            int32_t v = (int32_t)(uint32_t)w[k];
+            seg_combine(xf, xv, f, v);
+            xf = f;
+            xv = v;
+        }
+        seg_combine(cf, cv, aggf, agg);
+        cf = aggf;
+        cv = agg;
+    }
+    if (threadIdx.x == 0 && a.dbg_wscan) a.dbg_wscan[n] = cv;
+}
+
+// Per tile: the (head seen, sum since) pair of its winding changes.  The CTA
+// that finishes last scans the pairs of all tiles.
 template <int ITEMS, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_winding_reduce(const WindArgs a, uint64_t* __restrict__ tagg) {
+__global__ void __launch_bounds__(THREADS) k_winding_reduce(const WindArgs a, uint64_t* tagg,
+                                                            int32_t* __restrict__ tile_in, uint32_t* done) {
     constexpr int kTile = THREADS * ITEMS;
     __shared__ int32_t wv[THREADS / 32], wf[THREADS / 32];
+    __shared__ bool s_last;
     const int64_t n = a.n_dev ? (int64_t)min((uint64_t)*a.n_dev, (uint64_t)a.n) : a.n;
-    const int64_t tbase = (int64_t)blockIdx.x * kTile;
+    const int64_t tbase = (int64_t)blockIdx.x * kTile, tiles = (n + kTile - 1) / kTile;
     if (tbase >= n) return;
     const int64_t ibase = tbase + (int64_t)threadIdx.x * ITEMS;
     uint64_t kk[ITEMS];
@@ -300,78 +341,14 @@ __global__ void __launch_bounds__(THREADS) k_winding_reduce(const WindArgs a, ui
     int32_t tv, ve, agg;
     run_heads<ITEMS>(a, ibase, n, kk, kprev, wbits, tf, tv);
     cta_seg_scan<THREADS>(tf, tv, wv, wf, fe, ve, aggf, agg);
-    if (threadIdx.x == 0) tagg[blockIdx.x] = (aggf ? kHeadBit : 0ull) | (uint32_t)agg;
-}
-
-// The tiles' incoming winding prefixes: an exclusive segmented scan of the
-// tile pairs in one CTA, 1,024 tiles a round.  Also writes the scan's total
-// (the winding scan's last entry) when the stages are kept.
-__global__ void __launch_bounds__(1024) k_winding_scan_tiles(const uint64_t* __restrict__ tagg,
-                                                            int32_t* __restrict__ tile_in, const WindArgs a,
-                                                            int tile_records) {
-    __shared__ int32_t wv[32], wf[32];
-    const int64_t n = a.n_dev ? (int64_t)min((uint64_t)*a.n_dev, (uint64_t)a.n) : a.n;
-    const int64_t tiles = (n + tile_records - 1) / tile_records;
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    bool cf = false;
-    int32_t cv = 0;
-    for (int64_t base = 0; base < tiles; base += 1024) {
-        const int64_t t = base + threadIdx.x;
-        const uint64_t w = t < tiles ? tagg[t] : 0ull;
-        bool fi = (w & kHeadBit) != 0;
-        int32_t vi = (int32_t)(uint32_t)w;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const bool fp = __shfl_up_sync(0xFFFFFFFFu, (int)fi, d) != 0;
-            const int32_t vp = __shfl_up_sync(0xFFFFFFFFu, vi, d);
-            if ((int)lane >= d) seg_combine(fp, vp, fi, vi);
-        }
-        if (lane == 31) {
-            wv[warp] = vi;
-            wf[warp] = fi ? 1 : 0;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            bool f2 = wf[lane] != 0;
-            int32_t v2 = wv[lane];
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const bool fp = __shfl_up_sync(0xFFFFFFFFu, (int)f2, d) != 0;
-                const int32_t vp = __shfl_up_sync(0xFFFFFFFFu, v2, d);
-                if ((int)lane >= d) seg_combine(fp, vp, f2, v2);
-            }
-            wv[lane] = v2;   // inclusive over warps 0..lane
-            wf[lane] = f2 ? 1 : 0;
-        }
-        __syncthreads();
-        // the pair before this tile: the carry, the warps before, the lanes before
-        bool pf = cf;
-        int32_t pv = cv;
-        if (warp > 0) {
-            bool f2 = wf[warp - 1] != 0;
-            int32_t v2 = wv[warp - 1];
-            seg_combine(pf, pv, f2, v2);
-            pf = f2;
-            pv = v2;
-        }
-        // lanes before: the inclusive pair of lane - 1 within the warp
-        bool lf = __shfl_up_sync(0xFFFFFFFFu, (int)fi, 1) != 0;
-        int32_t lv = __shfl_up_sync(0xFFFFFFFFu, vi, 1);
-        if (lane > 0) seg_combine(pf, pv, lf, lv);
-        else {
-            lf = pf;
-            lv = pv;
-        }
-        // the value since the last head entering the tile, whatever lf says
-        if (t < tiles) tile_in[t] = lv;
-        bool nf = wf[31] != 0;
-        int32_t nv = wv[31];
-        seg_combine(cf, cv, nf, nv);
-        __syncthreads();
-        cf = nf;
-        cv = nv;
+    if (threadIdx.x == 0) {
+        st_relaxed_u64(&tagg[blockIdx.x], (aggf ? kHeadBit : 0ull) | (uint32_t)agg);
+        __threadfence();
+        s_last = atomicAdd(done, 1u) == (uint32_t)tiles - 1u;
+        __threadfence();
     }
-    if (threadIdx.x == 0 && a.dbg_wscan) a.dbg_wscan[n] = cv;
+    __syncthreads();
+    if (s_last) scan_tile_pairs<THREADS>(tagg, tile_in, a, n, tiles, wv, wf);
 }
 
 // Each thread owns ITEMS consecutive sorted records (a blocked layout): its
@@ -588,11 +565,11 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
         if (lane < THREADS / 32) S.warpB[lane] = wi - w;
         const uint32_t agg16 = __shfl_sync(0xFFFFFFFFu, wi, THREADS / 32 - 1);
         const uint64_t aggB = ((uint64_t)(agg16 >> 16) << kFragShift) | (uint64_t)(agg16 & 0xFFFFu);
-        if (lane == 0) st_release_u64(&tstatB[tile], (tile == 0 ? kFlagP : kFlagA) | aggB);
+        if (lane == 0) st_relaxed_u64(&tstatB[tile], (tile == 0 ? kFlagP : kFlagA) | aggB);
         uint64_t excl = 0;
         if (tile > 0) {
-            excl = lookback<false>(tstatB, tile, status, spin_limit);
-            if (lane == 0) st_release_u64(&tstatB[tile], kFlagP | (excl + aggB));
+            excl = lookback(tstatB, tile, status, spin_limit);
+            if (lane == 0) st_relaxed_u64(&tstatB[tile], kFlagP | (excl + aggB));
         }
         if (lane == 0) {
             S.prefixB = excl;
@@ -706,30 +683,28 @@ static int64_t wind_tile(int items) { return items == 4 ? 1024 : 2048; }
 
 size_t winding_status_words(int64_t n, int items) {
     const int64_t tile = wind_tile(items);
-    // look-back words of the output slots, tile pairs, tile prefixes
-    return 3 * (size_t)((n + tile - 1) / tile + 1);
+    return (size_t)((n + tile - 1) / tile + 1);
 }
+// tile pairs (64-bit), then tile prefixes (32-bit)
+size_t winding_tile_words(int64_t n, int items) { return 2 * winding_status_words(n, items); }
 
 template <int ITEMS, int THREADS>
 static void launch_wind(const WindArgs& a, int64_t tiles, uint64_t* sB, uint64_t* tagg, int32_t* tile_in,
-                        uint32_t* tile_counter, uint32_t* status, cudaStream_t st) {
-    k_winding_reduce<ITEMS, THREADS><<<(unsigned)tiles, THREADS, 0, st>>>(a, tagg);
-    k_winding_scan_tiles<<<1, 1024, 0, st>>>(tagg, tile_in, a, ITEMS * THREADS);
-    k_winding_emit<ITEMS, THREADS><<<(unsigned)tiles, THREADS, 0, st>>>(a, tile_in, sB, tile_counter, status,
+                        uint32_t* counters, uint32_t* status, cudaStream_t st) {
+    k_winding_reduce<ITEMS, THREADS><<<(unsigned)tiles, THREADS, 0, st>>>(a, tagg, tile_in, counters + 1);
+    k_winding_emit<ITEMS, THREADS><<<(unsigned)tiles, THREADS, 0, st>>>(a, tile_in, sB, counters, status,
                                                                         spin_limit());
 }
 
-void launch_winding_emit(const WindArgs& a, int items, uint64_t* tile_status, uint32_t* tile_counter,
+void launch_winding_emit(const WindArgs& a, int items, uint64_t* tile_status, uint64_t* tile_sums, uint32_t* counters,
                          uint32_t* status, cudaStream_t st) {
     if (a.n <= 0) return;
     const int64_t tile = wind_tile(items);
     const int64_t tiles = (a.n + tile - 1) / tile;
-    uint64_t* sB = tile_status;
-    uint64_t* tagg = tile_status + (tiles + 1);
-    int32_t* tile_in = reinterpret_cast<int32_t*>(tile_status + 2 * (tiles + 1));
-    count_launches(3);
-    if (items == 4) launch_wind<4, 256>(a, tiles, sB, tagg, tile_in, tile_counter, status, st);
-    else launch_wind<8, 256>(a, tiles, sB, tagg, tile_in, tile_counter, status, st);
+    int32_t* tile_in = reinterpret_cast<int32_t*>(tile_sums + (tiles + 1));
+    count_launches(2);
+    if (items == 4) launch_wind<4, 256>(a, tiles, tile_status, tile_sums, tile_in, counters, status, st);
+    else launch_wind<8, 256>(a, tiles, tile_status, tile_sums, tile_in, counters, status, st);
 }
 
 }  // namespace sr
