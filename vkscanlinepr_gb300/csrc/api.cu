@@ -1995,14 +1995,13 @@ sr_status sr_sizer_train(sr_sizer* s, const float* d_x, const float* d_t, uint32
         }
         for (uint32_t b0 = 0; b0 < n; b0 += d.batch) {
             const uint32_t nb = std::min(d.batch, n - b0);
-            CUDA_TRY(sr::launch_mlp_grad(s->wb.p, s->master.as<float>(), s->norm.as<float>(), d_x, d_t,
-                                         idx ? idx + b0 : nullptr, nb, s->grad.as<float>(), s->loss.as<float>(),
-                                         st));
             ++s->step;
             const float bc1 = (float)(1.0 - std::pow(b1, (double)s->step));
             const float bc2 = (float)(1.0 - std::pow(b2, (double)s->step));
-            sr::launch_adam(s->master.as<float>(), s->wb.p, s->grad.as<float>(), s->m.as<float>(), s->v.as<float>(),
-                            d.lr, d.beta1, d.beta2, d.eps, bc1, bc2, st);
+            CUDA_TRY(sr::launch_mlp_step(s->wb.p, s->master.as<float>(), s->norm.as<float>(), d_x, d_t,
+                                         idx ? idx + b0 : nullptr, nb, s->grad.as<float>(), s->loss.as<float>(),
+                                         s->m.as<float>(), s->v.as<float>(), d.lr, d.beta1, d.beta2, d.eps, bc1, bc2,
+                                         s->ctl.as<uint32_t>() + 1, st));
             if (!idx) {   // unshuffled minibatches are consecutive rows
                 d_x += (size_t)nb * sr::kMlpIn;
                 d_t += (size_t)nb * sr::kMlpOut;

@@ -17,6 +17,8 @@
 //   norm = x_mean[6] x_inv_std[6] y_mean[2] y_std[2]
 // so the network works in standard units; predictions are returned in
 // log(1 + count) units.
+#include <atomic>
+
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -31,8 +33,20 @@ constexpr int oW1 = 0, oB1 = oW1 + kH * kIn, oW2 = oB1 + kH, oB2 = oW2 + kH * kH
 static_assert(kParams == kMlpParams, "parameter layout");
 constexpr int nXm = 0, nXs = kIn, nYm = 2 * kIn, nYs = 2 * kIn + kOut;
 static_assert(nYs + kOut == kMlpNorm, "normaliser layout");
-constexpr int kSamples = 64;   // samples per training block (one per thread)
-constexpr int kPad = kH + 1;   // shared-memory row stride: row q starts in bank q
+// Shared-memory copies of the parameters: weights rounded to BF16 as the
+// forward pass uses them, biases FP32.  W1 is transposed (neighbouring lanes
+// take neighbouring units); a row of W2, as of the activations, is padded to
+// 68 floats, so that 16-byte reads of eight neighbouring rows meet no bank
+// twice.
+constexpr int kRow = kH + 4;
+struct Params {
+    __align__(16) float w2[kH][kRow];
+    __align__(16) float w1t[kIn][kH];
+    __align__(16) float w3[kOut][kH];
+    __align__(16) float b1[kH], b2[kH];
+    float b3[kOut];
+    float norm[kMlpNorm];
+};
 
 SR_DEV float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 // d/dx [x Phi(x)] = Phi(x) + x phi(x)
@@ -42,11 +56,33 @@ SR_DEV float gelu_grad(float x) {
     return fmaf(x, pdf, cdf);
 }
 
-SR_DEV bool is_bias(int i) { return (i >= oB1 && i < oW2) || (i >= oB2 && i < oW3) || i >= oB3; }
-
-// Parameters as the forward pass uses them: weights rounded to BF16, biases FP32.
-SR_DEV void load_params(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ master, float* s) {
-    for (int i = threadIdx.x; i < kParams; i += blockDim.x) s[i] = is_bias(i) ? master[i] : __bfloat162float(wb[i]);
+SR_DEV float bf(const __nv_bfloat16& w) { return __bfloat162float(w); }
+SR_DEV void load_params(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ master,
+                        const float* __restrict__ norm, Params& P) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    static_assert(oW2 % 8 == 0 && kH % 8 == 0, "16-byte reads of W2");
+    for (int i = tid; i < kH * kH / 8; i += nt) {
+        const uint4 v = reinterpret_cast<const uint4*>(wb + oW2)[i];
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+        float4 f[2];
+        float* q = reinterpret_cast<float*>(f);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {   // a BF16 is the upper half of its float
+            q[2 * k] = __uint_as_float(u[k] << 16);
+            q[2 * k + 1] = __uint_as_float(u[k] & 0xFFFF0000u);
+        }
+        float4* row = reinterpret_cast<float4*>(&P.w2[8 * i / kH][8 * i % kH]);
+        row[0] = f[0];
+        row[1] = f[1];
+    }
+    for (int i = tid; i < kH * kIn; i += nt) P.w1t[i % kIn][i / kIn] = bf(wb[oW1 + i]);
+    for (int i = tid; i < kOut * kH; i += nt) P.w3[i / kH][i % kH] = bf(wb[oW3 + i]);
+    for (int i = tid; i < kH; i += nt) {
+        P.b1[i] = master[oB1 + i];
+        P.b2[i] = master[oB2 + i];
+    }
+    if (tid < kOut) P.b3[tid] = master[oB3 + tid];
+    if (tid < kMlpNorm) P.norm[tid] = norm[tid];
 }
 }  // namespace
 
@@ -122,152 +158,336 @@ __global__ void k_path_labels(const uint32_t* __restrict__ path_first_curve, uin
 }
 
 // ------------------------------------------------------------ inference --
-// One path per thread; parameters staged once per block in shared memory.
-__global__ void __launch_bounds__(128) k_mlp_predict(const __nv_bfloat16* __restrict__ wb,
-                                                     const float* __restrict__ master,
-                                                     const float* __restrict__ norm, const float* __restrict__ x,
-                                                     uint32_t n, float* __restrict__ y) {
-    __shared__ float s[kParams];
-    __shared__ float nm[kMlpNorm];
-    load_params(wb, master, s);
-    if (threadIdx.x < kMlpNorm) nm[threadIdx.x] = norm[threadIdx.x];
+// A warp takes eight paths, a lane two of the 64 units of each layer for all
+// eight: a weight read from shared memory serves eight multiply-adds, and 16
+// sums are in flight a lane.  FP32 issue bounds it (4,608 multiply-adds and
+// 128 erf a path; 70% of the issue slots used): 200,000 paths take 70 us and
+// 5,000 take 8.3, where a path a thread (64 values in 247 registers, one sum
+// in flight) took 141 and 27.
+constexpr int kPredictThreads = 256, kPredictCtas = 3, kWarpPaths = 8;
+struct PredictSmem {
+    Params P;
+    __align__(16) float h[kPredictThreads / 32][kWarpPaths][kRow];
+};
+__global__ void __launch_bounds__(kPredictThreads, kPredictCtas) k_mlp_predict(
+    const __nv_bfloat16* __restrict__ wb, const float* __restrict__ master, const float* __restrict__ norm,
+    const float* __restrict__ x, uint32_t n, float* __restrict__ y) {
+    __shared__ PredictSmem S;
+    const Params& P = S.P;
+    load_params(wb, master, norm, S.P);
     __syncthreads();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float in[kIn];
-#pragma unroll
-        for (int k = 0; k < kIn; ++k) in[k] = (x[(size_t)i * kIn + k] - nm[nXm + k]) * nm[nXs + k];
-        float h1[kH];
-#pragma unroll
-        for (int j = 0; j < kH; ++j) {
-            float a = s[oB1 + j];
-#pragma unroll
-            for (int k = 0; k < kIn; ++k) a = fmaf(s[oW1 + j * kIn + k], in[k], a);
-            h1[j] = gelu(a);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float(*h)[kRow] = S.h[warp];
+    const uint32_t warps = gridDim.x * (kPredictThreads / 32);
+    for (uint32_t g = blockIdx.x * (kPredictThreads / 32) + warp; g * kWarpPaths < n; g += warps) {
+        const uint32_t p0 = g * kWarpPaths;
+        // layer 1: units lane and lane + 32
+        float v0 = 0.0f, v1 = 0.0f;   // the eight paths' 48 inputs, standardised
+        {
+            const uint32_t i0 = p0 * kIn + lane, i1 = i0 + 32;
+            const int k0 = lane % kIn, k1 = (lane + 32) % kIn;
+            if (i0 < n * kIn) v0 = (x[i0] - P.norm[nXm + k0]) * P.norm[nXs + k0];
+            if (lane < kWarpPaths * kIn - 32 && i1 < n * kIn) v1 = (x[i1] - P.norm[nXm + k1]) * P.norm[nXs + k1];
         }
-        float o0 = s[oB3], o1 = s[oB3 + 1];
-        for (int j = 0; j < kH; ++j) {
-            float a = s[oB2 + j];
 #pragma unroll
-            for (int k = 0; k < kH; ++k) a = fmaf(s[oW2 + j * kH + k], h1[k], a);
-            const float h2 = gelu(a);
-            o0 = fmaf(s[oW3 + j], h2, o0);
-            o1 = fmaf(s[oW3 + kH + j], h2, o1);
+        for (int q = 0; q < kWarpPaths; ++q) {
+            float a0 = P.b1[lane], a1 = P.b1[lane + 32];
+#pragma unroll
+            for (int k = 0; k < kIn; ++k) {
+                const int e = q * kIn + k;
+                const float in = __shfl_sync(0xFFFFFFFFu, e < 32 ? v0 : v1, e & 31);
+                a0 = fmaf(P.w1t[k][lane], in, a0);
+                a1 = fmaf(P.w1t[k][lane + 32], in, a1);
+            }
+            h[q][lane] = gelu(a0);
+            h[q][lane + 32] = gelu(a1);
         }
-        y[(size_t)i * kOut] = fmaf(o0, nm[nYs], nm[nYm]);
-        y[(size_t)i * kOut + 1] = fmaf(o1, nm[nYs + 1], nm[nYm + 1]);
+        __syncwarp();
+        // layer 2
+        float a0[kWarpPaths], a1[kWarpPaths];
+#pragma unroll
+        for (int q = 0; q < kWarpPaths; ++q) {
+            a0[q] = P.b2[lane];
+            a1[q] = P.b2[lane + 32];
+        }
+#pragma unroll 2
+        for (int k = 0; k < kH; k += 4) {
+            const float4 w0 = *reinterpret_cast<const float4*>(&P.w2[lane][k]);
+            const float4 w1 = *reinterpret_cast<const float4*>(&P.w2[lane + 32][k]);
+#pragma unroll
+            for (int q = 0; q < kWarpPaths; ++q) {
+                const float4 u = *reinterpret_cast<const float4*>(&h[q][k]);
+                a0[q] = fmaf(w0.x, u.x, a0[q]); a1[q] = fmaf(w1.x, u.x, a1[q]);
+                a0[q] = fmaf(w0.y, u.y, a0[q]); a1[q] = fmaf(w1.y, u.y, a1[q]);
+                a0[q] = fmaf(w0.z, u.z, a0[q]); a1[q] = fmaf(w1.z, u.z, a1[q]);
+                a0[q] = fmaf(w0.w, u.w, a0[q]); a1[q] = fmaf(w1.w, u.w, a1[q]);
+            }
+        }
+        // layer 3: 16 sums over the lanes, halving the sums a lane holds with
+        // every exchange: lane l ends with output l & 15 (path l / 2 & 7,
+        // output l & 1), the two halves of the warp added last
+        float o[2 * kWarpPaths];
+        const float w30 = P.w3[0][lane], w31 = P.w3[0][lane + 32], w40 = P.w3[1][lane], w41 = P.w3[1][lane + 32];
+#pragma unroll
+        for (int q = 0; q < kWarpPaths; ++q) {
+            const float g0 = gelu(a0[q]), g1 = gelu(a1[q]);
+            o[2 * q] = fmaf(w31, g1, w30 * g0);
+            o[2 * q + 1] = fmaf(w41, g1, w40 * g0);
+        }
+#pragma unroll
+        for (int d = 8; d; d >>= 1) {
+            const bool up = (lane & d) != 0;
+#pragma unroll
+            for (int i = 0; i < d; ++i) {
+                const float mine = up ? o[i + d] : o[i], other = up ? o[i] : o[i + d];
+                o[i] = mine + __shfl_xor_sync(0xFFFFFFFFu, other, d);
+            }
+        }
+        const float sum = o[0] + __shfl_xor_sync(0xFFFFFFFFu, o[0], 16);
+        const uint32_t at = p0 * kOut + lane;
+        const int k = lane & 1;
+        if (lane < 2 * kWarpPaths && at < n * kOut) y[at] = fmaf(sum + P.b3[k], P.norm[nYs + k], P.norm[nYm + k]);
+        __syncwarp();
     }
 }
 
 // ------------------------------------------------------------- training --
-// Forward and backward of the mean squared error (in standard units) over
-// one minibatch: rows idx[0..n) of (x, t), or rows 0..n when idx is NULL.
-// Each block takes 64 samples, one per thread, keeps their activations in
-// shared memory, then reduces its parameter gradients over the samples and
-// adds them into grad.  loss_sum receives the sum of squared errors.
-__global__ void __launch_bounds__(kSamples) k_mlp_grad(const __nv_bfloat16* __restrict__ wb,
-                                                       const float* __restrict__ master,
-                                                       const float* __restrict__ norm, const float* __restrict__ x,
-                                                       const float* __restrict__ t, const uint32_t* __restrict__ idx,
-                                                       uint32_t n, float scale, float* __restrict__ grad,
-                                                       float* __restrict__ loss_sum) {
-    extern __shared__ float sm[];
-    float* s = sm;                          // parameters [kParams]
-    float* a1 = s + kParams;                // layer-1 pre-activations [kSamples][kPad]
-    float* h1 = a1 + kSamples * kPad;       // layer-1 outputs
-    float* a2 = h1 + kSamples * kPad;       // layer-2 pre-activations
-    float* h2 = a2 + kSamples * kPad;       // layer-2 outputs
-    float* d2 = h2 + kSamples * kPad;       // dL/da2
-    float* d1 = d2 + kSamples * kPad;       // dL/da1
-    float* xin = d1 + kSamples * kPad;      // standardised inputs [kSamples][kIn]
-    float* dy = xin + kSamples * kIn;       // dL/dy [kSamples][kOut]
-    float* nm = dy + kSamples * kOut;       // normaliser [kMlpNorm]
-    load_params(wb, master, s);
-    const int tid = threadIdx.x;
-    if (tid < kMlpNorm) nm[tid] = norm[tid];
-    const uint32_t sidx = blockIdx.x * kSamples + tid;
-    const bool live = sidx < n;
-    const uint32_t row = live ? (idx ? idx[sidx] : sidx) : 0u;
-    __syncthreads();
+// Adam on the FP32 master copy (bias-corrected moments); refreshes the BF16
+// weights and clears the gradient for the next step.
+struct AdamArgs {
+    float *master, *m, *v;
+    __nv_bfloat16* wb;
+    float lr, b1, b2, eps, bc1, bc2;
+};
+// By a CTA of kThreads; every load before the first store, so that they are
+// in flight together.
+template <int kThreads> SR_DEV void adam_all(const AdamArgs& A, float* grad) {
+    constexpr int K = (kParams + kThreads - 1) / kThreads;
+    float g[K], m[K], v[K], w[K];
 #pragma unroll
-    for (int k = 0; k < kIn; ++k)
-        xin[tid * kIn + k] = live ? (x[(size_t)row * kIn + k] - nm[nXm + k]) * nm[nXs + k] : 0.0f;
-    for (int j = 0; j < kH; ++j) {
-        float a = s[oB1 + j];
+    for (int k = 0; k < K; ++k) {
+        const int i = threadIdx.x + k * kThreads;
+        if (i >= kParams) continue;
+        g[k] = __ldcg(grad + i);
+        m[k] = A.m[i];
+        v[k] = A.v[i];
+        w[k] = A.master[i];
+    }
 #pragma unroll
-        for (int k = 0; k < kIn; ++k) a = fmaf(s[oW1 + j * kIn + k], xin[tid * kIn + k], a);
-        a1[tid * kPad + j] = a;
-        h1[tid * kPad + j] = gelu(a);
-    }
-    float y0 = s[oB3], y1 = s[oB3 + 1];
-    for (int j = 0; j < kH; ++j) {
-        float a = s[oB2 + j];
-        for (int k = 0; k < kH; ++k) a = fmaf(s[oW2 + j * kH + k], h1[tid * kPad + k], a);
-        a2[tid * kPad + j] = a;
-        const float hv = gelu(a);
-        h2[tid * kPad + j] = hv;
-        y0 = fmaf(s[oW3 + j], hv, y0);
-        y1 = fmaf(s[oW3 + kH + j], hv, y1);
-    }
-    float e0 = 0.0f, e1 = 0.0f;
-    if (live) {
-        e0 = y0 - (t[(size_t)row * kOut] - nm[nYm]) / nm[nYs];
-        e1 = y1 - (t[(size_t)row * kOut + 1] - nm[nYm + 1]) / nm[nYs + 1];
-        atomicAdd(loss_sum, e0 * e0 + e1 * e1);
-    }
-    // d(mean squared error)/dy with scale = 1 / (samples * outputs)
-    const float g0 = 2.0f * scale * e0, g1 = 2.0f * scale * e1;
-    dy[tid * kOut] = g0;
-    dy[tid * kOut + 1] = g1;
-    for (int j = 0; j < kH; ++j)
-        d2[tid * kPad + j] = (s[oW3 + j] * g0 + s[oW3 + kH + j] * g1) * gelu_grad(a2[tid * kPad + j]);
-    for (int k = 0; k < kH; ++k) {
-        float a = 0.0f;
-        for (int j = 0; j < kH; ++j) a = fmaf(s[oW2 + j * kH + k], d2[tid * kPad + j], a);
-        d1[tid * kPad + k] = a * gelu_grad(a1[tid * kPad + k]);
-    }
-    __syncthreads();
-    // parameter gradients: sums over the block's samples
-    for (int e = tid; e < kParams; e += kSamples) {
-        float acc = 0.0f;
-        if (e < oB1) {                       // W1[j][k]
-            const int j = e / kIn, k = e % kIn;
-            for (int q = 0; q < kSamples; ++q) acc = fmaf(d1[q * kPad + j], xin[q * kIn + k], acc);
-        } else if (e < oW2) {                // b1
-            const int j = e - oB1;
-            for (int q = 0; q < kSamples; ++q) acc += d1[q * kPad + j];
-        } else if (e < oB2) {                // W2[j][k]
-            const int j = (e - oW2) / kH, k = (e - oW2) % kH;
-            for (int q = 0; q < kSamples; ++q) acc = fmaf(d2[q * kPad + j], h1[q * kPad + k], acc);
-        } else if (e < oW3) {                // b2
-            const int j = e - oB2;
-            for (int q = 0; q < kSamples; ++q) acc += d2[q * kPad + j];
-        } else if (e < oB3) {                // W3[o][j]
-            const int o = (e - oW3) / kH, j = (e - oW3) % kH;
-            for (int q = 0; q < kSamples; ++q) acc = fmaf(dy[q * kOut + o], h2[q * kPad + j], acc);
-        } else {                             // b3
-            const int o = e - oB3;
-            for (int q = 0; q < kSamples; ++q) acc += dy[q * kOut + o];
-        }
-        atomicAdd(&grad[e], acc);
+    for (int k = 0; k < K; ++k) {
+        const int i = threadIdx.x + k * kThreads;
+        if (i >= kParams) continue;
+        const float mi = A.b1 * m[k] + (1.0f - A.b1) * g[k];
+        const float vi = A.b2 * v[k] + (1.0f - A.b2) * g[k] * g[k];
+        A.m[i] = mi;
+        A.v[i] = vi;
+        const float wi = w[k] - A.lr * (mi / A.bc1) / (sqrtf(vi / A.bc2) + A.eps);
+        A.master[i] = wi;
+        A.wb[i] = __float2bfloat16_rn(wi);
+        grad[i] = 0.0f;
     }
 }
 
-// Adam on the FP32 master copy (bias-corrected moments); refreshes the BF16
-// weights and clears the gradient for the next step.
-__global__ void k_adam(float* __restrict__ master, __nv_bfloat16* __restrict__ wb, float* __restrict__ grad,
-                       float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2, float eps,
-                       float bc1, float bc2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kParams) return;
-    const float g = grad[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * g;
-    const float vi = b2 * v[i] + (1.0f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    const float w = master[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    master[i] = w;
-    wb[i] = __float2bfloat16_rn(w);
-    grad[i] = 0.0f;
+SR_DEV void red_add4(float* p, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// Forward and backward of the mean squared error (in standard units) over
+// one minibatch: rows idx[0..n) of (x, t), or rows 0..n when idx is NULL.
+// A CTA takes 32 samples: a minibatch of 4,096 is 128 CTAs, one wave with 16
+// warps on an SM.  Every layer is a small product out of shared memory in
+// which a thread owns 2 to 8 outputs, read in 16-byte pieces; the CTA's
+// parameter gradients are summed over its samples in registers and added into
+// grad.  loss_sum receives the sum of squared errors.  With `adam`, the CTA
+// that finishes last takes the optimiser step (a launch and its gap saved).
+// Shared-memory reads and the latency of its eight phases bound it: a step
+// of 4,096 samples takes 23 us, where 64 CTAs of 64 threads, a sample each,
+// and a separate optimiser launch took 84.
+constexpr int kSamples = 32, kGradThreads = 512;
+struct GradSmem {
+    Params P;
+    __align__(16) float a1[kSamples][kRow], h1[kSamples][kRow], a2[kSamples][kRow], h2[kSamples][kRow];
+    __align__(16) float d2[kSamples][kRow], d1[kSamples][kRow];
+    float xin[kSamples][kIn];
+    float ty[kSamples][kOut];   // standardised targets
+    float dy[kSamples][kOut];
+    bool last;
+};
+
+__global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const __nv_bfloat16* __restrict__ wb,
+                                                           const float* __restrict__ master,
+                                                           const float* __restrict__ norm, const float* __restrict__ x,
+                                                           const float* __restrict__ t,
+                                                           const uint32_t* __restrict__ idx, uint32_t n, float scale,
+                                                           float* grad, float* loss_sum, int adam, AdamArgs A,
+                                                           uint32_t* done) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
+    const Params& P = S.P;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t s0 = blockIdx.x * kSamples;
+    load_params(wb, master, norm, S.P);
+    if (tid < kSamples * kIn) {
+        const int q = tid / kIn, k = tid % kIn;
+        const uint32_t sidx = s0 + q;
+        float v = 0.0f;
+        if (sidx < n) v = (x[(size_t)(idx ? idx[sidx] : sidx) * kIn + k] - norm[nXm + k]) * norm[nXs + k];
+        S.xin[q][k] = v;
+    } else if (tid >= kGradThreads - kSamples * kOut) {
+        const int i = tid - (kGradThreads - kSamples * kOut), q = i / kOut, k = i % kOut;
+        const uint32_t sidx = s0 + q;
+        float v = 0.0f;
+        if (sidx < n) v = (t[(size_t)(idx ? idx[sidx] : sidx) * kOut + k] - norm[nYm + k]) / norm[nYs + k];
+        S.ty[q][k] = v;
+    }
+    __syncthreads();
+    // layer 1: 4 outputs a thread
+#pragma unroll
+    for (int i = 0; i < kSamples * kH / kGradThreads; ++i) {
+        const int q = (tid + i * kGradThreads) / kH, j = tid % kH;
+        float a = P.b1[j];
+#pragma unroll
+        for (int k = 0; k < kIn; ++k) a = fmaf(P.w1t[k][j], S.xin[q][k], a);
+        S.a1[q][j] = a;
+        S.h1[q][j] = gelu(a);
+    }
+    __syncthreads();
+    // layer 2: two units of two samples a thread
+    {
+        const int q = 2 * warp, j = lane;
+        float a00 = P.b2[j], a01 = P.b2[j + 32], a10 = a00, a11 = a01;
+#pragma unroll 4
+        for (int k = 0; k < kH; k += 4) {
+            const float4 u = *reinterpret_cast<const float4*>(&S.h1[q][k]);
+            const float4 v = *reinterpret_cast<const float4*>(&S.h1[q + 1][k]);
+            const float4 w0 = *reinterpret_cast<const float4*>(&P.w2[j][k]);
+            const float4 w1 = *reinterpret_cast<const float4*>(&P.w2[j + 32][k]);
+            a00 = fmaf(w0.x, u.x, a00); a01 = fmaf(w1.x, u.x, a01); a10 = fmaf(w0.x, v.x, a10); a11 = fmaf(w1.x, v.x, a11);
+            a00 = fmaf(w0.y, u.y, a00); a01 = fmaf(w1.y, u.y, a01); a10 = fmaf(w0.y, v.y, a10); a11 = fmaf(w1.y, v.y, a11);
+            a00 = fmaf(w0.z, u.z, a00); a01 = fmaf(w1.z, u.z, a01); a10 = fmaf(w0.z, v.z, a10); a11 = fmaf(w1.z, v.z, a11);
+            a00 = fmaf(w0.w, u.w, a00); a01 = fmaf(w1.w, u.w, a01); a10 = fmaf(w0.w, v.w, a10); a11 = fmaf(w1.w, v.w, a11);
+        }
+        S.a2[q][j] = a00; S.a2[q][j + 32] = a01; S.a2[q + 1][j] = a10; S.a2[q + 1][j + 32] = a11;
+        S.h2[q][j] = gelu(a00); S.h2[q][j + 32] = gelu(a01);
+        S.h2[q + 1][j] = gelu(a10); S.h2[q + 1][j + 32] = gelu(a11);
+    }
+    __syncwarp();
+    // layer 3 and the error: a warp its two samples, a lane two units of each
+    {
+        float sq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int q = 2 * warp + i;
+            float y0 = fmaf(P.w3[0][lane + 32], S.h2[q][lane + 32], P.w3[0][lane] * S.h2[q][lane]);
+            float y1 = fmaf(P.w3[1][lane + 32], S.h2[q][lane + 32], P.w3[1][lane] * S.h2[q][lane]);
+#pragma unroll
+            for (int d = 16; d; d >>= 1) {
+                y0 += __shfl_xor_sync(0xFFFFFFFFu, y0, d);
+                y1 += __shfl_xor_sync(0xFFFFFFFFu, y1, d);
+            }
+            const uint32_t sidx = s0 + q;
+            if (lane < kOut) {
+                float e = 0.0f;
+                if (sidx < n) {
+                    e = ((lane ? y1 : y0) + P.b3[lane]) - S.ty[q][lane];
+                    sq = fmaf(e, e, sq);
+                }
+                // d(mean squared error)/dy with scale = 1 / (samples * outputs)
+                S.dy[q][lane] = 2.0f * scale * e;
+            }
+        }
+        sq += __shfl_xor_sync(0xFFFFFFFFu, sq, 1);
+        if (lane == 0) atomicAdd(loss_sum, sq);
+        __syncwarp();
+        // dL/da2
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int q = 2 * warp + i;
+            const float g0 = S.dy[q][0], g1 = S.dy[q][1];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = lane + 32 * h;
+                S.d2[q][j] = (P.w3[0][j] * g0 + P.w3[1][j] * g1) * gelu_grad(S.a2[q][j]);
+            }
+        }
+    }
+    __syncthreads();
+    // dL/da1: four units of a sample a thread
+    {
+        const int q = tid / 16, k = (tid % 16) * 4;
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+        for (int j = 0; j < kH; j += 4) {
+            const float4 d = *reinterpret_cast<const float4*>(&S.d2[q][j]);
+            const float dj[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 w = *reinterpret_cast<const float4*>(&P.w2[j + i][k]);
+                a.x = fmaf(w.x, dj[i], a.x);
+                a.y = fmaf(w.y, dj[i], a.y);
+                a.z = fmaf(w.z, dj[i], a.z);
+                a.w = fmaf(w.w, dj[i], a.w);
+            }
+        }
+        a.x *= gelu_grad(S.a1[q][k]);
+        a.y *= gelu_grad(S.a1[q][k + 1]);
+        a.z *= gelu_grad(S.a1[q][k + 2]);
+        a.w *= gelu_grad(S.a1[q][k + 3]);
+        *reinterpret_cast<float4*>(&S.d1[q][k]) = a;
+    }
+    // parameter gradients, summed over the CTA's samples.  W2: eight inputs
+    // of a unit a thread
+    {
+        const int j = tid / 8, k = (tid % 8) * 8;
+        float g[8] = {};
+#pragma unroll 4
+        for (int q = 0; q < kSamples; ++q) {
+            const float d = S.d2[q][j];
+            const float4 u = *reinterpret_cast<const float4*>(&S.h1[q][k]);
+            const float4 v = *reinterpret_cast<const float4*>(&S.h1[q][k + 4]);
+            g[0] = fmaf(d, u.x, g[0]); g[1] = fmaf(d, u.y, g[1]); g[2] = fmaf(d, u.z, g[2]); g[3] = fmaf(d, u.w, g[3]);
+            g[4] = fmaf(d, v.x, g[4]); g[5] = fmaf(d, v.y, g[5]); g[6] = fmaf(d, v.z, g[6]); g[7] = fmaf(d, v.w, g[7]);
+        }
+        red_add4(grad + oW2 + j * kH + k, g[0], g[1], g[2], g[3]);
+        red_add4(grad + oW2 + j * kH + k + 4, g[4], g[5], g[6], g[7]);
+    }
+    __syncthreads();
+    // the others, one a thread and round
+    for (int e = tid; e < kParams - kH * kH; e += kGradThreads) {
+        float acc = 0.0f;
+        int at;
+        if (e < oB1) {                       // W1[j][k]
+            const int j = e / kIn, k = e % kIn;
+            for (int q = 0; q < kSamples; ++q) acc = fmaf(S.d1[q][j], S.xin[q][k], acc);
+            at = e;
+        } else if (e < oW2) {                // b1
+            for (int q = 0; q < kSamples; ++q) acc += S.d1[q][e - oB1];
+            at = e;
+        } else if (e < oW2 + kH) {           // b2
+            for (int q = 0; q < kSamples; ++q) acc += S.d2[q][e - oW2];
+            at = oB2 + (e - oW2);
+        } else if (e < oW2 + kH + kOut * kH) {   // W3[o][j]
+            const int i = e - (oW2 + kH), o = i / kH, j = i % kH;
+            for (int q = 0; q < kSamples; ++q) acc = fmaf(S.dy[q][o], S.h2[q][j], acc);
+            at = oW3 + i;
+        } else {                             // b3
+            const int o = e - (oW2 + kH + kOut * kH);
+            for (int q = 0; q < kSamples; ++q) acc += S.dy[q][o];
+            at = oB3 + o;
+        }
+        atomicAdd(&grad[at], acc);
+    }
+    if (!adam) return;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        S.last = atomicAdd(done, 1u) == gridDim.x - 1u;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!S.last) return;
+    adam_all<kGradThreads>(A, grad);
+    if (tid == 0) *done = 0;
 }
 
 __global__ void k_to_bf16(const float* __restrict__ master, __nv_bfloat16* __restrict__ wb) {
@@ -357,10 +577,6 @@ __global__ void k_judge(const uint32_t* __restrict__ path_first_curve, uint32_t 
 }
 
 // ------------------------------------------------------------- launches --
-size_t mlp_grad_smem() {
-    return sizeof(float) * (kParams + 6 * kSamples * kPad + kSamples * kIn + kSamples * kOut + kMlpNorm);
-}
-
 void launch_path_features(const GeomArgs& g, const uint32_t* path_first_curve, uint32_t n_paths, float* feats,
                           cudaStream_t st) {
     if (!n_paths) return;
@@ -379,30 +595,41 @@ void launch_mlp_predict(const void* wb, const float* master, const float* norm, 
                         int sm_count, cudaStream_t st) {
     if (!n) return;
     count_launches(1);
-    unsigned blocks = (n + 127) / 128;
-    const unsigned cap = 8u * (unsigned)(sm_count > 0 ? sm_count : 148);
+    constexpr unsigned per = kPredictThreads / 32 * kWarpPaths;
+    unsigned blocks = (n + per - 1) / per;
+    const unsigned cap = (unsigned)kPredictCtas * (unsigned)(sm_count > 0 ? sm_count : 148);   // one wave
     if (blocks > cap) blocks = cap;
-    k_mlp_predict<<<blocks, 128, 0, st>>>(static_cast<const __nv_bfloat16*>(wb), master, norm, x, n, y);
+    k_mlp_predict<<<blocks, kPredictThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(wb), master, norm, x, n, y);
+}
+
+static cudaError_t grad_launch(const void* wb, const float* master, const float* norm, const float* x, const float* t,
+                               const uint32_t* idx, uint32_t n, float* grad, float* loss_sum, bool adam,
+                               const AdamArgs& A, uint32_t* done, cudaStream_t st) {
+    static std::atomic<uint32_t> attr{0};
+    cudaError_t e = cudaSuccess;
+    once_per_device(attr, [&] {
+        e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem));
+    });
+    if (e != cudaSuccess) return e;
+    count_launches(1);
+    k_mlp_grad<<<(n + kSamples - 1) / kSamples, kGradThreads, sizeof(GradSmem), st>>>(
+        static_cast<const __nv_bfloat16*>(wb), master, norm, x, t, idx, n, 1.0f / ((float)n * (float)kOut), grad,
+        loss_sum, adam ? 1 : 0, A, done);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_mlp_grad(const void* wb, const float* master, const float* norm, const float* x, const float* t,
                             const uint32_t* idx, uint32_t n, float* grad, float* loss_sum, cudaStream_t st) {
     if (!n) return cudaSuccess;
-    const size_t smem = mlp_grad_smem();
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    count_launches(1);
-    k_mlp_grad<<<(n + kSamples - 1) / kSamples, kSamples, smem, st>>>(
-        static_cast<const __nv_bfloat16*>(wb), master, norm, x, t, idx, n, 1.0f / ((float)n * (float)kOut), grad,
-        loss_sum);
-    return cudaGetLastError();
+    return grad_launch(wb, master, norm, x, t, idx, n, grad, loss_sum, false, AdamArgs{}, nullptr, st);
 }
 
-void launch_adam(float* master, void* wb, float* grad, float* m, float* v, float lr, float b1, float b2, float eps,
-                 float bc1, float bc2, cudaStream_t st) {
-    count_launches(1);
-    k_adam<<<(kParams + 255) / 256, 256, 0, st>>>(master, static_cast<__nv_bfloat16*>(wb), grad, m, v, lr, b1, b2,
-                                                  eps, bc1, bc2);
+cudaError_t launch_mlp_step(void* wb, float* master, const float* norm, const float* x, const float* t,
+                            const uint32_t* idx, uint32_t n, float* grad, float* loss_sum, float* m, float* v, float lr,
+                            float b1, float b2, float eps, float bc1, float bc2, uint32_t* done, cudaStream_t st) {
+    if (!n) return cudaSuccess;
+    const AdamArgs A{master, m, v, static_cast<__nv_bfloat16*>(wb), lr, b1, b2, eps, bc1, bc2};
+    return grad_launch(wb, master, norm, x, t, idx, n, grad, loss_sum, true, A, done, st);
 }
 
 void launch_to_bf16(const float* master, void* wb, cudaStream_t st) {
