@@ -254,11 +254,11 @@ void sr_destroy(sr_ctx* ctx);
  * d_out[n] = the total (n+1 outputs; d_in and d_out may be the same
  * buffer), wrapping on overflow.  Replaces the reference's standalone scan
  * kernel workdir/shaders/common/naive_scan.comp:27-73 (one workgroup,
- * 1023-element batches) with a single-pass decoupled look-back scan.
- * Asynchronous on `stream`; its look-back scratch comes from
- * cudaMallocAsync/cudaFreeAsync on the same stream.  0 <= n < 2^31.
- * A look-back wait that gives up (SR_ERR_TIMEOUT) leaves a wrong prefix in
- * d_out; it is reported by sr_scan_status, not by this call. */
+ * 1023-element batches) with one CTA for short inputs and a sum and a scan of
+ * chunks for longer ones.  Asynchronous on `stream`; the chunk sums come from
+ * a memory pool of the library's (stream-ordered allocation on the same
+ * stream), which keeps up to 32 MB a device until sr_scan_status or the end of
+ * the process.  0 <= n < 2^31. */
 sr_status sr_exclusive_scan_i32(const int32_t* d_in, int32_t* d_out, int64_t n, void* stream);
 
 /* The same scan for callers that cannot allocate device memory: a host that
@@ -268,25 +268,26 @@ sr_status sr_exclusive_scan_i32(const int32_t* d_in, int32_t* d_out, int64_t n, 
  * This entry point calls no cudaMalloc, cudaFree or other allocating routine.
  * It has no counterpart in the reference.
  *
- * Its look-back scratch is a fixed array of SR_NOALLOC_SCAN_SCRATCH_BYTES
+ * Its scratch is a fixed array of SR_NOALLOC_SCAN_SCRATCH_BYTES
  * compiled into the library: every GPU that loads the library holds it until
  * the process exits.  n is limited to SR_NOALLOC_SCAN_MAX_N; larger n is
  * rejected with SR_ERR_INVALID_ARG.  The first call on a device looks up the
  * array's device address (with that device current); make that first call
  * before any stream capture; the address does not survive a cudaDeviceReset.
- * Every call uses the same array and clears the part it needs, so calls that
- * overlap on the GPU (on different streams, or from different threads) race:
- * serialise them on one stream.  Inputs, outputs and results are as for
- * sr_exclusive_scan_i32 (timeouts included, reported by sr_scan_status);
+ * Every call uses the same array, so calls that overlap on the GPU (on
+ * different streams, or from different threads) race: serialise them on one
+ * stream.  Inputs, outputs and results are as for sr_exclusive_scan_i32;
  * asynchronous on `stream`. */
 #define SR_NOALLOC_SCAN_MAX_N (1ll << 24)
 #define SR_NOALLOC_SCAN_SCRATCH_BYTES (4104u * 8u)
 sr_status sr_exclusive_scan_i32_noalloc(const int32_t* d_in, int32_t* d_out, int64_t n, void* stream);
 
-/* Waits for `stream`, then reports whether a look-back wait of a standalone
- * scan (sr_exclusive_scan_i32 or sr_exclusive_scan_i32_noalloc) on the
- * current device gave up since the last call: SR_ERR_TIMEOUT if one did
- * (that scan's output is wrong), else SR_OK.  It clears the report.  Scans
+/* Waits for `stream`, gives back the pool memory that sr_exclusive_scan_i32
+ * keeps on the current device, and reports whether a wait of a standalone
+ * scan there gave up since the last call: SR_ERR_TIMEOUT if one did (that
+ * scan's output is wrong), else SR_OK.  (sr_exclusive_scan_i32 and its
+ * allocation-free form hold no waits; sr_debug_scan_without_first_tile's
+ * single-pass scan does.)  It clears the report.  Scans
  * still running on other streams are reported by a later call.  The
  * reference's scan has no wait to give up (naive_scan.comp runs in one
  * workgroup), so this has no counterpart there.  Allocates nothing. */

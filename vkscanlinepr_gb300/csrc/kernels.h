@@ -132,12 +132,16 @@ void launch_fragment(const GeomArgs& g, const int2* rec, int64_t n_cap, const ui
                      uint8_t* wnp, const DebugOut& dbg, cudaStream_t st);
 
 // ---- scan.cu
-// Exclusive scan of n int32 values into out[0..n] (out[n] = total), single
-// pass with decoupled look-back.  in and out may alias.  tile_status must
-// hold scan_status_words(n) zeroed uint64 words.
-size_t scan_status_words(int64_t n);
-void launch_exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, uint64_t* tile_status,
-                               uint32_t* tile_counter, uint32_t* status, cudaStream_t st);
+// Exclusive scan of n int32 values into out[0..n] (out[n] = total).  in and
+// out may alias.  scratch: scan_scratch_bytes(n) bytes (0 for short inputs),
+// no need to clear them.
+size_t scan_scratch_bytes(int64_t n);
+void launch_scan_i32(const int32_t* in, int32_t* out, int64_t n, void* scratch, cudaStream_t st);
+// The same in a single pass with decoupled look-back (n > 0), as the frame's
+// kernels scan: tile_status holds lookback_scan_words(n) zeroed words.
+size_t lookback_scan_words(int64_t n);
+void launch_lookback_scan_i32(const int32_t* in, int32_t* out, int64_t n, uint64_t* tile_status,
+                              uint32_t* tile_counter, uint32_t* status, cudaStream_t st);
 
 // ---- sort.cu  (onesweep LSD radix sort, 8-bit digits)
 struct SortPlan {

@@ -1,7 +1,7 @@
 // noalloc.cu — the exclusive scan for callers that cannot allocate device
 // memory.
 //
-// sr_exclusive_scan_i32 takes its look-back scratch from cudaMallocAsync.
+// sr_exclusive_scan_i32 takes its scratch from a memory pool.
 // Some callers cannot allow that: a host that hands all device memory to
 // its own allocator or runs under a hard memory budget forbids third-party
 // allocations, and a frame loop with a fixed latency budget cannot risk an
@@ -22,8 +22,7 @@ sr_status report_error(sr_status s, const char* msg);   // api.cu
 
 namespace {
 
-// Look-back words for the largest scan, then the tile counter
-// (scan_status_words(n) + 1 words of 8 bytes, with a few to spare).
+// More than any scan's scratch (scan_scratch_bytes).
 constexpr size_t kNoallocWords = SR_NOALLOC_SCAN_SCRATCH_BYTES / sizeof(uint64_t);
 
 static __device__ __align__(256) uint64_t g_noalloc_scan_scratch[kNoallocWords];
@@ -73,21 +72,11 @@ extern "C" sr_status sr_exclusive_scan_i32_noalloc(const int32_t* d_in, int32_t*
     uint32_t* status = nullptr;
     sr_status s = scratch_on_current_device(&scratch, &status);
     if (s != SR_OK) return s;
-    cudaError_t e;
-    if (n == 0) {
-        e = cudaMemsetAsync(d_out, 0, sizeof(int32_t), st);
-        return e == cudaSuccess ? SR_OK : sr::report_error(SR_ERR_CUDA, cudaGetErrorString(e));
-    }
-    const size_t words = sr::scan_status_words(n) + 1;
-    if (words > kNoallocWords) return sr::report_error(SR_ERR_INTERNAL, "scan scratch too small");
-    // the previous call's look-back words and tile counter stay in the
-    // array: clear the part this call uses.  A look-back that gives up sets
-    // a bit in the status word, which sr_scan_status reports.
-    e = cudaMemsetAsync(scratch, 0, words * sizeof(uint64_t), st);
-    if (e != cudaSuccess) return sr::report_error(SR_ERR_CUDA, cudaGetErrorString(e));
-    uint32_t* counter = reinterpret_cast<uint32_t*>(scratch + words - 1);
-    sr::launch_exclusive_scan_i32(d_in, d_out, n, scratch, counter, status, st);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return sr::report_error(SR_ERR_CUDA, cudaGetErrorString(e));
-    return SR_OK;
+    // the sums of the previous call stay in the array; a scan writes what it
+    // reads of it
+    if (sr::scan_scratch_bytes(n) > sizeof(uint64_t) * kNoallocWords)
+        return sr::report_error(SR_ERR_INTERNAL, "scan scratch too small");
+    sr::launch_scan_i32(d_in, d_out, n, scratch, st);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? SR_OK : sr::report_error(SR_ERR_CUDA, cudaGetErrorString(e));
 }

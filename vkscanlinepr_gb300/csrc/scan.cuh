@@ -36,7 +36,9 @@ SR_DEV int32_t warp_incl_scan(int32_t v) {
 }
 
 // Warp-cooperative look-back over 64-bit tile words (flag in bits 62-63,
-// value in bits 0-31).  Returns the sum of all predecessors of `tile`.
+// value in bits 0-31).  Returns the sum of all predecessors of `tile`.  (Steps
+// over four windows of 32 words were slower: the polls of the CTAs that wait
+// slow each other down.)
 SR_DEV int32_t lookback_i32(uint64_t* tstat, uint32_t tile, uint32_t* status, uint32_t spin_limit) {
     const uint32_t lane = lane_id();
     int32_t excl = 0;
@@ -69,10 +71,11 @@ SR_DEV int32_t lookback_i32(uint64_t* tstat, uint32_t tile, uint32_t* status, ui
 // Exclusive prefix of one value per thread over all tiles (tile ids from a
 // counter, so every predecessor is running or done): the CTA's own scan, then
 // the look-back.  s_warp: THREADS / 32 + 1 words.  Every thread gets its
-// prefix; *tile_total, the sum up to and including this tile.
+// prefix; *tile_total, the sum up to and including this tile.  tstat NULL: the
+// only tile, starting from `carry`.
 template <int THREADS>
 SR_DEV int32_t scan_thread_values(int32_t v, uint32_t tile, uint64_t* tstat, uint32_t* status, uint32_t spin_limit,
-                                  int32_t* s_warp, int32_t* tile_total) {
+                                  int32_t* s_warp, int32_t* tile_total, int32_t carry = 0) {
     constexpr int kWarps = THREADS / 32;
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const int32_t incl = warp_incl_scan(v);
@@ -82,8 +85,8 @@ SR_DEV int32_t scan_thread_values(int32_t v, uint32_t tile, uint64_t* tstat, uin
         const int32_t w = lane < kWarps ? s_warp[lane] : 0;
         const int32_t wi = warp_incl_scan(w);
         const int32_t agg = __shfl_sync(0xFFFFFFFFu, wi, kWarps - 1);
-        if (lane == 0) st_relaxed_u64(&tstat[tile], (tile == 0 ? kScanFlagP : kScanFlagA) | (uint32_t)agg);
-        int32_t excl = 0;
+        if (tstat && lane == 0) st_relaxed_u64(&tstat[tile], (tile == 0 ? kScanFlagP : kScanFlagA) | (uint32_t)agg);
+        int32_t excl = carry;
         if (tile > 0) {
             excl = lookback_i32(tstat, tile, status, spin_limit);
             if (lane == 0) st_relaxed_u64(&tstat[tile], kScanFlagP | (uint32_t)wadd(excl, agg));
@@ -96,30 +99,16 @@ SR_DEV int32_t scan_thread_values(int32_t v, uint32_t tile, uint64_t* tstat, uin
     return wadd(s_warp[warp], wadd(incl, -v));
 }
 
-// One tile of the exclusive scan of in[0, n) into out[0, n]: THREADS x 4 x
-// ROWS values.  A warp owns 128 x ROWS consecutive values and reads a row of
-// 128 at a time, four neighbouring values a lane, so loads and stores are
-// whole lines.  Returns true in the tile that holds the end (it has written
-// out[n]).  in and out may alias.
+// The tile's values in registers (row r of a warp: 128 consecutive values,
+// four neighbouring ones a lane), scanned into out.  Returns true in the tile
+// that holds the end (it has written out[n]).
 template <int ROWS, int THREADS>
-SR_DEV bool scan_tile_i32(const int32_t* in, int32_t* out, int64_t n, uint32_t tile, uint64_t* tstat,
-                          uint32_t* status, uint32_t spin_limit, int32_t* s_warp, int32_t* total) {
+SR_DEV bool scan_tile_values(const int4 (&v)[ROWS], int32_t* out, int64_t n, uint32_t tile, uint64_t* tstat,
+                             uint32_t* status, uint32_t spin_limit, int32_t* s_warp, int32_t* total,
+                             int32_t carry = 0) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const int64_t base = ((int64_t)tile * (THREADS / 32) + warp) * (128 * ROWS) + lane * 4;
-    const bool in4 = (reinterpret_cast<uintptr_t>(in) & 15) == 0, out4 = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-    int4 v[ROWS];
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-        const int64_t i = base + r * 128;
-        if (in4 && i + 4 <= n) {
-            v[r] = *reinterpret_cast<const int4*>(in + i);
-        } else {
-            v[r].x = i < n ? in[i] : 0;
-            v[r].y = i + 1 < n ? in[i + 1] : 0;
-            v[r].z = i + 2 < n ? in[i + 2] : 0;
-            v[r].w = i + 3 < n ? in[i + 3] : 0;
-        }
-    }
+    const bool out4 = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     // the lane's prefix in each row, and the warp's sum
     int32_t ex[ROWS];
     int32_t run = 0;
@@ -132,7 +121,7 @@ SR_DEV bool scan_tile_i32(const int32_t* in, int32_t* out, int64_t n, uint32_t t
     }
     // the warps' sums: lane 0 brings its warp's into the CTA's scan, whose
     // value for lane 0 is what comes before the warp
-    int32_t before = scan_thread_values<THREADS>(lane == 0 ? run : 0, tile, tstat, status, spin_limit, s_warp, total);
+    int32_t before = scan_thread_values<THREADS>(lane == 0 ? run : 0, tile, tstat, status, spin_limit, s_warp, total, carry);
     before = __shfl_sync(0xFFFFFFFFu, before, 0);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
@@ -154,6 +143,37 @@ SR_DEV bool scan_tile_i32(const int32_t* in, int32_t* out, int64_t n, uint32_t t
     const bool last = (int64_t)(tile + 1) * (THREADS * 4 * ROWS) >= n;
     if (last && threadIdx.x == 0) out[n] = *total;
     return last;
+}
+
+// The tile's values from memory: whole lines, zeros past n.
+template <int ROWS, int THREADS>
+SR_DEV void load_tile_values(int4 (&v)[ROWS], const int32_t* in, int64_t n, uint32_t tile) {
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const int64_t base = ((int64_t)tile * (THREADS / 32) + warp) * (128 * ROWS) + lane * 4;
+    const bool in4 = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        const int64_t i = base + r * 128;
+        if (in4 && i + 4 <= n) {
+            v[r] = *reinterpret_cast<const int4*>(in + i);
+        } else {
+            v[r].x = i < n ? in[i] : 0;
+            v[r].y = i + 1 < n ? in[i + 1] : 0;
+            v[r].z = i + 2 < n ? in[i + 2] : 0;
+            v[r].w = i + 3 < n ? in[i + 3] : 0;
+        }
+    }
+}
+
+// One tile of the exclusive scan of in[0, n) into out[0, n]: THREADS x 4 x
+// ROWS values.  Returns true in the tile that holds the end.  in and out may
+// alias.
+template <int ROWS, int THREADS>
+SR_DEV bool scan_tile_i32(const int32_t* in, int32_t* out, int64_t n, uint32_t tile, uint64_t* tstat,
+                          uint32_t* status, uint32_t spin_limit, int32_t* s_warp, int32_t* total, int32_t carry = 0) {
+    int4 v[ROWS];
+    load_tile_values<ROWS, THREADS>(v, in, n, tile);
+    return scan_tile_values<ROWS, THREADS>(v, out, n, tile, tstat, status, spin_limit, s_warp, total, carry);
 }
 
 }  // namespace sr
