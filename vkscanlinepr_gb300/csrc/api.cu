@@ -304,7 +304,7 @@ struct Pipeline {
     // pass the control block, path_visible and the offset scan's words; after
     // it the tables sized by the capacity (back_layout)
     DevBuf ctl, zeroed;
-    DevBuf cbuf, rec, keys, keys_alt, wnp, skeys, svals, vals_alt, sort_scratch, wind_sums, draw, draw_row;
+    DevBuf cbuf, rec, keys, keys_alt, wnp, skeys, svals, vals_alt, sort_scratch, wind_sums, draw, draw_row, draw_list;
     DevBuf rkeys, rvals, rkeys_alt, rvals_alt, row_sort_scratch, row_start, image;
     DevBuf d_fkey, d_fwn, d_fleft, d_wscan, d_fflag, d_sflag, d_skey;
     // learned sizing: per-path curve ranges, draw counters, features,
@@ -334,6 +334,15 @@ struct Pipeline {
     // a frame's records carry no flag bits: they are merged again with them
     // when they are dumped, with the arguments of the frame
     bool rec_flags = false;
+    // a frame paints runs; its draw list is written when it is dumped, from
+    // the frame's sorted records and its scene's fill arrays, which the next
+    // scene's do not overwrite (fill_kept).  A rendered draw list is its own.
+    enum class DrawList { kNone, kWritten, kFromFrame, kCallers } draw_state = DrawList::kNone;
+    sr::WindArgs frame_wind{};
+    size_t frame_wind_at = 0;   // its look-back words in `zeroed`
+    int frame_wind_items = 8;
+    DevBuf fill_rule_kept, fill_info_kept;
+    bool fill_in_use = false;   // the frame's fill arrays are fill_rule and fill_info
     sr::GeomArgs frame_geom{};
     bool last_segsort = false;   // the last frame sorted its records per path (segsort.cu)
     // profiling
@@ -345,9 +354,9 @@ struct Pipeline {
         DevBuf* all[] = {&pos, &pos_path, &curve_pos, &curve_type, &curve_path, &fill_rule, &fill_info, &path_scene,
                          &scenes_d, &cta_base_d, &tpos, &curve_end, &path_begin, &cut, &count, &offs, &ctl, &zeroed,
                          &pieces, &chain_lists, &cbuf, &rec, &keys, &keys_alt,
-                         &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_sums, &draw, &draw_row,
+                         &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_sums, &draw, &draw_row, &draw_list,
                          &rkeys, &rvals, &rkeys_alt, &rvals_alt, &row_sort_scratch, &row_start, &image, &d_fkey, &d_fwn, &d_fleft, &d_wscan, &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw,
-                         &feats, &preds, &allot, &plan_tot, &judge_out, &seg_tiles, &cta_narrow_d, &paints_d, &aa_acc};
+                         &feats, &preds, &allot, &plan_tot, &judge_out, &seg_tiles, &cta_narrow_d, &paints_d, &aa_acc, &fill_rule_kept, &fill_info_kept};
         for (DevBuf* b : all) release(*b);
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
@@ -528,6 +537,11 @@ struct Pipeline {
     // pinned).
     sr_status upload_single(const sr_scene_view* s, int32_t W, int32_t H, const float* mvp) {
         CUDA_TRY(cudaSetDevice(device));
+        if (fill_in_use) {   // for a dump of the last frame's draw list
+            std::swap(fill_rule, fill_rule_kept);
+            std::swap(fill_info, fill_info_kept);
+            fill_in_use = false;
+        }
         S = 1;
         V = s->n_points;
         C = s->n_curves;
@@ -799,12 +813,12 @@ struct Pipeline {
                                &path_scene, &scenes_d, &cta_base_d, &tpos, &curve_end, &path_begin, &cut, &count, &offs,
                                &ctl, &zeroed, &pieces, &chain_lists, &cbuf,
                                &rec, &keys, &keys_alt, &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_sums,
-                               &draw, &draw_row, &rkeys, &rvals, &rkeys_alt, &rvals_alt,
+                               &draw, &draw_row, &draw_list, &rkeys, &rvals, &rkeys_alt, &rvals_alt,
                                &row_sort_scratch, &row_start, &image, &d_fkey,
                                &d_fwn, &d_fleft,
                                &d_wscan,
                                &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw, &feats, &preds, &allot,
-                               &plan_tot, &judge_out, &seg_tiles, &cta_narrow_d};
+                               &plan_tot, &judge_out, &seg_tiles, &cta_narrow_d, &fill_rule_kept, &fill_info_kept};
         uint64_t t = 0;
         for (const DevBuf* b : all) t += b->cap;
         return t;
@@ -933,6 +947,11 @@ struct Pipeline {
         wa.cut_segs = cut_segs();
         wa.row_count = reinterpret_cast<uint32_t*>(zero + at.row_count);
         wa.row_px = reinterpret_cast<unsigned long long*>(zero + at.row_px);
+        frame_wind = wa;
+        frame_wind_at = at.wind;
+        frame_wind_items = tune.wind_items;
+        draw_state = DrawList::kFromFrame;
+        fill_in_use = true;
         mark(ST_WINDING, false);
         launch_winding_emit(wa, tune.wind_items, reinterpret_cast<uint64_t*>(zero + at.wind), wind_sums.as<uint64_t>(),
                             ctlp + CTL_WIND_COUNTERS, status, st);
@@ -981,6 +1000,27 @@ struct Pipeline {
                          ctl.as<uint32_t>() + CTL_STATUS, nullptr);
         CUDA_TRY(cudaGetLastError());
         rec_flags = true;
+        return SR_OK;
+    }
+
+    // The last frame's draw list in draw_list (or a caller's own in draw).
+    sr_status write_draw_list(const void** src) {
+        *src = draw_state == DrawList::kCallers ? draw.p : draw_list.p;
+        if (draw_state != DrawList::kFromFrame || last_O <= 0) return SR_OK;
+        CUDA_TRY(ensure(draw_list, sizeof(int4) * (size_t)last_O));
+        *src = draw_list.p;
+        sr::WindArgs a = frame_wind;
+        a.draw = draw_list.as<int4>();
+        a.draw_capacity = last_O;
+        a.dbg_wscan = a.dbg_fflag = a.dbg_sflag = a.dbg_skey = nullptr;
+        uint64_t* words = reinterpret_cast<uint64_t*>(zeroed.as<char>() + frame_wind_at);
+        uint32_t* ctlp = ctl.as<uint32_t>();
+        CUDA_TRY(cudaMemsetAsync(words, 0, sizeof(uint64_t) * sr::winding_status_words(a.n, frame_wind_items), nullptr));
+        CUDA_TRY(cudaMemsetAsync(ctlp + CTL_WIND_COUNTERS, 0, sizeof(uint32_t), nullptr));
+        sr::launch_draw_list(a, frame_wind_items, words, wind_sums.as<uint64_t>(), ctlp + CTL_WIND_COUNTERS,
+                             ctlp + CTL_STATUS, nullptr);
+        CUDA_TRY(cudaGetLastError());
+        draw_state = DrawList::kWritten;
         return SR_OK;
     }
 
@@ -1360,6 +1400,7 @@ sr_status sr_render_draw_list(sr_ctx* c, const int32_t* records, int64_t n, void
         int32_t y = records[4 * i] >> 16;
         row[(size_t)i] = (y < 0 || y >= c->H) ? (uint32_t)rows : (uint32_t)(y / p.F);
     }
+    p.draw_state = Pipeline::DrawList::kCallers;
     CUDA_TRY(ensure(p.draw, sizeof(int4) * n1));
     CUDA_TRY(ensure(p.draw_row, sizeof(uint32_t) * n1));
     CUDA_TRY(ensure(p.rkeys, sizeof(uint32_t) * n1));
@@ -1452,9 +1493,8 @@ sr_status sr_debug_dump(sr_ctx* c, int stage, void* dst, size_t* bytes) {
     if (*bytes < need) return fail(SR_ERR_INVALID_ARG, "buffer of %zu bytes, need %zu", *bytes, need);
     if (need && !src) return fail(SR_ERR_INVALID_ARG, "stage %d not available", stage);
     CUDA_TRY(cudaSetDevice(p.device));
-    if (stage == SR_STAGE_INTERSECTION && need) {
-        SR_TRY(p.merge_records());
-    }
+    if (stage == SR_STAGE_INTERSECTION && need) SR_TRY(p.merge_records());
+    if (stage == SR_STAGE_DRAW_LIST && need) SR_TRY(p.write_draw_list(&src));
     if (need) CUDA_TRY(cudaMemcpy(dst, src, need, cudaMemcpyDeviceToHost));
     *bytes = need;
     return SR_OK;

@@ -221,20 +221,20 @@ struct WindArgs {
     int32_t pixel_mode;
     KeyLayout L;
     SceneTable st;
-    int4* draw;                     // [capacity] draw records
+    int4* draw;                     // [capacity] paint runs {y << 16 | x, width, fill_info, 0}
     int64_t draw_capacity;
-    uint32_t* draw_row;             // [capacity] global cell row of each draw record
-    uint64_t* totals;               // [2] merged fragments, spans
-    uint32_t* n_draw;               // [1] merged fragments + spans
+    uint32_t* draw_row;             // [capacity] global cell row of each paint run
+    uint64_t* totals;               // [2] merged fragments, spans; zeroed before
+    uint32_t* n_draw;               // [1] paint runs
     uint32_t* path_draw;            // [P] draw records per path (NULL unless labelling)
-    // [cut_rows][cut_segs]: 1 + the last draw index of a span that covers a
+    // [cut_rows][cut_segs]: 1 + the last index of a run that covers a
     // resolve segment (kResolveSeg pixels) entirely and leaves nothing of
-    // what was under it (opaque in pixel mode, any span in reference mode);
-    // zeroed before the emit, NULL to skip
+    // what was under it (opaque in pixel mode, any run in reference mode);
+    // zeroed before the emit
     uint32_t* seg_cut;
     uint32_t cut_rows, cut_segs;
-    uint32_t* row_count;            // [cut_rows] draw records per global cell row (zeroed before), or NULL
-    unsigned long long* row_px;     // [cut_rows] pixels of a row's records (widths summed; zeroed before), or NULL
+    uint32_t* row_count;            // [cut_rows] paint runs per global cell row (zeroed before)
+    unsigned long long* row_px;     // [cut_rows] pixels of a row's runs (widths summed; zeroed before)
     // parity dumps (NULL in production)
     int32_t* dbg_wscan;             // [N+1]
     int32_t* dbg_fflag;             // [N]
@@ -248,6 +248,11 @@ size_t winding_status_words(int64_t n, int items = 8);
 size_t winding_tile_words(int64_t n, int items = 8);
 void launch_winding_emit(const WindArgs& a, int items, uint64_t* tile_status, uint64_t* tile_sums, uint32_t* counters,
                          uint32_t* status, cudaStream_t st);
+// The reference's draw list (for a read-back), from the same sorted records
+// and tile prefixes: draw records into a.draw; tile_status and counters[0]
+// zeroed before.
+void launch_draw_list(const WindArgs& a, int items, uint64_t* tile_status, const uint64_t* tile_sums,
+                      uint32_t* counters, uint32_t* status, cudaStream_t st);
 
 // ---- resolve.cu
 // A gradient paint ready for the resolve (built on the host from an

@@ -89,6 +89,10 @@ SR_DEV uint64_t lookback(uint64_t* tstat, uint32_t tile, uint32_t* status, uint3
     return excl;
 }
 
+// What the emit writes.  A frame paints paint runs; the reference's draw list
+// is written when it is read back.
+enum EmitKind { kEmitRuns, kEmitDraws };
+
 // A tile's draw records in output order, as items of shared memory: the
 // record's index in the tile (bits 13..), a span bit (12) and, for a merged
 // fragment, its index among the tile's fragments (0..11).  A record gives at
@@ -96,11 +100,12 @@ SR_DEV uint64_t lookback(uint64_t* tstat, uint32_t tile, uint32_t* status, uint3
 constexpr uint32_t kItemSpan = 1u << 12;
 constexpr int kItemRecShift = 13;
 
-template <int ITEMS, int THREADS> struct Smem {
+template <int ITEMS, int THREADS, EmitKind KIND> struct Smem {
     uint32_t tile;
     int32_t warpA[THREADS / 32];
     int32_t warpAf[THREADS / 32];
     uint32_t warpB[THREADS / 32];
+    uint32_t warpC[THREADS / 32];                   // fragments << 16 | spans of a warp
     uint64_t prefixB;
     uint32_t count;
     uint32_t lo_prev;                               // low key half of the record before the tile
@@ -111,7 +116,10 @@ template <int ITEMS, int THREADS> struct Smem {
     uint32_t run_all[THREADS];
     uint64_t next_key;                              // the record after the tile, ~0 if none
     int32_t next_c;                                 // its centre part
-    uint32_t items[2 * THREADS * ITEMS];
+    // draw records: the items.  Paint runs: the j-th start (record << 16 |
+    // first cell) in items[j], the j-th end (cell after the last) in ends[j]
+    uint32_t items[(KIND == kEmitDraws ? 2 : 1) * THREADS * ITEMS];
+    uint16_t ends[KIND == kEmitDraws ? 1 : THREADS * ITEMS];
     __align__(16) uint32_t lo[THREADS * ITEMS];     // low key half (row rank, x + 1) of each record
     __align__(16) uint32_t paint[THREADS * ITEMS];  // fill_info of each record's path
 };
@@ -357,15 +365,29 @@ __global__ void __launch_bounds__(THREADS) k_winding_reduce(const WindArgs a, ui
 // registers.  The tile's draw records are contiguous in the output, so they
 // are listed as items in shared memory and written an item a thread:
 // consecutive threads write consecutive records.
-template <int ITEMS, int THREADS>
-__global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
+//
+// Paint runs.  The draw records of one path in one row paint disjoint cells in
+// one paint: a merged fragment its cell, a span the cells between two.  Where
+// they touch, one run stands for all of them: [first cell, cell after the
+// last) of a row.  A simple shape's row is one run instead of a fragment, a
+// fragment and a span, so the row sort and the resolve have a third of the
+// records to order and to paint.  In a row's order the painted cells and
+// gaps come as alternating starts and ends of runs, so the j-th start of a
+// tile and the j-th end belong together and are listed independently, each at
+// its own rank.  Runs are cut where a warp's records end.  On the 4096^2
+// frame 15.4 M draw records became 4.1 M runs: the row sort went from 0.246
+// to 0.107 ms and the resolve from 0.256 to 0.158, the emit from 0.43 to 0.465
+// (64 registers and 4 CTAs an SM; 48 and 5 spill: 0.500); in a batch of 64
+// uneven scenes the resolve went from 1.53 to 0.70 ms.
+template <int ITEMS, int THREADS, EmitKind KIND>
+__global__ void __launch_bounds__(THREADS, 4) k_winding_emit(const WindArgs a,
                                                               const int32_t* __restrict__ tile_in,
                                                               uint64_t* __restrict__ tstatB, uint32_t* counter,
                                                               uint32_t* status, uint32_t spin_limit) {
     constexpr int kTile = THREADS * ITEMS;
     static_assert(ITEMS % 2 == 0 && ITEMS <= 8, "records per thread");
     static_assert(kTile <= 4096, "record and fragment index of an item");
-    __shared__ Smem<ITEMS, THREADS> S;
+    __shared__ Smem<ITEMS, THREADS, KIND> S;
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) S.tile = atomicAdd(counter, 1u);
     __syncthreads();
@@ -377,8 +399,6 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
         // launched for the capacity: nothing here; an empty frame still
         // reports its (zero) totals
         if (n == 0 && tile == 0 && threadIdx.x == 0) {
-            a.totals[0] = 0;
-            a.totals[1] = 0;
             *a.n_draw = 0;
             if (a.dbg_wscan) a.dbg_wscan[0] = 0;
         }
@@ -507,7 +527,7 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
     }
 
     // ---- flags (mark_merged_fragment_and_span.comp:22-93)
-    uint32_t ffm = 0, sfm = 0;
+    uint32_t ffm = 0, sfm = 0, hdm = 0;   // fragments, spans, first records of a cell
     const int32_t F = a.F;
     // on the canvas: a row of it, and 0 <= x = (xo - 1) F < W, i.e. 1 <= xo <= ceil(W / F)
     const uint32_t xo_max1 = (uint32_t)div_F(a.W + F - 1, F);
@@ -523,7 +543,8 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
         const uint32_t xo_max = multi ? (uint32_t)div_F(scene_of_path(a.st, p1).W + F - 1, F) : xo_max1;
         const bool on = rank1 != off_rank && xo1 >= 1u && xo1 <= xo_max;
         const bool first = ibase + k == 0;
-        bool ff = on && (first || p0 != p1 || l0 != l1);
+        const bool head = first || p0 != p1 || l0 != l1;
+        bool ff = on && head;
         bool sf = !first && p0 == p1 && (l0 >> xbits) == rank1 && (l0 & xmask) + 1u < xo1;
         if (sf || (ff && a.pixel_mode)) {
             if (p1 != rule_path) {
@@ -544,6 +565,8 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
         }
         ffm |= (ff ? 1u : 0u) << k;
         sfm |= (sf ? 1u : 0u) << k;
+        hdm |= (head ? 1u : 0u) << k;
+        if (KIND == kEmitRuns && a.path_draw && (ff || sf)) atomicAdd(&a.path_draw[p1], (ff ? 1u : 0u) + (sf ? 1u : 0u));
         if (a.dbg_wscan) {
             const int64_t i = ibase + k;
             a.dbg_wscan[i] = wscan;
@@ -553,9 +576,48 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
         }
     }
 
-    // ---- output slots.  Within the CTA the counts are packed 16:16 (a tile
-    // has at most 2 x 2048 outputs); across tiles 31:31 with a look-back.
-    const uint32_t bsum = ((uint32_t)__popc(ffm) << 16) | (uint32_t)__popc(sfm);
+    // ---- output slots.  Within the CTA the counts are packed 16:16 (starts
+    // and ends of runs, or fragments and spans: a tile has at most 2048 of
+    // each); across tiles a look-back, over the runs, or over fragments and
+    // spans packed 31:31.
+    uint32_t bsum = ((uint32_t)__popc(ffm) << 16) | (uint32_t)__popc(sfm);
+    const uint32_t drawn = __reduce_add_sync(0xFFFFFFFFu, bsum);
+    if (lane == 0) S.warpC[warp] = drawn;
+    // runs: is the cell before this thread's first head painted?  That of the
+    // last head of a lane before, of this warp
+    bool painted_in = false;
+    const auto run_events = [&](bool painted, auto&& start, auto&& end) {
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            if (!((hdm >> k) & 1u)) continue;
+            const uint32_t p1 = kp[k], l1 = kl[k];
+            const uint32_t p0 = k == 0 ? pprev : kp[k - 1], l0 = k == 0 ? lprev : kl[k - 1];
+            const uint32_t x0 = l0 & xmask, x1 = l1 & xmask;   // cells are x - 1
+            const bool span = (sfm >> k) & 1u, cell = (ffm >> k) & 1u;
+            const bool joined = painted && p0 == p1 && (l0 >> xbits) == (l1 >> xbits) && (span || (cell && x1 == x0 + 1u));
+            if (painted && !joined) end(x0);
+            if (span) {
+                if (!joined) start(k, x0);
+                if (!cell) end(x1 - 1u);
+            } else if (cell && !joined) {
+                start(k, x1 - 1u);
+            }
+            painted = cell;
+        }
+        return painted;
+    };
+    if (KIND == kEmitRuns) {
+        const uint32_t hm = __ballot_sync(0xFFFFFFFFu, hdm != 0);
+        const uint32_t pm = __ballot_sync(0xFFFFFFFFu, hdm != 0 && ((ffm >> (31 - __clz(hdm | 1u))) & 1u));
+        const uint32_t vm = __ballot_sync(0xFFFFFFFFu, nvalid > 0);
+        const uint32_t below = hm & lanemask_lt();
+        painted_in = below && ((pm >> (31 - __clz(below))) & 1u);
+        uint32_t ns = 0, ne = 0;
+        const bool painted = run_events(painted_in, [&](int, uint32_t) { ++ns; }, [&](uint32_t) { ++ne; });
+        // the warp's last records: a run does not go on into the next warp
+        if (painted && vm && lane == 31u - (uint32_t)__clz(vm)) ++ne;
+        bsum = (ns << 16) | ne;
+    }
     const uint32_t inclB = warp_incl<uint32_t>(bsum);
     if (lane == 31) S.warpB[warp] = inclB;
     __syncthreads();
@@ -564,8 +626,17 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
         const uint32_t wi = warp_incl<uint32_t>(w);
         if (lane < THREADS / 32) S.warpB[lane] = wi - w;
         const uint32_t agg16 = __shfl_sync(0xFFFFFFFFu, wi, THREADS / 32 - 1);
-        const uint64_t aggB = ((uint64_t)(agg16 >> 16) << kFragShift) | (uint64_t)(agg16 & 0xFFFFu);
+        const uint64_t aggB = KIND == kEmitRuns
+                                  ? (uint64_t)(agg16 >> 16)
+                                  : ((uint64_t)(agg16 >> 16) << kFragShift) | (uint64_t)(agg16 & 0xFFFFu);
         if (lane == 0) st_relaxed_u64(&tstatB[tile], (tile == 0 ? kFlagP : kFlagA) | aggB);
+        if (KIND == kEmitRuns) {
+            const uint32_t d = __reduce_add_sync(0xFFFFFFFFu, lane < THREADS / 32 ? S.warpC[lane] : 0u);
+            if (lane < 2) {
+                const uint32_t v = lane ? d & 0xFFFFu : d >> 16;
+                if (v) atomicAdd(reinterpret_cast<unsigned long long*>(&a.totals[lane]), (unsigned long long)v);
+            }
+        }
         uint64_t excl = 0;
         if (tile > 0) {
             excl = lookback(tstatB, tile, status, spin_limit);
@@ -573,106 +644,114 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_emit(const WindArgs a,
         }
         if (lane == 0) {
             S.prefixB = excl;
-            S.count = (agg16 >> 16) + (agg16 & 0xFFFFu);
-            if (tile == num_tiles - 1) {
-                const uint64_t tot = excl + aggB;
-                a.totals[0] = tot >> kFragShift;
-                a.totals[1] = tot & kSpanMask;
-                *a.n_draw = (uint32_t)((tot >> kFragShift) + (tot & kSpanMask));
-            }
+            S.count = KIND == kEmitRuns ? agg16 >> 16 : (agg16 >> 16) + (agg16 & 0xFFFFu);
+            if (KIND == kEmitRuns && tile == num_tiles - 1) *a.n_draw = (uint32_t)(excl + aggB);
         }
     }
     __syncthreads();
-    // this thread's items: in record order, a record's fragment before its span
+    // this thread's items: starts and ends at their ranks, or in record order
+    // a record's fragment before its span
     {
         const uint32_t l0 = S.warpB[warp] + (inclB - bsum);
-        uint32_t lf = l0 >> 16, slot = lf + (l0 & 0xFFFFu);
-        if (ffm | sfm) {
+        if (KIND == kEmitRuns) {
+            uint32_t rs = l0 >> 16, re = l0 & 0xFFFFu;
+            const uint32_t re_end = re + (bsum & 0xFFFFu);
+            run_events(painted_in,
+                       [&](int k, uint32_t x) { S.items[rs++] = ((uint32_t)(threadIdx.x * ITEMS + k) << 16) | x; },
+                       [&](uint32_t x) { S.ends[re++] = (uint16_t)x; });
+            // the warp's last end: the cell of its last record
+            if (re < re_end) S.ends[re] = (uint16_t)(S.lo[threadIdx.x * ITEMS + nvalid - 1] & xmask);
+        } else {
+            uint32_t lf = l0 >> 16, slot = lf + (l0 & 0xFFFFu);
+            if (ffm | sfm) {
 #pragma unroll
-            for (int k = 0; k < ITEMS; ++k) {
-                const uint32_t rec = (threadIdx.x * ITEMS + k) << kItemRecShift;
-                if ((ffm >> k) & 1u) S.items[slot++] = rec | lf++;
-                if ((sfm >> k) & 1u) S.items[slot++] = rec | kItemSpan;
+                for (int k = 0; k < ITEMS; ++k) {
+                    const uint32_t rec = (threadIdx.x * ITEMS + k) << kItemRecShift;
+                    if ((ffm >> k) & 1u) S.items[slot++] = rec | lf++;
+                    if ((sfm >> k) & 1u) S.items[slot++] = rec | kItemSpan;
+                }
             }
         }
     }
     __syncthreads();
 
-    // ---- emit draw records (gen_merged_fragment_and_span.comp:33-103), an
-    // item a thread, from the key halves and paint staged in shared memory.
-    // An emitted record's cell is on the canvas: y = yy F with yy its row
-    // (rank Hy is row 0, rank r < Hy - 1 is row r + 1), x = (xo - 1) F.  A
-    // span's left end is the cell after the record before it (same path and
-    // row: only its x bits are read).  Each record also adds to its row's record count and pixel
-    // sum (summed over the lanes of a warp that share the row), and an opaque
-    // span to the cuts of the resolve segments it covers whole.
+    // ---- output, an item a thread, from the key halves and paint staged in
+    // shared memory.  A painted record's cell is on the canvas: y = yy F with
+    // yy its row (rank Hy is row 0, rank r < Hy - 1 is row r + 1), x =
+    // (xo - 1) F.
     const uint64_t tprefix = S.prefixB;
-    const int64_t tile_first = (int64_t)((tprefix >> kFragShift) + (tprefix & kSpanMask));
-    const uint64_t frag0 = tprefix >> kFragShift;
     const uint32_t tile_cnt = S.count;
-    const bool need_path = multi || a.path_draw;
-    // every lane of a warp runs the same rounds (the row sums are warp-wide)
-    const uint32_t rounds_end = (tile_cnt + THREADS - 1) / THREADS * THREADS;
-    for (uint32_t j = threadIdx.x; j < rounds_end; j += THREADS) {
-        const bool live = j < tile_cnt;
-        uint32_t row = 0xFFFFFFFFu, written = 0, px = 0;
-        if (live) {
-            const uint32_t it = S.items[j];
-            const bool span = (it & kItemSpan) != 0;
-            const uint32_t r = it >> kItemRecShift;
-            const uint32_t l1 = S.lo[r], info = S.paint[r];
-            uint32_t path1 = 0;
-            if (need_path) {
-                path1 = (uint32_t)(key_part(a.L, a.skeys[tbase + r]) >> pshift);
-                if (path1 >= a.n_paths) path1 = 0;
-            }
-            const uint32_t rank1 = (l1 >> xbits) & rmask;
-            const int32_t yy = rank1 == (uint32_t)a.L.Hy ? 0 : (int32_t)rank1 + 1;
-            row = (multi ? scene_of_path(a.st, path1).row_base : 0u) + (uint32_t)yy;
-            const int32_t y = yy * F, x1 = ((int32_t)(l1 & xmask) - 1) * F;
-            const int64_t o = tile_first + j;
+    if (KIND == kEmitDraws) {
+        // gen_merged_fragment_and_span.comp:33-103
+        const int64_t tile_first = (int64_t)((tprefix >> kFragShift) + (tprefix & kSpanMask));
+        const uint64_t frag0 = tprefix >> kFragShift;
+        for (uint32_t j = threadIdx.x; j < tile_cnt; j += THREADS) {
+            const uint32_t it = S.items[j], r = it >> kItemRecShift;
+            const uint32_t l1 = S.lo[r], rank1 = (l1 >> xbits) & rmask;
+            const int32_t y = (rank1 == (uint32_t)a.L.Hy ? 0 : (int32_t)rank1 + 1) * F;
+            const int32_t x1 = ((int32_t)(l1 & xmask) - 1) * F;
             int4 d;
-            if (!span) {
-                d = make_int4((int32_t)((uint32_t)y << 16) | x1, F, (int32_t)info,
+            if (!(it & kItemSpan)) {
+                d = make_int4((int32_t)((uint32_t)y << 16) | x1, F, (int32_t)S.paint[r],
                               (int32_t)(frag0 + (it & (kItemSpan - 1u)) + 1u));
-                px = (uint32_t)F;
             } else {
                 // the span's left cell is the record before it, in the same
                 // path and row (a span is never record 0)
                 const uint32_t l0 = r > 0 ? S.lo[r - 1] : S.lo_prev;
                 const int32_t x0 = imax(0, wadd(((int32_t)(l0 & xmask) - 1) * F, F));
-                d = make_int4((int32_t)((uint32_t)y << 16) | x0, x1 - x0, (int32_t)info, 0);
+                d = make_int4((int32_t)((uint32_t)y << 16) | x0, x1 - x0, (int32_t)S.paint[r], 0);
+            }
+            if (tile_first + j < a.draw_capacity) a.draw[tile_first + j] = d;
+        }
+        return;
+    }
+    // Runs.  Each also adds to its row's run count and pixel sum (summed over
+    // the lanes of a warp that share the row), and an opaque one to the cuts of
+    // the resolve segments it covers whole.  Every lane of a warp runs the same
+    // rounds (the row sums are warp-wide).
+    const int64_t tile_first = (int64_t)tprefix;
+    const uint32_t rounds_end = (tile_cnt + THREADS - 1) / THREADS * THREADS;
+    for (uint32_t j = threadIdx.x; j < rounds_end; j += THREADS) {
+        uint32_t row = 0xFFFFFFFFu, px = 0;
+        bool counted = false;
+        if (j < tile_cnt) {
+            const uint32_t it = S.items[j], r = it >> 16;
+            const uint32_t l1 = S.lo[r], info = S.paint[r];
+            const uint32_t rank1 = (l1 >> xbits) & rmask;
+            const int32_t yy = rank1 == (uint32_t)a.L.Hy ? 0 : (int32_t)rank1 + 1;
+            row = (uint32_t)yy;
+            if (multi) {
+                uint32_t path1 = (uint32_t)(key_part(a.L, a.skeys[tbase + r]) >> pshift);
+                if (path1 >= a.n_paths) path1 = 0;
+                row += scene_of_path(a.st, path1).row_base;
+            }
+            const int32_t x0 = (int32_t)(it & 0xFFFFu) * F, x1 = (int32_t)S.ends[j] * F;
+            const int64_t o = tile_first + j;
+            // only runs inside the capacity are written and counted, so that
+            // the row sort and the resolve stay inside the buffers
+            if (o < a.draw_capacity) {
+                a.draw[o] = make_int4((int32_t)((uint32_t)(yy * F) << 16) | x0, x1 - x0, (int32_t)info, 0);
+                a.draw_row[o] = row;
                 px = (uint32_t)imax(x1 - x0, 0);
-                // a span that hides everything under it ends the resolve's
-                // work before it in each segment it covers whole
-                if (a.seg_cut && o < a.draw_capacity && row < a.cut_rows && (!a.pixel_mode || (info >> 24) == 255u)) {
+                counted = row < a.cut_rows;
+                // a run that hides everything under it ends the resolve's work
+                // before it in each segment it covers whole
+                if (a.seg_cut && counted && (!a.pixel_mode || (info >> 24) == 255u)) {
                     const int32_t s_hi = imin(x1 / kResolveSeg, (int32_t)a.cut_segs);
                     for (int32_t sg = (x0 + kResolveSeg - 1) / kResolveSeg; sg < s_hi; ++sg)
                         atomicMax(&a.seg_cut[(size_t)row * a.cut_segs + (uint32_t)sg], (uint32_t)o + 1u);
                 }
-            }
-            if (a.path_draw) atomicAdd(&a.path_draw[path1], 1u);
-            // only records inside the draw capacity are written and counted,
-            // so that the row sort and the resolve stay inside the buffers
-            if (o < a.draw_capacity) {
-                a.draw[o] = d;
-                a.draw_row[o] = row;
-                written = 1;
             } else {
                 set_error(status, ERR_CAPACITY);
-                px = 0;
             }
         }
-        if (a.row_count) {
-            const bool counted = written != 0 && row < a.cut_rows;
-            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, counted ? row : 0xFFFFFFFFu);
-            if (counted) {
-                const uint32_t cnt = __popc(peers);
-                const uint32_t psum = __reduce_add_sync(peers, px);
-                if (lane == (uint32_t)(__ffs(peers) - 1)) {
-                    atomicAdd(&a.row_count[row], cnt);
-                    if (a.row_px) atomicAdd(&a.row_px[row], (unsigned long long)psum);
-                }
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, counted ? row : 0xFFFFFFFFu);
+        if (counted) {
+            const uint32_t cnt = __popc(peers);
+            const uint32_t psum = __reduce_add_sync(peers, px);
+            if (lane == (uint32_t)(__ffs(peers) - 1)) {
+                atomicAdd(&a.row_count[row], cnt);
+                atomicAdd(&a.row_px[row], (unsigned long long)psum);
             }
         }
     }
@@ -692,8 +771,8 @@ template <int ITEMS, int THREADS>
 static void launch_wind(const WindArgs& a, int64_t tiles, uint64_t* sB, uint64_t* tagg, int32_t* tile_in,
                         uint32_t* counters, uint32_t* status, cudaStream_t st) {
     k_winding_reduce<ITEMS, THREADS><<<(unsigned)tiles, THREADS, 0, st>>>(a, tagg, tile_in, counters + 1);
-    k_winding_emit<ITEMS, THREADS><<<(unsigned)tiles, THREADS, 0, st>>>(a, tile_in, sB, counters, status,
-                                                                        spin_limit());
+    k_winding_emit<ITEMS, THREADS, kEmitRuns><<<(unsigned)tiles, THREADS, 0, st>>>(a, tile_in, sB, counters, status,
+                                                                                   spin_limit());
 }
 
 void launch_winding_emit(const WindArgs& a, int items, uint64_t* tile_status, uint64_t* tile_sums, uint32_t* counters,
@@ -705,6 +784,21 @@ void launch_winding_emit(const WindArgs& a, int items, uint64_t* tile_status, ui
     count_launches(2);
     if (items == 4) launch_wind<4, 256>(a, tiles, tile_status, tile_sums, tile_in, counters, status, st);
     else launch_wind<8, 256>(a, tiles, tile_status, tile_sums, tile_in, counters, status, st);
+}
+
+void launch_draw_list(const WindArgs& a, int items, uint64_t* tile_status, const uint64_t* tile_sums,
+                      uint32_t* counters, uint32_t* status, cudaStream_t st) {
+    if (a.n <= 0) return;
+    const int64_t tile = wind_tile(items);
+    const int64_t tiles = (a.n + tile - 1) / tile;
+    const int32_t* tile_in = reinterpret_cast<const int32_t*>(tile_sums + (tiles + 1));
+    count_launches(1);
+    if (items == 4)
+        k_winding_emit<4, 256, kEmitDraws><<<(unsigned)tiles, 256, 0, st>>>(a, tile_in, tile_status, counters, status,
+                                                                            spin_limit());
+    else
+        k_winding_emit<8, 256, kEmitDraws><<<(unsigned)tiles, 256, 0, st>>>(a, tile_in, tile_status, counters, status,
+                                                                            spin_limit());
 }
 
 }  // namespace sr
