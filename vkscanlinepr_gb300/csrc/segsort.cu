@@ -27,11 +27,8 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;   // records a CTA sorts or merges
 constexpr int kGroup = kTile / 2;          // largest segment packed into a group tile
-// 9-bit digits: a tile's compact items need 2.3 passes a record on the
-// 4096^2 frame against 2.7 with 8-bit ones, for a histogram of 8 x 512 words
-constexpr int kRadixBits = 9;
+constexpr int kRadixBits = 9;   // digits of the 64-bit tile sort
 constexpr int kRadix = 1 << kRadixBits;
-constexpr int kDigitsPerThread = kRadix / 256;   // of the pass's digit scan
 constexpr uint32_t kChunkBit = 1u << 31;   // descriptor .z: a chunk of a large segment
 // Lanes with the same digit: __match_any_sync (tiles hold runs of nearly
 // sorted keys, so a warp sees few distinct digits), or one ballot per bit.
@@ -177,27 +174,47 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_tiles(const SegArgs s, uint
 // from a counter, so the grid does not follow the table's bound on them).
 //   * The tile reaches shared memory by one bulk copy (TMA) of its 16-byte
 //     aligned span; an odd last key comes by a plain load.
-//   * Within a tile the order is that of a compact item: the fields
-//     (path - pmin, row-rank code, x - xmin) packed in the fewest bits their
-//     ranges need (the rank codes of k_tile_sort32 are compacted, see
-//     TileRanges).  It usually needs 2-3 digit passes where the whole key
-//     needs 4-6, and a digit is one shift of a 32-bit word.
-//   * k_tile_sort32 sorts the tiles whose compact fields and payload fit one
-//     32-bit word: half the shared memory, so more CTAs per SM.  It hands
-//     the others to k_local_sort, whose items are 64-bit (rank - rmin codes,
-//     the payload in the high word, or the raw key when the fields need
-//     more than 32 bits), sorted through global memory.
-//   * A pass ranks the digits per warp (match_any + a per-warp histogram),
-//     scans the counts and scatters into the other buffer (stable: digit,
-//     then warp, then slot).  Rows of slots past the tile's end are skipped.
+//   * k_tile_sort spreads the records over up to 4096 bins, in key order: the
+//     tile's paths in turn, each with bins for its part of the range of (row,
+//     x) and one each for its off-canvas records and for row 0 (BinPlan).  A
+//     shared atomic gives a record its place in its bin; then a thread counts
+//     the records of its slot's bin that come before (by the code below the
+//     bin, then by index: the sort is stable) and writes the key to its place.
+//     Bins hold some eight records, so the count is short, and a record is
+//     moved once instead of once a digit: digit passes (2.3 a record, each a
+//     match, two histogram updates and a scatter) took 340 us for the 21 M
+//     records of a 4096^2 frame, this takes 276, and 21 instead of 38 us for a
+//     stage of 0.37 M records.  It is bound by instructions: the counts a
+//     third, the rest spread over the phases.  512 threads and 2 CTAs an SM
+//     (256 and 3: 266 us, but 29 for the small frame; 512 and 3, 40 registers:
+//     27).  8192 and 16384 bins cost more to clear and scan than they save.
+//     Off-canvas records share one key a path, so counting would be quadratic:
+//     their place is by index, from ballots.
+//   * A tile with a bin of more than 384 records, or with too many paths for
+//     the bins, is sorted by digit passes: compact 32-bit items ((path - pmin,
+//     row-rank code, x - xmin) in the fewest bits, the payload above), 8-bit
+//     digits ranked per warp (match_any and a histogram a warp), scanned and
+//     scattered.  (At 128 records 465 instead of 457 us for the stage, at 1024
+//     no change.)
+//   * A tile whose compact fields and payload do not fit 32 bits is handed to
+//     k_local_sort, whose items are 64-bit (rank - rmin codes, the payload in
+//     the high word, or the raw key when the fields need more than 32 bits),
+//     sorted through global memory by 9-bit digits.
 
-// Fields of a key: path, row rank, x (payload bits above the key ignored).
+// Fields of a key: path, row rank, x and the payload above them.  Row rank
+// and x share the low word (at most 31 bits), so a funnel shift takes the path.
 struct KeyFields {
     uint32_t xb, rb, pb;
     uint32_t off_rank;   // rank of the off-canvas records (Hy - 1); row 0 ranks one above
-    SR_DEV uint32_t x(uint64_t k) const { return (uint32_t)(k & ((1ull << xb) - 1)); }
-    SR_DEV uint32_t r(uint64_t k) const { return (uint32_t)((k >> xb) & ((1ull << rb) - 1)); }
-    SR_DEV uint32_t p(uint64_t k) const { return (uint32_t)((k >> (xb + rb)) & ((1ull << pb) - 1)); }
+    SR_DEV uint32_t x(uint64_t k) const { return (uint32_t)k & ((1u << xb) - 1u); }
+    SR_DEV uint32_t r(uint64_t k) const { return ((uint32_t)k >> xb) & ((1u << rb) - 1u); }
+    SR_DEV uint32_t p(uint64_t k) const {
+        return __funnelshift_r((uint32_t)k, (uint32_t)(k >> 32), xb + rb) & ((1u << pb) - 1u);
+    }
+    SR_DEV uint32_t pay(uint64_t k) const {
+        return kbits() >= 32u ? (uint32_t)(k >> 32) >> (kbits() - 32u)
+                              : __funnelshift_r((uint32_t)k, (uint32_t)(k >> 32), kbits());
+    }
     SR_DEV uint32_t kbits() const { return xb + rb + pb; }
 };
 
@@ -220,9 +237,8 @@ struct PassSmem {
     uint32_t warp_hist[kWarps][kRadix];
     uint32_t digit_start[kRadix];
     uint32_t scan_tmp[kWarps];
-    uint32_t red[kWarps][10];
+    uint32_t red[kWarps][6];
     uint64_t kred[kWarps][3];
-    uint64_t bar;
     uint32_t next;
 };
 
@@ -252,11 +268,12 @@ SR_DEV bool tile_span(const TileTables& u, uint32_t tile, uint32_t n_cap, uint32
 // Stages keys [a, a + len) in buf: [a & ~1, e & ~1) by one bulk copy, key
 // e - 1 by a load when e is odd.  Returns the slot of key a (0 or 1), or -1
 // when the copy wait gave up (uniform over the CTA, which then leaves).
+template <int THREADS>
 SR_DEV int stage_tile(uint64_t* buf, uint64_t* bar, uint32_t& phase, const uint64_t* __restrict__ keys_in,
                       uint32_t a, uint32_t len, uint32_t* status, uint32_t spin_limit) {
     const uint32_t e = a + len;
     if ((reinterpret_cast<uintptr_t>(keys_in) & 15u) != 0) {
-        for (uint32_t j = threadIdx.x; j < len; j += kThreads) buf[j] = keys_in[a + j];
+        for (uint32_t j = threadIdx.x; j < len; j += THREADS) buf[j] = keys_in[a + j];
         __syncthreads();
         return 0;
     }
@@ -360,89 +377,65 @@ struct Unpack {
     }
 };
 
-// Ranges of a tile for its 32-bit items, with the row ranks compacted: the
-// ranks in use below the off-canvas rank (a band), then the off-canvas rank,
-// then row 0's rank above it take consecutive codes, so a tile holding off-
-// canvas or row-0 records does not need the whole rank range; the x of the
-// off-canvas records (all the same when they are packed as keys are) is kept
-// aside, so they do not widen the x range either.  The order of the codes
+// Ranges of a tile's fields, with the row ranks compacted: the ranks in use
+// below the off-canvas rank (a band), then the off-canvas rank, then row 0's
+// rank above it take consecutive codes, so a tile holding off-canvas or row-0
+// records does not need the whole rank range.  Off-canvas records have x 0
+// (how keys are packed) and do not widen the x range.  The order of the codes
 // is the order of the ranks, and equal keys keep equal codes.
 struct TileRanges {
-    uint32_t pmin, pmax, bmin, bmax, xmin, xmax, xomin, xomax, has_off, has_top;
-    uint64_t top;   // the whole key's max (its payload's max)
+    uint32_t pmin, pmax, bmin, bmax, xmin, xmax, pay_max;
+    uint32_t flags;   // kHasOff | kHasTop | kOffX
+    static constexpr uint32_t kHasOff = 1, kHasTop = 2, kOffX = 4;
     SR_DEV void init() {
-        pmin = bmin = xmin = xomin = ~0u;
-        pmax = bmax = xmax = xomax = 0;
-        has_off = has_top = 0;
-        top = 0;
+        pmin = bmin = xmin = ~0u;
+        pmax = bmax = xmax = pay_max = flags = 0;
     }
     SR_DEV void add(const KeyFields& kf, uint64_t k) {
         const uint32_t p = kf.p(k), r = kf.r(k), x = kf.x(k);
         pmin = min(pmin, p); pmax = max(pmax, p);
         if (r == kf.off_rank) {
-            has_off = 1;
-            xomin = min(xomin, x); xomax = max(xomax, x);
+            flags |= x ? kHasOff | kOffX : kHasOff;
         } else {
             if (r < kf.off_rank) {
                 bmin = min(bmin, r); bmax = max(bmax, r);
             } else {
-                has_top = 1;
+                flags |= kHasTop;
             }
             xmin = min(xmin, x); xmax = max(xmax, x);
         }
-        top = max(top, k);
+        pay_max = max(pay_max, kf.pay(k));
     }
-    SR_DEV void reduce(PassSmem& S) {
+    // over the CTA's warps, through red[warps][8] (a barrier inside)
+    template <int WARPS> SR_DEV void reduce(uint32_t (*red)[8]) {
+        static_assert(WARPS <= 32, "a lane a warp");
         const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            pmin = min(pmin, __shfl_xor_sync(0xFFFFFFFFu, pmin, o));
-            pmax = max(pmax, __shfl_xor_sync(0xFFFFFFFFu, pmax, o));
-            bmin = min(bmin, __shfl_xor_sync(0xFFFFFFFFu, bmin, o));
-            bmax = max(bmax, __shfl_xor_sync(0xFFFFFFFFu, bmax, o));
-            xmin = min(xmin, __shfl_xor_sync(0xFFFFFFFFu, xmin, o));
-            xmax = max(xmax, __shfl_xor_sync(0xFFFFFFFFu, xmax, o));
-            xomin = min(xomin, __shfl_xor_sync(0xFFFFFFFFu, xomin, o));
-            xomax = max(xomax, __shfl_xor_sync(0xFFFFFFFFu, xomax, o));
-            top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-        }
-        has_off = __any_sync(0xFFFFFFFFu, has_off) ? 1u : 0u;
-        has_top = __any_sync(0xFFFFFFFFu, has_top) ? 1u : 0u;
+        warp_reduce();
         if (lane == 0) {
-            uint32_t* w = S.red[warp];
-            w[0] = pmin; w[1] = pmax; w[2] = bmin; w[3] = bmax; w[4] = xmin;
-            w[5] = xmax; w[6] = xomin; w[7] = xomax; w[8] = has_off; w[9] = has_top;
-            S.kred[warp][2] = top;
+            uint32_t* w = red[warp];
+            w[0] = pmin; w[1] = pmax; w[2] = bmin; w[3] = bmax;
+            w[4] = xmin; w[5] = xmax; w[6] = pay_max; w[7] = flags;
         }
         __syncthreads();
-        load(S);
-        top = S.kred[0][2];
-#pragma unroll
-        for (int w = 1; w < kWarps; ++w) top = max(top, S.kred[w][2]);
-    }
-    // the reduced values from the warps' shared words (also used to reload
-    // them after the passes, with fewer live registers through them)
-    SR_DEV void load(const PassSmem& S) {
         init();
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const uint32_t* v = S.red[w];
-            pmin = min(pmin, v[0]); pmax = max(pmax, v[1]);
-            bmin = min(bmin, v[2]); bmax = max(bmax, v[3]);
-            xmin = min(xmin, v[4]); xmax = max(xmax, v[5]);
-            xomin = min(xomin, v[6]); xomax = max(xomax, v[7]);
-            has_off |= v[8]; has_top |= v[9];
+        if (lane < WARPS) {
+            const uint32_t* w = red[lane];
+            pmin = w[0]; pmax = w[1]; bmin = w[2]; bmax = w[3];
+            xmin = w[4]; xmax = w[5]; pay_max = w[6]; flags = w[7];
         }
-        // off-canvas records of different x (not how keys are packed) share
-        // the x range like the others
-        if (has_off && xomin != xomax) {
-            xmin = min(xmin, xomin);
-            xmax = max(xmax, xomax);
-        }
+        warp_reduce();
     }
-    SR_DEV bool off_x_apart() const { return has_off && xomin == xomax; }
+    SR_DEV void warp_reduce() {
+        constexpr uint32_t all = 0xFFFFFFFFu;
+        pmin = __reduce_min_sync(all, pmin); pmax = __reduce_max_sync(all, pmax);
+        bmin = __reduce_min_sync(all, bmin); bmax = __reduce_max_sync(all, bmax);
+        xmin = __reduce_min_sync(all, xmin); xmax = __reduce_max_sync(all, xmax);
+        pay_max = __reduce_max_sync(all, pay_max); flags = __reduce_or_sync(all, flags);
+    }
+    SR_DEV uint32_t has_off() const { return flags & kHasOff; }
+    SR_DEV uint32_t has_top() const { return (flags & kHasTop) >> 1; }
     SR_DEV uint32_t band() const { return bmin <= bmax ? bmax - bmin + 1u : 0u; }
-    SR_DEV uint32_t rank_codes() const { return band() + has_off + has_top; }
+    SR_DEV uint32_t rank_codes() const { return band() + has_off() + has_top(); }
     SR_DEV uint32_t bits_p() const { return bits_of(pmax - pmin); }
     SR_DEV uint32_t bits_r() const { return bits_of(rank_codes() - 1u); }
     SR_DEV uint32_t bits_x() const { return xmin <= xmax ? bits_of(xmax - xmin) : 0u; }
@@ -451,8 +444,8 @@ struct TileRanges {
         const uint32_t p = kf.p(k), r = kf.r(k), x = kf.x(k);
         const uint32_t nb = band();
         const bool off = r == kf.off_rank;
-        const uint32_t rc = r < kf.off_rank ? r - bmin : (off ? nb : nb + has_off);
-        const uint32_t xc = off && off_x_apart() ? 0u : x - xmin;
+        const uint32_t rc = r < kf.off_rank ? r - bmin : (off ? nb : nb + has_off());
+        const uint32_t xc = off ? 0u : x - xmin;
         const uint32_t pc = bits_p() ? (p - pmin) << (br + bx) : 0u;
         return pc | (br ? rc << bx : 0u) | xc;
     }
@@ -462,17 +455,20 @@ struct TileRanges {
         const uint32_t rc = (uint32_t)(((uint64_t)c >> bx) & low_mask(br));
         const uint32_t p = pmin + (uint32_t)((uint64_t)c >> (br + bx));
         const uint32_t nb = band();
-        const uint32_t r = rc < nb ? bmin + rc : (has_off && rc == nb ? kf.off_rank : kf.off_rank + 1u);
-        const uint32_t x = r == kf.off_rank && off_x_apart() ? xomin : xmin + xc;
+        const uint32_t r = rc < nb ? bmin + rc : (has_off() && rc == nb ? kf.off_rank : kf.off_rank + 1u);
+        const uint32_t x = r == kf.off_rank ? 0u : xmin + xc;
         return ((uint64_t)p << (kf.xb + kf.rb)) | ((uint64_t)r << kf.xb) | (uint64_t)x;
     }
 };
 
 // `passes` digit passes over items buf[cur][0, len), each into the other
-// buffer; returns the buffer holding the result.  digit(item, shift).
-template <typename T, typename Digit>
-SR_DEV uint32_t radix_passes(PassSmem& S, T* buf0, T* buf1, uint32_t cur, uint32_t len, uint32_t passes,
-                             Digit digit) {
+// buffer; returns the buffer holding the result.  digit(item, shift).  hist:
+// a histogram of 1 << BITS counts a warp.
+template <typename T, int THREADS, int BITS, typename H, typename Digit>
+SR_DEV uint32_t radix_passes(H* hist, uint32_t* digit_start, uint32_t* scan_tmp, T* buf0, T* buf1, uint32_t cur,
+                             uint32_t len, uint32_t passes, Digit digit) {
+    constexpr int kWarps = THREADS / 32, kItems = kTile / THREADS, kRadix = 1 << BITS, kRadixBits = BITS;
+    constexpr int kDigitsPerThread = kRadix > THREADS ? kRadix / THREADS : 1;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     const uint32_t wfirst = warp * (32u * kItems);
     const uint32_t rows = wfirst >= len ? 0u : min((uint32_t)kItems, (len - wfirst + 31u) / 32u);
@@ -480,7 +476,7 @@ SR_DEV uint32_t radix_passes(PassSmem& S, T* buf0, T* buf1, uint32_t cur, uint32
         const uint32_t shift = pass * kRadixBits;
         const T* in = cur ? buf1 : buf0;
         T* out = cur ? buf0 : buf1;
-        for (int i = tid; i < kWarps * kRadix; i += kThreads) (&S.warp_hist[0][0])[i] = 0;
+        for (int i = tid; i < kWarps * kRadix; i += THREADS) hist[i] = 0;
         __syncthreads();
         // rank within the warp: warp w holds slots [w*512, w*512 + 512)
         uint32_t rd[kItems];   // rank | digit << 16
@@ -494,8 +490,8 @@ SR_DEV uint32_t radix_passes(PassSmem& S, T* buf0, T* buf1, uint32_t cur, uint32
             const uint32_t leader = (uint32_t)(__ffs(peers) - 1);
             uint32_t before = 0;
             if (ok && lane == leader) {
-                before = S.warp_hist[warp][dg];
-                S.warp_hist[warp][dg] = before + (uint32_t)__popc(peers);
+                before = hist[warp * kRadix + dg];
+                hist[warp * kRadix + dg] = (H)(before + (uint32_t)__popc(peers));
             }
             before = __shfl_sync(0xFFFFFFFFu, before, leader);
             rd[it] = (before + (uint32_t)__popc(peers & lanemask_lt())) | (dg << 16);
@@ -504,18 +500,20 @@ SR_DEV uint32_t radix_passes(PassSmem& S, T* buf0, T* buf1, uint32_t cur, uint32
         __syncthreads();
         // per digit: exclusive over warps, then over digits (a thread takes
         // kDigitsPerThread adjacent digits)
-        static_assert(kThreads * kDigitsPerThread == kRadix, "digits per thread");
+        static_assert(kDigitsPerThread == 1 || THREADS * kDigitsPerThread == kRadix, "digits per thread");
         uint32_t dcnt[kDigitsPerThread];
         uint32_t cnt = 0;
 #pragma unroll
         for (int q = 0; q < kDigitsPerThread; ++q) {
             const uint32_t dd = tid * kDigitsPerThread + (uint32_t)q;
             uint32_t sum = 0;
+            if (dd < (uint32_t)kRadix) {
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const uint32_t c = S.warp_hist[w][dd];
-                S.warp_hist[w][dd] = sum;
-                sum += c;
+                for (int w = 0; w < kWarps; ++w) {
+                    const uint32_t c = hist[w * kRadix + dd];
+                    hist[w * kRadix + dd] = (H)sum;
+                    sum += c;
+                }
             }
             dcnt[q] = sum;
             cnt += sum;
@@ -526,23 +524,24 @@ SR_DEV uint32_t radix_passes(PassSmem& S, T* buf0, T* buf1, uint32_t cur, uint32
             const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
             if ((int)lane >= o) x += y;
         }
-        if (lane == 31) S.scan_tmp[warp] = x;
+        if (lane == 31) scan_tmp[warp] = x;
         __syncthreads();
         if (warp == 0) {
-            const uint32_t w = lane < kWarps ? S.scan_tmp[lane] : 0u;
+            const uint32_t w = lane < kWarps ? scan_tmp[lane] : 0u;
             uint32_t wi = w;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, wi, o);
                 if ((int)lane >= o) wi += y;
             }
-            if (lane < kWarps) S.scan_tmp[lane] = wi - w;
+            if (lane < kWarps) scan_tmp[lane] = wi - w;
         }
         __syncthreads();
-        uint32_t start = S.scan_tmp[warp] + x - cnt;
+        uint32_t start = scan_tmp[warp] + x - cnt;
 #pragma unroll
         for (int q = 0; q < kDigitsPerThread; ++q) {
-            S.digit_start[tid * kDigitsPerThread + (uint32_t)q] = start;
+            const uint32_t dd = tid * kDigitsPerThread + (uint32_t)q;
+            if (dd < (uint32_t)kRadix) digit_start[dd] = start;
             start += dcnt[q];
         }
         __syncthreads();
@@ -551,7 +550,7 @@ SR_DEV uint32_t radix_passes(PassSmem& S, T* buf0, T* buf1, uint32_t cur, uint32
             if ((uint32_t)it >= rows) break;
             const uint32_t j = wfirst + (uint32_t)it * 32u + lane;
             const uint32_t dg = rd[it] >> 16;
-            if (j < len) out[S.digit_start[dg] + S.warp_hist[warp][dg] + (rd[it] & 0xFFFFu)] = in[j];
+            if (j < len) out[digit_start[dg] + hist[warp * kRadix + dg] + (rd[it] & 0xFFFFu)] = in[j];
         }
         __syncthreads();
         cur ^= 1u;
@@ -559,44 +558,291 @@ SR_DEV uint32_t radix_passes(PassSmem& S, T* buf0, T* buf1, uint32_t cur, uint32
     return cur;
 }
 
-// ---- 32-bit items
-struct Sort32Smem {
+// ---- the tile sort
+// Bins of a tile and where a bin is too full for the search in it.
+constexpr int kSortThreads = 512;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kSortRows = kTile / kSortThreads;
+constexpr uint32_t kBins = 4096;
+constexpr uint32_t kHeavyBin = 384;
+constexpr uint32_t kIndexBits = 12;   // a record's index in its tile
+constexpr int kSortBits = 8;          // digits of the radix passes
+constexpr int kBinRounds = (int)kBins / (8 * kSortThreads);   // of eight bins a thread
+static_assert(kTile == 1 << kIndexBits && kBins == 8u * kBinRounds * kSortThreads && kBins <= 1u << 14, "tile geometry");
+
+struct TileSmem {
     union {
         uint64_t keys[kTile + 2];        // the staged tile
-        uint32_t items[2][kTile + 4];    // the passes' buffers, once the keys are read
+        uint32_t items[2][kTile + 4];    // radix passes: their buffers, once the keys are read
     };
-    PassSmem ps;
+    union {
+        struct {
+            uint4 slot4[kTile / 4];      // low code << 12 | index, bin by bin; before, a path's first off-canvas place
+            uint4 bins4[kBins / 8];      // two 16-bit counts a word; then the bins' starts
+            uint16_t slot_bin[kTile];    // bin | kOffSlot of a slot
+        };
+        struct {
+            uint16_t hist[kSortWarps * (1 << kSortBits)];
+            uint32_t digit_start[1 << kSortBits];
+        };
+    };
+    uint32_t red[kSortWarps][8];
+    uint32_t warp_off[kSortWarps];   // off-canvas records of a warp
+    uint32_t scan_tmp[kSortWarps];
+    TileRanges ranges;
+    uint64_t bar;
+    uint32_t next;
+};
+constexpr uint16_t kOffSlot = 1u << 14;
+
+// How a tile's records fall into bins: `stride` bins a path, `band` of them
+// for its rows on the canvas but row 0 (rank code and x, shifted right), then
+// one for its off-canvas records and one for row 0.
+struct BinPlan {
+    uint32_t stride, band, shift;
+    bool ok;
+    SR_DEV BinPlan(const TileRanges& R, uint32_t bx) {
+        const uint32_t paths = R.pmax - R.pmin + 1u;
+        const uint32_t per_path = paths < kBins ? (kBins - 1u) / paths : 0u;   // one bin more holds the end
+        const uint32_t nb = R.band();
+        band = shift = 0;
+        ok = per_path >= 3u && paths <= (uint32_t)kTile;
+        if (ok && nb) {
+            const uint32_t most = per_path - 2u, last = (nb << bx) - 1u;
+            const uint32_t lb = bits_of(last), fl = 31u - (uint32_t)__clz((int)most);
+            shift = lb > fl + 1u ? lb - fl - 1u : 0u;
+            while ((last >> shift) >= most) ++shift;
+            band = (last >> shift) + 1u;
+        }
+        stride = band + 2u;
+        ok = ok && shift <= 32u - kIndexBits && bx <= 32u - kIndexBits;
+    }
 };
 
-// Sorts tile `tile` with 32-bit items (payload above the compact fields), or
-// hands it to the 64-bit kernel (queued in u.fallback).  False when a copy
+// The tile's records in order, by bins: false when a bin is too full.
+SR_DEV bool sort_by_bins(TileSmem& S, const TileRanges& R, const BinPlan& B, uint32_t bx, uint32_t base, uint32_t len,
+                         const KeyFields& kf, uint64_t* __restrict__ out) {
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const uint32_t rows = (len + kSortThreads - 1) / kSortThreads;
+    const uint32_t wfirst = warp * rows * 32u;
+    uint32_t* slot = reinterpret_cast<uint32_t*>(S.slot4);
+    uint32_t* bins = reinterpret_cast<uint32_t*>(S.bins4);
+    // ---- counts: each record's bin, its place in it (as the counts go, in no
+    // order) and the code that orders it there.  An off-canvas record's place
+    // among its path's is by index: its rank among the tile's off-canvas
+    // records (as warp << 12 | rank in the warp, until the warps' counts are
+    // known) less the first one's of its path.
+    uint32_t at[kSortRows], low[kSortRows];   // bin | off << 14 | place << 16; low code (off canvas: path)
+    uint32_t n_off = 0;
+    bool heavy = false;
+#pragma unroll
+    for (int it = 0; it < kSortRows; ++it) {
+        if ((uint32_t)it >= rows) break;
+        const uint32_t j = wfirst + (uint32_t)it * 32u + lane;
+        const bool live = j < len;
+        uint32_t bin = 0, place = 0;
+        bool off = false;
+        low[it] = 0;
+        if (live) {
+            const uint64_t k = S.keys[base + j];
+            const uint32_t r = kf.r(k), x = kf.x(k);
+            const uint32_t path = kf.p(k) - R.pmin;
+            bin = path * B.stride;
+            off = r == kf.off_rank;
+            if (r < kf.off_rank) {
+                const uint32_t c = ((r - R.bmin) << bx) | (x - R.xmin);
+                bin += c >> B.shift;
+                low[it] = c & ((1u << B.shift) - 1u);
+            } else {
+                bin += B.band + (off ? 0u : 1u);
+                low[it] = off ? path : x - R.xmin;
+            }
+        }
+        const uint32_t om = __ballot_sync(0xFFFFFFFFu, off);
+        if (om) {
+            if (off) place = (warp << kIndexBits) | (n_off + (uint32_t)__popc(om & lanemask_lt()));
+            n_off += (uint32_t)__popc(om);
+            uint32_t left = om;
+            while (left) {   // one path's at a time; mostly there is one
+                const int leader = __ffs(left) - 1;
+                const uint32_t lbin = __shfl_sync(0xFFFFFFFFu, bin, leader);
+                const uint32_t peers = __ballot_sync(0xFFFFFFFFu, off && bin == lbin);
+                if ((int)lane == leader) {
+                    atomicAdd(&bins[bin >> 1], (uint32_t)__popc(peers) << (16u * (bin & 1u)));
+                    atomicMin(&slot[low[it]], place);
+                }
+                left &= ~peers;
+            }
+        }
+        if (live && !off) {
+            const uint32_t sh = 16u * (bin & 1u);
+            place = (atomicAdd(&bins[bin >> 1], 1u << sh) >> sh) & 0xFFFFu;
+            heavy = heavy || place >= kHeavyBin;
+        }
+        at[it] = bin | (off ? (uint32_t)kOffSlot : 0u) | (place << 16);
+    }
+    if (lane == 0) S.warp_off[warp] = n_off;
+    if (__syncthreads_or(heavy)) return false;
+    // ---- the bins' starts over their counts: a warp's bins are `rounds` times
+    // 256, eight a lane
+    const uint32_t rounds = ((R.pmax - R.pmin + 1u) * B.stride + 8u * kSortThreads) / (8u * kSortThreads);
+    const uint32_t word0 = warp * rounds * 32u + lane;
+    uint32_t sums[kBinRounds], wsum = 0;
+#pragma unroll
+    for (int q = 0; q < kBinRounds; ++q) {
+        sums[q] = 0;
+        if ((uint32_t)q >= rounds) break;
+        const uint4 w = S.bins4[word0 + (uint32_t)q * 32u];
+        const uint32_t two = w.x + w.y + w.z + w.w;   // no half carries: a tile's records
+        sums[q] = (two & 0xFFFFu) + (two >> 16);
+        wsum += __reduce_add_sync(0xFFFFFFFFu, sums[q]);
+    }
+    if (lane == 0) S.scan_tmp[warp] = wsum;
+    if (R.has_off()) {
+        // lane v: off-canvas records of the warps before v
+        uint32_t before = lane < kSortWarps ? S.warp_off[lane] : 0u;
+        const uint32_t own = before;
+#pragma unroll
+        for (int o = 1; o < kSortWarps; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, before, o);
+            if ((int)lane >= o) before += y;
+        }
+        before -= own;
+        const uint32_t mine = __shfl_sync(0xFFFFFFFFu, before, warp);
+#pragma unroll
+        for (int it = 0; it < kSortRows; ++it) {
+            if ((uint32_t)it >= rows) break;
+            const bool off = (at[it] & kOffSlot) != 0;
+            const uint32_t first = off ? slot[low[it]] : 0u;
+            const uint32_t before_first = __shfl_sync(0xFFFFFFFFu, before, first >> kIndexBits);
+            if (off) {
+                constexpr uint32_t m = (1u << kIndexBits) - 1u;
+                const uint32_t place = mine + ((at[it] >> 16) & m) - before_first - (first & m);
+                at[it] = (at[it] & 0xFFFFu) | (place << 16);
+            }
+        }
+    }
+    __syncthreads();
+    uint32_t wstart = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? S.scan_tmp[lane] : 0u);
+#pragma unroll
+    for (int q = 0; q < kBinRounds; ++q) {
+        if ((uint32_t)q >= rounds) break;
+        uint32_t incl = sums[q];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if ((int)lane >= o) incl += y;
+        }
+        const uint4 w = S.bins4[word0 + (uint32_t)q * 32u];
+        const uint32_t c4[4] = {w.x, w.y, w.z, w.w};
+        uint32_t s4[4], at0 = wstart + incl - sums[q];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t second = at0 + (c4[i] & 0xFFFFu);
+            s4[i] = at0 | (second << 16);
+            at0 = second + (c4[i] >> 16);
+        }
+        S.bins4[word0 + (uint32_t)q * 32u] = make_uint4(s4[0], s4[1], s4[2], s4[3]);
+        wstart += __shfl_sync(0xFFFFFFFFu, incl, 31);
+    }
+    __syncthreads();
+    // ---- records to their bins
+    const uint16_t* start = reinterpret_cast<const uint16_t*>(S.bins4);
+#pragma unroll
+    for (int it = 0; it < kSortRows; ++it) {
+        if ((uint32_t)it >= rows) break;
+        const uint32_t j = wfirst + (uint32_t)it * 32u + lane;
+        if (j < len) {
+            const uint32_t p = start[at[it] & (kBins - 1u)] + (at[it] >> 16);
+            slot[p] = (low[it] << kIndexBits) | j;
+            S.slot_bin[p] = (uint16_t)(at[it] & (kBins - 1u + kOffSlot));
+        }
+    }
+    __syncthreads();
+    // ---- a slot a thread: its record's rank in its bin (code, then index),
+    // counted; its key goes from the staged tile straight to its place.  The
+    // lanes of a warp read the same few bins and write next to each other.
+    for (uint32_t q = tid; q < len; q += kSortThreads) {
+        const uint32_t v = slot[q], b = S.slot_bin[q];
+        uint32_t pos = q;
+        if (!(b & kOffSlot)) {
+            const uint32_t s0 = start[b], s1 = start[b + 1];
+            pos = s0;
+            for (uint32_t i = s0; i < s1; ++i) pos += slot[i] < v ? 1u : 0u;
+        }
+        out[pos] = S.keys[base + (v & ((1u << kIndexBits) - 1u))];
+    }
+    return true;
+}
+
+// The same by radix passes over 32-bit items (payload above the compact
+// fields): the tiles with a crowded bin, or of too many paths for bins.
+SR_DEV void sort_by_digits(TileSmem& S, const TileRanges& R, uint32_t base, uint32_t len, const KeyFields& kf,
+                           uint64_t* __restrict__ out) {
+    const uint32_t tid = threadIdx.x;
+    const uint32_t kbits = kf.kbits();
+    const uint32_t br = R.bits_r(), bx = R.bits_x(), bits = R.bits_p() + br + bx;
+    if (tid == 0) S.ranges = R;
+    // a field shifts only when it is not empty, so no shift reaches 32; through
+    // registers: the items overwrite the staged keys
+    uint32_t iv[kSortRows];
+#pragma unroll
+    for (int i = 0; i < kSortRows; ++i) {
+        const uint32_t j = tid + (uint32_t)i * kSortThreads;
+        iv[i] = 0;
+        if (j < len) {
+            const uint64_t k = S.keys[base + j];
+            iv[i] = (bits < 32u ? kf.pay(k) << bits : 0u) | R.code(kf, k, br, bx);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSortRows; ++i) {
+        const uint32_t j = tid + (uint32_t)i * kSortThreads;
+        if (j < len) S.items[0][j] = iv[i];
+    }
+    const uint32_t cmask = low_mask(bits);
+    const uint32_t passes = (bits + kSortBits - 1) / kSortBits;
+    const uint32_t cur = radix_passes<uint32_t, kSortThreads, kSortBits, uint16_t>(
+        S.hist, S.digit_start, S.scan_tmp, S.items[0], S.items[1], 0u, len, passes,
+        [cmask](uint32_t v, uint32_t shift) -> uint32_t { return ((v & cmask) >> shift) & ((1u << kSortBits) - 1u); });
+    const TileRanges U = S.ranges;   // read back: fewer live registers through the passes
+    const uint32_t ubr = U.bits_r(), ubx = U.bits_x(), ubits = U.bits_p() + ubr + ubx;
+    const uint32_t umask = low_mask(ubits);
+    for (uint32_t j = tid; j < len; j += kSortThreads) {
+        const uint32_t v = S.items[cur][j];
+        const uint64_t pay = ubits < 32u ? (uint64_t)(v >> ubits) : 0ull;
+        out[j] = (pay << kbits) | U.key(kf, v & umask, ubr, ubx);
+    }
+}
+
+// Sorts tile `tile`, or hands it to the 64-bit kernel when its compact fields
+// and payload do not fit 32 bits (queued in u.fallback).  False when a copy
 // wait gave up.
-SR_DEV bool sort_tile32(Sort32Smem& S, uint32_t tile, uint32_t& phase, const uint64_t* __restrict__ keys_in,
-                        uint64_t* __restrict__ keys_out, uint64_t* __restrict__ keys_alt, const KeyFields& kf,
-                        uint32_t n_cap, const TileTables& u, bool wide, uint32_t* status,
-                        uint32_t spin_limit) {
+SR_DEV bool sort_tile(TileSmem& S, uint32_t tile, uint32_t& phase, const uint64_t* __restrict__ keys_in,
+                      uint64_t* __restrict__ keys_out, uint64_t* __restrict__ keys_alt, const KeyFields& kf,
+                      uint32_t n_cap, const TileTables& u, bool wide, uint32_t* status, uint32_t spin_limit) {
     const uint32_t tid = threadIdx.x;
     uint32_t a, len;
     bool to_alt;
     if (!tile_span(u, tile, n_cap, a, len, to_alt)) return true;
-    uint64_t* dst = to_alt ? keys_alt : keys_out;
-    const int off = stage_tile(S.keys, &S.ps.bar, phase, keys_in, a, len, status, spin_limit);
+    uint64_t* out = (to_alt ? keys_alt : keys_out) + a;
+    // (the copy's wait publishes these)
+#pragma unroll
+    for (int i = 0; i < kBinRounds; ++i) S.bins4[tid + (uint32_t)i * kSortThreads] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int i = 0; i < kTile / 4 / kSortThreads; ++i)
+        S.slot4[tid + (uint32_t)i * kSortThreads] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    const int off = stage_tile<kSortThreads>(S.keys, &S.bar, phase, keys_in, a, len, status, spin_limit);
     if (off < 0) return false;
-
-    // the tile's ranges
-    const uint32_t kbits = kf.kbits();
-    const uint64_t kmask = (1ull << kbits) - 1ull;
     const uint32_t base = (uint32_t)off;
     TileRanges R;
     R.init();
-    for (uint32_t j = tid; j < len; j += kThreads) R.add(kf, S.keys[base + j]);
-    R.reduce(S.ps);
-    const uint32_t br = R.bits_r(), bx = R.bits_x();
-    const uint32_t bits = R.bits_p() + br + bx;
-    const uint64_t pay_max = R.top >> kbits;
-    const uint32_t payb = pay_max > 0xFFFFFFFFull ? 33u : bits_of((uint32_t)pay_max);
-    (void)kmask;
-    if (bits + payb > 32u) {
+    for (uint32_t j = tid; j < len; j += kSortThreads) R.add(kf, S.keys[base + j]);
+    R.reduce<kSortWarps>(S.red);
+    const uint32_t bx = R.bits_x();
+    const uint32_t bits = R.bits_p() + R.bits_r() + bx;
+    if (bits + bits_of(R.pay_max) > 32u || (R.flags & TileRanges::kOffX)) {
         if (tid == 0) {
             u.fallback[atomicAdd(u.wide_count, 1u)] = tile;
             if (!wide) set_error(status, ERR_CAPACITY);   // k_local_sort is not launched: the frame is redone
@@ -604,70 +850,37 @@ SR_DEV bool sort_tile32(Sort32Smem& S, uint32_t tile, uint32_t& phase, const uin
         return true;
     }
     if (bits == 0) {   // one key: already in order
-        for (uint32_t j = tid; j < len; j += kThreads) dst[a + j] = S.keys[base + j];
+        for (uint32_t j = tid; j < len; j += kSortThreads) out[j] = S.keys[base + j];
         return true;
     }
-    // the items (payload above the fields; a field shifts only when it is
-    // not empty, so no shift reaches 32), through registers: they overwrite
-    // the staged keys
-    uint32_t iv[kItems];
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        if ((uint32_t)i * kThreads >= len) break;
-        const uint32_t j = tid + (uint32_t)i * kThreads;
-        if (j < len) {
-            const uint64_t k = S.keys[base + j];
-            iv[i] = (bits < 32u ? (uint32_t)(k >> kbits) << bits : 0u) | R.code(kf, k, br, bx);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        if ((uint32_t)i * kThreads >= len) break;
-        const uint32_t j = tid + (uint32_t)i * kThreads;
-        if (j < len) S.items[0][j] = iv[i];
-    }
-    const uint32_t cmask = low_mask(bits);
-    const uint32_t passes = (bits + kRadixBits - 1) / kRadixBits;
-    const uint32_t cur = radix_passes<uint32_t>(S.ps, S.items[0], S.items[1], 0u, len, passes,
-                                                [cmask](uint32_t v, uint32_t shift) -> uint32_t {
-                                                    return ((v & cmask) >> shift) & (kRadix - 1);
-                                                });
-    TileRanges U;
-    U.load(S.ps);
-    const uint32_t ubr = U.bits_r(), ubx = U.bits_x(), ubits = U.bits_p() + ubr + ubx;
-    const uint32_t umask = low_mask(ubits);
-    for (uint32_t j = tid; j < len; j += kThreads) {
-        const uint32_t v = S.items[cur][j];
-        const uint64_t pay = ubits < 32u ? (uint64_t)(v >> ubits) : 0ull;
-        dst[a + j] = (pay << kbits) | U.key(kf, v & umask, ubr, ubx);
-    }
+    const BinPlan B(R, bx);
+    if (B.ok && sort_by_bins(S, R, B, bx, base, len, kf, out)) return true;
+    sort_by_digits(S, R, base, len, kf, out);
     return true;
 }
 
-__global__ void __launch_bounds__(kThreads, 4) k_tile_sort32(const uint64_t* __restrict__ keys_in,
-                                                             uint64_t* __restrict__ keys_out,
-                                                             uint64_t* __restrict__ keys_alt,
-                                                             KeyFields kf, uint32_t n_cap, uint32_t mt,
-                                                             TileTables u, bool wide, uint32_t* status,
-                                                             uint32_t spin_limit) {
+__global__ void __launch_bounds__(kSortThreads, 2) k_tile_sort(const uint64_t* __restrict__ keys_in,
+                                                               uint64_t* __restrict__ keys_out,
+                                                               uint64_t* __restrict__ keys_alt, KeyFields kf,
+                                                               uint32_t n_cap, uint32_t mt, TileTables u, bool wide,
+                                                               uint32_t* status, uint32_t spin_limit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Sort32Smem& S = *reinterpret_cast<Sort32Smem*>(smem_raw);
+    TileSmem& S = *reinterpret_cast<TileSmem*>(smem_raw);
     // tiles past the table exist only in a frame whose records overflowed (redone)
     const uint32_t n_tiles = min(u.ctl[kCtlTiles], mt);
-    if (threadIdx.x == 0) mbar_init(&S.ps.bar, 1);
+    if (threadIdx.x == 0) mbar_init(&S.bar, 1);
     uint32_t phase = 0;
     for (;;) {
-        if (threadIdx.x == 0) S.ps.next = atomicAdd(&u.ctl[kCtlSortNext], 1u);
+        if (threadIdx.x == 0) S.next = atomicAdd(&u.ctl[kCtlSortNext], 1u);
         __syncthreads();   // also: the previous tile is done with the buffers
-        const uint32_t tile = S.ps.next;
+        const uint32_t tile = S.next;
         __syncthreads();
         if (tile >= n_tiles) break;
-        if (!sort_tile32(S, tile, phase, keys_in, keys_out, keys_alt, kf, n_cap, u, wide, status, spin_limit)) return;
+        if (!sort_tile(S, tile, phase, keys_in, keys_out, keys_alt, kf, n_cap, u, wide, status, spin_limit)) return;
     }
 }
 
-// ---- 64-bit items (the tiles k_tile_sort32 handed over; rare).  The
+// ---- 64-bit items (the tiles k_tile_sort handed over; rare).  The
 // passes run between the tile's range of the input array (scratch by now:
 // the 32-bit kernel has staged every tile) and of the output, with the
 // histograms in static shared memory (the kernel is launched every frame,
@@ -707,7 +920,8 @@ SR_DEV void sort_tile64(PassSmem& S, uint32_t tile, uint64_t* keys_in, uint64_t*
         first[j] = compact ? ((k >> kbits) << 32) | c : k;
     }
     if (compact) {
-        radix_passes<uint64_t>(S, first, other, 0u, len, passes, [](uint64_t v, uint32_t shift) -> uint32_t {
+        radix_passes<uint64_t, kThreads, kRadixBits, uint32_t>(
+            &S.warp_hist[0][0], S.digit_start, S.scan_tmp, first, other, 0u, len, passes, [](uint64_t v, uint32_t shift) -> uint32_t {
             return ((uint32_t)v >> shift) & (kRadix - 1);
         });
         Unpack U;
@@ -717,7 +931,8 @@ SR_DEV void sort_tile64(PassSmem& S, uint32_t tile, uint64_t* keys_in, uint64_t*
             dst[j] = ((v >> 32) << kbits) | U.key(kf, (uint32_t)v);
         }
     } else {
-        radix_passes<uint64_t>(S, first, other, 0u, len, passes, [kmask](uint64_t v, uint32_t shift) -> uint32_t {
+        radix_passes<uint64_t, kThreads, kRadixBits, uint32_t>(
+            &S.warp_hist[0][0], S.digit_start, S.scan_tmp, first, other, 0u, len, passes, [kmask](uint64_t v, uint32_t shift) -> uint32_t {
             return (uint32_t)((v & kmask) >> shift) & (kRadix - 1);
         });
     }
@@ -894,25 +1109,25 @@ void launch_segsort(const SegArgs& sa, uint64_t* keys_in, uint64_t* keys_out, ui
     // resident CTAs per SM of the two persistent kernels (same on every
     // device of the build's architecture)
     static std::atomic<uint32_t> attr{0};
-    static std::atomic<int> occ_sort32{0}, occ_merge{0};
+    static std::atomic<int> occ_sort{0}, occ_merge{0};
     once_per_device(attr, [] {
-        cudaFuncSetAttribute(k_tile_sort32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Sort32Smem));
+        cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
         cudaFuncSetAttribute(k_merge_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MergeSmem));
         int a = 0, c = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_tile_sort32, kThreads, sizeof(Sort32Smem));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_tile_sort, kSortThreads, sizeof(TileSmem));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_merge_level, kThreads, sizeof(MergeSmem));
-        occ_sort32.store(std::max(a, 1));
+        occ_sort.store(std::max(a, 1));
         occ_merge.store(std::max(c, 1));
     });
     const size_t sms = (size_t)std::max(sm_count, 1);
-    const unsigned g_sort32 = (unsigned)std::min<size_t>(mt, sms * (size_t)std::max(occ_sort32.load(), 1));
+    const unsigned g_tile = (unsigned)std::min<size_t>(mt, sms * (size_t)std::max(occ_sort.load(), 1));
     // the 64-bit sort takes the few tiles the 32-bit one hands over
     const unsigned g_sort = (unsigned)std::min<size_t>(mt, sms);
     const unsigned g_merge =
         (unsigned)std::min<size_t>(kMergeParts * mt, sms * (size_t)std::max(occ_merge.load(), 1));
     count_launches(1 + (sa.wide ? 1 : 0) + (uint32_t)levels);
     const uint32_t n_cap = (uint32_t)sa.cap;
-    k_tile_sort32<<<g_sort32, kThreads, sizeof(Sort32Smem), st>>>(keys_in, keys_out, keys_alt, kf, n_cap,
+    k_tile_sort<<<g_tile, kSortThreads, sizeof(TileSmem), st>>>(keys_in, keys_out, keys_alt, kf, n_cap,
                                                                   (uint32_t)mt, u, sa.wide, status, spin_limit());
     if (sa.wide) k_local_sort<<<g_sort, kThreads, 0, st>>>(keys_in, keys_out, keys_alt, kf, n_cap, u);
     for (int lv = 0; lv < levels; ++lv)
