@@ -1178,10 +1178,10 @@ static_assert(SR_SIZER_PARAMS == sr::kMlpParams && SR_SIZER_FEATURES == sr::kMlp
 // on one device.
 struct sr_sizer {
     int device = 0, sm_count = 148;
-    DevBuf master, wb, grad, m, v, norm, loss;   // loss: one float
+    DevBuf master, wb, grad, m, v, norm, loss;   // loss: one double
     DevBuf keys, perm, keys_out, alt_k, alt_v, sort_scratch, ctl;
     int64_t step = 0;
-    float* h_loss = nullptr;
+    float* h_loss = nullptr;   // the loss (a double), then the status word
     ~sr_sizer() {
         DevBuf* all[] = {&master, &wb, &grad, &m, &v, &norm, &loss, &keys, &perm, &keys_out, &alt_k, &alt_v,
                          &sort_scratch, &ctl};
@@ -2034,14 +2034,14 @@ sr_status sr_sizer_loss_grad(sr_sizer* s, const float* d_x, const float* d_t, ui
     CUDA_TRY(cudaSetDevice(s->device));
     const size_t pb = sizeof(float) * sr::kMlpParams;
     CUDA_TRY(cudaMemset(s->grad.p, 0, pb));
-    CUDA_TRY(cudaMemset(s->loss.p, 0, sizeof(float)));
+    CUDA_TRY(cudaMemset(s->loss.p, 0, sizeof(double)));
     CUDA_TRY(sr::launch_mlp_grad(s->wb.p, s->master.as<float>(), s->norm.as<float>(), d_x, d_t, nullptr, n,
-                                 s->grad.as<float>(), s->loss.as<float>(), nullptr));
-    float loss = 0.0f;
-    CUDA_TRY(cudaMemcpy(&loss, s->loss.p, sizeof(float), cudaMemcpyDeviceToHost));
+                                 s->grad.as<float>(), s->loss.as<double>(), nullptr));
+    double loss = 0.0;
+    CUDA_TRY(cudaMemcpy(&loss, s->loss.p, sizeof(double), cudaMemcpyDeviceToHost));
     if (h_grad) CUDA_TRY(cudaMemcpy(h_grad, s->grad.p, pb, cudaMemcpyDeviceToHost));
     CUDA_TRY(cudaMemset(s->grad.p, 0, pb));
-    if (h_loss) *h_loss = loss / ((float)n * (float)sr::kMlpOut);
+    if (h_loss) *h_loss = (float)(loss / ((double)n * sr::kMlpOut));
     return SR_OK;
 }
 
@@ -2081,7 +2081,7 @@ sr_status sr_sizer_train(sr_sizer* s, const float* d_x, const float* d_t, uint32
     CUDA_TRY(cudaMemsetAsync(s->ctl.p, 0, sizeof(uint32_t) * 4, st));
     const double b1 = d.beta1, b2 = d.beta2;
     for (uint32_t ep = 0; ep < d.epochs; ++ep) {
-        CUDA_TRY(cudaMemsetAsync(s->loss.p, 0, sizeof(float), st));
+        CUDA_TRY(cudaMemsetAsync(s->loss.p, 0, sizeof(double), st));
         if (d.shuffle) {
             sr::launch_perm_keys(s->keys.as<uint32_t>(), n, d.seed * 0x100000001B3ull + ep, st);
             sr::launch_sort_u32(sp, s->keys.as<uint32_t>(), nullptr, s->keys_out.as<uint32_t>(), idx,
@@ -2094,7 +2094,7 @@ sr_status sr_sizer_train(sr_sizer* s, const float* d_x, const float* d_t, uint32
             const float bc1 = (float)(1.0 - std::pow(b1, (double)s->step));
             const float bc2 = (float)(1.0 - std::pow(b2, (double)s->step));
             CUDA_TRY(sr::launch_mlp_step(s->wb.p, s->master.as<float>(), s->norm.as<float>(), d_x, d_t,
-                                         idx ? idx + b0 : nullptr, nb, s->grad.as<float>(), s->loss.as<float>(),
+                                         idx ? idx + b0 : nullptr, nb, s->grad.as<float>(), s->loss.as<double>(),
                                          s->m.as<float>(), s->v.as<float>(), d.lr, d.beta1, d.beta2, d.eps, bc1, bc2,
                                          s->ctl.as<uint32_t>() + 1, st));
             if (!idx) {   // unshuffled minibatches are consecutive rows
@@ -2108,13 +2108,15 @@ sr_status sr_sizer_train(sr_sizer* s, const float* d_x, const float* d_t, uint32
         }
     }
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemcpyAsync(s->h_loss, s->loss.p, sizeof(float), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(s->h_loss + 1, s->ctl.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(s->h_loss, s->loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(s->h_loss + 2, s->ctl.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     uint32_t status = 0;
-    std::memcpy(&status, s->h_loss + 1, sizeof status);
+    std::memcpy(&status, s->h_loss + 2, sizeof status);
     SR_TRY(check_status_word(status));
-    if (h_loss) *h_loss = s->h_loss[0] / ((float)n * (float)sr::kMlpOut);
+    double loss;
+    std::memcpy(&loss, s->h_loss, sizeof loss);
+    if (h_loss) *h_loss = (float)(loss / ((double)n * sr::kMlpOut));
     return SR_OK;
 }
 

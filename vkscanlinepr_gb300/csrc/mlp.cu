@@ -298,7 +298,9 @@ SR_DEV void red_add4(float* p, float a, float b, float c, float d) {
 // warps on an SM.  Every layer is a small product out of shared memory in
 // which a thread owns 2 to 8 outputs, read in 16-byte pieces; the CTA's
 // parameter gradients are summed over its samples in registers and added into
-// grad.  loss_sum receives the sum of squared errors.  With `adam`, the CTA
+// grad.  loss_sum receives the sum of squared errors (a double: a float sum
+// in the order the warps come differs by up to 3e-6 from run to run).  With
+// `adam`, the CTA
 // that finishes last takes the optimiser step (a launch and its gap saved).
 // Shared-memory reads and the latency of its eight phases bound it: a step
 // of 4,096 samples takes 23 us, where 64 CTAs of 64 threads, a sample each,
@@ -319,7 +321,7 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const __nv_bfloat16* 
                                                            const float* __restrict__ norm, const float* __restrict__ x,
                                                            const float* __restrict__ t,
                                                            const uint32_t* __restrict__ idx, uint32_t n, float scale,
-                                                           float* grad, float* loss_sum, int adam, AdamArgs A,
+                                                           float* grad, double* loss_sum, int adam, AdamArgs A,
                                                            uint32_t* done) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const __nv_bfloat16* 
             }
         }
         sq += __shfl_xor_sync(0xFFFFFFFFu, sq, 1);
-        if (lane == 0) atomicAdd(loss_sum, sq);
+        if (lane == 0) atomicAdd(loss_sum, (double)sq);
         __syncwarp();
         // dL/da2
 #pragma unroll
@@ -603,7 +605,7 @@ void launch_mlp_predict(const void* wb, const float* master, const float* norm, 
 }
 
 static cudaError_t grad_launch(const void* wb, const float* master, const float* norm, const float* x, const float* t,
-                               const uint32_t* idx, uint32_t n, float* grad, float* loss_sum, bool adam,
+                               const uint32_t* idx, uint32_t n, float* grad, double* loss_sum, bool adam,
                                const AdamArgs& A, uint32_t* done, cudaStream_t st) {
     static std::atomic<uint32_t> attr{0};
     cudaError_t e = cudaSuccess;
@@ -619,13 +621,13 @@ static cudaError_t grad_launch(const void* wb, const float* master, const float*
 }
 
 cudaError_t launch_mlp_grad(const void* wb, const float* master, const float* norm, const float* x, const float* t,
-                            const uint32_t* idx, uint32_t n, float* grad, float* loss_sum, cudaStream_t st) {
+                            const uint32_t* idx, uint32_t n, float* grad, double* loss_sum, cudaStream_t st) {
     if (!n) return cudaSuccess;
     return grad_launch(wb, master, norm, x, t, idx, n, grad, loss_sum, false, AdamArgs{}, nullptr, st);
 }
 
 cudaError_t launch_mlp_step(void* wb, float* master, const float* norm, const float* x, const float* t,
-                            const uint32_t* idx, uint32_t n, float* grad, float* loss_sum, float* m, float* v, float lr,
+                            const uint32_t* idx, uint32_t n, float* grad, double* loss_sum, float* m, float* v, float lr,
                             float b1, float b2, float eps, float bc1, float bc2, uint32_t* done, cudaStream_t st) {
     if (!n) return cudaSuccess;
     const AdamArgs A{master, m, v, static_cast<__nv_bfloat16*>(wb), lr, b1, b2, eps, bc1, bc2};
