@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(256) k_transform(const float2* __restrict__ po
                                                    const uint32_t* __restrict__ pos_path, uint32_t n_points,
                                                    const SceneTable t, float2* __restrict__ tpos,
                                                    int32_t* __restrict__ path_visible) {
+    wait_for_stream();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t lane = lane_id();
     uint32_t pidx = 0xFFFFFFFFu;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(256) k_arc_fixup(const uint32_t* __restrict__ 
                                                    const uint32_t* __restrict__ curve_path, uint32_t n_curves,
                                                    const float2* __restrict__ pos, const SceneTable t,
                                                    float2* __restrict__ tpos, int32_t* __restrict__ path_visible) {
+    wait_for_stream();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n_curves || curve_type[c] != kArc) return;
     const uint32_t first = curve_pos[c], path = curve_path[c];
@@ -240,6 +242,7 @@ __global__ void __launch_bounds__(256) k_count(const GeomArgs g, float* __restri
                                                uint32_t* __restrict__ chain_items, uint8_t* __restrict__ chain_keys,
                                                uint32_t list_cap, uint32_t* __restrict__ chain_count,
                                                uint32_t* __restrict__ class_count, uint32_t* __restrict__ status) {
+    wait_for_stream();
     __shared__ uint32_t s_hist[kChainClasses], s_total, s_base;
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = c < g.n_curves;
@@ -438,6 +441,7 @@ __global__ void __launch_bounds__(256) k_offsets_and_order(
     const uint32_t* __restrict__ items, const uint8_t* __restrict__ keys, uint32_t list_cap,
     const uint32_t* __restrict__ chain_count, const uint32_t* __restrict__ class_count,
     uint32_t* __restrict__ class_next, uint32_t* __restrict__ sorted) {
+    wait_for_stream();
     __shared__ uint32_t s_start[kChainClasses], s_hist[kChainClasses], s_at[kChainClasses];
     __shared__ uint32_t s_tile;
     __shared__ int32_t s_warp[256 / 32 + 1];
@@ -840,6 +844,7 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
                                                 const uint32_t* __restrict__ items, uint32_t list_cap,
                                                 const uint32_t* __restrict__ class_count,
                                                 uint32_t* __restrict__ queue, int32_t* __restrict__ cbuf) {
+    wait_for_stream();
     ChainTickets<true> T;
     T.build(class_count);
     for (;;) {
@@ -905,6 +910,7 @@ __global__ void __launch_bounds__(128) k_order_records(const GeomArgs g, const i
                                                        const uint32_t* __restrict__ class_count,
                                                        const int32_t* __restrict__ cbuf, int2* __restrict__ rec,
                                                        uint32_t* __restrict__ status) {
+    wait_for_stream();
     ChainTickets<false> T;
     T.build(class_count);
     const uint32_t warps = gridDim.x * (blockDim.x / 32u);
@@ -1044,6 +1050,7 @@ __global__ void __launch_bounds__(32 * kFragWarps) k_fragment(const GeomArgs g, 
                                                               int64_t n_cap, const uint32_t* __restrict__ n_dev,
                                                               uint64_t* __restrict__ keys, uint8_t* __restrict__ wnp,
                                                               DebugOut dbg) {
+    wait_for_stream();
     const int64_t n = (int64_t)min((uint64_t)*n_dev, (uint64_t)n_cap);
     const int64_t b = ((int64_t)blockIdx.x * kFragWarps + (threadIdx.x >> 5)) * kFragOut;
     if (b >= n) return;
@@ -1130,7 +1137,8 @@ void launch_arc_fixup(const uint32_t* curve_type, const uint32_t* curve_pos, con
                       cudaStream_t st) {
     if (n_curves == 0) return;
     count_launches(1);
-    k_arc_fixup<<<(n_curves + 255) / 256, 256, 0, st>>>(curve_type, curve_pos, curve_path, n_curves, pos, t, tpos,
+    launch_after(k_arc_fixup, (n_curves + 255) / 256, 256, 0, st, curve_type, curve_pos, curve_path, n_curves, pos,
+                 t, tpos,
                                                         path_visible);
 }
 
@@ -1138,7 +1146,7 @@ void launch_transform(const float2* pos, const uint32_t* pos_path, uint32_t n_po
                       float2* tpos, int32_t* path_visible, cudaStream_t st) {
     if (n_points == 0) return;
     count_launches(1);
-    k_transform<<<(n_points + 255) / 256, 256, 0, st>>>(pos, pos_path, n_points, t, tpos, path_visible);
+    launch_after(k_transform, (n_points + 255) / 256, 256, 0, st, pos, pos_path, n_points, t, tpos, path_visible);
 }
 
 size_t piece_table_bytes(uint32_t n_curves) { return sizeof(uint4) * kMaxPieces * (size_t)n_curves; }
@@ -1148,7 +1156,8 @@ void launch_count(const GeomArgs& g, float* cut_cache, int32_t* count, const Cha
                   cudaStream_t st) {
     if (g.n_curves == 0) return;
     count_launches(1);
-    k_count<<<(g.n_curves + 255) / 256, 256, 0, st>>>(g, cut_cache, count, w.pieces, w.chain_items, w.chain_keys,
+    launch_after(k_count, (g.n_curves + 255) / 256, 256, 0, st, g, cut_cache, count, w.pieces, w.chain_items,
+                 w.chain_keys,
                                                       w.list_cap, w.chain_count, w.class_count, status);
 }
 
@@ -1165,7 +1174,8 @@ void launch_offsets_and_order(const GeomArgs& g, const int32_t* count, int32_t* 
     count_launches(1);
     const uint32_t tiles = offset_tiles(g.n_curves);
     const unsigned order = (unsigned)std::min<size_t>(((size_t)w.list_cap + 255) / 256, (size_t)sm_count * 4);
-    k_offsets_and_order<<<tiles + order, 256, 0, st>>>(count, offs, g.n_curves, tiles, tile_status, tile_counter,
+    launch_after(k_offsets_and_order, tiles + order, 256, 0, st, count, offs, g.n_curves, tiles, tile_status,
+                 tile_counter,
                                                        report_n, status, spin_limit(), w.chain_items, w.chain_keys,
                                                        w.list_cap, w.chain_count, w.class_count, w.class_next,
                                                        w.sorted_items);
@@ -1175,7 +1185,8 @@ void launch_chains(const GeomArgs& g, const int32_t* offs, const ChainWork& w, i
                    cudaStream_t st) {
     if (g.n_curves == 0) return;
     count_launches(1);
-    k_chains<<<sm_count * kChainCtas, 128, 0, st>>>(g, offs, w.pieces, w.sorted_items, w.list_cap, w.class_count,
+    launch_after(k_chains, sm_count * kChainCtas, 128, 0, st, g, offs, w.pieces, w.sorted_items, w.list_cap,
+                 w.class_count,
                                                     w.chain_queue, cbuf);
 }
 
@@ -1191,7 +1202,8 @@ void launch_order_records(const GeomArgs& g, const int32_t* offs, const ChainWor
                           uint32_t* status, int sm_count, cudaStream_t st) {
     if (g.n_curves == 0) return;
     count_launches(1);
-    k_order_records<<<sm_count * 32, 128, 0, st>>>(g, offs, w.pieces, w.sorted_items, w.list_cap, w.class_count, cbuf,
+    launch_after(k_order_records, sm_count * 32, 128, 0, st, g, offs, w.pieces, w.sorted_items, w.list_cap,
+                 w.class_count, cbuf,
                                                    rec, status);
 }
 
@@ -1200,7 +1212,8 @@ void launch_fragment(const GeomArgs& g, const int2* rec, int64_t n_cap, const ui
     if (n_cap <= 0 || g.n_curves == 0) return;
     count_launches(1);
     constexpr int64_t per = kFragWarps * kFragOut;
-    k_fragment<<<(unsigned)((n_cap + per - 1) / per), 32 * kFragWarps, 0, st>>>(g, rec, n_cap, n_dev, keys, wnp, dbg);
+    launch_after(k_fragment, (unsigned)((n_cap + per - 1) / per), 32 * kFragWarps, 0, st, g, rec, n_cap, n_dev, keys,
+                 wnp, dbg);
 }
 
 }  // namespace sr

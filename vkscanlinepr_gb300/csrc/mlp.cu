@@ -172,6 +172,7 @@ struct PredictSmem {
 __global__ void __launch_bounds__(kPredictThreads, kPredictCtas) k_mlp_predict(
     const __nv_bfloat16* __restrict__ wb, const float* __restrict__ master, const float* __restrict__ norm,
     const float* __restrict__ x, uint32_t n, float* __restrict__ y) {
+    wait_for_stream();
     __shared__ PredictSmem S;
     const Params& P = S.P;
     load_params(wb, master, norm, S.P);
@@ -323,6 +324,7 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const __nv_bfloat16* 
                                                            const uint32_t* __restrict__ idx, uint32_t n, float scale,
                                                            float* grad, double* loss_sum, int adam, AdamArgs A,
                                                            uint32_t* done) {
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
     const Params& P = S.P;
@@ -488,17 +490,22 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const __nv_bfloat16* 
     }
     __syncthreads();
     if (!S.last) return;
+    // (the next step's CTAs wait here, not at the start: among this step's they
+    // would crowd its free SMs)
+    release_next();
     adam_all<kGradThreads>(A, grad);
     if (tid == 0) *done = 0;
 }
 
 __global__ void k_to_bf16(const float* __restrict__ master, __nv_bfloat16* __restrict__ wb) {
+    wait_for_stream();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < kParams) wb[i] = __float2bfloat16_rn(master[i]);
 }
 
 // Shuffle keys for one epoch: a splitmix64 hash of (seed, i).
 __global__ void k_perm_keys(uint32_t* __restrict__ keys, uint32_t n, uint64_t seed) {
+    wait_for_stream();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint64_t z = seed + 0x9E3779B97F4A7C15ull * (uint64_t)(i + 1);
@@ -601,7 +608,8 @@ void launch_mlp_predict(const void* wb, const float* master, const float* norm, 
     unsigned blocks = (n + per - 1) / per;
     const unsigned cap = (unsigned)kPredictCtas * (unsigned)(sm_count > 0 ? sm_count : 148);   // one wave
     if (blocks > cap) blocks = cap;
-    k_mlp_predict<<<blocks, kPredictThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(wb), master, norm, x, n, y);
+    launch_after(k_mlp_predict, blocks, kPredictThreads, 0, st, static_cast<const __nv_bfloat16*>(wb), master, norm,
+                 x, n, y);
 }
 
 static cudaError_t grad_launch(const void* wb, const float* master, const float* norm, const float* x, const float* t,
@@ -614,9 +622,9 @@ static cudaError_t grad_launch(const void* wb, const float* master, const float*
     });
     if (e != cudaSuccess) return e;
     count_launches(1);
-    k_mlp_grad<<<(n + kSamples - 1) / kSamples, kGradThreads, sizeof(GradSmem), st>>>(
-        static_cast<const __nv_bfloat16*>(wb), master, norm, x, t, idx, n, 1.0f / ((float)n * (float)kOut), grad,
-        loss_sum, adam ? 1 : 0, A, done);
+    launch_after(k_mlp_grad, (n + kSamples - 1) / kSamples, kGradThreads, sizeof(GradSmem), st,
+                 static_cast<const __nv_bfloat16*>(wb), master, norm, x, t, idx, n, 1.0f / ((float)n * (float)kOut), grad,
+                 loss_sum, adam ? 1 : 0, A, done);
     return cudaGetLastError();
 }
 
@@ -636,13 +644,13 @@ cudaError_t launch_mlp_step(void* wb, float* master, const float* norm, const fl
 
 void launch_to_bf16(const float* master, void* wb, cudaStream_t st) {
     count_launches(1);
-    k_to_bf16<<<(kParams + 255) / 256, 256, 0, st>>>(master, static_cast<__nv_bfloat16*>(wb));
+    launch_after(k_to_bf16, (kParams + 255) / 256, 256, 0, st, master, static_cast<__nv_bfloat16*>(wb));
 }
 
 void launch_perm_keys(uint32_t* keys, uint32_t n, uint64_t seed, cudaStream_t st) {
     if (!n) return;
     count_launches(1);
-    k_perm_keys<<<(n + 255) / 256, 256, 0, st>>>(keys, n, seed);
+    launch_after(k_perm_keys, (n + 255) / 256, 256, 0, st, keys, n, seed);
 }
 
 void launch_allot(const float* y, uint32_t n_paths, const uint32_t* path_scene, const float margins[4],

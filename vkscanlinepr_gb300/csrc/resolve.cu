@@ -478,6 +478,7 @@ SR_DEV void resolve_pixel_rows(const ResolveArgs& a, const ResolveWork& w, int32
 // the chunk already staged); a warp skips the records before its own cut.
 template <int WARPS, bool GRAD>
 __global__ void __launch_bounds__(32 * WARPS) k_resolve_pixel_rows(const ResolveArgs a) {
+    wait_for_stream();
     __shared__ PixRec slots[WARPS * 32];
     __shared__ RunBuf bufs[WARPS];
     if (!a.cta_narrow[blockIdx.x]) return;
@@ -488,6 +489,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_resolve_pixel_rows(const Resolve
 
 template <int WARPS, bool GRAD>
 __global__ void __launch_bounds__(32 * WARPS) k_resolve_pixel(const ResolveArgs a) {
+    wait_for_stream();
     if (a.any_narrow && a.cta_narrow[blockIdx.x]) return;   // k_resolve_pixel_rows
     __shared__ PixRec sq[kChunk];
     __shared__ RunBuf bufs[WARPS];
@@ -577,6 +579,7 @@ struct RefRec {
 
 template <int WARPS, bool GRAD>
 __global__ void __launch_bounds__(32 * WARPS) k_resolve_ref(const ResolveArgs a) {
+    wait_for_stream();
     __shared__ RefRec sq[kChunk];
     const ResolveWork w = resolve_work<WARPS>(a);
     const int tid = threadIdx.x, lane = tid & 31;
@@ -657,10 +660,12 @@ __global__ void __launch_bounds__(32 * WARPS) k_resolve_ref(const ResolveArgs a)
 
 template <int WARPS, bool GRAD> static void launch_resolve_t(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st) {
     if (a.pixel_mode) {
-        if (a.any_wide) k_resolve_pixel<WARPS, GRAD><<<n_ctas, 32 * WARPS, 0, st>>>(a);
+        if (a.any_wide) launch_after(k_resolve_pixel<WARPS, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
+        // (not launch_after: placed early it takes the other kernel's SMs, 0.72
+        // instead of 0.70 ms in a batch of 64 uneven scenes)
         if (a.any_narrow) k_resolve_pixel_rows<WARPS, GRAD><<<n_ctas, 32 * WARPS, 0, st>>>(a);
     } else {
-        k_resolve_ref<WARPS, GRAD><<<n_ctas, 32 * WARPS, 0, st>>>(a);
+        launch_after(k_resolve_ref<WARPS, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
     }
 }
 
@@ -680,6 +685,7 @@ void launch_resolve(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st) {
 // Multisampling: the sample frames summed per channel (ushort4; 16 samples
 // of 255 fit), then the rounded average (sum + k/2) / k per channel.
 __global__ void k_aa_accumulate(const uint32_t* __restrict__ img, ushort4* __restrict__ acc, size_t n, int first) {
+    wait_for_stream();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t c = img[i];
@@ -692,6 +698,7 @@ __global__ void k_aa_accumulate(const uint32_t* __restrict__ img, ushort4* __res
 }
 
 __global__ void k_aa_resolve(const ushort4* __restrict__ acc, uint32_t* __restrict__ img, size_t n, uint32_t k) {
+    wait_for_stream();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const ushort4 v = acc[i];
@@ -702,13 +709,14 @@ __global__ void k_aa_resolve(const ushort4* __restrict__ acc, uint32_t* __restri
 void launch_aa_accumulate(const uint32_t* img, void* acc, size_t n, bool first, cudaStream_t st) {
     if (!n) return;
     count_launches(1);
-    k_aa_accumulate<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(img, static_cast<ushort4*>(acc), n, first ? 1 : 0);
+    launch_after(k_aa_accumulate, (unsigned)((n + 255) / 256), 256, 0, st, img, static_cast<ushort4*>(acc), n,
+                 first ? 1 : 0);
 }
 
 void launch_aa_resolve(const void* acc, uint32_t* img, size_t n, uint32_t k, cudaStream_t st) {
     if (!n) return;
     count_launches(1);
-    k_aa_resolve<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(static_cast<const ushort4*>(acc), img, n, k);
+    launch_after(k_aa_resolve, (unsigned)((n + 255) / 256), 256, 0, st, static_cast<const ushort4*>(acc), img, n, k);
 }
 
 void launch_row_bounds(const uint32_t* srows, int64_t n, const uint32_t* n_dev, int32_t rows, int32_t* row_start,

@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(kThreads) k_scan_i32(const int32_t* in, int32_
 }
 
 __global__ void __launch_bounds__(kOneThreads) k_scan_one(const int32_t* in, int32_t* out, int64_t n) {
+    wait_for_stream();
     __shared__ int32_t s_warp[2][kOneThreads / 32 + 1];
     int32_t carry = 0;
     int par = 0;
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(kOneThreads) k_scan_one(const int32_t* in, int
 // first is what the L2 holds.
 __global__ void __launch_bounds__(kThreads, 8) k_chunk_sums(const int32_t* __restrict__ in, int64_t n, uint32_t tiles,
                                                             int32_t* __restrict__ sums) {
+    wait_for_stream();
     __shared__ int32_t s_warp[kThreads / 32];
     uint32_t t0, t1;
     chunk_tiles(tiles, t0, t1);
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_chunk_sums(const int32_t* __res
 // The chunks' scans, the next tile's loads under way while one is scanned.
 __global__ void __launch_bounds__(kThreads, kChunkCtas) k_chunk_scan(const int32_t* in, int32_t* out, int64_t n,
                                                                      uint32_t tiles, const int32_t* __restrict__ sums) {
+    wait_for_stream();
     __shared__ int32_t s_warp[2][kThreads / 32 + 1];
     uint32_t t0, t1;
     chunk_tiles(tiles, t0, t1);
@@ -139,14 +142,14 @@ void launch_scan_i32(const int32_t* in, int32_t* out, int64_t n, void* scratch, 
     }
     if (n <= kOneTo) {
         count_launches(1);
-        k_scan_one<<<1, kOneThreads, 0, st>>>(in, out, n);
+        launch_after(k_scan_one, 1, kOneThreads, 0, st, in, out, n);
         return;
     }
     count_launches(2);
     const uint32_t tiles = tiles_of(n);
     const unsigned grid = std::min(tiles, kChunksMax);
-    k_chunk_sums<<<grid, kThreads, 0, st>>>(in, n, tiles, static_cast<int32_t*>(scratch));
-    k_chunk_scan<<<grid, kThreads, 0, st>>>(in, out, n, tiles, static_cast<const int32_t*>(scratch));
+    launch_after(k_chunk_sums, grid, kThreads, 0, st, in, n, tiles, static_cast<int32_t*>(scratch));
+    launch_after(k_chunk_scan, grid, kThreads, 0, st, in, out, n, tiles, static_cast<const int32_t*>(scratch));
 }
 
 size_t lookback_scan_words(int64_t n) { return (size_t)tiles_of(n) + 1; }

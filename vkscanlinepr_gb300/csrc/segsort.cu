@@ -126,6 +126,7 @@ __global__ void k_seg_largest(const SegArgs s) {
 // launches, 3.6-8 us each.)
 __global__ void __launch_bounds__(kSegThreads) k_seg_tiles(const SegArgs s, uint32_t mt, TileTables u,
                                                            uint32_t* status, uint32_t spin_limit) {
+    wait_for_stream();
     __shared__ uint32_t s_tile;
     __shared__ int32_t s_warp[kSegThreads / 32 + 1];
     if (threadIdx.x == 0) s_tile = atomicAdd(&u.ctl[0], 1u);
@@ -864,6 +865,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_tile_sort(const uint64_t* _
                                                                uint64_t* __restrict__ keys_alt, KeyFields kf,
                                                                uint32_t n_cap, uint32_t mt, TileTables u, bool wide,
                                                                uint32_t* status, uint32_t spin_limit) {
+    wait_for_stream();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileSmem& S = *reinterpret_cast<TileSmem*>(smem_raw);
     // tiles past the table exist only in a frame whose records overflowed (redone)
@@ -941,6 +943,7 @@ SR_DEV void sort_tile64(PassSmem& S, uint32_t tile, uint64_t* keys_in, uint64_t*
 __global__ void __launch_bounds__(kThreads) k_local_sort(uint64_t* keys_in, uint64_t* __restrict__ keys_out,
                                                          uint64_t* __restrict__ keys_alt, KeyFields kf, uint32_t n_cap,
                                                          TileTables u) {
+    wait_for_stream();
     __shared__ PassSmem S;
     const uint32_t n_tiles = *u.wide_count;
     if (n_tiles == 0) return;   // the usual case: nothing handed over
@@ -1059,6 +1062,7 @@ SR_DEV void merge_item(MergeSmem& S, uint32_t item, uint64_t* __restrict__ keys_
 __global__ void __launch_bounds__(kThreads) k_merge_level(uint64_t* __restrict__ keys_out,
                                                           uint64_t* __restrict__ keys_alt, uint32_t level,
                                                           uint32_t key_bits, uint32_t n_cap, TileTables u) {
+    wait_for_stream();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MergeSmem& S = *reinterpret_cast<MergeSmem*>(smem_raw);
     __shared__ uint32_t next;
@@ -1102,7 +1106,8 @@ void launch_segsort(const SegArgs& sa, uint64_t* keys_in, uint64_t* keys_out, ui
     TileTables u = carve(sa);
     const size_t mt = max_tiles(sa.n_paths, sa.cap);
     count_launches(1);
-    k_seg_tiles<<<(sa.n_paths + kSegThreads - 1) / kSegThreads, kSegThreads, 0, st>>>(sa, (uint32_t)mt, u, status,
+    launch_after(k_seg_tiles, (sa.n_paths + kSegThreads - 1) / kSegThreads, kSegThreads, 0, st, sa, (uint32_t)mt, u,
+                 status,
                                                                                       spin_limit());
     const uint32_t key_bits = L.pbits + L.rbits + L.xbits;
     const KeyFields kf{L.xbits, L.rbits, L.pbits, (uint32_t)(L.Hy - 1)};
@@ -1127,11 +1132,12 @@ void launch_segsort(const SegArgs& sa, uint64_t* keys_in, uint64_t* keys_out, ui
         (unsigned)std::min<size_t>(kMergeParts * mt, sms * (size_t)std::max(occ_merge.load(), 1));
     count_launches(1 + (sa.wide ? 1 : 0) + (uint32_t)levels);
     const uint32_t n_cap = (uint32_t)sa.cap;
-    k_tile_sort<<<g_tile, kSortThreads, sizeof(TileSmem), st>>>(keys_in, keys_out, keys_alt, kf, n_cap,
+    launch_after(k_tile_sort, g_tile, kSortThreads, sizeof(TileSmem), st, keys_in, keys_out, keys_alt, kf, n_cap,
                                                                   (uint32_t)mt, u, sa.wide, status, spin_limit());
-    if (sa.wide) k_local_sort<<<g_sort, kThreads, 0, st>>>(keys_in, keys_out, keys_alt, kf, n_cap, u);
+    if (sa.wide) launch_after(k_local_sort, g_sort, kThreads, 0, st, keys_in, keys_out, keys_alt, kf, n_cap, u);
     for (int lv = 0; lv < levels; ++lv)
-        k_merge_level<<<g_merge, kThreads, sizeof(MergeSmem), st>>>(keys_out, keys_alt, (uint32_t)lv, key_bits, n_cap,
+        launch_after(k_merge_level, g_merge, kThreads, sizeof(MergeSmem), st, keys_out, keys_alt, (uint32_t)lv,
+                     key_bits, n_cap,
                                                                     u);
 }
 

@@ -98,6 +98,7 @@ template <typename K>
 __global__ void __launch_bounds__(kThreads) k_hist(const K* __restrict__ keys, int64_t n_max,
                                                    const uint32_t* __restrict__ n_dev, uint32_t passes,
                                                    uint32_t key_bits, uint32_t* __restrict__ hist) {
+    wait_for_stream();
     __shared__ uint32_t sh[kMaxPasses][kRadix];
     const int64_t n = n_dev ? (int64_t)min((uint64_t)*n_dev, (uint64_t)n_max) : n_max;
     for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kThreads) (&sh[0][0])[i] = 0;
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(kThreads) k_row_starts(const uint32_t* __restr
                                                          uint32_t key_bits, uint32_t* __restrict__ hist,
                                                          uint64_t* tstat, uint32_t* counter, uint32_t* status,
                                                          uint32_t spin_limit) {
+    wait_for_stream();
     __shared__ uint32_t sh[kMaxPasses][kRadix];
     __shared__ uint32_t s_tile;
     __shared__ int32_t s_warp[kWarps + 1];
@@ -182,6 +184,7 @@ __global__ void __launch_bounds__(kThreads, onesweep_min_blocks(kVals, ITEMS)) k
                                                        const uint32_t* __restrict__ digit_count,
                                                        uint32_t* __restrict__ lookback, uint32_t* counter,
                                                        uint32_t* status, uint32_t spin_limit) {
+    wait_for_stream();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int kItems = ITEMS, kTile = kThreads * ITEMS;
     OnesweepSmem<K, kVals, ITEMS>& S = *reinterpret_cast<OnesweepSmem<K, kVals, ITEMS>*>(smem_raw);
@@ -335,7 +338,7 @@ static void sort_impl(const SortPlan& p, const K* keys_in, const uint32_t* vals_
         int hb = (int)((p.n + kThreads - 1) / kThreads);
         if (hb > kHistBlocks) hb = kHistBlocks;
         count_launches(1);
-        k_hist<K><<<hb, kThreads, 0, st>>>(keys_in, p.n, p.n_dev, p.passes, p.key_bits, s.hist);
+        launch_after(k_hist<K>, hb, kThreads, 0, st, keys_in, p.n, p.n_dev, p.passes, p.key_bits, s.hist);
     }
     const size_t smem = sizeof(OnesweepSmem<K, kVals, ITEMS>);
     static std::atomic<uint32_t> attr_set{0};
@@ -349,7 +352,7 @@ static void sort_impl(const SortPlan& p, const K* keys_in, const uint32_t* vals_
         K* kdst = to_out ? keys_out : keys_alt;
         uint32_t* vdst = to_out ? vals_out : vals_alt;
         count_launches(1);
-        k_onesweep<K, kVals, ITEMS><<<p.tiles, kThreads, smem, st>>>(ksrc, vsrc, kdst, vdst, p.n, p.n_dev,
+        launch_after(k_onesweep<K, kVals, ITEMS>, p.tiles, kThreads, smem, st, ksrc, vsrc, kdst, vdst, p.n, p.n_dev,
                                                              pass * kRadixBits,
                                                              digit_mask(p.key_bits, pass * kRadixBits),
                                                              s.hist + pass * kRadix,
@@ -396,7 +399,8 @@ void launch_row_starts(SortPlan& p, const uint32_t* row_count, uint32_t rows, in
         return;
     }
     count_launches(1);
-    k_row_starts<<<(rows + kRowTile - 1) / kRowTile, kThreads, 0, st>>>(row_count, rows, row_start, p.passes, p.key_bits,
+    launch_after(k_row_starts, (rows + kRowTile - 1) / kRowTile, kThreads, 0, st, row_count, rows, row_start,
+                 p.passes, p.key_bits,
                                                                         carve(p, scratch).hist, tile_status,
                                                                         tile_counter, status, spin_limit());
 }

@@ -708,6 +708,7 @@ SR_DEV void winding_prefix(uint32_t heads, uint32_t wbits, int32_t* wv, int32_t*
 template <int ITEMS, int THREADS, int SPLIT, bool MULTI>
 __global__ void __launch_bounds__(THREADS, 4) k_winding_reduce(const WindArgs a, uint64_t* tagg,
                                                             int32_t* __restrict__ tile_in, uint32_t* done) {
+    wait_for_previous();
     constexpr int kTile = 256 * ITEMS, kWarps = THREADS / 32 / SPLIT, kRounds = kTile / 64 / SPLIT;
     constexpr int kFlight = kRounds < 8 ? kRounds : 8;
     static_assert(kRounds % kFlight == 0 && (SPLIT == 1 || kWarps == 1), "a warp a tile, or the CTA's warps");
@@ -796,6 +797,7 @@ __global__ void __launch_bounds__(THREADS, 4) k_winding_reduce(const WindArgs a,
         __threadfence();
     }
     __syncthreads();
+    release_next();
     if (s_last) scan_tile_pairs<THREADS>(tagg, tile_in, a, n, tiles, wv, wf);
 }
 
@@ -847,6 +849,7 @@ template <int ITEMS, int THREADS, bool MULTI>
 __global__ void __launch_bounds__(THREADS, 5) k_winding_runs(const WindArgs a, const int32_t* __restrict__ tile_in,
                                                              uint64_t* __restrict__ tstat, uint32_t* counter,
                                                              uint32_t* status, uint32_t spin_limit) {
+    wait_for_stream();
     constexpr int kTile = THREADS * ITEMS;
     static_assert(ITEMS % 2 == 0 && ITEMS <= 8, "records per thread");
     __shared__ RunSmem<ITEMS, THREADS> S;
@@ -1147,11 +1150,12 @@ template <int ITEMS, bool MULTI>
 static void launch_runs(const WindArgs& a, int64_t tiles, uint64_t* words, uint64_t* tagg, int32_t* tile_in,
                         uint32_t* counters, uint32_t* status, cudaStream_t st) {
     if (tiles >= kWarpTiles)
-        k_winding_reduce<ITEMS, 256, 1, MULTI><<<(unsigned)((tiles + 7) / 8), 256, 0, st>>>(a, tagg, tile_in,
+        launch_after(k_winding_reduce<ITEMS, 256, 1, MULTI>, (unsigned)((tiles + 7) / 8), 256, 0, st, a, tagg, tile_in,
                                                                                         counters + 1);
     else
-        k_winding_reduce<ITEMS, 256, 8, MULTI><<<(unsigned)tiles, 256, 0, st>>>(a, tagg, tile_in, counters + 1);
-    k_winding_runs<ITEMS, 256, MULTI><<<(unsigned)tiles, 256, 0, st>>>(a, tile_in, words, counters, status,
+        launch_after(k_winding_reduce<ITEMS, 256, 8, MULTI>, (unsigned)tiles, 256, 0, st, a, tagg, tile_in,
+                     counters + 1);
+    launch_after(k_winding_runs<ITEMS, 256, MULTI>, (unsigned)tiles, 256, 0, st, a, tile_in, words, counters, status,
                                                                        spin_limit());
 }
 
