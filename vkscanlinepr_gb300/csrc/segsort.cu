@@ -872,13 +872,14 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_tile_sort(const uint64_t* _
     const uint32_t n_tiles = min(u.ctl[kCtlTiles], mt);
     if (threadIdx.x == 0) mbar_init(&S.bar, 1);
     uint32_t phase = 0;
-    for (;;) {
-        if (threadIdx.x == 0) S.next = atomicAdd(&u.ctl[kCtlSortNext], 1u);
-        __syncthreads();   // also: the previous tile is done with the buffers
-        const uint32_t tile = S.next;
-        __syncthreads();
-        if (tile >= n_tiles) break;
+    // the first tiles by the CTAs' numbers: an SM's second CTA takes one only
+    // when every SM has one
+    for (uint32_t tile = blockIdx.x; tile < n_tiles;) {
+        __syncthreads();   // the previous tile is done with the buffers (before the first: the barrier is set up)
+        if (threadIdx.x == 0) S.next = gridDim.x + atomicAdd(&u.ctl[kCtlSortNext], 1u);
         if (!sort_tile(S, tile, phase, keys_in, keys_out, keys_alt, kf, n_cap, u, wide, status, spin_limit)) return;
+        __syncthreads();
+        tile = S.next;
     }
 }
 
