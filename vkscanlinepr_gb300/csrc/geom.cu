@@ -166,15 +166,20 @@ SR_DEV int32_t cut_range(int32_t size, int32_t F, int32_t& b, int32_t& e) {
 
 // Pieces of a curve: at most 4 monotonic cuts + the end at t = 1.
 constexpr int kMaxPieces = 5;
-// A lane of a split chain takes at least 1 << kSegLog bisected roots.  With
-// 8 / 16 / 32 the chain stage of the 4096^2 frame of 20,000 paths took 0.379 /
-// 0.311 / 0.281 ms (longer stretches waste fewer run-up and repeated roots),
-// that of the 1024^2 frame of 500 paths 0.054 / 0.057 / 0.072 ms (a lane's
-// stretch is its latency) and that of a 2048^2 frame of 5,000 paths 0.142 /
-// 0.140 / 0.177 ms.  (One chain a lane, and the longest a warp each beside
-// them, took 1.35, 0.33 and 0.82 ms.)
-constexpr int32_t kSegLog = 4;
-constexpr int kChainCtas = 8;   // of four warps, an SM; 4 and 16 took the same
+// A lane of a split chain takes at least 1 << kSegLog bisected roots: 64 when
+// the chains are many waves of work (longer stretches waste fewer run-up and
+// repeated roots), 8 when they leave schedulers idle (a lane's stretch is its
+// latency).  "Many" and "few" by the warps' shares (tickets) that stretches of
+// 16 would give.  The chain stage in ms, with 8 / 16 / 32 / 64: 4096^2 frame
+// of 20,000 paths (45,000 tickets) 0.36 / 0.293 / 0.276 / 0.267, batch of 64
+// uneven scenes 0.26 / 0.212 / 0.205 / 0.192, 2048^2 frame of 5,000 paths
+// (10,291) 0.135 / 0.121 / 0.133, 1000x750 frame of 1,200 paths (1,906) 0.036 /
+// 0.041, 1024^2 frame of 500 paths (1,001) 0.041 / 0.045 (4: 0.037).  (One
+// chain a lane, and the longest a warp each beside them, took 1.35, 0.82 and
+// 0.33 ms for the 4096^2, 2048^2 and 1024^2 frames.)
+constexpr int32_t kSegShort = 3, kSegLog = 4, kSegLong = 6;
+constexpr uint32_t kShortTickets = 16, kLongTickets = 160;   // an SM
+constexpr int kChainCtas = 7;   // of four warps, an SM: all that fit with 72 registers a thread
 
 // Piece record layout in the output: [t0][x crossings][y crossings], the
 // crossing values of each side solved by one chain (k_chains), then merged
@@ -197,17 +202,17 @@ SR_DEV uint32_t chain_key(int32_t len, uint32_t type) {
     return ((14u - lg) << 2) | cls;
 }
 // How the chains of a class are shared out: 2^lanes lanes a chain and 2^warps
-// warps (warps only with 32 lanes).  Solving, a lane takes 16 to 31 bisected
-// roots or, a line's root being a closed form, 512 to 1,023 of a line, as far
-// as 32 lanes go (run_segments).  Ordering, a lane takes every 32nd root, up
+// warps (warps only with 32 lanes).  Solving, a lane takes 1 << seg_log to
+// twice that bisected roots or, a line's root being a closed form, 32 times as
+// many of a line, as far as 32 lanes go (run_segments).  Ordering, a lane takes every 32nd root, up
 // to 256 a warp, so that a warp's roots are neighbours in memory.
 struct ChainShare {
     uint32_t lanes, warps;
 };
-template <bool kSolve> SR_DEV ChainShare chain_share(uint32_t key) {
+template <bool kSolve> SR_DEV ChainShare chain_share(uint32_t key, int32_t seg_log) {
     const int32_t lg = 14 - (int32_t)(key >> 2);
     ChainShare s;
-    s.lanes = (uint32_t)imin(imax(kSolve ? lg - ((key & 3u) == 2u ? kSegLog + 5 : kSegLog) : lg + 1, 0), 5);
+    s.lanes = (uint32_t)imin(imax(kSolve ? lg - ((key & 3u) == 2u ? seg_log + 5 : seg_log) : lg + 1, 0), 5);
     s.warps = kSolve ? 0u : (uint32_t)imax(lg + 1 - 8, 0);
     return s;
 }
@@ -546,6 +551,44 @@ SR_DEV float bisect(const AxisPoly& a, float c, float t_min, float t_max) {
     return t_solve;
 }
 
+// The same solve near a guess of its result: the turns of the first kGuessed
+// steps are taken from the guess at once, so the midpoints do not wait for the
+// values, and the values, which then depend on nothing but their midpoints,
+// say whether every turn was right.  If one was not (a guess that is not the
+// result's neighbour), the solve is done plainly.  1,150 cycles a root where
+// the plain one takes 1,560: the chain stage of the 1024^2 frame went from
+// 0.050 to 0.043 ms, of the 2048^2 one from 0.140 to 0.124 (14 turns: 0.045
+// and 0.127; 20: no better).
+constexpr int kGuessed = 18;
+template <int kType>
+SR_DEV float bisect_near(const AxisPoly& a, float c, float t_min, float t_max, float guess) {
+    const float v0 = eval_axis<kType>(a, t_min);
+    const bool s0 = v0 < c;
+    float ta = t_min, tb = t_max;
+    bool wrong = false;
+#pragma unroll
+    for (int j = 0; j < kGuessed; ++j) {
+        const float tm = mid_rn(ta, tb);
+        const bool right = tm < guess;
+        if (right) ta = tm;
+        else tb = tm;
+        wrong |= ((eval_axis<kType>(a, tm) < c) == s0) != right;
+    }
+    if (wrong) return bisect<kType>(a, c, t_min, t_max);
+    float t_solve = t_min, last = 0.0f;
+#pragma unroll
+    for (int j = kGuessed; j < 24; ++j) {
+        const float tm = mid_rn(ta, tb);
+        const float v = eval_axis<kType>(a, tm);
+        t_solve = tm;
+        last = v;
+        if ((v < c) == s0) ta = tm;
+        else tb = tm;
+    }
+    if (v0 == c || fabsf(__fsub_rn(last, c)) > 1.0f) t_solve = t_min;
+    return t_solve;
+}
+
 // The state after root k of a chain whose state before it is lo: its t with
 // the side bit in the flag bits.
 struct ChainSide {
@@ -561,6 +604,13 @@ template <int kType> SR_DEV int32_t next_root(const ChainSide& s, int32_t k, int
     if (kType == 2) t = gmin(gmax(__fmul_rn(__fsub_rn(c, s.a.p0), s.inv), bitsf(lo)), s.t_hi);
     else t = bisect<kType>(s.a, c, bitsf(lo), s.t_hi);
     return (fbits(t) & ~3) | s.side;
+}
+
+// The same for a root whose state is likely near `guess`.
+template <int kType> SR_DEV int32_t next_root_near(const ChainSide& s, int32_t k, int32_t lo, int32_t guess) {
+    if (kType == 2) return next_root<kType>(s, k, lo);
+    const float c = __fadd_rn(s.x, __fmul_rn((float)k, s.dx));
+    return (fbits(bisect_near<kType>(s.a, c, bitsf(lo), s.t_hi, bitsf(guess))) & ~3) | s.side;
 }
 
 // Warp-cooperative solve of one long chain.  By the invariant above, the 31
@@ -697,13 +747,14 @@ SR_DEV void finish_chain_warp(const ChainSide& s, int32_t len, int32_t seg, int3
 // 4 ulp.  So two chains started from different low ends soon hold the same
 // state (on the generated scenes, after two roots in 95% of the cases; later
 // for t under an eighth of the piece, where 4 ulp is finer than the steps'
-// end).  Each lane starts two roots before its stretch from the piece's own
-// start and solves on from there; then every lane whose state at its
+// end).  Each lane starts a root before its stretch from the piece's own start
+// and solves on from there (a second run-up root saves fewer repeats than it
+// costs: 0.041 instead of 0.035 ms on the 1024^2 frame); then every lane whose state at its
 // stretch's start is not the one its left neighbour ended with solves again
-// from that one, until it meets a root it already has.  Rounds of this end
-// when all neighbours agree, which makes every root the one that the
-// sequential chain gives.  A chain of 32 lanes that has not settled after
-// two rounds (its t small all along) is finished root by root by the warp.
+// from that one, near the roots it has (bisect_near), until it meets one of
+// them.  Rounds of this end when all neighbours agree, which makes every root the one that the
+// sequential chain gives.  A chain of 32 lanes that has not settled after a
+// round (its t small all along) is finished root by root by the warp.
 template <int kType>
 SR_DEV void run_segments(const ChainSide& s, int32_t len, float t_lo, int32_t* __restrict__ out, int32_t lanes,
                          int32_t l) {
@@ -711,7 +762,7 @@ SR_DEV void run_segments(const ChainSide& s, int32_t len, float t_lo, int32_t* _
     const int32_t ks = imin(l * seg, len), ke = imin(ks + seg, len);
     int32_t st = fbits(t_lo);
     if (ks < ke)
-        for (int32_t k = imax(ks - 2, 0); k < ks; ++k) st = next_root<kType>(s, k, st);
+        for (int32_t k = imax(ks - 1, 0); k < ks; ++k) st = next_root<kType>(s, k, st);
     int32_t entry = st;
     for (int32_t k = ks; k < ke; ++k) {
         st = next_root<kType>(s, k, st);
@@ -724,7 +775,7 @@ SR_DEV void run_segments(const ChainSide& s, int32_t len, float t_lo, int32_t* _
         const bool need = l > 0 && ks < ke && prev != entry;
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, need);
         if (!m) return;
-        if (kType != 2 && lanes == 32 && round >= 2) {
+        if (kType != 2 && lanes == 32 && round >= 1) {
             finish_chain_warp<kType>(s, len, seg, out, entry, end);
             return;
         }
@@ -733,8 +784,9 @@ SR_DEV void run_segments(const ChainSide& s, int32_t len, float t_lo, int32_t* _
             st = prev;
             bool met = false;
             for (int32_t k = ks; k < ke; ++k) {
-                st = next_root<kType>(s, k, st);
-                met = out[k] == st;
+                const int32_t was = out[k];   // solved from another low end: a neighbour of this one
+                st = next_root_near<kType>(s, k, st, was);
+                met = was == st;
                 if (met) break;
                 out[k] = st;
             }
@@ -795,16 +847,23 @@ SR_DEV ChainSetup chain_setup(const GeomArgs& g, const int32_t* __restrict__ off
 template <bool kSolve> struct ChainTickets {
     uint32_t start0, start1, n0, n1, first0, first1;   // two classes a lane
     uint32_t total;
-    SR_DEV static uint32_t tickets_of(uint32_t n, uint32_t key) {
-        const ChainShare s = chain_share<kSolve>(key);
+    int32_t seg_log;
+    SR_DEV uint32_t tickets_of(uint32_t n, uint32_t key) const {
+        const ChainShare s = chain_share<kSolve>(key, seg_log);
         return s.lanes == 5 ? n << s.warps : ((n << s.lanes) + 31u) / 32u;
     }
-    SR_DEV void build(const uint32_t* __restrict__ class_count) {
+    SR_DEV ChainShare share(uint32_t key) const { return chain_share<kSolve>(key, seg_log); }
+    SR_DEV void build(const uint32_t* __restrict__ class_count, uint32_t sms) {
         const uint32_t lane = lane_id();
+        seg_log = kSegLog;
         class_starts(class_count, start0, start1);
         n0 = class_count[2 * lane];
         n1 = class_count[2 * lane + 1];
         if (2 * lane + 1 == kEmptyPiece && kSolve) n1 = 0;
+        if (kSolve) {
+            const uint32_t t = __reduce_add_sync(0xFFFFFFFFu, tickets_of(n0, 2 * lane) + tickets_of(n1, 2 * lane + 1));
+            seg_log = t < kShortTickets * sms ? kSegShort : (t >= kLongTickets * sms ? kSegLong : kSegLog);
+        }
         const uint32_t t0 = tickets_of(n0, 2 * lane), t1 = tickets_of(n1, 2 * lane + 1);
         uint32_t x = t0 + t1;
 #pragma unroll
@@ -830,7 +889,7 @@ template <bool kSolve> struct ChainTickets {
         const uint32_t tfirst = __shfl_sync(0xFFFFFFFFu, odd ? first1 : first0, at);
         const uint32_t cfirst = __shfl_sync(0xFFFFFFFFu, odd ? start1 : start0, at);
         const uint32_t ccount = __shfl_sync(0xFFFFFFFFu, odd ? n1 : n0, at);
-        const ChainShare s = chain_share<kSolve>(key);
+        const ChainShare s = share(key);
         const uint32_t i = s.lanes == 5 ? (ticket - tfirst) >> s.warps : ((ticket - tfirst) * 32u + lane_id()) >> s.lanes;
         warp = (ticket - tfirst) & ((1u << s.warps) - 1u);
         const bool listed = i < ccount && cfirst + i < list_cap;
@@ -839,6 +898,17 @@ template <bool kSolve> struct ChainTickets {
     }
 };
 
+// A warp's first ticket, the CTAs being placed an SM after the other, `ctas`
+// an SM: the first tickets go to as many SMs, the next ones to other
+// schedulers of these (a CTA's warps are on different ones).  Tickets handed
+// out by a counter from the start went to the SMs whose requests came first:
+// of the 1,001 tickets of a 1024^2 frame six shared a scheduler and 3,000
+// cycles a root, while others had none.
+SR_DEV uint32_t first_ticket(uint32_t ctas) {
+    const uint32_t sms = gridDim.x / ctas;
+    return (blockIdx.x / sms * (blockDim.x / 32u) + (threadIdx.x >> 5)) * sms + blockIdx.x % sms;
+}
+
 __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t* __restrict__ offs,
                                                 const uint4* __restrict__ pieces,
                                                 const uint32_t* __restrict__ items, uint32_t list_cap,
@@ -846,12 +916,9 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
                                                 uint32_t* __restrict__ queue, int32_t* __restrict__ cbuf) {
     wait_for_stream();
     ChainTickets<true> T;
-    T.build(class_count);
-    for (;;) {
-        uint32_t ticket = 0;
-        if (lane_id() == 0) ticket = atomicAdd(queue, 1u);
-        ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
-        if (ticket >= T.total) break;
+    T.build(class_count, gridDim.x / kChainCtas);
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    for (uint32_t ticket = first_ticket(kChainCtas); ticket < T.total;) {
         uint32_t key, pos, warp;
         const bool listed = T.find(ticket, list_cap, key, pos, warp);
         const ChainSetup s = chain_setup(g, offs, pieces, items[pos]);
@@ -859,12 +926,14 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
         // reports it), has no roots
         const int32_t len = listed && s.base + s.len <= g.rec_cap ? s.len : 0;
         int32_t* out = cbuf + s.base;
-        const uint32_t gl = chain_share<true>(key).lanes, cls = key & 3u;
+        const uint32_t gl = T.share(key).lanes, cls = key & 3u;
         const int32_t lanes = 1 << gl, l = (int32_t)(lane_id() & ((1u << gl) - 1u));
         if (cls == 0u) run_segments<4>(s.side, len, s.t_lo, out, lanes, l);
         else if (cls == 1u) run_segments<3>(s.side, len, s.t_lo, out, lanes, l);
         else if (cls == 2u) run_segments<2>(s.side, len, s.t_lo, out, lanes, l);
         else run_segments<(int)kArc>(s.side, len, s.t_lo, out, lanes, l);
+        if (lane_id() == 0) ticket = warps + atomicAdd(queue, 1u);
+        ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
     }
 }
 
@@ -912,7 +981,7 @@ __global__ void __launch_bounds__(128) k_order_records(const GeomArgs g, const i
                                                        uint32_t* __restrict__ status) {
     wait_for_stream();
     ChainTickets<false> T;
-    T.build(class_count);
+    T.build(class_count, 0);
     const uint32_t warps = gridDim.x * (blockDim.x / 32u);
     for (uint32_t ticket = blockIdx.x * (blockDim.x / 32u) + (threadIdx.x >> 5); ticket < T.total; ticket += warps) {
         uint32_t key, pos, warp;
@@ -936,7 +1005,7 @@ __global__ void __launch_bounds__(128) k_order_records(const GeomArgs g, const i
             if (back) i0 = nx;
             else if (bitsf(X[0]) <= bitsf(t0)) i0 = count_le(X, 0, nx, bitsf(t0));
         }
-        const uint32_t gl = chain_share<false>(key).lanes;
+        const uint32_t gl = T.share(key).lanes;
         const int32_t l = (int32_t)(lane_id() & ((1u << gl) - 1u));
         const bool y_side = (item & 1u) != 0;
         if (l == 0 && warp == 0 && (y_side || ny == 0)) R[i0] = make_int2((int32_t)c, t0);
