@@ -291,13 +291,11 @@ struct Pipeline {
     uint32_t S = 0, V = 0, C = 0, P = 0;
     int32_t Wmax = 1, Hmax = 1;
     uint32_t total_rows = 0, res_ctas = 0;
+    int res_seg = sr::kResolveSeg;
     uint64_t total_pixels = 0;
     std::vector<sr::SceneInfo> info;
     std::vector<uint32_t> cta_base;
-    std::vector<uint8_t> cta_narrow;
-    bool any_narrow = false, any_wide = false;
     DevBuf pos, pos_path, curve_pos, curve_type, curve_path, fill_rule, fill_info, path_scene, scenes_d, cta_base_d;
-    DevBuf cta_narrow_d;
     // frame
     DevBuf tpos, curve_end, path_begin, cut, count, offs, pieces, chain_lists;
     // what starts a frame zeroed, cleared by one memset each: before the count
@@ -356,7 +354,7 @@ struct Pipeline {
                          &pieces, &chain_lists, &cbuf, &rec, &keys, &keys_alt,
                          &wnp, &skeys, &svals, &vals_alt, &sort_scratch, &wind_sums, &draw, &draw_row, &draw_list,
                          &rkeys, &rvals, &rkeys_alt, &rvals_alt, &row_sort_scratch, &row_start, &image, &d_fkey, &d_fwn, &d_fleft, &d_wscan, &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw,
-                         &feats, &preds, &allot, &plan_tot, &judge_out, &seg_tiles, &cta_narrow_d, &paints_d, &aa_acc, &fill_rule_kept, &fill_info_kept};
+                         &feats, &preds, &allot, &plan_tot, &judge_out, &seg_tiles, &paints_d, &aa_acc, &fill_rule_kept, &fill_info_kept};
         for (DevBuf* b : all) release(*b);
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
@@ -439,8 +437,7 @@ struct Pipeline {
         Wmax = 1;
         Hmax = 1;
         cta_base.assign(S + 1, 0);
-        cta_narrow.clear();
-        any_narrow = any_wide = false;
+        uint64_t segs = 0;   // of kResolveSeg pixels
         for (uint32_t s = 0; s < S; ++s) {
             sr::SceneInfo& si = info[s];
             si.rows = (uint32_t)((si.H + F - 1) / F);
@@ -450,29 +447,29 @@ struct Pipeline {
             total_pixels += (uint64_t)si.W * (uint64_t)si.H;
             Wmax = std::max(Wmax, si.W);
             Hmax = std::max(Hmax, si.H);
+            segs += (uint64_t)si.rows * (uint64_t)((si.W + sr::kResolveSeg - 1) / sr::kResolveSeg);
+        }
+        res_seg = sr::resolve_segment(segs, mode == SR_MODE_PIXEL, sm_count);
+        for (uint32_t s = 0; s < S; ++s) {
+            const sr::SceneInfo& si = info[s];
             cta_base[s] = res_ctas;
-            uint32_t rpc = sr::resolve_rows_per_cta(si.W, tune.resolve_warps);
-            res_ctas += (si.rows + rpc - 1) / rpc;
-            cta_narrow.resize(res_ctas, rpc > 1 ? 1 : 0);
-            (rpc > 1 ? any_narrow : any_wide) = true;
+            res_ctas += sr::resolve_ctas(si.W, si.rows, mode == SR_MODE_PIXEL, res_seg, tune.resolve_warps);
         }
         cta_base[S] = res_ctas;
         CUDA_TRY(ensure(scenes_d, sizeof(sr::SceneInfo) * std::max<uint32_t>(S, 1)));
         CUDA_TRY(ensure(cta_base_d, sizeof(uint32_t) * (S + 1)));
         CUDA_TRY(ensure(image, 4 * std::max<uint64_t>(total_pixels, 1)));
-        CUDA_TRY(ensure(cta_narrow_d, std::max<size_t>(res_ctas, 1)));
         if (!flush) return SR_OK;   // upload() stages the table with the scenes
         SR_TRY(stage_reserve(table_stage_bytes()));
         stage_table();
         return stage_flush();
     }
     size_t table_stage_bytes() const {
-        return staged_size(sizeof(sr::SceneInfo) * S) + staged_size(sizeof(uint32_t) * (S + 1)) + staged_size(res_ctas);
+        return staged_size(sizeof(sr::SceneInfo) * S) + staged_size(sizeof(uint32_t) * (S + 1));
     }
     void stage_table() {
         stage(scenes_d.p, info.data(), sizeof(sr::SceneInfo) * S);
         stage(cta_base_d.p, cta_base.data(), sizeof(uint32_t) * (S + 1));
-        stage(cta_narrow_d.p, cta_narrow.data(), res_ctas);
     }
 
     sr_status upload(const HostScenes& h) {
@@ -784,8 +781,7 @@ struct Pipeline {
             &Pipeline::rkeys_alt, &Pipeline::rvals_alt, &Pipeline::row_sort_scratch, &Pipeline::row_start,
             &Pipeline::image,
             &Pipeline::path_first, &Pipeline::path_draw, &Pipeline::feats, &Pipeline::preds, &Pipeline::allot,
-            &Pipeline::plan_tot, &Pipeline::judge_out, &Pipeline::seg_tiles,
-            &Pipeline::cta_narrow_d};
+            &Pipeline::plan_tot, &Pipeline::judge_out, &Pipeline::seg_tiles};
         *moved = false;
         CUDA_TRY(cudaSetDevice(device));
         for (DevBuf Pipeline::* b : bufs) {
@@ -818,7 +814,7 @@ struct Pipeline {
                                &d_fwn, &d_fleft,
                                &d_wscan,
                                &d_fflag, &d_sflag, &d_skey, &path_first, &path_draw, &feats, &preds, &allot,
-                               &plan_tot, &judge_out, &seg_tiles, &cta_narrow_d, &fill_rule_kept, &fill_info_kept};
+                               &plan_tot, &judge_out, &seg_tiles, &fill_rule_kept, &fill_info_kept};
         uint64_t t = 0;
         for (const DevBuf* b : all) t += b->cap;
         return t;
@@ -975,14 +971,12 @@ struct Pipeline {
         ra.n_scenes = S;
         ra.F = F;
         ra.warps = tune.resolve_warps;
+        ra.seg = res_seg;
         ra.pixel_mode = g.pixel_mode;
         ra.image = image.as<uint32_t>();
         ra.seg_cut = wa.seg_cut;
         ra.cut_segs = cut_segs();
         ra.row_px = wa.row_px;
-        ra.cta_narrow = cta_narrow_d.as<uint8_t>();
-        ra.any_narrow = any_narrow ? 1 : 0;
-        ra.any_wide = any_wide ? 1 : 0;
         ra.paints = n_paints ? paints_d.as<DevPaint>() : nullptr;
         ra.n_paints = n_paints;
         mark(ST_RESOLVE, false);
@@ -1428,14 +1422,12 @@ sr_status sr_render_draw_list(sr_ctx* c, const int32_t* records, int64_t n, void
     ra.n_scenes = p.S;
     ra.F = p.F;
     ra.warps = p.tune.resolve_warps;
+    ra.seg = p.res_seg;
     ra.pixel_mode = p.mode == SR_MODE_PIXEL;
     ra.image = p.image.as<uint32_t>();
     ra.seg_cut = nullptr;
     ra.cut_segs = 0;
     ra.row_px = nullptr;
-    ra.cta_narrow = p.cta_narrow_d.as<uint8_t>();
-    ra.any_narrow = p.any_narrow ? 1 : 0;
-    ra.any_wide = p.any_wide ? 1 : 0;
     ra.paints = p.n_paints ? p.paints_d.as<sr::DevPaint>() : nullptr;
     ra.n_paints = p.n_paints;
     sr::launch_resolve(ra, p.res_ctas, st);

@@ -294,8 +294,8 @@ __host__ __device__ __forceinline__ int32_t fill_paint(uint32_t info) {
     return (info >> 24) == 0u && (info & 0x00FFFFFFu) != 0u ? (int32_t)(info & 0x00FFFFFFu) - 1 : -1;
 }
 
-// Resolve work: each CTA paints rows_per_cta cell rows of one scene;
-// cta_base[s] is the first CTA of scene s (host-built, n_scenes+1 entries).
+// Resolve work: a CTA paints segments or rows of one scene; cta_base[s] is the
+// first CTA of scene s (host-built, n_scenes+1 entries).
 struct ResolveArgs {
     const int4* draw;
     const uint32_t* row_sorted_idx;   // draw indices sorted by global cell row
@@ -306,18 +306,20 @@ struct ResolveArgs {
     int32_t F;
     int32_t pixel_mode;
     int32_t warps;                    // warps per CTA: 8 or 16
+    int32_t seg;                      // pixels per warp: kResolveSeg, or 128 or 64 (pixel mode)
     uint32_t* image;                  // all scenes' RGBA8 framebuffers
     const uint32_t* seg_cut;          // [rows][cut_segs] from the emit, or NULL
     const unsigned long long* row_px; // [rows] summed record widths from the emit, or NULL (every row searched)
     uint32_t cut_segs;
-    const uint8_t* cta_narrow;        // [CTAs] 1 for a CTA of several rows
-    int any_narrow, any_wide;         // some CTA is, some is not (pixel mode has a kernel for each)
     const DevPaint* paints;           // gradient paints of the scene (single-scene contexts), or NULL
     uint32_t n_paints;
 };
-// Pixels per warp of a resolve CTA.
+// Pixels per warp of the resolve (of a large frame), and of a cut.
 constexpr int kResolveSeg = 256;
-uint32_t resolve_rows_per_cta(int32_t W, int warps);
+// Pixels per warp for a frame of `segs` segments of kResolveSeg pixels.
+int resolve_segment(uint64_t segs, int pixel_mode, int sm_count);
+// CTAs that a scene of `rows` cell rows takes.
+uint32_t resolve_ctas(int32_t W, uint32_t rows, int pixel_mode, int seg, int warps);
 void launch_resolve(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st);
 // Multisampling: sum a sample frame into acc (first: start the sums), and
 // write the rounded averages of k frames.

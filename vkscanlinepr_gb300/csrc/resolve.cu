@@ -6,12 +6,12 @@
 // [x, x+width) x [y, y+FRAG_SIZE), the framebuffer is cleared to white, and
 // records land in draw order.  Reference mode overwrites (blending is off in
 // the reference pipeline); pixel mode composites source-over with integer
-// arithmetic.  Draw records are first sorted stably by cell row (onesweep),
-// so a CTA owns one cell row (or several short ones), stages its records in
-// shared memory, and applies them in path order; a thread owns a fixed set
-// of pixels, so no barrier is needed between records.  In pixel mode a warp
-// first finds where its 256-pixel segment's painting may start (the
-// collapse cut below) and skips the records before it.
+// arithmetic.  Draw records are first sorted stably by cell row (onesweep), so
+// a row's records are applied in path order; a thread owns a fixed set of
+// pixels, so no barrier is needed between records.  In pixel mode a warp paints
+// a segment of a row and first finds where its painting may start (the collapse
+// cut below); in reference mode a CTA owns one cell row (or several short ones)
+// and stages its records in shared memory.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -44,8 +44,9 @@ __global__ void k_row_bounds(const uint32_t* __restrict__ srows, int64_t n_cap, 
 // (checked exhaustively by the CPU tests).  Alpha stays 255:
 // (255*a + 255*(255-a) + 127) / 255 = 255.
 constexpr float kRound = 12582912.0f;   // 1.5 * 2^23
-constexpr int kK = kResolveSeg / 32;   // pixels per lane; a warp owns kResolveSeg pixels
+constexpr int kK = kResolveSeg / 32;   // pixels per lane of a whole segment
 constexpr int kChunk = 1024;
+constexpr uint64_t kHalfSegs = 200, kQuarterSegs = 40;   // segments of kResolveSeg an SM
 
 struct PixRec {
     int32_t x0, x1;     // [x0, x1) clipped to >= 0
@@ -65,17 +66,32 @@ template <class Rec> SR_DEV void blend3(uint32_t& rb, float& g, const Rec& q) {
     g = __fsub_rn(__fmaf_rn(ug, 1.0f / 255.0f, kRound), kRound);
 }
 
-uint32_t resolve_rows_per_cta(int32_t W, int warps) {
-    int32_t segs = (W + kResolveSeg - 1) / kResolveSeg;
-    return segs >= warps ? 1u : (uint32_t)(warps / segs);
+int resolve_segment(uint64_t segs, int pixel_mode, int sm_count) {
+    const uint64_t sms = (uint64_t)(sm_count > 0 ? sm_count : 1);
+    if (!pixel_mode || segs >= kHalfSegs * sms) return kResolveSeg;
+    return segs >= kQuarterSegs * sms ? kResolveSeg / 2 : kResolveSeg / 4;
 }
 
-// Which rows and segment a warp paints: a CTA holds rows_per_cta cell rows
-// of one scene; small canvases give each row fewer warps than the CTA has.
-// A warp skips the records before the last one that covers its whole
-// segment and hides what is under it (seg_cut, written by the emit): source-
-// over with a = 255 gives floor((255 s + 127) / 255) = s whatever the pixel
-// held, and an overwrite leaves nothing of it either.
+uint32_t resolve_ctas(int32_t W, uint32_t rows, int pixel_mode, int seg, int warps) {
+    const uint32_t segs = (uint32_t)((W + seg - 1) / seg);
+    if (pixel_mode) return (rows * segs + (uint32_t)warps - 1) / (uint32_t)warps;
+    const uint32_t rpc = segs >= (uint32_t)warps ? 1u : (uint32_t)warps / segs;
+    return (rows + rpc - 1) / rpc;
+}
+
+SR_DEV uint32_t scene_of_cta(const ResolveArgs& a) {   // last s with cta_base[s] <= blockIdx.x
+    uint32_t lo = 0, hi = a.n_scenes;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (a.cta_base[mid] <= blockIdx.x) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Reference mode: which rows and segment a warp paints.  A CTA holds
+// rows_per_cta cell rows of one scene; small canvases give each row fewer
+// warps than the CTA has.
 struct ResolveWork {
     const SceneInfo* si;
     int32_t W, r0, nr, segs, groups, my_row;
@@ -84,13 +100,7 @@ struct ResolveWork {
 
 template <int WARPS> SR_DEV ResolveWork resolve_work(const ResolveArgs& a) {
     constexpr int kResolveWarps = WARPS;
-    // scene of this CTA: last s with cta_base[s] <= blockIdx.x
-    uint32_t lo = 0, hi = a.n_scenes;
-    while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (a.cta_base[mid] <= blockIdx.x) lo = mid;
-        else hi = mid;
-    }
+    const uint32_t lo = scene_of_cta(a);
     ResolveWork w;
     w.si = &a.scenes[lo];
     w.W = w.si->W;
@@ -111,10 +121,12 @@ template <int WARPS> SR_DEV ResolveWork resolve_work(const ResolveArgs& a) {
     return w;
 }
 
-SR_DEV uint32_t resolve_cut(const ResolveArgs& a, const ResolveWork& w, int32_t seg, bool live) {
-    if (!a.seg_cut || !live) return 0u;
-    return a.seg_cut[(size_t)(w.si->row_base + (uint32_t)(w.r0 + w.my_row)) * a.cut_segs +
-                     (uint32_t)(seg / kResolveSeg)];
+// A warp skips the records before the last one that covers its whole segment
+// and hides what is under it (seg_cut, written by the emit): source-over with
+// a = 255 gives floor((255 s + 127) / 255) = s whatever the pixel held, and an
+// overwrite leaves nothing of it either.
+SR_DEV uint32_t resolve_cut(const ResolveArgs& a, uint32_t global_row, int32_t seg) {
+    return a.seg_cut ? a.seg_cut[(size_t)global_row * a.cut_segs + (uint32_t)(seg / kResolveSeg)] : 0u;
 }
 
 template <int WARPS> SR_DEV int32_t resolve_seg(const ResolveWork& w, int group) {
@@ -227,12 +239,13 @@ template <bool GRAD> SR_DEV PixRec pix_rec(const int4 d, uint32_t di) {
 // A gradient record: each lane blends its covered pixels with the paint's
 // colour at their centres (row centre yc); a paint the table lacks paints
 // nothing.
+template <int K>
 SR_DEV void apply_gradient(const ResolveArgs& a, const PixRec& pr, int32_t seg, int lane, float yc,
-                           uint32_t (&rb)[kK], float (&g)[kK]) {
+                           uint32_t (&rb)[K], float (&g)[K]) {
     if (!a.paints || pr.sab >= a.n_paints) return;
     const DevPaint& P = a.paints[pr.sab];
 #pragma unroll
-    for (int j = 0; j < kK; ++j) {
+    for (int j = 0; j < K; ++j) {
         const int32_t p = seg + lane + 32 * j;
         if (p >= pr.x0 && p < pr.x1) {
             const uint32_t col = paint_color(P, __fadd_rn((float)p, 0.5f), yc);
@@ -244,32 +257,32 @@ SR_DEV void apply_gradient(const ResolveArgs& a, const PixRec& pr, int32_t seg, 
 // A record on this warp's segment: a one-pixel record is a uniform branch on
 // its register slot; a record over the whole segment blends every slot;
 // otherwise each lane tests its pixels.
-template <bool GRAD>
-SR_DEV void apply_pix(const ResolveArgs& a, const PixRec& pr, int32_t seg, int lane, float yc, uint32_t (&rb)[kK],
-                      float (&g)[kK]) {
+template <bool GRAD, int K>
+SR_DEV void apply_pix(const ResolveArgs& a, const PixRec& pr, int32_t seg, int lane, float yc, uint32_t (&rb)[K],
+                      float (&g)[K]) {
     if (GRAD && pr.iau == kGradient) {
         apply_gradient(a, pr, seg, lane, yc, rb, g);
-    } else if (pr.x1 - pr.x0 == 1) {
+    } else if (K == 8 && pr.x1 - pr.x0 == 1) {
         const int32_t off = pr.x0 - seg;
         const int j = off >> 5;
         if (lane == (off & 31)) {
             switch (j) {
                 case 0: blend3(rb[0], g[0], pr); break;
-                case 1: blend3(rb[1], g[1], pr); break;
-                case 2: blend3(rb[2], g[2], pr); break;
-                case 3: blend3(rb[3], g[3], pr); break;
-                case 4: blend3(rb[4], g[4], pr); break;
-                case 5: blend3(rb[5], g[5], pr); break;
-                case 6: blend3(rb[6], g[6], pr); break;
-                default: blend3(rb[7], g[7], pr); break;
+                case 1: blend3(rb[1 % K], g[1 % K], pr); break;
+                case 2: blend3(rb[2 % K], g[2 % K], pr); break;
+                case 3: blend3(rb[3 % K], g[3 % K], pr); break;
+                case 4: blend3(rb[4 % K], g[4 % K], pr); break;
+                case 5: blend3(rb[5 % K], g[5 % K], pr); break;
+                case 6: blend3(rb[6 % K], g[6 % K], pr); break;
+                default: blend3(rb[7 % K], g[7 % K], pr); break;
             }
         }
-    } else if (pr.x0 <= seg && pr.x1 >= seg + kResolveSeg) {
+    } else if (pr.x0 <= seg && pr.x1 >= seg + 32 * K) {
 #pragma unroll
-        for (int j = 0; j < kK; ++j) blend3(rb[j], g[j], pr);
+        for (int j = 0; j < K; ++j) blend3(rb[j], g[j], pr);
     } else {
 #pragma unroll
-        for (int j = 0; j < kK; ++j) {
+        for (int j = 0; j < K; ++j) {
             int32_t p = seg + lane + 32 * j;
             if (p >= pr.x0 && p < pr.x1) blend3(rb[j], g[j], pr);
         }
@@ -387,43 +400,67 @@ struct RunWalk {
     }
 };
 
-template <bool GRAD> SR_DEV void stage_pix(const ResolveArgs& a, PixRec* sq, int32_t c0, int32_t cnt) {
-    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-        const uint32_t di = a.row_sorted_idx[c0 + q];
-        sq[q] = pix_rec<GRAD>(a.draw[di], di);
-    }
-}
-
-SR_DEV void init_pix(uint32_t (&rb)[kK], float (&g)[kK]) {
+template <int K> SR_DEV void init_pix(uint32_t (&rb)[K], float (&g)[K]) {
 #pragma unroll
-    for (int j = 0; j < kK; ++j) {
+    for (int j = 0; j < K; ++j) {
         rb[j] = 0x00FF00FFu;
         g[j] = 255.0f;
     }
 }
 
-SR_DEV void store_pix(const ResolveArgs& a, const ResolveWork& w, int32_t seg, int lane, const uint32_t (&rb)[kK],
-                      const float (&g)[kK]) {
-    uint32_t* out = a.image + w.si->image_off + (size_t)(w.r0 + w.my_row) * w.W;
+template <int K>
+SR_DEV void store_pix(uint32_t* __restrict__ row, int32_t W, int32_t seg, int lane, const uint32_t (&rb)[K],
+                      const float (&g)[K]) {
 #pragma unroll
-    for (int j = 0; j < kK; ++j) {
+    for (int j = 0; j < K; ++j) {
         int32_t p = seg + lane + 32 * j;
-        if (p < w.W) out[p] = rb[j] | ((uint32_t)__float2int_rn(g[j]) << 8) | 0xFF000000u;
+        if (p < W) row[p] = rb[j] | ((uint32_t)__float2int_rn(g[j]) << 8) | 0xFF000000u;
     }
 }
 
-// A CTA of several short rows (a canvas narrower than WARPS segments): each
-// warp finds its cut and streams its own row's records 32 at a time through
-// its own shared-memory slots, without waiting for the other warps.
-template <bool GRAD>
-SR_DEV void resolve_pixel_rows(const ResolveArgs& a, const ResolveWork& w, int32_t seg, PixRec* slot, RunBuf& buf) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t r = w.si->row_base + (uint32_t)(w.r0 + w.my_row);
+// A warp paints one segment of one row, by itself: it finds its cut and
+// streams the row's records from there, 32 at a time, through its own
+// shared-memory slots.  The warps of a CTA mostly share a row, so the records
+// come from L1, and no warp waits for another.  (A CTA a row that staged the
+// row's last 1,024 records for its warps, beside a kernel like this one for
+// canvases narrower than the CTA, each with a grid over all rows: 0.160 ms for
+// the 4096^2 frame and 0.70 for 64 uneven scenes, against 0.121 and 0.50.
+// Blank canvases took 0.257 of the 0.70, now 0.131.)  Instructions bound it,
+// some 20 a record and 7 a record and 32 pixels, and in a small frame the
+// latency of a row's records one after the other.
+//
+// So a warp's segment is shorter when the frame has few: 256 pixels, 128 below
+// 200 such segments an SM, 64 below 40.  With 256 / 128 / 64 the kernel took,
+// in ms: 4096^2 frame of 20,000 paths (431 segments an SM) 0.121 / 0.188 /
+// 0.354, 2048^2 frame of 5,000 (108) 0.078 / 0.060 / 0.076, of 3,000 stars
+// 0.070 / 0.060 / 0.078, 1024^2 frame of 3,000 (27) 0.109 / 0.080 / 0.059, of
+// 500 stars 0.0184 / 0.0164 / 0.0164, 512^2 frame of 3,000 0.144 / 0.106 /
+// 0.076, 256^2 frame of 3,000 0.301 / 0.180 / 0.147.  (Chosen by the scene in a
+// batch, the narrow ones at 128: 0.51 instead of 0.50.)
+template <int WARPS, int K, bool GRAD>
+__global__ void __launch_bounds__(32 * WARPS, (GRAD ? 32 : K == 8 ? 40 : 48) / WARPS) k_resolve_pixel(const ResolveArgs a) {
+    wait_for_stream();
+    constexpr int kSeg = 32 * K;
+    static_assert(kResolveSeg % kSeg == 0, "a cut covers whole segments");
+    __shared__ PixRec slots[WARPS * 32];
+    __shared__ RunBuf bufs[WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t scene = scene_of_cta(a);
+    const SceneInfo* si = &a.scenes[scene];
+    const int32_t W = si->W;
+    const uint32_t segs = (uint32_t)(W + kSeg - 1) / kSeg;
+    const uint32_t item = (blockIdx.x - a.cta_base[scene]) * WARPS + (uint32_t)warp;
+    const uint32_t y = item / segs;
+    if (y >= si->rows) return;
+    const int32_t seg = (int32_t)(item - y * segs) * kSeg;
+    PixRec* slot = slots + warp * 32;
+    RunBuf& buf = bufs[warp];
+    const uint32_t r = si->row_base + y;
     const int32_t beg = a.row_start[r], end = a.row_start[r + 1];
-    const int32_t segend = imin(seg + kResolveSeg, w.W);
-    const uint32_t cut = resolve_cut(a, w, seg, true);
+    const int32_t segend = imin(seg + kSeg, W);
+    const uint32_t cut = resolve_cut(a, r, seg);
     int32_t start = beg;
-    if (row_searched(a, r, w.W)) {
+    if (row_searched(a, r, W)) {
         RunWalk rw;
         const int32_t lim = imax(beg, end - kChunk);
         bool found = false;
@@ -434,7 +471,7 @@ SR_DEV void resolve_pixel_rows(const ResolveArgs& a, const ResolveWork& w, int32
             if (q >= lim) {
                 const uint32_t di = a.row_sorted_idx[q];
                 pr = pix_rec<GRAD>(a.draw[di], di);
-                ov = pr.x0 < seg + kResolveSeg && pr.x1 > seg;
+                ov = pr.x0 < seg + kSeg && pr.x1 > seg;
                 // a gradient's colour varies over the segment: it ends a run
                 cover = pr.x0 <= seg && pr.x1 >= segend && pr.iau != kGradient;
             }
@@ -442,17 +479,17 @@ SR_DEV void resolve_pixel_rows(const ResolveArgs& a, const ResolveWork& w, int32
         }
         if (found || rw.close(lane, buf)) start = rw.cut;
     }
-    uint32_t rb[kK];
-    float g[kK];
-    init_pix(rb, g);
-    const float yc = __fadd_rn((float)(w.r0 + w.my_row), 0.5f);
+    uint32_t rb[K];
+    float g[K];
+    init_pix<K>(rb, g);
+    const float yc = __fadd_rn((float)y, 0.5f);
     for (int32_t c0 = start; c0 < end; c0 += 32) {
         const int32_t q = c0 + lane;
         bool ov = false;
         if (q < end) {
             const uint32_t di = a.row_sorted_idx[q];
             const PixRec pr = pix_rec<GRAD>(a.draw[di], di);
-            ov = pr.x0 < seg + kResolveSeg && pr.x1 > seg && pr.idx1 >= cut;
+            ov = pr.x0 < seg + kSeg && pr.x1 > seg && pr.idx1 >= cut;
             if (ov) slot[lane] = pr;
         }
         uint32_t m = __ballot_sync(0xFFFFFFFFu, ov);
@@ -460,111 +497,11 @@ SR_DEV void resolve_pixel_rows(const ResolveArgs& a, const ResolveWork& w, int32
         while (m) {
             const PixRec p = slot[__ffs(m) - 1];
             m &= m - 1;
-            apply_pix<GRAD>(a, p, seg, lane, yc, rb, g);
+            apply_pix<GRAD, K>(a, p, seg, lane, yc, rb, g);
         }
         __syncwarp();
     }
-    store_pix(a, w, seg, lane, rb, g);
-}
-
-// CTAs of several rows (canvases narrower than WARPS segments) run the path
-// above in their own kernel, with little shared memory; the kernel below
-// skips them.  The two run one after the other over the same grid.
-//
-// A CTA per cell row (a canvas of at least half as many segments as the CTA
-// has warps; warps beyond the row's segments idle): the row's last kChunk
-// records are staged once, every warp finds its segment's cut in them, and the CTA
-// stages from the earliest cut on (chunks end-aligned, so the last one is
-// the chunk already staged); a warp skips the records before its own cut.
-template <int WARPS, bool GRAD>
-__global__ void __launch_bounds__(32 * WARPS) k_resolve_pixel_rows(const ResolveArgs a) {
-    wait_for_stream();
-    __shared__ PixRec slots[WARPS * 32];
-    __shared__ RunBuf bufs[WARPS];
-    if (!a.cta_narrow[blockIdx.x]) return;
-    const ResolveWork w = resolve_work<WARPS>(a);
-    const int warp = threadIdx.x >> 5;
-    if (w.active) resolve_pixel_rows<GRAD>(a, w, resolve_seg<WARPS>(w, 0) * kResolveSeg, slots + warp * 32, bufs[warp]);
-}
-
-template <int WARPS, bool GRAD>
-__global__ void __launch_bounds__(32 * WARPS) k_resolve_pixel(const ResolveArgs a) {
-    wait_for_stream();
-    if (a.any_narrow && a.cta_narrow[blockIdx.x]) return;   // k_resolve_pixel_rows
-    __shared__ PixRec sq[kChunk];
-    __shared__ RunBuf bufs[WARPS];
-    __shared__ int32_t cta_start[2];   // by group parity: a warp may still read the last group's
-    const ResolveWork w = resolve_work<WARPS>(a);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int32_t W = w.W;
-    const uint32_t r = w.si->row_base + (uint32_t)w.r0;
-    const int32_t beg = a.row_start[r], end = a.row_start[r + 1];
-    const int32_t tail0 = imax(beg, end - kChunk);
-    const bool search = row_searched(a, r, W);
-    bool tail_staged = false;   // sq holds [tail0, end)
-    if (search) {
-        stage_pix<GRAD>(a, sq, tail0, end - tail0);
-        tail_staged = true;
-    }
-    for (int group = 0; group < w.groups; ++group) {
-        const int32_t seg = resolve_seg<WARPS>(w, group) * kResolveSeg;
-        const bool live = w.active && seg < W;   // a row of fewer segments than warps leaves some idle
-        int32_t start = beg, s0 = beg;
-        if (search) {
-            if (threadIdx.x == 0) cta_start[group & 1] = end;
-            __syncthreads();
-            if (live) {
-                const int32_t segend = imin(seg + kResolveSeg, W);
-                RunWalk rw;
-                bool found = false;
-                for (int32_t c1 = end - tail0; c1 > 0 && !found; c1 -= 32) {
-                    const int32_t i = c1 - 32 + lane;
-                    bool ov = false, cover = false;
-                    if (i >= 0) {
-                        const int32_t x0 = sq[i].x0, x1 = sq[i].x1;
-                        ov = x0 < seg + kResolveSeg && x1 > seg;
-                        cover = x0 <= seg && x1 >= segend && sq[i].iau != kGradient;
-                    }
-                    found = rw.feed(__ballot_sync(0xFFFFFFFFu, ov), __ballot_sync(0xFFFFFFFFu, cover),
-                                    sq[i < 0 ? 0 : i], tail0 + i, lane, bufs[warp]);
-                }
-                if (found || rw.close(lane, bufs[warp])) start = rw.cut;
-                if (lane == 0) atomicMin(&cta_start[group & 1], start);
-            }
-            __syncthreads();
-            s0 = cta_start[group & 1];
-        }
-        const uint32_t cut = resolve_cut(a, w, seg, live);
-        uint32_t rb[kK];
-        float g[kK];
-        init_pix(rb, g);
-        const float yc = __fadd_rn((float)w.r0, 0.5f);
-        const int32_t nchunks = (end - s0 + kChunk - 1) / kChunk;
-        for (int k = nchunks - 1; k >= 0; --k) {
-            const int32_t c0 = imax(s0, end - (k + 1) * kChunk), c1 = end - k * kChunk;
-            const int32_t base = k ? c0 : tail0;
-            if (k || !tail_staged) {
-                __syncthreads();
-                stage_pix<GRAD>(a, sq, base, c1 - base);
-                __syncthreads();
-                tail_staged = k == 0;
-            }
-            if (!live) continue;
-            const int32_t hi = c1 - base;
-            for (int32_t g0 = imax(c0, start) - base; g0 < hi; g0 += 32) {
-                const int32_t qi = g0 + lane;
-                bool ov = false;
-                if (qi < hi) ov = sq[qi].x0 < seg + kResolveSeg && sq[qi].x1 > seg && sq[qi].idx1 >= cut;
-                uint32_t m = __ballot_sync(0xFFFFFFFFu, ov);
-                while (m) {
-                    const PixRec pr = sq[g0 + __ffs(m) - 1];
-                    m &= m - 1;
-                    apply_pix<GRAD>(a, pr, seg, lane, yc, rb, g);
-                }
-            }
-        }
-        if (live) store_pix(a, w, seg, lane, rb, g);
-    }
+    store_pix<K>(a.image + si->image_off + (size_t)y * W, W, seg, lane, rb, g);
 }
 
 // ------------------------------------------------------- reference mode --
@@ -589,7 +526,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_resolve_ref(const ResolveArgs a)
     for (int group = 0; group < w.groups; ++group) {
         const int32_t seg = resolve_seg<WARPS>(w, group) * kResolveSeg;
         const bool live = w.active && seg < W;
-        const uint32_t cut = resolve_cut(a, w, seg, live);
+        const uint32_t cut = live ? resolve_cut(a, w.si->row_base + (uint32_t)(w.r0 + w.my_row), seg) : 0u;
         uint32_t px[kK];
 #pragma unroll
         for (int j = 0; j < kK; ++j) px[j] = 0xFFFFFFFFu;
@@ -660,10 +597,9 @@ __global__ void __launch_bounds__(32 * WARPS) k_resolve_ref(const ResolveArgs a)
 
 template <int WARPS, bool GRAD> static void launch_resolve_t(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st) {
     if (a.pixel_mode) {
-        if (a.any_wide) launch_after(k_resolve_pixel<WARPS, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
-        // (not launch_after: placed early it takes the other kernel's SMs, 0.72
-        // instead of 0.70 ms in a batch of 64 uneven scenes)
-        if (a.any_narrow) k_resolve_pixel_rows<WARPS, GRAD><<<n_ctas, 32 * WARPS, 0, st>>>(a);
+        if (a.seg == 64) launch_after(k_resolve_pixel<WARPS, 2, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
+        else if (a.seg == 128) launch_after(k_resolve_pixel<WARPS, 4, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
+        else launch_after(k_resolve_pixel<WARPS, 8, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
     } else {
         launch_after(k_resolve_ref<WARPS, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
     }
@@ -671,7 +607,7 @@ template <int WARPS, bool GRAD> static void launch_resolve_t(const ResolveArgs& 
 
 void launch_resolve(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st) {
     if (n_ctas == 0) return;
-    count_launches(a.pixel_mode ? (a.any_wide ? 1 : 0) + (a.any_narrow ? 1 : 0) : 1);
+    count_launches(1);
     const bool grad = a.paints && a.n_paints;
     if (a.warps == 8) {
         if (grad) launch_resolve_t<8, true>(a, n_ctas, st);
