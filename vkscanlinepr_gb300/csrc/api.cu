@@ -12,6 +12,8 @@
 // enqueues without waiting, an overflow is detected on the device, and the
 // frame can be captured as a CUDA graph.  A single-scene context is a
 // one-scene batch.
+#include <cuda.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -268,6 +270,37 @@ static void append_scene(HostScenes& h, uint32_t w, uint32_t hgt, const sr_scene
     }
 }
 
+// Whether kernels on `device` may write `bytes` at p: device memory of that
+// device, all of it in one allocation, 4-byte aligned.  Anything else (another
+// device's memory, managed or host memory, a range that runs past its
+// allocation) is left to cudaMemcpyAsync, which copies or refuses it.
+static bool kernels_may_write(const void* p, size_t bytes, int device) {
+    if ((reinterpret_cast<uintptr_t>(p) & 3u) != 0) return false;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
+    using RangeFn = CUresult(CUDAAPI*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const RangeFn range = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 12000, cudaEnableDefault, &found) !=
+                cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<RangeFn>(fn);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr at_p = reinterpret_cast<CUdeviceptr>(p);
+    return range && range(&base, &size, at_p) == CUDA_SUCCESS && at_p - base <= size && bytes <= size - (at_p - base);
+}
+
+
 // --------------------------------------------------------------------------
 // The device pipeline of one set of scenes.
 struct Pipeline {
@@ -322,6 +355,7 @@ struct Pipeline {
         size_t off, bytes;
     };
     std::vector<StagedCopy> staged;
+    uint32_t* image2 = nullptr;     // device memory of the caller that the frame being enqueued goes to as well
     uint32_t* h_report = nullptr;   // pinned copy of the control block's report
     // results
     sr_stats stats{};
@@ -979,6 +1013,7 @@ struct Pipeline {
         ra.row_px = wa.row_px;
         ra.paints = n_paints ? paints_d.as<DevPaint>() : nullptr;
         ra.n_paints = n_paints;
+        ra.image2 = image2;
         mark(ST_RESOLVE, false);
         launch_resolve(ra, res_ctas, st);
         mark(ST_RESOLVE, true);
@@ -1276,6 +1311,16 @@ sr_status sr_set_paints(sr_ctx* c, const sr_paint* paints, uint32_t n) {
 static sr_status render_core(sr_ctx* c, void* rgba_out, int out_is_device, cudaStream_t st) {
     Pipeline& p = c->p;
     const size_t bytes = (size_t)c->W * c->H * 4;
+    // the resolve writes device memory of this device itself
+    struct Direct {
+        Pipeline& p;
+        ~Direct() { p.image2 = nullptr; }
+    } direct{p};
+    CUDA_TRY(cudaSetDevice(p.device));
+    if (rgba_out && out_is_device && kernels_may_write(rgba_out, bytes, p.device)) {
+        p.image2 = static_cast<uint32_t*>(rgba_out);
+        rgba_out = nullptr;
+    }
     const bool presized = c->hint_valid && p.loaded && c->hint_C == p.C && c->hint_P == p.P;
     const uint64_t launches0 = sr::launches_so_far();
     sr_status s = SR_ERR_OVERFLOW_REFIT;
@@ -1365,7 +1410,12 @@ sr_status sr_render_aa(sr_ctx* c, uint32_t samples, void* rgba_out, int out_is_d
     if (s2 == SR_OK) s2 = upload_paints(c);
     SR_TRY(s);
     SR_TRY(s2);
-    sr::launch_aa_resolve(p.aa_acc.p, p.image.as<uint32_t>(), npx, samples, st);
+    uint32_t* img2 = nullptr;
+    if (rgba_out && out_is_device && kernels_may_write(rgba_out, npx * 4, p.device)) {
+        img2 = static_cast<uint32_t*>(rgba_out);
+        rgba_out = nullptr;
+    }
+    sr::launch_aa_resolve(p.aa_acc.p, p.image.as<uint32_t>(), img2, npx, samples, st);
     CUDA_TRY(cudaGetLastError());
     if (rgba_out)
         CUDA_TRY(cudaMemcpyAsync(rgba_out, p.image.p, npx * 4,
@@ -1866,7 +1916,14 @@ sr_status sr_batch_get_image(sr_batch* b, uint32_t index, void* rgba_out, int ou
     const sr::SceneInfo& si = b->p.info[index];
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     CUDA_TRY(cudaSetDevice(b->p.device));
-    CUDA_TRY(cudaMemcpyAsync(rgba_out, b->p.image.as<uint32_t>() + si.image_off, (size_t)si.W * si.H * 4,
+    const uint32_t* img = b->p.image.as<uint32_t>() + si.image_off;
+    const size_t npx = (size_t)si.W * si.H;
+    if (out_is_device && kernels_may_write(rgba_out, npx * 4, b->p.device)) {
+        sr::launch_copy_image(img, static_cast<uint32_t*>(rgba_out), npx, b->p.sm_count, st);
+        CUDA_TRY(cudaGetLastError());
+        return SR_OK;
+    }
+    CUDA_TRY(cudaMemcpyAsync(rgba_out, img, npx * 4,
                              out_is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
     if (!out_is_device) CUDA_TRY(cudaStreamSynchronize(st));
     return SR_OK;

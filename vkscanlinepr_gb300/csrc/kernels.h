@@ -308,6 +308,7 @@ struct ResolveArgs {
     int32_t warps;                    // warps per CTA: 8 or 16
     int32_t seg;                      // pixels per warp: kResolveSeg, or 128 or 64 (pixel mode)
     uint32_t* image;                  // all scenes' RGBA8 framebuffers
+    uint32_t* image2 = nullptr;       // the caller's memory for them too, or NULL
     const uint32_t* seg_cut;          // [rows][cut_segs] from the emit, or NULL
     const unsigned long long* row_px; // [rows] summed record widths from the emit, or NULL (every row searched)
     uint32_t cut_segs;
@@ -324,7 +325,10 @@ void launch_resolve(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st);
 // Multisampling: sum a sample frame into acc (first: start the sums), and
 // write the rounded averages of k frames.
 void launch_aa_accumulate(const uint32_t* img, void* acc, size_t n, bool first, cudaStream_t st);
-void launch_aa_resolve(const void* acc, uint32_t* img, size_t n, uint32_t k, cudaStream_t st);
+// (img2: a second copy, or NULL)
+void launch_aa_resolve(const void* acc, uint32_t* img, uint32_t* img2, size_t n, uint32_t k, cudaStream_t st);
+// n pixels from a framebuffer to device memory of this device.
+void launch_copy_image(const uint32_t* src, uint32_t* dst, size_t n, int sm_count, cudaStream_t st);
 // n_dev (optional) holds the record count; n is the capacity.
 void launch_row_bounds(const uint32_t* srows, int64_t n, const uint32_t* n_dev, int32_t rows, int32_t* row_start,
                        cudaStream_t st);

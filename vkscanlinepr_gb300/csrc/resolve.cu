@@ -12,6 +12,8 @@
 // a segment of a row and first finds where its painting may start (the collapse
 // cut below); in reference mode a CTA owns one cell row (or several short ones)
 // and stages its records in shared memory.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -408,13 +410,19 @@ template <int K> SR_DEV void init_pix(uint32_t (&rb)[K], float (&g)[K]) {
     }
 }
 
+// The row's pixels into the framebuffer, and into the caller's (a copy of the
+// framebuffer would read it again, and be one more launch).
 template <int K>
-SR_DEV void store_pix(uint32_t* __restrict__ row, int32_t W, int32_t seg, int lane, const uint32_t (&rb)[K],
+SR_DEV void store_pix(const ResolveArgs& a, uint64_t row, int32_t W, int32_t seg, int lane, const uint32_t (&rb)[K],
                       const float (&g)[K]) {
 #pragma unroll
     for (int j = 0; j < K; ++j) {
         int32_t p = seg + lane + 32 * j;
-        if (p < W) row[p] = rb[j] | ((uint32_t)__float2int_rn(g[j]) << 8) | 0xFF000000u;
+        if (p < W) {
+            const uint32_t v = rb[j] | ((uint32_t)__float2int_rn(g[j]) << 8) | 0xFF000000u;
+            a.image[row + (uint32_t)p] = v;
+            if (a.image2) a.image2[row + (uint32_t)p] = v;
+        }
     }
 }
 
@@ -501,7 +509,7 @@ __global__ void __launch_bounds__(32 * WARPS, (GRAD ? 32 : K == 8 ? 40 : 48) / W
         }
         __syncwarp();
     }
-    store_pix<K>(a.image + si->image_off + (size_t)y * W, W, seg, lane, rb, g);
+    store_pix<K>(a, si->image_off + (uint64_t)y * (uint32_t)W, W, seg, lane, rb, g);
 }
 
 // ------------------------------------------------------- reference mode --
@@ -584,11 +592,14 @@ __global__ void __launch_bounds__(32 * WARPS) k_resolve_ref(const ResolveArgs a)
             const int32_t y0 = (w.r0 + w.my_row) * a.F;
             const int32_t nrows = imin(a.F, w.si->H - y0);
             for (int32_t yy = 0; yy < nrows; ++yy) {
-                uint32_t* out = a.image + w.si->image_off + (size_t)(y0 + yy) * W;
+                const uint64_t row = w.si->image_off + (uint64_t)(y0 + yy) * (uint32_t)W;
 #pragma unroll
                 for (int j = 0; j < kK; ++j) {
                     int32_t p = seg + lane + 32 * j;
-                    if (p < W) out[p] = px[j];
+                    if (p < W) {
+                        a.image[row + (uint32_t)p] = px[j];
+                        if (a.image2) a.image2[row + (uint32_t)p] = px[j];
+                    }
                 }
             }
         }
@@ -633,13 +644,35 @@ __global__ void k_aa_accumulate(const uint32_t* __restrict__ img, ushort4* __res
     acc[i] = v;
 }
 
-__global__ void k_aa_resolve(const ushort4* __restrict__ acc, uint32_t* __restrict__ img, size_t n, uint32_t k) {
+__global__ void k_aa_resolve(const ushort4* __restrict__ acc, uint32_t* __restrict__ img, uint32_t* __restrict__ img2,
+                             size_t n, uint32_t k) {
     wait_for_stream();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const ushort4 v = acc[i];
     const uint32_t h = k / 2u;
-    img[i] = ((v.x + h) / k) | (((v.y + h) / k) << 8) | (((v.z + h) / k) << 16) | (((v.w + h) / k) << 24);
+    const uint32_t c = ((v.x + h) / k) | (((v.y + h) / k) << 8) | (((v.z + h) / k) << 16) | (((v.w + h) / k) << 24);
+    img[i] = c;
+    if (img2) img2[i] = c;
+}
+
+// A framebuffer to the caller's device memory: four 16-byte loads in flight a
+// thread, or 4-byte ones where either lies off 16 bytes.  The 64 images (423
+// MB) of a batch take 228 us, a launch each (3.5 us of host time), where
+// cudaMemcpyAsync took 687.
+template <class T>
+__global__ void __launch_bounds__(256) k_copy(const T* __restrict__ src, T* __restrict__ dst, size_t n) {
+    wait_for_stream();
+    const size_t stride = (size_t)gridDim.x * 1024;
+    for (size_t i = (size_t)blockIdx.x * 1024 + threadIdx.x; i < n; i += stride) {
+        T v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + 256 * k < n) v[k] = src[i + 256 * k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + 256 * k < n) dst[i + 256 * k] = v[k];
+    }
 }
 
 void launch_aa_accumulate(const uint32_t* img, void* acc, size_t n, bool first, cudaStream_t st) {
@@ -649,10 +682,24 @@ void launch_aa_accumulate(const uint32_t* img, void* acc, size_t n, bool first, 
                  first ? 1 : 0);
 }
 
-void launch_aa_resolve(const void* acc, uint32_t* img, size_t n, uint32_t k, cudaStream_t st) {
+void launch_aa_resolve(const void* acc, uint32_t* img, uint32_t* img2, size_t n, uint32_t k, cudaStream_t st) {
     if (!n) return;
     count_launches(1);
-    launch_after(k_aa_resolve, (unsigned)((n + 255) / 256), 256, 0, st, static_cast<const ushort4*>(acc), img, n, k);
+    launch_after(k_aa_resolve, (unsigned)((n + 255) / 256), 256, 0, st, static_cast<const ushort4*>(acc), img, img2, n,
+                 k);
+}
+
+void launch_copy_image(const uint32_t* src, uint32_t* dst, size_t n, int sm_count, cudaStream_t st) {
+    if (!n) return;
+    count_launches(1);
+    const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0 && n % 4 == 0;
+    const size_t items = vec ? n / 4 : n;
+    const unsigned grid = (unsigned)std::min<size_t>((items + 1023) / 1024, (size_t)std::max(sm_count, 1) * 8);
+    if (vec)
+        launch_after(k_copy<uint4>, grid, 256, 0, st, reinterpret_cast<const uint4*>(src), reinterpret_cast<uint4*>(dst),
+                     items);
+    else
+        launch_after(k_copy<uint32_t>, grid, 256, 0, st, src, dst, items);
 }
 
 void launch_row_bounds(const uint32_t* srows, int64_t n, const uint32_t* n_dev, int32_t rows, int32_t* row_start,
