@@ -355,8 +355,10 @@ struct Pipeline {
         size_t off, bytes;
     };
     std::vector<StagedCopy> staged;
+    bool back_cleared = false;      // enqueue_front cleared the back half's buffer
     uint32_t* image2 = nullptr;     // device memory of the caller that the frame being enqueued goes to as well
-    uint32_t* h_report = nullptr;   // pinned copy of the control block's report
+    uint32_t* h_report = nullptr;   // pinned copy of the control block's report, written by the resolve
+    uint32_t* d_report = nullptr;   // its device address
     // results
     sr_stats stats{};
     int64_t last_N = 0, last_O = 0, last_cap = 0, last_dcap = 0;
@@ -438,6 +440,7 @@ struct Pipeline {
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
         if (sm_count <= 0) sm_count = 148;
         CUDA_TRY(cudaMallocHost(&h_report, sizeof(uint32_t) * CTL_REPORT));
+        CUDA_TRY(cudaHostGetDevicePointer(&d_report, h_report, 0));
         CUDA_TRY(ensure(ctl, sizeof(uint32_t) * CTL_WORDS));
         return SR_OK;
     }
@@ -876,15 +879,17 @@ struct Pipeline {
     }
 
     // Transform, count, chain order and offset scan (no allocation, no wait).
-    sr_status enqueue_front(cudaStream_t st) {
+    // cap >= 0: also clears what enqueue_back needs cleared for that capacity.
+    sr_status enqueue_front(cudaStream_t st, int64_t cap, int64_t dcap) {
         using namespace sr;
         uint32_t* ctlp = ctl.as<uint32_t>();
         uint32_t* status = ctlp + CTL_STATUS;
         CUDA_TRY(cudaMemsetAsync(ctl.p, 0, front_bytes(), st));
         if (count_paths) CUDA_TRY(cudaMemsetAsync(path_draw.p, 0, sizeof(uint32_t) * std::max<uint32_t>(P, 1), st));
         mark(ST_TRANSFORM, false);
-        launch_transform(pos.as<float2>(), pos_path.as<uint32_t>(), V, table(), tpos.as<float2>(),
-                         path_visible(), st);
+        back_cleared = cap >= 0;
+        launch_transform(pos.as<float2>(), pos_path.as<uint32_t>(), V, table(), tpos.as<float2>(), path_visible(),
+                         zeroed.p, back_cleared ? back_layout(cap, dcap).total : 0, sm_count, st);
         if (arcs)
             launch_arc_fixup(curve_type.as<uint32_t>(), curve_pos.as<uint32_t>(), curve_path.as<uint32_t>(), C,
                              pos.as<float2>(), table(), tpos.as<float2>(), path_visible(), st);
@@ -912,7 +917,8 @@ struct Pipeline {
         const uint32_t* n_dev = reinterpret_cast<const uint32_t*>(offs.as<int32_t>() + C);
         const BackLayout at = back_layout(cap, dcap_req);
         char* zero = zeroed.as<char>();
-        CUDA_TRY(cudaMemsetAsync(zero, 0, at.total, st));
+        if (!back_cleared) CUDA_TRY(cudaMemsetAsync(zero, 0, at.total, st));
+        back_cleared = false;
         const GeomArgs g = geom(cap);
         const ChainWork cw = chain_work();
         DebugOut dbg{nullptr, nullptr, nullptr};
@@ -1014,6 +1020,9 @@ struct Pipeline {
         ra.paints = n_paints ? paints_d.as<DevPaint>() : nullptr;
         ra.n_paints = n_paints;
         ra.image2 = image2;
+        ra.control = ctlp;
+        ra.report = d_report;
+        ra.report_words = CTL_REPORT;
         mark(ST_RESOLVE, false);
         launch_resolve(ra, res_ctas, st);
         mark(ST_RESOLVE, true);
@@ -1056,7 +1065,7 @@ struct Pipeline {
     // Read N back (the reference's count read-back, scanline_rasterizer.cpp:355-356).
     sr_status read_count(cudaStream_t st, int64_t* N) {
         if (segmented()) sr::launch_segsort_largest(seg_args(1, nullptr), st);
-        SR_TRY(enqueue_readback(st));
+        CUDA_TRY(cudaMemcpyAsync(h_report, ctl.p, sizeof(uint32_t) * CTL_REPORT, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
         SR_TRY(check_status_word(h_report[CTL_STATUS]));
         seg_levels = levels_for(h_report[CTL_LARGEST]);
@@ -1094,14 +1103,15 @@ struct Pipeline {
         seg_check = cap < 0 ? 0u : (uint32_t)sr::segsort_tile() << levels;
         seg_levels = levels;
         seg_wide = wide || cap < 0;
-        SR_TRY(enqueue_front(st));
+        if (cap >= 0) SR_TRY(reserve(cap, dcap));
+        SR_TRY(enqueue_front(st, cap, dcap));
         if (cap < 0) {
             int64_t N = 0;
             SR_TRY(read_count(st, &N));
             cap = N;
             dcap = -1;
+            SR_TRY(reserve(cap, dcap));
         }
-        SR_TRY(reserve(cap, dcap));
         SR_TRY(enqueue_back(st, cap, dcap));
         stats.kernel_launches = (uint32_t)(sr::launches_so_far() - launches0);
         ev_pending = (flags & SR_FLAG_PROFILE) != 0;
@@ -1110,14 +1120,7 @@ struct Pipeline {
         return SR_OK;
     }
 
-    // Queues the copy of the frame's report into pinned host memory.
-    sr_status enqueue_readback(cudaStream_t st) {
-        CUDA_TRY(cudaMemcpyAsync(h_report, ctl.p, sizeof(uint32_t) * CTL_REPORT, cudaMemcpyDeviceToHost, st));
-        return SR_OK;
-    }
-
     sr_status finish(cudaStream_t st) {
-        SR_TRY(enqueue_readback(st));
         CUDA_TRY(cudaStreamSynchronize(st));
         return collect();
     }
@@ -1819,7 +1822,7 @@ static sr_status batch_enqueue(sr_batch* b, const sr_batch_render_opts& d, cudaS
             cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
             sr_status s1 = SR_OK, s2 = SR_OK;
             if (e == cudaSuccess) {
-                s1 = p.enqueue_front(cs);
+                s1 = p.enqueue_front(cs, cap, dcap);
                 if (s1 == SR_OK) s2 = p.enqueue_back(cs, cap, dcap);
                 cudaError_t e2 = cudaStreamEndCapture(cs, &b->graph);   // always end the capture
                 if (e2 != cudaSuccess) e = e2;
@@ -1841,7 +1844,6 @@ static sr_status batch_enqueue(sr_batch* b, const sr_batch_render_opts& d, cudaS
     } else {
         SR_TRY(p.frame(st, cap, dcap));
     }
-    SR_TRY(p.enqueue_readback(st));
     if (!b->done) CUDA_TRY(cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming));
     CUDA_TRY(cudaEventRecord(b->done, st));
     b->inflight = true;
@@ -2188,7 +2190,7 @@ sr_status sr_batch_path_features(sr_batch* b, float* d_feats, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     CUDA_TRY(cudaMemsetAsync(p.path_visible(), 0, sizeof(int32_t) * std::max<uint32_t>(p.P, 1), st));
     sr::launch_transform(p.pos.as<float2>(), p.pos_path.as<uint32_t>(), p.V, p.table(), p.tpos.as<float2>(),
-                         p.path_visible(), st);
+                         p.path_visible(), nullptr, 0, p.sm_count, st);
     if (p.arcs)
         sr::launch_arc_fixup(p.curve_type.as<uint32_t>(), p.curve_pos.as<uint32_t>(), p.curve_path.as<uint32_t>(), p.C,
                              p.pos.as<float2>(), p.table(), p.tpos.as<float2>(), p.path_visible(), st);

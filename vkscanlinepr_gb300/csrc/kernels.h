@@ -121,8 +121,9 @@ uint32_t chain_list_capacity(uint32_t n_curves);
 void launch_arc_fixup(const uint32_t* curve_type, const uint32_t* curve_pos, const uint32_t* curve_path,
                       uint32_t n_curves, const float2* pos, const SceneTable& t, float2* tpos, int32_t* path_visible,
                       cudaStream_t st);
+// zero: zero_bytes (a multiple of 16) to clear beside it.
 void launch_transform(const float2* pos, const uint32_t* pos_path, uint32_t n_points, const SceneTable& t,
-                      float2* tpos, int32_t* path_visible, cudaStream_t st);
+                      float2* tpos, int32_t* path_visible, void* zero, size_t zero_bytes, int sm_count, cudaStream_t st);
 void launch_count(const GeomArgs& g, float* cut_cache, int32_t* count, const ChainWork& w, uint32_t* status,
                   cudaStream_t st);
 // After the count pass: the curves' record offsets offs[0..C] (exclusive scan
@@ -309,6 +310,9 @@ struct ResolveArgs {
     int32_t seg;                      // pixels per warp: kResolveSeg, or 128 or 64 (pixel mode)
     uint32_t* image;                  // all scenes' RGBA8 framebuffers
     uint32_t* image2 = nullptr;       // the caller's memory for them too, or NULL
+    const uint32_t* control = nullptr; // control block, whose first report_words words go to report (host memory)
+    uint32_t* report = nullptr;
+    uint32_t report_words = 0;
     const uint32_t* seg_cut;          // [rows][cut_segs] from the emit, or NULL
     const unsigned long long* row_px; // [rows] summed record widths from the emit, or NULL (every row searched)
     uint32_t cut_segs;

@@ -426,6 +426,13 @@ SR_DEV void store_pix(const ResolveArgs& a, uint64_t row, int32_t W, int32_t seg
     }
 }
 
+// The frame's report: the control block's first words into page-locked host
+// memory (every kernel that writes them is done), for the wait at the frame's
+// end; a copy of its own would be one more launch.
+SR_DEV void write_report(const ResolveArgs& a) {
+    if (blockIdx.x == 0 && threadIdx.x < a.report_words) a.report[threadIdx.x] = a.control[threadIdx.x];
+}
+
 // A warp paints one segment of one row, by itself: it finds its cut and
 // streams the row's records from there, 32 at a time, through its own
 // shared-memory slots.  The warps of a CTA mostly share a row, so the records
@@ -448,6 +455,7 @@ SR_DEV void store_pix(const ResolveArgs& a, uint64_t row, int32_t W, int32_t seg
 template <int WARPS, int K, bool GRAD>
 __global__ void __launch_bounds__(32 * WARPS, (GRAD ? 32 : K == 8 ? 40 : 48) / WARPS) k_resolve_pixel(const ResolveArgs a) {
     wait_for_stream();
+    write_report(a);
     constexpr int kSeg = 32 * K;
     static_assert(kResolveSeg % kSeg == 0, "a cut covers whole segments");
     __shared__ PixRec slots[WARPS * 32];
@@ -525,6 +533,7 @@ struct RefRec {
 template <int WARPS, bool GRAD>
 __global__ void __launch_bounds__(32 * WARPS) k_resolve_ref(const ResolveArgs a) {
     wait_for_stream();
+    write_report(a);
     __shared__ RefRec sq[kChunk];
     const ResolveWork w = resolve_work<WARPS>(a);
     const int tid = threadIdx.x, lane = tid & 31;
