@@ -608,8 +608,8 @@ void launch_mlp_predict(const void* wb, const float* master, const float* norm, 
     unsigned blocks = (n + per - 1) / per;
     const unsigned cap = (unsigned)kPredictCtas * (unsigned)(sm_count > 0 ? sm_count : 148);   // one wave
     if (blocks > cap) blocks = cap;
-    launch_after(k_mlp_predict, blocks, kPredictThreads, 0, st, static_cast<const __nv_bfloat16*>(wb), master, norm,
-                 x, n, y);
+    launch_after(k_mlp_predict, blocks, kPredictThreads, 0, st, static_cast<const __nv_bfloat16*>(wb), master, norm, x,
+                 n, y);
 }
 
 static cudaError_t grad_launch(const void* wb, const float* master, const float* norm, const float* x, const float* t,
@@ -623,8 +623,8 @@ static cudaError_t grad_launch(const void* wb, const float* master, const float*
     if (e != cudaSuccess) return e;
     count_launches(1);
     launch_after(k_mlp_grad, (n + kSamples - 1) / kSamples, kGradThreads, sizeof(GradSmem), st,
-                 static_cast<const __nv_bfloat16*>(wb), master, norm, x, t, idx, n, 1.0f / ((float)n * (float)kOut), grad,
-                 loss_sum, adam ? 1 : 0, A, done);
+                 static_cast<const __nv_bfloat16*>(wb), master, norm, x, t, idx, n, 1.0f / ((float)n * (float)kOut),
+                 grad, loss_sum, adam ? 1 : 0, A, done);
     return cudaGetLastError();
 }
 

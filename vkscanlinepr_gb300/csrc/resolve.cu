@@ -705,8 +705,8 @@ void launch_copy_image(const uint32_t* src, uint32_t* dst, size_t n, int sm_coun
     const size_t items = vec ? n / 4 : n;
     const unsigned grid = (unsigned)std::min<size_t>((items + 1023) / 1024, (size_t)std::max(sm_count, 1) * 8);
     if (vec)
-        launch_after(k_copy<uint4>, grid, 256, 0, st, reinterpret_cast<const uint4*>(src), reinterpret_cast<uint4*>(dst),
-                     items);
+        launch_after(k_copy<uint4>, grid, 256, 0, st, reinterpret_cast<const uint4*>(src),
+                     reinterpret_cast<uint4*>(dst), items);
     else
         launch_after(k_copy<uint32_t>, grid, 256, 0, st, src, dst, items);
 }

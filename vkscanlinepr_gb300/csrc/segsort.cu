@@ -1108,8 +1108,7 @@ void launch_segsort(const SegArgs& sa, uint64_t* keys_in, uint64_t* keys_out, ui
     const size_t mt = max_tiles(sa.n_paths, sa.cap);
     count_launches(1);
     launch_after(k_seg_tiles, (sa.n_paths + kSegThreads - 1) / kSegThreads, kSegThreads, 0, st, sa, (uint32_t)mt, u,
-                 status,
-                                                                                      spin_limit());
+                 status, spin_limit());
     const uint32_t key_bits = L.pbits + L.rbits + L.xbits;
     const KeyFields kf{L.xbits, L.rbits, L.pbits, (uint32_t)(L.Hy - 1)};
     // resident CTAs per SM of the two persistent kernels (same on every
@@ -1134,12 +1133,11 @@ void launch_segsort(const SegArgs& sa, uint64_t* keys_in, uint64_t* keys_out, ui
     count_launches(1 + (sa.wide ? 1 : 0) + (uint32_t)levels);
     const uint32_t n_cap = (uint32_t)sa.cap;
     launch_after(k_tile_sort, g_tile, kSortThreads, sizeof(TileSmem), st, keys_in, keys_out, keys_alt, kf, n_cap,
-                                                                  (uint32_t)mt, u, sa.wide, status, spin_limit());
+                 (uint32_t)mt, u, sa.wide, status, spin_limit());
     if (sa.wide) launch_after(k_local_sort, g_sort, kThreads, 0, st, keys_in, keys_out, keys_alt, kf, n_cap, u);
     for (int lv = 0; lv < levels; ++lv)
         launch_after(k_merge_level, g_merge, kThreads, sizeof(MergeSmem), st, keys_out, keys_alt, (uint32_t)lv,
-                     key_bits, n_cap,
-                                                                    u);
+                     key_bits, n_cap, u);
 }
 
 }  // namespace sr

@@ -1151,12 +1151,12 @@ static void launch_runs(const WindArgs& a, int64_t tiles, uint64_t* words, uint6
                         uint32_t* counters, uint32_t* status, cudaStream_t st) {
     if (tiles >= kWarpTiles)
         launch_after(k_winding_reduce<ITEMS, 256, 1, MULTI>, (unsigned)((tiles + 7) / 8), 256, 0, st, a, tagg, tile_in,
-                                                                                        counters + 1);
+                     counters + 1);
     else
         launch_after(k_winding_reduce<ITEMS, 256, 8, MULTI>, (unsigned)tiles, 256, 0, st, a, tagg, tile_in,
                      counters + 1);
     launch_after(k_winding_runs<ITEMS, 256, MULTI>, (unsigned)tiles, 256, 0, st, a, tile_in, words, counters, status,
-                                                                       spin_limit());
+                 spin_limit());
 }
 
 void launch_winding_emit(const WindArgs& a, int items, uint64_t* tile_status, uint64_t* tile_sums, uint32_t* counters,
