@@ -641,8 +641,9 @@ struct Pipeline {
     sr::ChainWork chain_work() const {
         sr::ChainWork cw;
         uint32_t* ctlp = ctl.as<uint32_t>();
-        uint32_t* cl = chain_lists.as<uint32_t>();
         const uint32_t lc = list_cap();
+        cw.chain_piece = chain_lists.as<uint4>();
+        uint32_t* cl = chain_lists.as<uint32_t>() + 4 * (size_t)lc;
         cw.pieces = pieces.as<uint4>();
         cw.chain_items = cl;
         cw.sorted_items = cl + lc;
@@ -665,7 +666,7 @@ struct Pipeline {
         CUDA_TRY(ensure(count, sizeof(int32_t) * ((size_t)C + 1)));
         CUDA_TRY(ensure(offs, sizeof(int32_t) * ((size_t)C + 1)));
         CUDA_TRY(ensure(pieces, sr::piece_table_bytes(std::max<uint32_t>(C, 1))));
-        CUDA_TRY(ensure(chain_lists, 9 * (size_t)list_cap()));
+        CUDA_TRY(ensure(chain_lists, 25 * (size_t)list_cap()));
         CUDA_TRY(ensure(row_start, sizeof(int32_t) * ((size_t)total_rows + 1)));
         return SR_OK;
     }
@@ -789,7 +790,7 @@ struct Pipeline {
         add(8 * v1); add(8 * c1); add(front_bytes()); add(4 * (p1 + 1)); add(20 * c1); add(4 * (c1 + 1)); add(4 * (c1 + 1));
         add(sr::piece_table_bytes((uint32_t)c1));
         const size_t lc = list_cap();
-        add(9 * lc);
+        add(25 * lc);
         add(4 * ((size_t)total_rows + 1));
         post_count_buffers(cap, dcap, [&](DevBuf&, size_t b) { add(b); });
         return total;

@@ -802,7 +802,10 @@ SR_DEV void run_segments(const ChainSide& s, int32_t len, float t_lo, int32_t* _
     }
 }
 
+constexpr uint32_t kBackwards = 0x8000u;   // a piece that runs backwards (its x crossings take 15 bits)
+
 struct ChainSetup {
+    uint4 piece;   // of the record order: first record, crossings (pack_n without signs, kBackwards), start bits, item
     ChainSide side;
     uint32_t type;
     int32_t len;
@@ -826,10 +829,13 @@ SR_DEV ChainSetup chain_setup(const GeomArgs& g, const int32_t* __restrict__ off
     const int32_t nx = piece_nx(me.x), ny = piece_ny(me.x);
     s.base = base + 1 + (side ? nx : 0);
     s.len = side ? ny : nx;
+    const uint32_t t0 = piece == 0 ? 0u : pt[piece - 1].y;   // bits of 0.0f for the first piece
+    const bool back = __uint_as_float(me.y) < __uint_as_float(t0);
+    s.piece = make_uint4((uint32_t)base, (uint32_t)nx | ((uint32_t)ny << 16) | (back ? kBackwards : 0u), t0, item);
     const bool neg = side ? (me.x & 0x80000000u) != 0 : (me.x & 0x8000u) != 0;
     s.side.x = __uint_as_float(side ? me.w : me.z);
     s.side.dx = neg ? -(float)g.F : (float)g.F;
-    s.t_lo = piece == 0 ? 0.0f : __uint_as_float(pt[piece - 1].y);
+    s.t_lo = __uint_as_float(t0);
     s.side.t_hi = __uint_as_float(me.y);
     const float2* cp = g.tpos + g.curve_pos[c];
     const uint32_t np = curve_slots(s.type);
@@ -919,7 +925,8 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
                                                 const uint4* __restrict__ pieces,
                                                 const uint32_t* __restrict__ items, uint32_t list_cap,
                                                 const uint32_t* __restrict__ class_count,
-                                                uint32_t* __restrict__ queue, int32_t* __restrict__ cbuf) {
+                                                uint32_t* __restrict__ queue, int32_t* __restrict__ cbuf,
+                                                uint4* __restrict__ chain_piece) {
     wait_for_stream();
     ChainTickets<true> T;
     T.build(class_count, gridDim.x / kChainCtas);
@@ -934,6 +941,7 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
         int32_t* out = cbuf + s.base;
         const uint32_t gl = T.share(key).lanes, cls = key & 3u;
         const int32_t lanes = 1 << gl, l = (int32_t)(lane_id() & ((1u << gl) - 1u));
+        if (listed && l == 0) chain_piece[pos] = s.piece;
         if (cls == 0u) run_segments<4>(s.side, len, s.t_lo, out, lanes, l);
         else if (cls == 1u) run_segments<3>(s.side, len, s.t_lo, out, lanes, l);
         else if (cls == 2u) run_segments<2>(s.side, len, s.t_lo, out, lanes, l);
@@ -957,11 +965,14 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
 // roots, then t0, then all y roots: i0 is all of them.
 //
 // A lane finds the place of a root by a binary search; a warp's roots are
-// neighbours, so its loads and stores are too.  Those dependent loads bound
-// it: 0.183 ms on the 4096^2 frame of 21 M records (0.014 ms on the 1024^2
-// frame of 0.37 M), where a thread per short and a CTA per long piece took
-// 0.295 (0.027); a lane walking a stretch of 16 consecutive roots took 0.52,
-// its 4-byte accesses being scattered.
+// neighbours, so its loads and stores are too.  The dependent loads bound it,
+// of a chain's piece first: k_chains leaves it in one 16-byte word a chain (the
+// curve's offset and its pieces summed up again took 0.184 instead of 0.158 ms
+// on the 4096^2 frame of 21 M records, 0.127 instead of 0.106 in a batch of 64
+// uneven scenes); then of the search, but a search by windows of 32 roots held
+// by a warp, with a third of the loads, was no faster (0.197).  A thread per
+// short and a CTA per long piece took 0.295; a lane walking a stretch of 16
+// consecutive roots 0.52, its 4-byte accesses being scattered.
 SR_DEV int32_t count_le(const int32_t* a, int32_t lo, int32_t hi, float v) {   // elements <= v, of a[lo, hi) sorted, + lo
     while (lo < hi) {
         const int32_t mid = (lo + hi) >> 1;
@@ -983,6 +994,7 @@ __global__ void __launch_bounds__(128) k_order_records(const GeomArgs g, const i
                                                        const uint4* __restrict__ pieces,
                                                        const uint32_t* __restrict__ items, uint32_t list_cap,
                                                        const uint32_t* __restrict__ class_count,
+                                                       const uint4* __restrict__ chain_piece,
                                                        const int32_t* __restrict__ cbuf, int2* __restrict__ rec,
                                                        uint32_t* __restrict__ status) {
     wait_for_stream();
@@ -992,21 +1004,20 @@ __global__ void __launch_bounds__(128) k_order_records(const GeomArgs g, const i
     for (uint32_t ticket = blockIdx.x * (blockDim.x / 32u) + (threadIdx.x >> 5); ticket < T.total; ticket += warps) {
         uint32_t key, pos, warp;
         if (!T.find(ticket, list_cap, key, pos, warp)) continue;
-        const uint32_t item = items[pos], c = item >> 4, piece = (item >> 1) & 7u;
-        const uint4* pt = pieces + (size_t)c * kMaxPieces;
-        int64_t base = offs[c];
-        for (uint32_t j = 0; j < piece; ++j) base += 1 + piece_nx(pt[j].x) + piece_ny(pt[j].x);
-        const uint4 me = pt[piece];
-        const int32_t nx = piece_nx(me.x), ny = piece_ny(me.x);
+        // (k_chains left out the pieces without crossings)
+        const uint4 pc = key == kEmptyPiece ? chain_setup(g, offs, pieces, items[pos]).piece : chain_piece[pos];
+        const uint32_t item = pc.w, c = item >> 4;
+        const int64_t base = (int64_t)pc.x;
+        const int32_t nx = piece_nx(pc.y), ny = piece_ny(pc.y);
         if (base + 1 + nx + ny > g.rec_cap) {
             set_error(status, ERR_CAPACITY);
             continue;
         }
-        const int32_t t0 = piece == 0 ? 0 : (int32_t)pt[piece - 1].y;   // bits of 0.0f for the first piece
+        const int32_t t0 = (int32_t)pc.z;
         const int32_t *X = cbuf + base + 1, *Y = X + nx;
         int2* R = rec + base;
         int32_t i0 = 0;
-        const bool back = __uint_as_float(me.y) < bitsf(t0);
+        const bool back = (pc.y & kBackwards) != 0;
         if (nx > 0 && ny > 0) {
             if (back) i0 = nx;
             else if (bitsf(X[0]) <= bitsf(t0)) i0 = count_le(X, 0, nx, bitsf(t0));
@@ -1263,7 +1274,7 @@ void launch_chains(const GeomArgs& g, const int32_t* offs, const ChainWork& w, i
     // (not launch_after: placed while the offset scan drains, its CTAs do not
     // spread over the SMs, 1,725 instead of 1,675 us for a 4096^2 frame)
     k_chains<<<sm_count * kChainCtas, 128, 0, st>>>(g, offs, w.pieces, w.sorted_items, w.list_cap, w.class_count,
-                                                    w.chain_queue, cbuf);
+                                                    w.chain_queue, cbuf, w.chain_piece);
 }
 
 void launch_merge(const GeomArgs& g, const int32_t* offs, const ChainWork& w, const int32_t* cbuf, int2* rec,
@@ -1279,7 +1290,7 @@ void launch_order_records(const GeomArgs& g, const int32_t* offs, const ChainWor
     if (g.n_curves == 0) return;
     count_launches(1);
     launch_after(k_order_records, sm_count * 32, 128, 0, st, g, offs, w.pieces, w.sorted_items, w.list_cap,
-                 w.class_count, cbuf, rec, status);
+                 w.class_count, w.chain_piece, cbuf, rec, status);
 }
 
 void launch_fragment(const GeomArgs& g, const int2* rec, int64_t n_cap, const uint32_t* n_dev, uint64_t* keys,

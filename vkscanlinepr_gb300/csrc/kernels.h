@@ -107,6 +107,7 @@ struct ChainWork {
     uint32_t* chain_items;    // [list_cap] (curve << 4 | piece << 1 | side), append order
     uint8_t* chain_keys;      // [list_cap] class of each: length class / type
     uint32_t* sorted_items;   // [list_cap] the same, longest class first
+    uint4* chain_piece;       // [list_cap] each sorted item's piece, for the record order
     uint32_t list_cap;
     uint32_t* chain_count;    // [1] zeroed before the count pass, as are the next three
     uint32_t* class_count;    // [kChainClassWords] chains of each class
