@@ -1128,9 +1128,10 @@ __global__ void __launch_bounds__(128) k_merge(const GeomArgs g, const int32_t* 
 // A warp takes 32 consecutive records and writes the first 31: each lane
 // evaluates the curve at its own record, and the next lane's point (or the
 // curve's end, from the count pass) is the piece's end.  Instruction issue
-// bounds it (70%): 0.209 ms on the 4096^2 frame of 21 M records; evaluating
-// both ends in every lane took 0.225.
-constexpr int kFragWarps = 8, kFragOut = 31;
+// and the latency of the curve's loads bound it: 0.206 ms on the 4096^2 frame
+// of 21 M records, 0.122 in a batch of 64 uneven scenes (CTAs of eight warps
+// 0.208 and 0.128; evaluating both ends in every lane took 0.225).
+constexpr int kFragWarps = 4, kFragOut = 31;
 
 __global__ void __launch_bounds__(32 * kFragWarps) k_fragment(const GeomArgs g, const int2* __restrict__ rec,
                                                               int64_t n_cap, const uint32_t* __restrict__ n_dev,
