@@ -14,6 +14,8 @@
 // scattered into shared memory in digit order, then written out in runs, so
 // global stores stay mostly contiguous.  An upfront kernel histograms every
 // pass's digits in one read of the keys.
+#include <algorithm>
+
 #include "kernels.h"
 #include "scan.cuh"
 
@@ -251,8 +253,9 @@ __global__ void __launch_bounds__(kThreads) k_row_sort(const uint32_t* __restric
         for (int q = 0; q < kPer; ++q)
 #pragma unroll
             for (int k = 0; k < kRowWindow; ++k)
-                w[q][k] = look[q] - k >= 0 ? ld_relaxed_u32(lookback + (size_t)(look[q] - k) * kR + threadIdx.x + q * kThreads)
-                                           : kFlagP;
+                w[q][k] = look[q] - k >= 0
+                              ? ld_relaxed_u32(lookback + (size_t)(look[q] - k) * kR + threadIdx.x + q * kThreads)
+                              : kFlagP;
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
             if (look[q] < 0) continue;
@@ -330,141 +333,147 @@ __global__ void __launch_bounds__(kThreads, onesweep_min_blocks(kVals, ITEMS)) k
     constexpr int kItems = ITEMS, kTile = kThreads * ITEMS;
     OnesweepSmem<K, kVals, ITEMS>& S = *reinterpret_cast<OnesweepSmem<K, kVals, ITEMS>*>(smem_raw);
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kWarps * kRadix; i += kThreads) (&S.warp_hist[0][0])[i] = 0;
-    if (threadIdx.x == 0) S.tile = atomicAdd(counter, 1u);
-    __syncthreads();
-    const uint32_t tile = S.tile;
     const int64_t n = n_dev ? (int64_t)min((uint64_t)*n_dev, (uint64_t)n_max) : n_max;
-    const int64_t tbase = (int64_t)tile * kTile;
-    if (tbase >= n) return;   // launched for a larger capacity than this sort has
-    const int64_t wbase = tbase + (int64_t)warp * (32 * kItems);
+    // tile after tile until the input's end: the grid follows the GPU, not the
+    // capacity, of which a frame's runs are a fraction (a CTA a tile of the
+    // capacity: 0.103 instead of 0.091 ms for the row sort of the 4096^2 frame,
+    // 0.105 instead of 0.079 for 64 uneven scenes)
+    for (;; __syncthreads()) {
+        for (int i = threadIdx.x; i < kWarps * kRadix; i += kThreads) (&S.warp_hist[0][0])[i] = 0;
+        if (threadIdx.x == 0) S.tile = atomicAdd(counter, 1u);
+        __syncthreads();
+        const uint32_t tile = S.tile;
+        const int64_t tbase = (int64_t)tile * kTile;
+        if (tbase >= n) return;
+        const int64_t wbase = tbase + (int64_t)warp * (32 * kItems);
 
-    // ---- load (warp-striped, coalesced) and rank within the warp
-    K k[kItems];
-    uint32_t v[kVals ? kItems : 1];
-    uint32_t rank[kItems];
+        // ---- load (warp-striped, coalesced) and rank within the warp
+        K k[kItems];
+        uint32_t v[kVals ? kItems : 1];
+        uint32_t rank[kItems];
 #pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-        int64_t idx = wbase + it * 32 + lane;
-        bool ok = idx < n;
-        k[it] = ok ? keys_in[idx] : (K)0;
-        if (kVals) v[it] = ok ? (vals_in ? vals_in[idx] : (uint32_t)idx) : 0u;
-    }
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-        int64_t idx = wbase + it * 32 + lane;
-        bool ok = idx < n;
-        uint32_t d = ok ? digit_of(k[it], shift, dmask) : (uint32_t)kRadix;   // kRadix = out of range
-        uint32_t peers = same_digit_lanes<sizeof(K) == 4>(d);
-        uint32_t leader = (uint32_t)(__ffs(peers) - 1);
-        uint32_t before = 0;
-        if (ok && lane == leader) {
-            before = S.warp_hist[warp][d];
-            S.warp_hist[warp][d] = before + (uint32_t)__popc(peers);
+        for (int it = 0; it < kItems; ++it) {
+            int64_t idx = wbase + it * 32 + lane;
+            bool ok = idx < n;
+            k[it] = ok ? keys_in[idx] : (K)0;
+            if (kVals) v[it] = ok ? (vals_in ? vals_in[idx] : (uint32_t)idx) : 0u;
         }
-        before = __shfl_sync(0xFFFFFFFFu, before, leader);
-        rank[it] = before + (uint32_t)__popc(peers & lanemask_lt());
-        __syncwarp();
-    }
-    __syncthreads();
-
-    // ---- per digit: exclusive offsets across warps; tile count; publish
-    const uint32_t d = threadIdx.x;   // kThreads == kRadix
-    uint32_t cnt = 0;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-        uint32_t t = S.warp_hist[w][d];
-        S.warp_hist[w][d] = cnt;
-        cnt += t;
-    }
-    uint32_t* lb_mine = lookback + (size_t)tile * kRadix + d;
-    st_relaxed_u32(lb_mine, (tile == 0 ? kFlagP : kFlagA) | cnt);
-
-    // tile-local digit starts and the digits' global starts: block exclusive
-    // scans over the tile's 256 counts and over the whole input's
-    const uint32_t all = digit_count[d];
-    uint32_t x = cnt, y = all;
-#pragma unroll
-    for (int dd = 1; dd < 32; dd <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, x, dd), u = __shfl_up_sync(0xFFFFFFFFu, y, dd);
-        if ((int)lane >= dd) {
-            x += t;
-            y += u;
-        }
-    }
-    if (lane == 31) S.scan_tmp[warp] = make_uint2(x, y);
-    __syncthreads();
-    uint32_t dstart = x - cnt, gstart = y - all;
-    for (uint32_t w = 0; w < warp; ++w) {
-        dstart += S.scan_tmp[w].x;
-        gstart += S.scan_tmp[w].y;
-    }
-    S.digit_start[d] = dstart;
-
-    // ---- look-back for this digit: 8 preceding tiles' words per step, all
-    // loads in flight together; stop at the first inclusive prefix, wait
-    // (bounded) at the first tile that has published nothing yet
-    uint32_t excl = 0;
-    if (tile > 0) {
-        const uint32_t* base = lookback + d;
-        int64_t look = (int64_t)tile - 1;
-        uint32_t spins = 0;
-        for (;;) {
-            uint32_t w[kLookWindow];
-#pragma unroll
-            for (int q = 0; q < kLookWindow; ++q)
-                w[q] = look - q >= 0 ? ld_relaxed_u32(base + (size_t)(look - q) * kRadix) : kFlagP;
-            int used = 0;
-            bool done = false;
-#pragma unroll
-            for (int q = 0; q < kLookWindow; ++q) {
-                if (done || used < q) continue;   // stopped at an earlier word
-                const uint32_t f = w[q] & ~kCountMask;
-                if (f == 0) continue;             // not published yet: used stays q
-                excl += w[q] & kCountMask;
-                used = q + 1;
-                done = f == kFlagP;
+        for (int it = 0; it < kItems; ++it) {
+            int64_t idx = wbase + it * 32 + lane;
+            bool ok = idx < n;
+            uint32_t d = ok ? digit_of(k[it], shift, dmask) : (uint32_t)kRadix;   // kRadix = out of range
+            uint32_t peers = same_digit_lanes<sizeof(K) == 4>(d);
+            uint32_t leader = (uint32_t)(__ffs(peers) - 1);
+            uint32_t before = 0;
+            if (ok && lane == leader) {
+                before = S.warp_hist[warp][d];
+                S.warp_hist[warp][d] = before + (uint32_t)__popc(peers);
             }
-            if (done) break;
-            look -= used;
-            if (used == 0) {
-                if (++spins > spin_limit) {
-                    set_error(status, ERR_LOOKBACK_TIMEOUT);
-                    break;
+            before = __shfl_sync(0xFFFFFFFFu, before, leader);
+            rank[it] = before + (uint32_t)__popc(peers & lanemask_lt());
+            __syncwarp();
+        }
+        __syncthreads();
+
+        // ---- per digit: exclusive offsets across warps; tile count; publish
+        const uint32_t d = threadIdx.x;   // kThreads == kRadix
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            uint32_t t = S.warp_hist[w][d];
+            S.warp_hist[w][d] = cnt;
+            cnt += t;
+        }
+        uint32_t* lb_mine = lookback + (size_t)tile * kRadix + d;
+        st_relaxed_u32(lb_mine, (tile == 0 ? kFlagP : kFlagA) | cnt);
+
+        // tile-local digit starts and the digits' global starts: block exclusive
+        // scans over the tile's 256 counts and over the whole input's
+        const uint32_t all = digit_count[d];
+        uint32_t x = cnt, y = all;
+#pragma unroll
+        for (int dd = 1; dd < 32; dd <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, x, dd), u = __shfl_up_sync(0xFFFFFFFFu, y, dd);
+            if ((int)lane >= dd) {
+                x += t;
+                y += u;
+            }
+        }
+        if (lane == 31) S.scan_tmp[warp] = make_uint2(x, y);
+        __syncthreads();
+        uint32_t dstart = x - cnt, gstart = y - all;
+        for (uint32_t w = 0; w < warp; ++w) {
+            dstart += S.scan_tmp[w].x;
+            gstart += S.scan_tmp[w].y;
+        }
+        S.digit_start[d] = dstart;
+
+        // ---- look-back for this digit: 8 preceding tiles' words per step, all
+        // loads in flight together; stop at the first inclusive prefix, wait
+        // (bounded) at the first tile that has published nothing yet
+        uint32_t excl = 0;
+        if (tile > 0) {
+            const uint32_t* base = lookback + d;
+            int64_t look = (int64_t)tile - 1;
+            uint32_t spins = 0;
+            for (;;) {
+                uint32_t w[kLookWindow];
+#pragma unroll
+                for (int q = 0; q < kLookWindow; ++q)
+                    w[q] = look - q >= 0 ? ld_relaxed_u32(base + (size_t)(look - q) * kRadix) : kFlagP;
+                int used = 0;
+                bool done = false;
+#pragma unroll
+                for (int q = 0; q < kLookWindow; ++q) {
+                    if (done || used < q) continue;   // stopped at an earlier word
+                    const uint32_t f = w[q] & ~kCountMask;
+                    if (f == 0) continue;             // not published yet: used stays q
+                    excl += w[q] & kCountMask;
+                    used = q + 1;
+                    done = f == kFlagP;
                 }
-                __nanosleep(32);
+                if (done) break;
+                look -= used;
+                if (used == 0) {
+                    if (++spins > spin_limit) {
+                        set_error(status, ERR_LOOKBACK_TIMEOUT);
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+            }
+            st_relaxed_u32(lb_mine, kFlagP | (excl + cnt));
+        }
+        S.digit_global[d] = gstart + excl - dstart;
+        __syncthreads();
+
+        // ---- scatter into shared memory in digit order
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            int64_t idx = wbase + it * 32 + lane;
+            if (idx < n) {
+                uint32_t dg = digit_of(k[it], shift, dmask);
+                uint32_t pos = S.digit_start[dg] + S.warp_hist[warp][dg] + rank[it];
+                S.keys[pos] = k[it];
+                if (kVals) S.vals[pos] = v[it];
             }
         }
-        st_relaxed_u32(lb_mine, kFlagP | (excl + cnt));
-    }
-    S.digit_global[d] = gstart + excl - dstart;
-    __syncthreads();
+        __syncthreads();
 
-    // ---- scatter into shared memory in digit order
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-        int64_t idx = wbase + it * 32 + lane;
-        if (idx < n) {
-            uint32_t dg = digit_of(k[it], shift, dmask);
-            uint32_t pos = S.digit_start[dg] + S.warp_hist[warp][dg] + rank[it];
-            S.keys[pos] = k[it];
-            if (kVals) S.vals[pos] = v[it];
-        }
-    }
-    __syncthreads();
-
-    // ---- write runs to global memory
-    int64_t valid = n - tbase;
-    if (valid > kTile) valid = kTile;
-    for (int j = threadIdx.x; j < valid; j += kThreads) {
-        K kk = S.keys[j];
-        uint32_t dg = digit_of(kk, shift, dmask);
-        uint32_t o = S.digit_global[dg] + (uint32_t)j;
-        if ((int64_t)o < n) {
-            keys_out[o] = kk;
-            if (kVals) vals_out[o] = S.vals[j];
-        } else {
-            set_error(status, ERR_BAD_INDEX);
+        // ---- write runs to global memory
+        int64_t valid = n - tbase;
+        if (valid > kTile) valid = kTile;
+        for (int j = threadIdx.x; j < valid; j += kThreads) {
+            K kk = S.keys[j];
+            uint32_t dg = digit_of(kk, shift, dmask);
+            uint32_t o = S.digit_global[dg] + (uint32_t)j;
+            if ((int64_t)o < n) {
+                keys_out[o] = kk;
+                if (kVals) vals_out[o] = S.vals[j];
+            } else {
+                set_error(status, ERR_BAD_INDEX);
+            }
         }
     }
 }
@@ -483,9 +492,16 @@ static void sort_impl(const SortPlan& p, const K* keys_in, const uint32_t* vals_
     }
     const size_t smem = sizeof(OnesweepSmem<K, kVals, ITEMS>);
     static std::atomic<uint32_t> attr_set{0};
+    static std::atomic<uint32_t> wave{1};   // CTAs the GPU holds (the same on every device of the build's architecture)
     once_per_device(attr_set, [&] {
         cudaFuncSetAttribute(k_onesweep<K, kVals, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int dev = 0, sms = 0, per = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_onesweep<K, kVals, ITEMS>, kThreads, smem);
+        wave.store((uint32_t)std::max(sms, 1) * (uint32_t)std::max(per, 1));
     });
+    const unsigned grid = std::min(p.tiles, wave.load());
     const K* ksrc = keys_in;
     const uint32_t* vsrc = vals_in;
     for (uint32_t pass = 0; pass < p.passes; ++pass) {
@@ -493,7 +509,7 @@ static void sort_impl(const SortPlan& p, const K* keys_in, const uint32_t* vals_
         K* kdst = to_out ? keys_out : keys_alt;
         uint32_t* vdst = to_out ? vals_out : vals_alt;
         count_launches(1);
-        launch_after(k_onesweep<K, kVals, ITEMS>, p.tiles, kThreads, smem, st, ksrc, vsrc, kdst, vdst, p.n, p.n_dev,
+        launch_after(k_onesweep<K, kVals, ITEMS>, grid, kThreads, smem, st, ksrc, vsrc, kdst, vdst, p.n, p.n_dev,
                      pass * kRadixBits, digit_mask(p.key_bits, pass * kRadixBits), s.hist + pass * kRadix,
                      s.lookback + (size_t)pass * (p.tiles + 1) * kRadix, s.counters + pass, status, spin_limit());
         ksrc = kdst;
