@@ -38,17 +38,21 @@ constexpr bool kMatchAny = true;
 // zeroed, in the zeroed buffer.
 struct TileTables {
     uint4* desc;           // [max_tiles] {start, segment size, k | rounds << 16 | chunk bit, -}
-    uint32_t* chunks;      // [max_tiles] the chunk tiles (of large segments), in no order
+    // [kMergeClasses][max_tiles] the chunk tiles of large segments by the merge
+    // rounds their segment needs (1, 2, ...), in no order
+    uint32_t* chunks;
+    uint32_t mt;           // max_tiles
     uint32_t* fallback;    // [max_tiles] tiles left to the 64-bit tile sort, in no order
     uint32_t* tile_end;    // [max_tiles] end of a group tile (atomic max over its segments); zeroed
     uint64_t* scan_status; // look-back words of the tile scan; zeroed
-    // zeroed: [0] scan counter, [1] chunk tiles, [2] next tile of the tile
-    // sort, [3] next of the 64-bit sort, [4] tiles, [5 + l] next work item of
-    // merge round l
+    // zeroed: [0] scan counter, [2] next tile of the tile sort, [3] next of the
+    // 64-bit sort, [4] tiles, [5 + l] next work item of merge round l, [16 + r]
+    // chunk tiles of segments of r rounds
     uint32_t* ctl;
     uint32_t* wide_count;  // tiles left to the 64-bit sort
 };
-constexpr int kCtlChunks = 1, kCtlSortNext = 2, kCtlFallbackNext = 3, kCtlTiles = 4, kCtlMergeNext = 5;
+constexpr int kCtlSortNext = 2, kCtlFallbackNext = 3, kCtlTiles = 4, kCtlMergeNext = 5, kCtlChunks = 16;
+constexpr uint32_t kMergeClasses = 5;   // the most rounds a frame takes
 constexpr int kSegThreads = 256;   // segments a CTA of the tile scan takes
 
 size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -71,7 +75,8 @@ TileTables carve(const SegArgs& a) {
     t.desc = reinterpret_cast<uint4*>(b);
     b += round256(mt * 16);
     t.chunks = reinterpret_cast<uint32_t*>(b);
-    b += round256(mt * 4);
+    t.mt = (uint32_t)mt;
+    b += round256(kMergeClasses * mt * 4);
     t.fallback = reinterpret_cast<uint32_t*>(b);
     char* z = static_cast<char*>(a.zeroed);
     t.ctl = reinterpret_cast<uint32_t*>(z);
@@ -156,10 +161,12 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_tiles(const SegArgs s, uint
     if (e - a > (uint32_t)kGroup) {
         const uint32_t rounds = rounds_of((uint32_t)n);
         const int32_t m = (int32_t)min((uint32_t)n, mt - min(mt, (uint32_t)first));   // chunks that fit the table
-        const uint32_t at = m > 0 ? atomicAdd(&u.ctl[kCtlChunks], (uint32_t)m) : 0u;
+        // (more rounds than that only in a frame that is redone)
+        const uint32_t cls = min(rounds, kMergeClasses);
+        const uint32_t at = cls && m > 0 ? atomicAdd(&u.ctl[kCtlChunks + cls], (uint32_t)m) : 0u;
         for (int32_t k = 0; k < m; ++k) {
             u.desc[first + k] = make_uint4(a, e - a, (uint32_t)k | (rounds << 16) | kChunkBit, 0u);
-            u.chunks[at + k] = (uint32_t)(first + k);
+            if (cls) u.chunks[(size_t)(cls - 1) * u.mt + at + k] = (uint32_t)(first + k);
         }
         return;
     }
@@ -569,7 +576,8 @@ constexpr uint32_t kHeavyBin = 384;
 constexpr uint32_t kIndexBits = 12;   // a record's index in its tile
 constexpr int kSortBits = 8;          // digits of the radix passes
 constexpr int kBinRounds = (int)kBins / (8 * kSortThreads);   // of eight bins a thread
-static_assert(kTile == 1 << kIndexBits && kBins == 8u * kBinRounds * kSortThreads && kBins <= 1u << 14, "tile geometry");
+static_assert(kTile == 1 << kIndexBits && kBins == 8u * kBinRounds * kSortThreads && kBins <= 1u << 14,
+              "tile geometry");
 
 struct TileSmem {
     union {
@@ -924,7 +932,8 @@ SR_DEV void sort_tile64(PassSmem& S, uint32_t tile, uint64_t* keys_in, uint64_t*
     }
     if (compact) {
         radix_passes<uint64_t, kThreads, kRadixBits, uint32_t>(
-            &S.warp_hist[0][0], S.digit_start, S.scan_tmp, first, other, 0u, len, passes, [](uint64_t v, uint32_t shift) -> uint32_t {
+            &S.warp_hist[0][0], S.digit_start, S.scan_tmp, first, other, 0u, len, passes,
+            [](uint64_t v, uint32_t shift) -> uint32_t {
             return ((uint32_t)v >> shift) & (kRadix - 1);
         });
         Unpack U;
@@ -935,7 +944,8 @@ SR_DEV void sort_tile64(PassSmem& S, uint32_t tile, uint64_t* keys_in, uint64_t*
         }
     } else {
         radix_passes<uint64_t, kThreads, kRadixBits, uint32_t>(
-            &S.warp_hist[0][0], S.digit_start, S.scan_tmp, first, other, 0u, len, passes, [kmask](uint64_t v, uint32_t shift) -> uint32_t {
+            &S.warp_hist[0][0], S.digit_start, S.scan_tmp, first, other, 0u, len, passes,
+            [kmask](uint64_t v, uint32_t shift) -> uint32_t {
             return (uint32_t)((v & kmask) >> shift) & (kRadix - 1);
         });
     }
@@ -1006,11 +1016,15 @@ SR_DEV uint32_t warp_merge_split(const uint64_t* A, uint32_t na, const uint64_t*
     return lo;
 }
 
-// Work item w is part w % kMergeParts of chunk tile chunks[w / kMergeParts]; the CTAs are
-// persistent (one wave) and take items from the round's counter.
-SR_DEV void merge_item(MergeSmem& S, uint32_t item, uint64_t* __restrict__ keys_out, uint64_t* __restrict__ keys_alt,
+// Work item w is part w % kMergeParts of the w / kMergeParts-th chunk of the
+// segments that still merge in this round (by classes of rounds: with all
+// chunks in one list the last round of the 4096^2 frame spent 19 us finding
+// that most had nothing to do, 10 now); the CTAs are persistent (one
+// wave) and take items from the round's counter.
+SR_DEV void merge_item(MergeSmem& S, uint32_t item, uint32_t chunk, uint64_t* __restrict__ keys_out,
+                       uint64_t* __restrict__ keys_alt,
                        uint32_t level, uint32_t key_bits, uint32_t n_cap, const TileTables& u) {
-    const uint4 desc = u.desc[u.chunks[item / kMergeParts]];
+    const uint4 desc = u.desc[chunk];
     const uint32_t k = desc.z & 0xFFFFu, rounds = (desc.z >> 16) & 0x7FFFu;
     if (level >= rounds) return;
     const uint64_t* src = ((rounds - level) & 1u) ? keys_alt : keys_out;
@@ -1067,21 +1081,33 @@ __global__ void __launch_bounds__(kThreads) k_merge_level(uint64_t* __restrict__
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MergeSmem& S = *reinterpret_cast<MergeSmem*>(smem_raw);
     __shared__ uint32_t next;
-    const uint32_t n_items = (uint32_t)kMergeParts * u.ctl[kCtlChunks];
+    uint32_t count[kMergeClasses], n_items = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < kMergeClasses; ++r) {
+        count[r] = r >= level ? min(u.ctl[kCtlChunks + 1 + r], u.mt) : 0u;
+        n_items += (uint32_t)kMergeParts * count[r];
+    }
     for (;;) {
         if (threadIdx.x == 0) next = atomicAdd(&u.ctl[kCtlMergeNext + level], 1u);
         __syncthreads();   // also: the previous item is done with the buffers
         const uint32_t item = next;
         __syncthreads();
         if (item >= n_items) break;
-        merge_item(S, item, keys_out, keys_alt, level, key_bits, n_cap, u);
+        uint32_t at = item / kMergeParts, cls = 0;
+#pragma unroll
+        for (uint32_t r = 0; r + 1 < kMergeClasses; ++r)
+            if (cls == r && at >= count[r]) {
+                at -= count[r];
+                cls = r + 1;
+            }
+        merge_item(S, item, u.chunks[(size_t)cls * u.mt + at], keys_out, keys_alt, level, key_bits, n_cap, u);
     }
 }
 
 // ------------------------------------------------------------- launches --
 size_t segsort_table_bytes(uint32_t P, int64_t cap) {
     const size_t mt = max_tiles(P, cap);
-    return round256(mt * 16) + 2 * round256(mt * 4);
+    return round256(mt * 16) + round256(kMergeClasses * mt * 4) + round256(mt * 4);
 }
 size_t segsort_zeroed_bytes(uint32_t P, int64_t cap) { return 256 + scan_area(P) + round256(max_tiles(P, cap) * 4); }
 
