@@ -52,10 +52,10 @@ ORACLE_SAMPLE = 64
 # What bounds each stage's main kernel (profiles/ncu_top_kernels_frame4096.md):
 # the HBM fraction is the roofline only for the stages that move bytes.
 LIMITS = {
-    "resolve": "latency of each segment's walk back to its collapse cut and of the record gathers",
+    "resolve": "instruction issue: the walk back to each segment's collapse cut, then some 20 a record",
     "chains": "instruction issue: 24 bisection steps a root, and the stretches solved again",
-    "sort": "shared-memory ranking latency of the tile sort and merge rounds",
-    "winding_emit": "latency of each tile's flag, look-back and emission phases at 4-5 CTAs per SM, DRAM ~14%",
+    "sort": "instruction issue of the tile sort (73%), shared-memory reads and load latency of the merge rounds",
+    "winding_emit": "instruction issue and the barriers between a tile's phases at 5 CTAs per SM",
 }
 STAGE_NAMES = ["transform", "count", "offset_scan", "chains", "merge", "fragment", "sort", "winding_emit",
                "row_sort", "resolve", "wide"]
@@ -178,10 +178,6 @@ class ClockSampler:
 def stage_bytes(st, n_curves, n_points, W, H):
     """Algorithmic bytes per stage for one frame."""
     N = st["n_intersections"]
-    O = st["n_draw_records"]
-    passes = st["sort_passes"]
-    rows_bits = max(1, int(np.ceil(np.log2(H + 1))))
-    row_passes = (rows_bits + 7) // 8
     return {
         "transform": n_points * (8 + 4 + 8),
         "count": n_curves * (12 + 32 + 20 + 4),
@@ -192,12 +188,11 @@ def stage_bytes(st, n_curves, n_points, W, H):
         # the per-path segmented sort: one read and one write of each 8-byte
         # key (the least any sort moves; large paths' merge rounds come on top)
         "sort": N * 2 * 8,
-        # sorted keys in; draw records (16 B) and their cell rows (4 B) out
-        "winding_emit": N * 8 + O * (16 + 4),
-        "row_sort": O * 4 + row_passes * O * 2 * (4 + 4),
-        # a latency walk to each segment's collapse cut bounds it, and the
-        # records it reads depend on where the cuts fall: no byte count
-        # comparable with the streaming stages (its time is reported)
+        # sorted keys in, twice (reduce and runs); the paint runs out come on top
+        "winding_emit": N * 8 * 2,
+        # the paint runs a frame has, and how many of them the resolve reads
+        # after its collapse cuts, are not reported: times only
+        "row_sort": 0,
         "resolve": 0,
         "wide": 0,   # not used
     }

@@ -12,12 +12,11 @@
 //                         winding changes, a fully parallel read of the keys;
 //                         its last CTA scans the tile pairs into each tile's
 //                         incoming winding prefix;
-//   k_winding_emit        the records' winding scan, fragment and span flags,
-//                         output slots (one decoupled look-back over packed
-//                         31:31-bit counts of merged fragments and spans) and
-//                         the draw records.
-// Draw records come out in the reference's order: a record's merged
-// fragment, then the span ending at it.
+//   k_winding_runs        the records' winding scan, fragment and span flags,
+//                         and the paint runs at their output slots (one
+//                         decoupled look-back over the tiles' run counts).
+// k_draw_list writes the reference's draw records, in its order (a record's
+// merged fragment, then the span ending at it), when they are read back.
 //
 // The reference's winding scan is global over its one scene's records
 // (scanline_rasterizer.cpp:479-506), so a path whose changes do not sum to
