@@ -160,14 +160,30 @@ __global__ void k_path_labels(const uint32_t* __restrict__ path_first_curve, uin
 // ------------------------------------------------------------ inference --
 // A warp takes eight paths, a lane two of the 64 units of each layer for all
 // eight: a weight read from shared memory serves eight multiply-adds, and 16
-// sums are in flight a lane.  FP32 issue bounds it (4,608 multiply-adds and
-// 128 erf a path; 70% of the issue slots used): 200,000 paths take 70 us and
-// 5,000 take 8.3, where a path a thread (64 values in 247 registers, one sum
-// in flight) took 141 and 27.
+// sums are in flight a lane.  The second layer's multiply-adds are done two
+// paths an instruction (fma.rn.f32x2, each half rounded as fmaf).  Instruction
+// issue bounds it (128 erf a path are the larger part): 200,000 paths take 62.6
+// us, 20,000 take 12.0 and 5,000 take 6.5; with an instruction a multiply-add
+// 67.3 for 200,000, with four CTAs an SM and 64 registers 61.6, but 14.5 for
+// 20,000; with sixteen paths a warp 64.4; a path a thread (64 values in 247
+// registers, one sum in flight) took 141, and 27 for 5,000.
+// Two floats in one register pair, and a * b + c of both (rounded as fmaf).
+SR_DEV uint64_t pair(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+SR_DEV void unpair(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+SR_DEV uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 constexpr int kPredictThreads = 256, kPredictCtas = 3, kWarpPaths = 8;
 struct PredictSmem {
     Params P;
-    __align__(16) float h[kPredictThreads / 32][kWarpPaths][kRow];
+    __align__(16) float h[kPredictThreads / 32][kH][kWarpPaths];   // a unit's values of the warp's paths
 };
 __global__ void __launch_bounds__(kPredictThreads, kPredictCtas) k_mlp_predict(
     const __nv_bfloat16* __restrict__ wb, const float* __restrict__ master, const float* __restrict__ norm,
@@ -178,7 +194,7 @@ __global__ void __launch_bounds__(kPredictThreads, kPredictCtas) k_mlp_predict(
     load_params(wb, master, norm, S.P);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float(*h)[kRow] = S.h[warp];
+    float(*h)[kWarpPaths] = S.h[warp];
     const uint32_t warps = gridDim.x * (kPredictThreads / 32);
     for (uint32_t g = blockIdx.x * (kPredictThreads / 32) + warp; g * kWarpPaths < n; g += warps) {
         const uint32_t p0 = g * kWarpPaths;
@@ -191,38 +207,54 @@ __global__ void __launch_bounds__(kPredictThreads, kPredictCtas) k_mlp_predict(
             if (lane < kWarpPaths * kIn - 32 && i1 < n * kIn) v1 = (x[i1] - P.norm[nXm + k1]) * P.norm[nXs + k1];
         }
 #pragma unroll
-        for (int q = 0; q < kWarpPaths; ++q) {
-            float a0 = P.b1[lane], a1 = P.b1[lane + 32];
+        for (int q0 = 0; q0 < kWarpPaths; q0 += 4) {
+            float4 g0, g1;
 #pragma unroll
-            for (int k = 0; k < kIn; ++k) {
-                const int e = q * kIn + k;
-                const float in = __shfl_sync(0xFFFFFFFFu, e < 32 ? v0 : v1, e & 31);
-                a0 = fmaf(P.w1t[k][lane], in, a0);
-                a1 = fmaf(P.w1t[k][lane + 32], in, a1);
+            for (int i = 0; i < 4; ++i) {
+                float a0 = P.b1[lane], a1 = P.b1[lane + 32];
+#pragma unroll
+                for (int k = 0; k < kIn; ++k) {
+                    const int e = (q0 + i) * kIn + k;
+                    const float in = __shfl_sync(0xFFFFFFFFu, e < 32 ? v0 : v1, e & 31);
+                    a0 = fmaf(P.w1t[k][lane], in, a0);
+                    a1 = fmaf(P.w1t[k][lane + 32], in, a1);
+                }
+                (&g0.x)[i] = gelu(a0);
+                (&g1.x)[i] = gelu(a1);
             }
-            h[q][lane] = gelu(a0);
-            h[q][lane + 32] = gelu(a1);
+            *reinterpret_cast<float4*>(&h[lane][q0]) = g0;
+            *reinterpret_cast<float4*>(&h[lane + 32][q0]) = g1;
         }
         __syncwarp();
-        // layer 2
-        float a0[kWarpPaths], a1[kWarpPaths];
+        // layer 2, two paths an instruction
+        uint64_t s0[kWarpPaths / 2], s1[kWarpPaths / 2];
 #pragma unroll
-        for (int q = 0; q < kWarpPaths; ++q) {
-            a0[q] = P.b2[lane];
-            a1[q] = P.b2[lane + 32];
+        for (int q = 0; q < kWarpPaths / 2; ++q) {
+            s0[q] = pair(P.b2[lane], P.b2[lane]);
+            s1[q] = pair(P.b2[lane + 32], P.b2[lane + 32]);
         }
 #pragma unroll 2
         for (int k = 0; k < kH; k += 4) {
             const float4 w0 = *reinterpret_cast<const float4*>(&P.w2[lane][k]);
             const float4 w1 = *reinterpret_cast<const float4*>(&P.w2[lane + 32][k]);
 #pragma unroll
-            for (int q = 0; q < kWarpPaths; ++q) {
-                const float4 u = *reinterpret_cast<const float4*>(&h[q][k]);
-                a0[q] = fmaf(w0.x, u.x, a0[q]); a1[q] = fmaf(w1.x, u.x, a1[q]);
-                a0[q] = fmaf(w0.y, u.y, a0[q]); a1[q] = fmaf(w1.y, u.y, a1[q]);
-                a0[q] = fmaf(w0.z, u.z, a0[q]); a1[q] = fmaf(w1.z, u.z, a1[q]);
-                a0[q] = fmaf(w0.w, u.w, a0[q]); a1[q] = fmaf(w1.w, u.w, a1[q]);
+            for (int i = 0; i < 4; ++i) {
+                const uint64_t d0 = pair((&w0.x)[i], (&w0.x)[i]), d1 = pair((&w1.x)[i], (&w1.x)[i]);
+#pragma unroll
+                for (int q = 0; q < kWarpPaths / 2; q += 2) {
+                    const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(&h[k + i][2 * q]);
+                    s0[q] = fma2(d0, u.x, s0[q]);
+                    s1[q] = fma2(d1, u.x, s1[q]);
+                    s0[q + 1] = fma2(d0, u.y, s0[q + 1]);
+                    s1[q + 1] = fma2(d1, u.y, s1[q + 1]);
+                }
             }
+        }
+        float a0[kWarpPaths], a1[kWarpPaths];
+#pragma unroll
+        for (int q = 0; q < kWarpPaths / 2; ++q) {
+            unpair(s0[q], a0[2 * q], a0[2 * q + 1]);
+            unpair(s1[q], a1[2 * q], a1[2 * q + 1]);
         }
         // layer 3: 16 sums over the lanes, halving the sums a lane holds with
         // every exchange: lane l ends with output l & 15 (path l / 2 & 7,
@@ -301,8 +333,8 @@ SR_DEV void red_add4(float* p, float a, float b, float c, float d) {
 // parameter gradients are summed over its samples in registers and added into
 // grad.  loss_sum receives the sum of squared errors (a double: a float sum
 // in the order the warps come differs by up to 3e-6 from run to run).  With
-// `adam`, the CTA
-// that finishes last takes the optimiser step (a launch and its gap saved).
+// `adam`, the CTA that finishes last takes the optimiser step (a launch and its
+// gap saved).
 // Shared-memory reads and the latency of its eight phases bound it: a step
 // of 4,096 samples takes 23 us, where 64 CTAs of 64 threads, a sample each,
 // and a separate optimiser launch took 84.
