@@ -17,7 +17,7 @@ REPO = os.path.dirname(HERE)
 
 CU_SOURCES = ["geom.cu", "scan.cu", "sort.cu", "winding.cu", "resolve.cu", "mlp.cu", "segsort.cu", "api.cu", "noalloc.cu"]
 CPP_SOURCES = ["host.cpp", "server.cpp", "image.cpp"]
-HEADERS = ["common.cuh", "scan.cuh", "kernels.h", "synth.h"]
+HEADERS = ["common.cuh", "scan.cuh", "segtiles.cuh", "kernels.h", "synth.h"]
 
 NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

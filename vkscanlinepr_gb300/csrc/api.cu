@@ -940,15 +940,16 @@ struct Pipeline {
         launch_order_records(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), rec.as<int2>(), status, sm_count, st);
         mark(ST_MERGE, true);
         mark(ST_FRAGMENT, false);
+        last_segsort = segmented() && seg_levels >= 0;
+        SegArgs seg = seg_args(cap, zero + at.seg);
         launch_fragment(g, rec.as<int2>(), cap, n_dev, keys.as<uint64_t>(), keep ? wnp.as<uint8_t>() : nullptr, dbg,
-                        st);
+                        last_segsort ? &seg : nullptr, status, st);
         mark(ST_FRAGMENT, true);
         const KeyLayout L = g.L;
         SortPlan sp = sort_plan(cap, L.pbits + L.rbits + L.xbits, n_dev, tune.sort_items);
         mark(ST_SORT, false);
-        last_segsort = segmented() && seg_levels >= 0;
         if (last_segsort)
-            launch_segsort(seg_args(cap, zero + at.seg), keys.as<uint64_t>(), skeys.as<uint64_t>(),
+            launch_segsort(seg, keys.as<uint64_t>(), skeys.as<uint64_t>(),
                            keys_alt.as<uint64_t>(), L, seg_levels, sm_count, status, st);
         else
             launch_sort_u64(sp, keys.as<uint64_t>(), nullptr, skeys.as<uint64_t>(),

@@ -9,6 +9,7 @@
 
 #include "kernels.h"
 #include "scan.cuh"
+#include "segtiles.cuh"
 
 namespace sr {
 
@@ -1133,13 +1134,24 @@ __global__ void __launch_bounds__(128) k_merge(const GeomArgs g, const int32_t* 
 // 0.208 and 0.128; evaluating both ends in every lane took 0.225).
 constexpr int kFragWarps = 4, kFragOut = 31;
 
-__global__ void __launch_bounds__(32 * kFragWarps) k_fragment(const GeomArgs g, const int2* __restrict__ rec,
-                                                              int64_t n_cap, const uint32_t* __restrict__ n_dev,
-                                                              uint64_t* __restrict__ keys, uint8_t* __restrict__ wnp,
-                                                              DebugOut dbg) {
+// SEG: the first seg_ctas CTAs build the tables of the per-path sort beside
+// that.  For a frame of few paths that saves the tables' launch, 3 us of the 154
+// of the 1024^2 frame; of many paths the kernel with the call in it is slower by
+// as much as the launch takes (0.212 instead of 0.205 ms on the 4096^2 frame).
+constexpr uint32_t kSegPaths = 4096;
+static_assert(kSegThreads == 32 * kFragWarps, "one launch");
+template <bool SEG>
+__global__ void __launch_bounds__(32 * kFragWarps) k_fragment(
+    const GeomArgs g, const int2* __restrict__ rec, int64_t n_cap, const uint32_t* __restrict__ n_dev,
+    uint64_t* __restrict__ keys, uint8_t* __restrict__ wnp, DebugOut dbg, uint32_t seg_ctas,
+    const __grid_constant__ SegArgs seg, const __grid_constant__ TileTables tables, uint32_t* status, uint32_t spin_limit) {
     wait_for_stream();
+    if (SEG && blockIdx.x < seg_ctas) {
+        seg_tiles(seg, tables, status, spin_limit);
+        return;
+    }
     const int64_t n = (int64_t)min((uint64_t)*n_dev, (uint64_t)n_cap);
-    const int64_t b = ((int64_t)blockIdx.x * kFragWarps + (threadIdx.x >> 5)) * kFragOut;
+    const int64_t b = ((int64_t)(blockIdx.x - (SEG ? seg_ctas : 0u)) * kFragWarps + (threadIdx.x >> 5)) * kFragOut;
     if (b >= n) return;
     const uint32_t lane = lane_id();
     const int64_t i = b + lane;
@@ -1295,12 +1307,20 @@ void launch_order_records(const GeomArgs& g, const int32_t* offs, const ChainWor
 }
 
 void launch_fragment(const GeomArgs& g, const int2* rec, int64_t n_cap, const uint32_t* n_dev, uint64_t* keys,
-                     uint8_t* wnp, const DebugOut& dbg, cudaStream_t st) {
+                     uint8_t* wnp, DebugOut dbg, SegArgs* seg, uint32_t* status, cudaStream_t st) {
     if (n_cap <= 0 || g.n_curves == 0) return;
     count_launches(1);
     constexpr int64_t per = kFragWarps * kFragOut;
-    launch_after(k_fragment, (unsigned)((n_cap + per - 1) / per), 32 * kFragWarps, 0, st, g, rec, n_cap, n_dev, keys,
-                 wnp, dbg);
+    const unsigned grid = (unsigned)((n_cap + per - 1) / per);
+    if (seg && seg->n_paths <= kSegPaths) {
+        const uint32_t seg_ctas = (seg->n_paths + kSegThreads - 1) / kSegThreads;
+        seg->tables_built = true;
+        launch_after(k_fragment<true>, grid + seg_ctas, 32 * kFragWarps, 0, st, g, rec, n_cap, n_dev, keys, wnp, dbg,
+                     seg_ctas, *seg, segsort_tables(*seg), status, spin_limit());
+    } else {
+        launch_after(k_fragment<false>, grid, 32 * kFragWarps, 0, st, g, rec, n_cap, n_dev, keys, wnp, dbg, 0u,
+                     SegArgs{}, TileTables{}, status, spin_limit());
+    }
 }
 
 }  // namespace sr

@@ -148,8 +148,13 @@ void launch_merge(const GeomArgs& g, const int32_t* offs, const ChainWork& w, co
 // centre part).  With wnp NULL the bits are stored above the key bits of
 // each key instead of in wnp[].
 // n_cap launches the grid; the record count is read from n_dev (offs[C]).
+struct SegArgs;
+struct TileTables;
+// seg: the per-path sort's segments (NULL: none), whose tables it builds when
+// they are few (seg->tables_built).
 void launch_fragment(const GeomArgs& g, const int2* rec, int64_t n_cap, const uint32_t* n_dev, uint64_t* keys,
-                     uint8_t* wnp, const DebugOut& dbg, cudaStream_t st);
+                     uint8_t* wnp, DebugOut dbg, SegArgs* seg, uint32_t* status, cudaStream_t st);
+TileTables segsort_tables(const SegArgs& a);
 
 // ---- scan.cu
 // Exclusive scan of n int32 values into out[0..n] (out[n] = total).  in and
@@ -215,6 +220,7 @@ struct SegArgs {
     bool wide;                    // those tiles are sorted (else flagged as a capacity overflow)
     void* tables;                 // segsort_table_bytes
     void* zeroed;                 // segsort_zeroed_bytes, zeroed before
+    bool tables_built = false;    // by launch_fragment
 };
 size_t segsort_table_bytes(uint32_t n_paths, int64_t cap);
 size_t segsort_zeroed_bytes(uint32_t n_paths, int64_t cap);
