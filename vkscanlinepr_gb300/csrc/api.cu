@@ -490,7 +490,7 @@ struct Pipeline {
         for (uint32_t s = 0; s < S; ++s) {
             const sr::SceneInfo& si = info[s];
             cta_base[s] = res_ctas;
-            res_ctas += sr::resolve_ctas(si.W, si.rows, mode == SR_MODE_PIXEL, res_seg, tune.resolve_warps);
+            res_ctas += sr::resolve_ctas(si.W, si.rows, res_seg, tune.resolve_warps);
         }
         cta_base[S] = res_ctas;
         CUDA_TRY(ensure(scenes_d, sizeof(sr::SceneInfo) * std::max<uint32_t>(S, 1)));

@@ -261,7 +261,7 @@ struct WindArgs {
     uint32_t* path_draw;            // [P] draw records per path (NULL unless labelling)
     // [cut_rows][cut_segs]: 1 + the last index of a run that covers a
     // resolve segment (kResolveSeg pixels) entirely and leaves nothing of
-    // what was under it (opaque in pixel mode, any run in reference mode);
+    // what was under it (an opaque one; pixel mode only);
     // zeroed before the emit
     uint32_t* seg_cut;
     uint32_t cut_rows, cut_segs;
@@ -320,7 +320,7 @@ struct ResolveArgs {
     int32_t F;
     int32_t pixel_mode;
     int32_t warps;                    // warps per CTA: 8 or 16
-    int32_t seg;                      // pixels per warp: kResolveSeg, or 128 or 64 (pixel mode)
+    int32_t seg;                      // pixels per warp: kResolveSeg, or 128 or 64
     uint32_t* image;                  // all scenes' RGBA8 framebuffers
     uint32_t* image2 = nullptr;       // the caller's memory for them too, or NULL
     const uint32_t* control = nullptr; // control block, whose first report_words words go to report (host memory)
@@ -337,7 +337,7 @@ constexpr int kResolveSeg = 256;
 // Pixels per warp for a frame of `segs` segments of kResolveSeg pixels.
 int resolve_segment(uint64_t segs, int pixel_mode, int sm_count);
 // CTAs that a scene of `rows` cell rows takes.
-uint32_t resolve_ctas(int32_t W, uint32_t rows, int pixel_mode, int seg, int warps);
+uint32_t resolve_ctas(int32_t W, uint32_t rows, int seg, int warps);
 void launch_resolve(const ResolveArgs& a, uint32_t n_ctas, cudaStream_t st);
 // Multisampling: sum a sample frame into acc (first: start the sums), and
 // write the rounded averages of k frames.

@@ -8,10 +8,9 @@
 // the reference pipeline); pixel mode composites source-over with integer
 // arithmetic.  Draw records are first sorted stably by cell row (onesweep), so
 // a row's records are applied in path order; a thread owns a fixed set of
-// pixels, so no barrier is needed between records.  In pixel mode a warp paints
-// a segment of a row and first finds where its painting may start (the collapse
-// cut below); in reference mode a CTA owns one cell row (or several short ones)
-// and stages its records in shared memory.
+// pixels, so no barrier is needed between records.  A warp paints a segment of a
+// row: in pixel mode it first finds where its painting may start (the collapse
+// cut below), in reference mode it takes the latest record of each pixel.
 #include <algorithm>
 
 #include "common.cuh"
@@ -46,7 +45,6 @@ __global__ void k_row_bounds(const uint32_t* __restrict__ srows, int64_t n_cap, 
 // (checked exhaustively by the CPU tests).  Alpha stays 255:
 // (255*a + 255*(255-a) + 127) / 255 = 255.
 constexpr float kRound = 12582912.0f;   // 1.5 * 2^23
-constexpr int kK = kResolveSeg / 32;   // pixels per lane of a whole segment
 constexpr int kChunk = 1024;
 constexpr uint64_t kHalfSegs = 200, kQuarterSegs = 40;   // segments of kResolveSeg an SM
 
@@ -70,15 +68,13 @@ template <class Rec> SR_DEV void blend3(uint32_t& rb, float& g, const Rec& q) {
 
 int resolve_segment(uint64_t segs, int pixel_mode, int sm_count) {
     const uint64_t sms = (uint64_t)(sm_count > 0 ? sm_count : 1);
-    if (!pixel_mode || segs >= kHalfSegs * sms) return kResolveSeg;
+    if (segs >= (pixel_mode ? kHalfSegs : kQuarterSegs) * sms) return kResolveSeg;
     return segs >= kQuarterSegs * sms ? kResolveSeg / 2 : kResolveSeg / 4;
 }
 
-uint32_t resolve_ctas(int32_t W, uint32_t rows, int pixel_mode, int seg, int warps) {
+uint32_t resolve_ctas(int32_t W, uint32_t rows, int seg, int warps) {
     const uint32_t segs = (uint32_t)((W + seg - 1) / seg);
-    if (pixel_mode) return (rows * segs + (uint32_t)warps - 1) / (uint32_t)warps;
-    const uint32_t rpc = segs >= (uint32_t)warps ? 1u : (uint32_t)warps / segs;
-    return (rows + rpc - 1) / rpc;
+    return (rows * segs + (uint32_t)warps - 1) / (uint32_t)warps;
 }
 
 SR_DEV uint32_t scene_of_cta(const ResolveArgs& a) {   // last s with cta_base[s] <= blockIdx.x
@@ -91,50 +87,11 @@ SR_DEV uint32_t scene_of_cta(const ResolveArgs& a) {   // last s with cta_base[s
     return lo;
 }
 
-// Reference mode: which rows and segment a warp paints.  A CTA holds
-// rows_per_cta cell rows of one scene; small canvases give each row fewer
-// warps than the CTA has.
-struct ResolveWork {
-    const SceneInfo* si;
-    int32_t W, r0, nr, segs, groups, my_row;
-    bool active;
-};
-
-template <int WARPS> SR_DEV ResolveWork resolve_work(const ResolveArgs& a) {
-    constexpr int kResolveWarps = WARPS;
-    const uint32_t lo = scene_of_cta(a);
-    ResolveWork w;
-    w.si = &a.scenes[lo];
-    w.W = w.si->W;
-    w.segs = (w.W + kResolveSeg - 1) / kResolveSeg;
-    const int32_t R = w.segs >= kResolveWarps ? 1 : kResolveWarps / w.segs;
-    w.r0 = (int32_t)(blockIdx.x - a.cta_base[lo]) * R;
-    w.nr = imin(R, (int32_t)w.si->rows - w.r0);
-    const int warp = threadIdx.x >> 5;
-    if (w.segs >= kResolveWarps) {
-        w.my_row = 0;
-        w.groups = (w.segs + kResolveWarps - 1) / kResolveWarps;
-        w.active = true;
-    } else {
-        w.my_row = warp / w.segs;
-        w.groups = 1;
-        w.active = w.my_row < w.nr;
-    }
-    return w;
-}
-
 // A warp skips the records before the last one that covers its whole segment
 // and hides what is under it (seg_cut, written by the emit): source-over with
-// a = 255 gives floor((255 s + 127) / 255) = s whatever the pixel held, and an
-// overwrite leaves nothing of it either.
+// a = 255 gives floor((255 s + 127) / 255) = s whatever the pixel held.
 SR_DEV uint32_t resolve_cut(const ResolveArgs& a, uint32_t global_row, int32_t seg) {
     return a.seg_cut ? a.seg_cut[(size_t)global_row * a.cut_segs + (uint32_t)(seg / kResolveSeg)] : 0u;
-}
-
-template <int WARPS> SR_DEV int32_t resolve_seg(const ResolveWork& w, int group) {
-    constexpr int kResolveWarps = WARPS;
-    const int warp = threadIdx.x >> 5;
-    return w.segs >= kResolveWarps ? group * kResolveWarps + warp : warp % w.segs;
 }
 
 // Colour of gradient paint P at the pixel-space point (x, y), packed RGBA8,
@@ -521,95 +478,84 @@ __global__ void __launch_bounds__(32 * WARPS, (GRAD ? 32 : K == 8 ? 40 : 48) / W
 }
 
 // ------------------------------------------------------- reference mode --
-// Overwrite in draw order (blending off); a cell row is FRAG_SIZE pixel
-// rows, painted alike.
+// Overwrite in draw order (blending off); a cell row is FRAG_SIZE pixel rows,
+// painted alike.  A pixel takes the latest record over it, so a warp walks its
+// row's records from the end back, 32 at a time, fills the pixels of its segment
+// that have none yet and stops when all have.  (A CTA a row or several short
+// ones that staged all their records for its warps, in draw order, took 18 us for
+// a 1000x750 frame of 1,200 paths and 82 for the 4096^2 one; this takes 8 and 43.)
+// 64 pixels a warp below 40 segments of 256 an SM, else 256: for 512^2 and 3,000
+// paths 8 us with 64 and 12 with 256, for 2048^2 and 5,000 24 and 18 (128: 20).
 struct RefRec {
     int32_t x0, x1;
     uint32_t col;
-    int32_t row;
-    uint32_t idx1;   // 1 + draw index
 };
 
-template <int WARPS, bool GRAD>
+template <int WARPS, int K, bool GRAD>
 __global__ void __launch_bounds__(32 * WARPS) k_resolve_ref(const ResolveArgs a) {
     wait_for_stream();
     write_report(a);
-    __shared__ RefRec sq[kChunk];
-    const ResolveWork w = resolve_work<WARPS>(a);
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int32_t W = w.W;
-    const uint32_t gr0 = w.si->row_base + (uint32_t)w.r0;
-    const int32_t beg = a.row_start[gr0], end = a.row_start[gr0 + (uint32_t)w.nr];
-    for (int group = 0; group < w.groups; ++group) {
-        const int32_t seg = resolve_seg<WARPS>(w, group) * kResolveSeg;
-        const bool live = w.active && seg < W;
-        const uint32_t cut = live ? resolve_cut(a, w.si->row_base + (uint32_t)(w.r0 + w.my_row), seg) : 0u;
-        uint32_t px[kK];
+    constexpr int kSeg = 32 * K;
+    __shared__ RefRec slots[WARPS * 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t scene = scene_of_cta(a);
+    const SceneInfo* si = &a.scenes[scene];
+    const int32_t W = si->W;
+    const uint32_t segs = (uint32_t)(W + kSeg - 1) / kSeg;
+    const uint32_t item = (blockIdx.x - a.cta_base[scene]) * WARPS + (uint32_t)warp;
+    const uint32_t y = item / segs;
+    if (y >= si->rows) return;
+    const int32_t seg = (int32_t)(item - y * segs) * kSeg;
+    RefRec* slot = slots + warp * 32;
+    const uint32_t r = si->row_base + y;
+    const int32_t beg = a.row_start[r], end = a.row_start[r + 1];
+    uint32_t px[K], open = 0;   // pixels on the canvas without a record yet
 #pragma unroll
-        for (int j = 0; j < kK; ++j) px[j] = 0xFFFFFFFFu;
-        for (int32_t c0 = beg; c0 < end; c0 += kChunk) {
-            const int32_t cnt = imin(kChunk, end - c0);
-            __syncthreads();
-            for (int q = tid; q < cnt; q += blockDim.x) {
-                const uint32_t di = a.row_sorted_idx[c0 + q];
-                int4 d = a.draw[di];
-                RefRec rr;
-                rr.idx1 = di + 1u;
-                rr.x0 = d.x & 0xFFFF;
-                rr.x1 = wadd(rr.x0, d.y);
-                rr.col = (uint32_t)d.z;
-                rr.row = div_F(d.x >> 16, a.F) - w.r0;
-                sq[q] = rr;
-            }
-            __syncthreads();
-            if (!live) continue;
-            for (int32_t g0 = 0; g0 < cnt; g0 += 32) {
-                const int32_t qi = g0 + lane;
-                bool ov = false;
-                if (qi < cnt)
-                    ov = sq[qi].row == w.my_row && sq[qi].x0 < seg + kResolveSeg && sq[qi].x1 > seg &&
-                         sq[qi].idx1 >= cut;
-                uint32_t m = __ballot_sync(0xFFFFFFFFu, ov);
-                while (m) {
-                    const int q = g0 + __ffs(m) - 1;
-                    m &= m - 1;
-                    const RefRec rr = sq[q];
-                    const int32_t paint = GRAD ? fill_paint(rr.col) : -1;
-                    if (paint >= 0) {
-                        // a gradient, sampled on the cell's centre row; a
-                        // paint the table lacks paints nothing
-                        if (a.paints && (uint32_t)paint < a.n_paints) {
-                            const DevPaint& P = a.paints[paint];
-                            const float yc = __fadd_rn((float)((w.r0 + w.my_row) * a.F), 1.0f);
+    for (int j = 0; j < K; ++j) {
+        px[j] = 0xFFFFFFFFu;
+        open |= (seg + lane + 32 * j < W ? 1u : 0u) << j;
+    }
+    for (int32_t c1 = end; c1 > beg && __any_sync(0xFFFFFFFFu, open != 0); c1 -= 32) {
+        const int32_t q = c1 - 32 + lane;
+        bool ov = false;
+        if (q >= beg) {
+            const int4 d = a.draw[a.row_sorted_idx[q]];
+            const int32_t x0 = d.x & 0xFFFF, x1 = wadd(x0, d.y);
+            ov = x0 < seg + kSeg && x1 > seg && div_F(d.x >> 16, a.F) == (int32_t)y;
+            // a gradient that the table lacks paints nothing
+            if (GRAD && ov && fill_paint((uint32_t)d.z) >= 0)
+                ov = a.paints && (uint32_t)fill_paint((uint32_t)d.z) < a.n_paints;
+            if (ov) slot[lane] = RefRec{x0, x1, (uint32_t)d.z};
+        }
+        uint32_t m = __ballot_sync(0xFFFFFFFFu, ov);
+        __syncwarp();
+        while (m) {
+            const int b = 31 - __clz((int)m);
+            m &= ~(1u << b);
+            const RefRec rr = slot[b];
+            const int32_t paint = GRAD ? fill_paint(rr.col) : -1;
+            // a gradient is sampled on the cell's centre row
+            const float yc = GRAD ? __fadd_rn((float)((int32_t)y * a.F), 1.0f) : 0.0f;
 #pragma unroll
-                            for (int j = 0; j < kK; ++j) {
-                                int32_t p = seg + lane + 32 * j;
-                                if (p >= rr.x0 && p < rr.x1) px[j] = paint_color(P, __fadd_rn((float)p, 0.5f), yc);
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < kK; ++j) {
-                            int32_t p = seg + lane + 32 * j;
-                            if (p >= rr.x0 && p < rr.x1) px[j] = rr.col;
-                        }
-                    }
+            for (int j = 0; j < K; ++j) {
+                const int32_t p = seg + lane + 32 * j;
+                if (((open >> j) & 1u) && p >= rr.x0 && p < rr.x1) {
+                    px[j] = paint >= 0 ? paint_color(a.paints[paint], __fadd_rn((float)p, 0.5f), yc) : rr.col;
+                    open &= ~(1u << j);
                 }
             }
         }
-        if (live) {
-            const int32_t y0 = (w.r0 + w.my_row) * a.F;
-            const int32_t nrows = imin(a.F, w.si->H - y0);
-            for (int32_t yy = 0; yy < nrows; ++yy) {
-                const uint64_t row = w.si->image_off + (uint64_t)(y0 + yy) * (uint32_t)W;
+        __syncwarp();
+    }
+    const int32_t y0 = (int32_t)y * a.F, nrows = imin(a.F, si->H - y0);
+    for (int32_t yy = 0; yy < nrows; ++yy) {
+        const uint64_t row = si->image_off + (uint64_t)(y0 + yy) * (uint32_t)W;
 #pragma unroll
-                for (int j = 0; j < kK; ++j) {
-                    int32_t p = seg + lane + 32 * j;
-                    if (p < W) {
-                        a.image[row + (uint32_t)p] = px[j];
-                        if (a.image2) a.image2[row + (uint32_t)p] = px[j];
-                    }
-                }
+        for (int j = 0; j < K; ++j) {
+            const int32_t p = seg + lane + 32 * j;
+            if (p < W) {
+                a.image[row + (uint32_t)p] = px[j];
+                if (a.image2) a.image2[row + (uint32_t)p] = px[j];
             }
         }
     }
@@ -621,7 +567,8 @@ template <int WARPS, bool GRAD> static void launch_resolve_t(const ResolveArgs& 
         else if (a.seg == 128) launch_after(k_resolve_pixel<WARPS, 4, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
         else launch_after(k_resolve_pixel<WARPS, 8, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
     } else {
-        launch_after(k_resolve_ref<WARPS, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
+        if (a.seg == kResolveSeg / 4) launch_after(k_resolve_ref<WARPS, 2, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
+        else launch_after(k_resolve_ref<WARPS, 8, GRAD>, n_ctas, 32 * WARPS, 0, st, a);
     }
 }
 

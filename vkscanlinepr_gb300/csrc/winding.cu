@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(THREADS, 5) k_winding_runs(const WindArgs a, c
                 counted = row < a.cut_rows;
                 // a run that hides everything under it ends the resolve's work
                 // before it in each segment it covers whole
-                if (counted && (!a.pixel_mode || (info >> 24) == 255u)) {
+                if (counted && a.pixel_mode && (info >> 24) == 255u) {
                     const int32_t s_hi = imin(x1 / kResolveSeg, (int32_t)a.cut_segs);
                     for (int32_t sg = (x0 + kResolveSeg - 1) / kResolveSeg; sg < s_hi; ++sg)
                         atomicMax(&a.seg_cut[(size_t)row * a.cut_segs + (uint32_t)sg], (uint32_t)o + 1u);
