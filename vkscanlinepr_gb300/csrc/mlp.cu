@@ -195,16 +195,16 @@ __global__ void __launch_bounds__(kPredictThreads, kPredictCtas) k_mlp_predict(
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float(*h)[kWarpPaths] = S.h[warp];
-    const uint32_t warps = gridDim.x * (kPredictThreads / 32);
-    for (uint32_t g = blockIdx.x * (kPredictThreads / 32) + warp; g * kWarpPaths < n; g += warps) {
-        const uint32_t p0 = g * kWarpPaths;
+    const uint32_t warps = gridDim.x * (kPredictThreads / 32), groups = n / kWarpPaths + (n % kWarpPaths ? 1u : 0u);
+    for (uint32_t g = blockIdx.x * (kPredictThreads / 32) + warp; g < groups; g += warps) {
+        const int here = g < n / kWarpPaths ? kWarpPaths : (int)(n % kWarpPaths);   // paths of this group
+        const float* xg = x + (size_t)g * (kWarpPaths * kIn);   // (6 n needs more than 32 bits)
         // layer 1: units lane and lane + 32
         float v0 = 0.0f, v1 = 0.0f;   // the eight paths' 48 inputs, standardised
         {
-            const uint32_t i0 = p0 * kIn + lane, i1 = i0 + 32;
             const int k0 = lane % kIn, k1 = (lane + 32) % kIn;
-            if (i0 < n * kIn) v0 = (x[i0] - P.norm[nXm + k0]) * P.norm[nXs + k0];
-            if (lane < kWarpPaths * kIn - 32 && i1 < n * kIn) v1 = (x[i1] - P.norm[nXm + k1]) * P.norm[nXs + k1];
+            if (lane < here * kIn) v0 = (xg[lane] - P.norm[nXm + k0]) * P.norm[nXs + k0];
+            if (lane + 32 < here * kIn) v1 = (xg[lane + 32] - P.norm[nXm + k1]) * P.norm[nXs + k1];
         }
 #pragma unroll
         for (int q0 = 0; q0 < kWarpPaths; q0 += 4) {
@@ -277,9 +277,9 @@ __global__ void __launch_bounds__(kPredictThreads, kPredictCtas) k_mlp_predict(
             }
         }
         const float sum = o[0] + __shfl_xor_sync(0xFFFFFFFFu, o[0], 16);
-        const uint32_t at = p0 * kOut + lane;
         const int k = lane & 1;
-        if (lane < 2 * kWarpPaths && at < n * kOut) y[at] = fmaf(sum + P.b3[k], P.norm[nYs + k], P.norm[nYm + k]);
+        if (lane < here * kOut)
+            y[(size_t)g * (kWarpPaths * kOut) + lane] = fmaf(sum + P.b3[k], P.norm[nYs + k], P.norm[nYm + k]);
         __syncwarp();
     }
 }
@@ -637,7 +637,7 @@ void launch_mlp_predict(const void* wb, const float* master, const float* norm, 
     if (!n) return;
     count_launches(1);
     constexpr unsigned per = kPredictThreads / 32 * kWarpPaths;
-    unsigned blocks = (n + per - 1) / per;
+    unsigned blocks = n / per + (n % per ? 1u : 0u);
     const unsigned cap = (unsigned)kPredictCtas * (unsigned)(sm_count > 0 ? sm_count : 148);   // one wave
     if (blocks > cap) blocks = cap;
     launch_after(k_mlp_predict, blocks, kPredictThreads, 0, st, static_cast<const __nv_bfloat16*>(wb), master, norm, x,
