@@ -1035,6 +1035,9 @@ struct Pipeline {
         ra.report_words = CTL_REPORT;
         mark(ST_RESOLVE, false);
         launch_resolve(ra, res_ctas, st);
+        // (a batch without scenes has no CTA that writes the report)
+        if (!res_ctas)
+            CUDA_TRY(cudaMemcpyAsync(h_report, ctl.p, sizeof(uint32_t) * CTL_REPORT, cudaMemcpyDeviceToHost, st));
         mark(ST_RESOLVE, true);
         CUDA_TRY(cudaGetLastError());
         return SR_OK;
