@@ -67,12 +67,14 @@ sr_status fail(sr_status s, const char* fmt, ...) {
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
+    uint32_t moves = 0;   // times the memory was replaced
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
 // Grows b to hold `bytes`, with `slack` (a quarter by default) to spare.
 cudaError_t ensure(DevBuf& b, size_t bytes, bool slack = true) {
     if (bytes <= b.cap && b.p) return cudaSuccess;
+    ++b.moves;
     if (b.p) {
         cudaFree(b.p);
         b.p = nullptr;
@@ -90,6 +92,7 @@ cudaError_t ensure(DevBuf& b, size_t bytes, bool slack = true) {
 }
 
 void release(DevBuf& b) {
+    ++b.moves;
     if (b.p) cudaFree(b.p);
     b.p = nullptr;
     b.cap = 0;
@@ -805,33 +808,42 @@ struct Pipeline {
         stages_valid = false;
     }
 
+    // The buffers whose addresses a batch's frame holds.
+    static constexpr DevBuf Pipeline::* kFrameBufs[] = {
+        &Pipeline::pos, &Pipeline::pos_path, &Pipeline::curve_pos, &Pipeline::curve_type, &Pipeline::curve_path,
+        &Pipeline::fill_rule, &Pipeline::fill_info, &Pipeline::path_scene, &Pipeline::scenes_d, &Pipeline::cta_base_d,
+        &Pipeline::tpos, &Pipeline::curve_end, &Pipeline::path_begin, &Pipeline::cut, &Pipeline::count,
+        &Pipeline::offs, &Pipeline::ctl, &Pipeline::zeroed, &Pipeline::pieces, &Pipeline::chain_lists,
+        &Pipeline::cbuf, &Pipeline::rec, &Pipeline::keys, &Pipeline::keys_alt, &Pipeline::wnp, &Pipeline::skeys,
+        &Pipeline::svals, &Pipeline::vals_alt, &Pipeline::sort_scratch, &Pipeline::wind_sums, &Pipeline::draw,
+        &Pipeline::draw_row, &Pipeline::rkeys, &Pipeline::rvals, &Pipeline::rkeys_alt, &Pipeline::rvals_alt,
+        &Pipeline::row_sort_scratch, &Pipeline::row_start, &Pipeline::image, &Pipeline::seg_tiles};
+    static constexpr DevBuf Pipeline::* kPlanBufs[] = {&Pipeline::path_first, &Pipeline::path_draw, &Pipeline::feats,
+                                                       &Pipeline::preds,      &Pipeline::allot,     &Pipeline::plan_tot,
+                                                       &Pipeline::judge_out};
+    // Changes whenever one of a frame's buffers has moved: a captured frame
+    // holds their addresses.
+    uint64_t frame_buffer_moves() const {
+        uint64_t n = 0;
+        for (DevBuf Pipeline::* b : kFrameBufs) n += (this->*b).moves;
+        return n;
+    }
+
     // Grows every device buffer to at least m's capacity for the same
     // buffer (a second batch that will see frames like m's); the pinned
     // plan totals too.  True when a buffer moved.
     sr_status reserve_like(const Pipeline& m, bool* moved) {
-        static DevBuf Pipeline::* const bufs[] = {
-            &Pipeline::pos, &Pipeline::pos_path, &Pipeline::curve_pos, &Pipeline::curve_type,
-            &Pipeline::curve_path, &Pipeline::fill_rule, &Pipeline::fill_info, &Pipeline::path_scene,
-            &Pipeline::scenes_d, &Pipeline::cta_base_d, &Pipeline::tpos, &Pipeline::curve_end, &Pipeline::path_begin, &Pipeline::cut,
-            &Pipeline::count, &Pipeline::offs, &Pipeline::ctl, &Pipeline::zeroed, &Pipeline::pieces,
-            &Pipeline::chain_lists, &Pipeline::cbuf,
-            &Pipeline::rec, &Pipeline::keys, &Pipeline::keys_alt, &Pipeline::wnp, &Pipeline::skeys,
-            &Pipeline::svals, &Pipeline::vals_alt, &Pipeline::sort_scratch, &Pipeline::wind_sums,
-            &Pipeline::draw, &Pipeline::draw_row, &Pipeline::rkeys, &Pipeline::rvals,
-            &Pipeline::rkeys_alt, &Pipeline::rvals_alt, &Pipeline::row_sort_scratch, &Pipeline::row_start,
-            &Pipeline::image,
-            &Pipeline::path_first, &Pipeline::path_draw, &Pipeline::feats, &Pipeline::preds, &Pipeline::allot,
-            &Pipeline::plan_tot, &Pipeline::judge_out, &Pipeline::seg_tiles};
         *moved = false;
         CUDA_TRY(cudaSetDevice(device));
-        for (DevBuf Pipeline::* b : bufs) {
+        auto grow = [&](DevBuf Pipeline::* b) {
             DevBuf& mine = this->*b;
             const size_t want = (m.*b).cap;
-            if (want > mine.cap) {
-                *moved = true;   // before: a failed ensure has freed the old buffer too
-                CUDA_TRY(ensure(mine, want, false));
-            }
-        }
+            if (want <= mine.cap) return cudaSuccess;
+            *moved = true;   // before: a failed ensure has freed the old buffer too
+            return ensure(mine, want, false);
+        };
+        for (DevBuf Pipeline::* b : kFrameBufs) CUDA_TRY(grow(b));
+        for (DevBuf Pipeline::* b : kPlanBufs) CUDA_TRY(grow(b));
         SR_TRY(stage_reserve(m.h_stage_cap));
         if (h_plan_words < m.h_plan_words) {
             if (h_plan_ptr) cudaFreeHost(h_plan_ptr);
@@ -1199,6 +1211,7 @@ struct sr_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int64_t graph_cap = -1, graph_dcap = -1;
+    uint64_t graph_moves = 0;   // frame_buffer_moves() at the capture
     uint32_t graph_launches = 0;
     uint32_t overflows = 0, refits = 0;
     cudaStream_t cap_stream = nullptr;   // captures run here: the legacy stream cannot be captured
@@ -1817,7 +1830,9 @@ static sr_status batch_enqueue(sr_batch* b, const sr_batch_render_opts& d, cudaS
     const int64_t cap = d.record_capacity;
     const int64_t dcap = cap >= 0 ? Pipeline::draw_cap_for(cap, d.draw_capacity) : -1;
     if (cap >= 0 && d.use_graph) {
-        if (!b->exec || b->graph_cap != cap || b->graph_dcap != dcap) {
+        // (a frame since the capture, exact or with more capacity, may have
+        // grown a buffer whose address the graph holds)
+        if (!b->exec || b->graph_cap != cap || b->graph_dcap != dcap || b->graph_moves != p.frame_buffer_moves()) {
             if (b->exec) cudaGraphExecDestroy(b->exec);
             if (b->graph) cudaGraphDestroy(b->graph);
             b->exec = nullptr;
@@ -1847,6 +1862,7 @@ static sr_status batch_enqueue(sr_batch* b, const sr_batch_render_opts& d, cudaS
             CUDA_TRY(cudaGraphInstantiate(&b->exec, b->graph, 0));
             b->graph_cap = cap;
             b->graph_dcap = dcap;
+            b->graph_moves = p.frame_buffer_moves();
             b->graph_launches = (uint32_t)(sr::launches_so_far() - l0);
         }
         CUDA_TRY(cudaGraphLaunch(b->exec, st));
