@@ -369,8 +369,9 @@ struct Pipeline {
     uint32_t last_wide = 0;      // its sort tiles that needed 64-bit items
     bool stages_valid = false;
     // a frame's records carry no flag bits: they are merged again with them
-    // when they are dumped, with the arguments of the frame
-    bool rec_flags = false;
+    // when they are dumped, with the arguments of the frame.  kNone: a frame
+    // that failed before its records has replaced what they came from
+    enum class Records { kNone, kPlain, kFlagged } rec_state = Records::kNone;
     // a frame paints runs; its draw list is written when it is dumped, from
     // the frame's sorted records and its scene's fill arrays, which the next
     // scene's do not overwrite (fill_kept).  A rendered draw list is its own.
@@ -946,7 +947,7 @@ struct Pipeline {
         mark(ST_CHAINS, false);
         launch_chains(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), sm_count, st);
         mark(ST_CHAINS, true);
-        rec_flags = false;   // sr_debug_dump adds them when asked
+        rec_state = Records::kPlain;   // sr_debug_dump adds the flags when asked
         frame_geom = g;
         mark(ST_MERGE, false);
         launch_order_records(g, offs.as<int32_t>(), cw, cbuf.as<int32_t>(), rec.as<int2>(), status, sm_count, st);
@@ -1058,17 +1059,19 @@ struct Pipeline {
     // The last frame's intersection records with their flags, from its chains
     // (which stay as they are until the next frame's).
     sr_status merge_records() {
-        if (rec_flags) return SR_OK;
+        if (rec_state == Records::kNone) return fail(SR_ERR_INVALID_ARG, "the last frame made no records");
+        if (rec_state == Records::kFlagged) return SR_OK;
         sr::launch_merge(frame_geom, offs.as<int32_t>(), chain_work(), cbuf.as<int32_t>(), rec.as<int2>(),
                          ctl.as<uint32_t>() + CTL_STATUS, nullptr);
         CUDA_TRY(cudaGetLastError());
-        rec_flags = true;
+        rec_state = Records::kFlagged;
         return SR_OK;
     }
 
     // The last frame's draw list in draw_list (or a caller's own in draw).
     sr_status write_draw_list(const void** src) {
         *src = draw_state == DrawList::kCallers ? draw.p : draw_list.p;
+        if (draw_state == DrawList::kNone) return fail(SR_ERR_INVALID_ARG, "the last frame made no draw list");
         if (draw_state != DrawList::kFromFrame || last_O <= 0) return SR_OK;
         CUDA_TRY(ensure(draw_list, sizeof(int4) * (size_t)last_O));
         *src = draw_list.p;
@@ -1120,6 +1123,10 @@ struct Pipeline {
         if (!loaded) return fail(SR_ERR_NO_SCENE, "render before a scene was loaded");
         cur = st;
         stages_valid = false;
+        // until enqueue_back: the buffers may move, and the counts and offsets
+        // become the new scene's
+        rec_state = Records::kNone;
+        draw_state = DrawList::kNone;
         const uint64_t launches0 = sr::launches_so_far();
         SR_TRY(prepare_front());
         // exact sizing reads the largest segment back; a pre-sized frame
