@@ -1083,9 +1083,13 @@ struct Pipeline {
         uint32_t* ctlp = ctl.as<uint32_t>();
         CUDA_TRY(cudaMemsetAsync(words, 0, sizeof(uint64_t) * sr::winding_status_words(a.n, frame_wind_items), nullptr));
         CUDA_TRY(cudaMemsetAsync(ctlp + CTL_WIND_COUNTERS, 0, sizeof(uint32_t), nullptr));
+        CUDA_TRY(cudaMemsetAsync(ctlp + CTL_STATUS, 0, sizeof(uint32_t), nullptr));
         sr::launch_draw_list(a, frame_wind_items, words, wind_sums.as<uint64_t>(), ctlp + CTL_WIND_COUNTERS,
                              ctlp + CTL_STATUS, nullptr);
         CUDA_TRY(cudaGetLastError());
+        uint32_t status = 0;
+        CUDA_TRY(cudaMemcpy(&status, ctlp + CTL_STATUS, sizeof status, cudaMemcpyDeviceToHost));
+        SR_TRY(check_status_word(status & sr::ERR_LOOKBACK_TIMEOUT));   // (a list that waits gave up on is not one)
         draw_state = DrawList::kWritten;
         return SR_OK;
     }
