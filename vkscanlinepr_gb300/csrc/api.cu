@@ -1099,11 +1099,12 @@ struct Pipeline {
         if (segmented()) sr::launch_segsort_largest(seg_args(1, nullptr), st);
         CUDA_TRY(cudaMemcpyAsync(h_report, ctl.p, sizeof(uint32_t) * CTL_REPORT, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
-        SR_TRY(check_status_word(h_report[CTL_STATUS]));
+        const uint32_t status = h_report[CTL_STATUS], n = h_report[CTL_N];
+        SR_TRY(check_status_word(status & ~(uint32_t)sr::ERR_CAPACITY));
+        if (n >= sr::kMaxRecords || (status & sr::ERR_CAPACITY))
+            return fail(SR_ERR_OVERFLOW_REFIT, "record count out of range (%u modulo 2^32)", n);
         seg_levels = levels_for(h_report[CTL_LARGEST]);
-        *N = (int64_t)(int32_t)h_report[CTL_N];
-        if (*N < 0 || *N >= (1ll << 30))
-            return fail(SR_ERR_OVERFLOW_REFIT, "record count %lld out of range", (long long)*N);
+        *N = (int64_t)n;
         return SR_OK;
     }
 

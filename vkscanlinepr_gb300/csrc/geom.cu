@@ -481,6 +481,8 @@ SR_DEV void class_starts(const uint32_t* __restrict__ class_count, uint32_t& s0,
 // count pass made (the radix sort that it replaced took five launches).  The
 // scan's last tile also leaves the record count in report_n.
 constexpr int kOffsetRows = 1;   // small tiles: 240 K curves are 234 of them
+// (a curve gives at most kMaxPieces * (1 + 2 * 16,387) records)
+static_assert(1024ull * kOffsetRows * kMaxPieces * (1 + 2 * 16387) < (1ull << 28), "records a tile adds");
 __global__ void __launch_bounds__(256) k_offsets_and_order(
     const int32_t* __restrict__ count, int32_t* __restrict__ offs, uint32_t n_curves, uint32_t scan_tiles,
     uint64_t* tstat, uint32_t* counter, uint32_t* report_n, uint32_t* status, uint32_t spin_limit,
@@ -495,9 +497,15 @@ __global__ void __launch_bounds__(256) k_offsets_and_order(
         if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
         __syncthreads();
         int32_t total;
-        if (scan_tile_i32<kOffsetRows, 256>(count, offs, n_curves, s_tile, tstat, status, spin_limit, s_warp, &total) &&
-            threadIdx.x == 0)
-            *report_n = (uint32_t)total;
+        const bool last =
+            scan_tile_i32<kOffsetRows, 256>(count, offs, n_curves, s_tile, tstat, status, spin_limit, s_warp, &total);
+        if (threadIdx.x == 0) {
+            if (last) *report_n = (uint32_t)total;
+            // More records than a frame takes, whatever the sum has become by
+            // the end: a tile adds less than 2^28, so no sum passes 2^31
+            // without a tile that ends between 2^30 and there.
+            if ((uint32_t)total >= kMaxRecords) set_error(status, ERR_CAPACITY);
+        }
         return;
     }
     const uint32_t n = imin((int32_t)*chain_count, (int32_t)list_cap);
@@ -984,8 +992,8 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
         const bool listed = T.find(ticket, list_cap, key, pos, warp);
         const ChainSetup s = chain_setup(g, offs, pieces, items[pos]);
         // a lane without a chain, or whose chain overflows (k_order_records
-        // reports it), has no roots
-        const int32_t len = listed && s.base + s.len <= g.rec_cap ? s.len : 0;
+        // reports it), has no roots; a base below 0 is an offset past 2^31
+        const int32_t len = listed && s.base >= 0 && s.base + s.len <= g.rec_cap ? s.len : 0;
         int32_t* out = cbuf + s.base;
         const uint32_t gl = T.share(key).lanes, cls = key & 3u;
         const int32_t lanes = 1 << gl, l = (int32_t)(lane_id() & ((1u << gl) - 1u));
@@ -1124,7 +1132,7 @@ SR_DEV void merge_piece(const GeomArgs& g, const int32_t* __restrict__ offs, con
                         uint32_t c, int j) {
     const int64_t start = offs[c], end = offs[c + 1];
     if (start >= end) return;
-    if (end > g.rec_cap) {
+    if (start < 0 || end > g.rec_cap) {
         if (j == 0) set_error(status, ERR_CAPACITY);
         return;
     }

@@ -115,6 +115,8 @@ struct ChainWork {
     uint32_t* chain_queue;    // [1] next ticket of the chains
 };
 constexpr int kChainClassWords = 64;
+// A frame has fewer records (its offsets and counts are 32-bit).
+constexpr uint32_t kMaxRecords = 1u << 30;
 size_t piece_table_bytes(uint32_t n_curves);
 uint32_t chain_list_capacity(uint32_t n_curves);
 
@@ -128,8 +130,8 @@ void launch_transform(const float2* pos, const uint32_t* pos_path, uint32_t n_po
 void launch_count(const GeomArgs& g, float* cut_cache, int32_t* count, const ChainWork& w, uint32_t* status,
                   cudaStream_t st);
 // After the count pass: the curves' record offsets offs[0..C] (exclusive scan
-// of count, look-back words and counter zeroed; the total also to report_n)
-// and the chains in class order.
+// of count, look-back words and counter zeroed; the total also to report_n; a
+// capacity error from kMaxRecords on) and the chains in class order.
 size_t offset_scan_words(uint32_t n_curves);
 void launch_offsets_and_order(const GeomArgs& g, const int32_t* count, int32_t* offs, const ChainWork& w,
                               uint64_t* tile_status, uint32_t* tile_counter, uint32_t* report_n, uint32_t* status,
