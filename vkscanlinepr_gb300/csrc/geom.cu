@@ -646,12 +646,28 @@ struct ChainSide {
     float x, dx, t_hi;    // first grid line, step, end of the piece
     int side;
 };
+//
+// A line's root is NaN where the line starts on the grid line and is so short
+// that 1 / (p1 - p0) overflows (0 * inf; it crosses no second line then), and
+// all its roots are where the matrix sent a point to infinity.  No comparison
+// holds for NaN, so the sequential merge never takes an x root that is one: t0
+// and the y roots go before, and the exhausted y side's 2.0 stands in its
+// place.  A y root that is NaN it takes at once, before any x root above t0.
+// Stored as 2.0 and as -inf the two have these places in the order of numbers
+// (k_order_records and k_merge write NaN for -inf).
+constexpr int32_t kPastEnd = 0x40000001;            // 2.0 with the y side's bit
+constexpr int32_t kNanY = (int32_t)0xFF800000u;     // -inf
+SR_DEV int32_t stored_t(int32_t root) { return root == kNanY ? 0x7FFFFFFD : root; }
 template <int kType> SR_DEV int32_t next_root(const ChainSide& s, int32_t k, int32_t lo) {
     // x + k dx: whole numbers below 2^15, exact like the repeated sum
     const float c = __fadd_rn(s.x, __fmul_rn((float)k, s.dx));
     float t;
-    if (kType == 2) t = gmin(gmax(__fmul_rn(__fsub_rn(c, s.a.p0), s.inv), bitsf(lo)), s.t_hi);
-    else t = bisect<kType>(s.a, c, bitsf(lo), s.t_hi);
+    if (kType == 2) {
+        t = gmin(gmax(__fmul_rn(__fsub_rn(c, s.a.p0), s.inv), bitsf(lo)), s.t_hi);
+        if (t != t) return s.side ? kNanY : kPastEnd;
+    } else {
+        t = bisect<kType>(s.a, c, bitsf(lo), s.t_hi);
+    }
     return (fbits(t) & ~3) | s.side;
 }
 
@@ -846,17 +862,9 @@ SR_DEV void run_segments(const ChainSide& s, int32_t len, float t_lo, int32_t* _
 }
 
 constexpr uint32_t kBackwards = 0x8000u;   // a piece that runs backwards (its x crossings take 15 bits)
-constexpr uint32_t kMaybeNan = 0x80000000u;   // a line some of whose roots may be NaN (its y crossings likewise)
-
-// Whether a line's roots (c - p0) * (1 / extent) on one axis can be NaN: where
-// p0 is not finite (the extent is infinite or NaN then), the extent is NaN, or
-// it is so small that 1 / extent overflows.
-SR_DEV bool roots_maybe_nan(float extent) { return !(fabsf(extent) > 1e-37f && fabsf(extent) < 3e38f); }
 
 struct ChainSetup {
-    // of the record order: first record, crossings (pack_n without signs,
-    // kBackwards, kMaybeNan), start bits, item
-    uint4 piece;
+    uint4 piece;   // of the record order: first record, crossings (pack_n without signs, kBackwards), start bits, item
     ChainSide side;
     uint32_t type;
     int32_t len;
@@ -891,16 +899,11 @@ SR_DEV ChainSetup chain_setup(const GeomArgs& g, const int32_t* __restrict__ off
     const float2* cp = g.tpos + g.curve_pos[c];
     const uint32_t np = curve_slots(s.type);
     float p[4];
-    float2 p0 = make_float2(0.0f, 0.0f), ext = p0;
 #pragma unroll
     for (uint32_t k = 0; k < 4; ++k) {
         float2 v = k < np ? cp[k] : make_float2(0.0f, 0.0f);
         p[k] = side ? v.y : v.x;
-        if (k == 0) p0 = v;
-        if (k == 1) ext = make_float2(__fsub_rn(v.x, p0.x), __fsub_rn(v.y, p0.y));
     }
-    if (s.type == 2u && ((nx > 0 && roots_maybe_nan(ext.x)) || (ny > 0 && roots_maybe_nan(ext.y))))
-        s.piece.y |= kMaybeNan;
     AxisPoly& a = s.side.a;
     a.p0 = p[0]; a.p1 = p[1]; a.p2 = p[2]; a.p3 = p[3];
     a.d01 = __fsub_rn(p[1], p[0]);
@@ -1020,14 +1023,6 @@ __global__ void __launch_bounds__(128) k_chains(const GeomArgs g, const int32_t*
 // below t0, and the sequential merge, which takes the lower head, takes all x
 // roots, then t0, then all y roots: i0 is all of them.
 //
-// A line's roots may be NaN (roots_maybe_nan): all of a chain then, or its
-// only one, as 0 * inf needs c = p0 and such an extent holds no second grid
-// line.  No comparison holds for them, so an x chain of NaN is never taken: t0
-// and the y roots come first, then for each x root the exhausted y side's 2.0.
-// A y chain of NaN is taken whole as soon as t0 has been, before the x roots
-// above t0.  (Looked up in the chains for every line, not noted by k_chains,
-// the NaN took 11 us more of the 4096^2 frame.)
-//
 // A lane finds the place of a root by a binary search; a warp's roots are
 // neighbours, so its loads and stores are too.  The dependent loads bound it,
 // of a chain's piece first: k_chains leaves it in one 16-byte word a chain (the
@@ -1093,15 +1088,6 @@ __global__ void __launch_bounds__(128) k_order_records(const GeomArgs g, const i
         const int32_t len = y_side ? ny : nx, m = y_side ? nx : ny;
         const int32_t *A = y_side ? Y : X, *B = y_side ? X : Y;
         const int32_t k0 = (int32_t)warp * 256, k1 = imin(k0 + 256, len);
-        if (pc.y & kMaybeNan) {
-            const bool x_nan = nx > 0 && bitsf(X[0]) != bitsf(X[0]), y_nan = ny > 0 && bitsf(Y[0]) != bitsf(Y[0]);
-            if (x_nan || y_nan) {   // (i0 is 0 with NaN in the x chain)
-                for (int32_t k = k0 + l; k < k1; k += 32)
-                    R[y_side ? 1 + i0 + k : (k < i0 ? k : 1 + ny + k)] =
-                        make_int2((int32_t)c, x_nan && !y_side ? fbits(2.0f) | 1 : A[k]);
-                continue;
-            }
-        }
         int32_t r = 0;   // roots of the other chain before this one (x roots equal to a y root come before it)
         for (int32_t k = k0 + l; k < k1; k += 32) {
             const int32_t t = A[k];
@@ -1115,7 +1101,7 @@ __global__ void __launch_bounds__(128) k_order_records(const GeomArgs g, const i
                 r = count_lt(B, r, m, bitsf(t));
                 o = k < i0 ? k : 1 + k + r;
             }
-            R[o] = make_int2((int32_t)c, t);
+            R[o] = make_int2((int32_t)c, stored_t(t));
         }
     }
 }
@@ -1171,7 +1157,7 @@ SR_DEV void merge_piece(const GeomArgs& g, const int32_t* __restrict__ offs, con
             out = av;
             ++ia;
         } else {
-            out = bv;
+            out = stored_t(bv);
             ++ib;
         }
         if ((out & ~3) == (last & ~3)) {
