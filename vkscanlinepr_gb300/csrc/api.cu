@@ -68,6 +68,7 @@ struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
     uint32_t moves = 0;   // times the memory was replaced
+    bool clear = false;   // new memory starts zeroed
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
@@ -88,7 +89,9 @@ cudaError_t ensure(DevBuf& b, size_t bytes, bool slack = true) {
         return e;
     }
     b.cap = want;
-    return cudaSuccess;
+    if (!b.clear) return cudaSuccess;
+    e = cudaMemset(b.p, 0, want);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
 }
 
 void release(DevBuf& b) {
@@ -446,6 +449,11 @@ struct Pipeline {
         CUDA_TRY(cudaMallocHost(&h_report, sizeof(uint32_t) * CTL_REPORT));
         CUDA_TRY(cudaHostGetDevicePointer(&d_report, h_report, 0));
         CUDA_TRY(ensure(ctl, sizeof(uint32_t) * CTL_WORDS));
+        // The row order's buffers hold indexes of draw records from their first
+        // day on: where a frame fails (keys left unsorted, a wait that gave up),
+        // it has places that nobody wrote in this frame, and the resolve reads
+        // what is there.
+        rvals.clear = rvals_alt.clear = true;
         return SR_OK;
     }
 

@@ -956,9 +956,11 @@ SR_DEV void merge_item(MergeSmem& S, uint32_t item, uint32_t chunk, uint64_t* __
         if (lane_id() == 0) S.split[warp] = sp;
     }
     __syncthreads();
-    const uint32_t ia0 = S.split[0], ia1 = S.split[1];
-    const uint32_t ib0 = d0 - ia0, ib1 = d1 - ia1;
-    const uint32_t nA = ia1 - ia0, nB = ib1 - ib0, n = d1 - d0;
+    // (Of sorted runs the second split is not below the first, nor further on
+    // than n.  A frame that is redone may merge a chunk that nobody sorted: its
+    // parts stay within the runs and the buffers too.)
+    const uint32_t n = d1 - d0, ia0 = S.split[0], ia1 = min(max(S.split[1], ia0), ia0 + n);
+    const uint32_t ib0 = d0 - ia0, nA = ia1 - ia0, nB = n - nA;
     for (uint32_t j = tid; j < nA; j += kThreads) S.in[j] = A[ia0 + j];
     for (uint32_t j = tid; j < nB; j += kThreads) S.in[nA + j] = B[ib0 + j];
     __syncthreads();

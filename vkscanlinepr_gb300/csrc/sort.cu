@@ -144,9 +144,13 @@ __global__ void __launch_bounds__(kThreads) k_row_starts(const uint32_t* __restr
     for (uint32_t i = threadIdx.x; i < passes * kRadix; i += kThreads) (&sh[0][0])[i] = 0;
     __syncthreads();
     const uint32_t tile = s_tile;
+    // A frame that has failed by now (its caller is told so) has rows without
+    // records: where a wait gave up, the counts may add up to more than the
+    // order has room for.
+    const uint32_t counted = *status ? 0u : rows;
     for (uint32_t q = 0; q < 4; ++q) {
         const uint32_t b = tile * kRowTile + q * kThreads + threadIdx.x;
-        const uint32_t c = b < rows ? counts[b] : 0u;
+        const uint32_t c = b < counted ? counts[b] : 0u;
         if (!c) continue;
         for (uint32_t p = 0; p < passes; ++p)
             atomicAdd(&sh[p][digit_of(b, p * kRadixBits, digit_mask(key_bits, p * kRadixBits))], c);
@@ -157,8 +161,9 @@ __global__ void __launch_bounds__(kThreads) k_row_starts(const uint32_t* __restr
         if (v) atomicAdd(&hist[i], v);
     }
     int32_t total;
-    scan_tile_i32<1, kThreads>(reinterpret_cast<const int32_t*>(counts), row_start, rows, tile, tstat, status,
-                               spin_limit, s_warp, &total);
+    int4 v[1];
+    load_tile_values<1, kThreads>(v, reinterpret_cast<const int32_t*>(counts), counted, tile);
+    scan_tile_values<1, kThreads>(v, row_start, rows, tile, tstat, status, spin_limit, s_warp, &total);
 }
 
 // ------------------------------------------------ row sort in one pass ---
