@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_tiles(const SegArgs s, Tile
 //     Off-canvas records share one key a path, so counting would be quadratic:
 //     their place is by index, from ballots.
 //   * A tile with a bin of more than 384 records, or with too many paths for
-//     the bins, is sorted by digit passes: compact 32-bit items ((path - pmin,
+//     the bins, and every tile of a frame that has failed by now, is sorted by
+//     digit passes: compact 32-bit items ((path - pmin,
 //     row-rank code, x - xmin) in the fewest bits, the payload above), 8-bit
 //     digits ranked per warp (match_any and a histogram a warp), scanned and
 //     scattered.  (At 128 records 465 instead of 457 us for the stage, at 1024
@@ -504,6 +505,7 @@ struct TileSmem {
     TileRanges ranges;
     uint64_t bar;
     uint32_t next;
+    bool grouped;   // the records are grouped by path
 };
 constexpr uint16_t kOffSlot = 1u << 14;
 
@@ -531,7 +533,8 @@ struct BinPlan {
     }
 };
 
-// The tile's records in order, by bins: false when a bin is too full.
+// The tile's records in order, by bins: false when a bin is too full.  The
+// records are grouped by path (an off-canvas record's place counts on it).
 SR_DEV bool sort_by_bins(TileSmem& S, const TileRanges& R, const BinPlan& B, uint32_t bx, uint32_t base, uint32_t len,
                          const KeyFields& kf, uint64_t* __restrict__ out) {
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
@@ -766,7 +769,7 @@ SR_DEV bool sort_tile(TileSmem& S, uint32_t tile, uint32_t& phase, const uint64_
         return true;
     }
     const BinPlan B(R, bx);
-    if (B.ok && sort_by_bins(S, R, B, bx, base, len, kf, out)) return true;
+    if (S.grouped && B.ok && sort_by_bins(S, R, B, bx, base, len, kf, out)) return true;
     sort_by_digits(S, R, base, len, kf, out);
     return true;
 }
@@ -781,7 +784,13 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_tile_sort(const uint64_t* _
     TileSmem& S = *reinterpret_cast<TileSmem*>(smem_raw);
     // tiles past the table exist only in a frame whose records overflowed (redone)
     const uint32_t n_tiles = min(u.ctl[kCtlTiles], mt);
-    if (threadIdx.x == 0) mbar_init(&S.bar, 1);
+    if (threadIdx.x == 0) {
+        mbar_init(&S.bar, 1);
+        // In a frame whose records overflowed, or whose offsets are wrong, there
+        // are records of the frame before between a path's own.  (Read by one
+        // thread: other CTAs may set it now.)
+        S.grouped = *status == 0u;
+    }
     uint32_t phase = 0;
     // the first tiles by the CTAs' numbers: an SM's second CTA takes one only
     // when every SM has one
