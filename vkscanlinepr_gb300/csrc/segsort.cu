@@ -204,8 +204,9 @@ SR_DEV int stage_tile(uint64_t* buf, uint64_t* bar, uint32_t& phase, const uint6
     __syncthreads();
     const bool ok = nb == 0 || mbar_wait_bounded(bar, phase, spin_limit, status);
     if (__syncthreads_or(!ok)) {
-        // gave up: let the copy land before the CTA leaves
-        if (nb) mbar_wait_bounded(bar, phase, spin_limit, nullptr);
+        // gave up: let the copy land before the CTA leaves, whatever limit it
+        // was that the wait ran into
+        if (nb) mbar_wait_bounded(bar, phase, max(spin_limit, kSpinLimitDefault), nullptr);
         return -1;
     }
     if (nb) phase ^= 1u;

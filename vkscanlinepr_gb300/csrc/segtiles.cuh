@@ -99,7 +99,8 @@ SR_DEV void seg_tiles(const SegArgs& s, const TileTables& u, uint32_t* status, u
         const uint32_t at = cls && m > 0 ? atomicAdd(&u.ctl[kCtlChunks + cls], (uint32_t)m) : 0u;
         for (int32_t k = 0; k < m; ++k) {
             u.desc[first + k] = make_uint4(a, e - a, (uint32_t)k | (rounds << 16) | kChunkBit, 0u);
-            if (cls) u.chunks[(size_t)(cls - 1) * u.mt + at + k] = (uint32_t)(first + k);
+            // (more than mt of a class only where a wait gave up and `first` is wrong)
+            if (cls && at + (uint32_t)k < mt) u.chunks[(size_t)(cls - 1) * mt + at + k] = (uint32_t)(first + k);
         }
         return;
     }
