@@ -2194,7 +2194,7 @@ sr_status sr_sizer_train(sr_sizer* s, const float* d_x, const float* d_t, uint32
             const float bc1 = (float)(1.0 - std::pow(b1, (double)s->step));
             const float bc2 = (float)(1.0 - std::pow(b2, (double)s->step));
             CUDA_TRY(sr::launch_mlp_step(s->wb.p, s->master.as<float>(), s->norm.as<float>(), d_x, d_t,
-                                         idx ? idx + b0 : nullptr, nb, s->grad.as<float>(), s->loss.as<double>(),
+                                         idx ? idx + b0 : nullptr, n, nb, s->grad.as<float>(), s->loss.as<double>(),
                                          s->m.as<float>(), s->v.as<float>(), d.lr, d.beta1, d.beta2, d.eps, bc1, bc2,
                                          s->ctl.as<uint32_t>() + 1, st));
             if (!idx) {   // unshuffled minibatches are consecutive rows

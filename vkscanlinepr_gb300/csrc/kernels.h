@@ -370,12 +370,13 @@ void launch_mlp_predict(const void* wb, const float* master, const float* norm, 
 // sum of squared errors into loss_sum.
 cudaError_t launch_mlp_grad(const void* wb, const float* master, const float* norm, const float* x, const float* t,
                             const uint32_t* idx, uint32_t n, float* grad, double* loss_sum, cudaStream_t st);
-// A training step: the gradient, then Adam (by the last CTA of the same
+// A training step on n of the `rows` rows: the gradient, then Adam (by the last CTA of the same
 // launch, which finds itself through `done`, a word zeroed before the first
 // step); grad is zero before and after.
 cudaError_t launch_mlp_step(void* wb, float* master, const float* norm, const float* x, const float* t,
-                            const uint32_t* idx, uint32_t n, float* grad, double* loss_sum, float* m, float* v, float lr,
-                            float b1, float b2, float eps, float bc1, float bc2, uint32_t* done, cudaStream_t st);
+                            const uint32_t* idx, uint32_t rows, uint32_t n, float* grad, double* loss_sum, float* m,
+                            float* v, float lr, float b1, float b2, float eps, float bc1, float bc2, uint32_t* done,
+                            cudaStream_t st);
 void launch_to_bf16(const float* master, void* wb, cudaStream_t st);
 void launch_perm_keys(uint32_t* keys, uint32_t n, uint64_t seed, cudaStream_t st);
 // allot[P][2] from predictions with the path margins (margins[0..1]);

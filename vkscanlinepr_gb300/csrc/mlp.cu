@@ -349,11 +349,18 @@ struct GradSmem {
     bool last;
 };
 
+// Row of sample i.  (A shuffle whose sort gave up, which the caller is told at
+// the end, leaves places of the order unwritten: what they hold may be no row.)
+SR_DEV uint32_t sample_row(const uint32_t* __restrict__ idx, uint32_t rows, uint32_t i) {
+    return idx ? min(idx[i], rows - 1u) : i;
+}
+
 __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const __nv_bfloat16* __restrict__ wb,
                                                            const float* __restrict__ master,
                                                            const float* __restrict__ norm, const float* __restrict__ x,
                                                            const float* __restrict__ t,
-                                                           const uint32_t* __restrict__ idx, uint32_t n, float scale,
+                                                           const uint32_t* __restrict__ idx, uint32_t rows, uint32_t n,
+                                                           float scale,
                                                            float* grad, double* loss_sum, int adam, AdamArgs A,
                                                            uint32_t* done) {
     wait_for_previous();
@@ -367,13 +374,13 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const __nv_bfloat16* 
         const int q = tid / kIn, k = tid % kIn;
         const uint32_t sidx = s0 + q;
         float v = 0.0f;
-        if (sidx < n) v = (x[(size_t)(idx ? idx[sidx] : sidx) * kIn + k] - norm[nXm + k]) * norm[nXs + k];
+        if (sidx < n) v = (x[(size_t)sample_row(idx, rows, sidx) * kIn + k] - norm[nXm + k]) * norm[nXs + k];
         S.xin[q][k] = v;
     } else if (tid >= kGradThreads - kSamples * kOut) {
         const int i = tid - (kGradThreads - kSamples * kOut), q = i / kOut, k = i % kOut;
         const uint32_t sidx = s0 + q;
         float v = 0.0f;
-        if (sidx < n) v = (t[(size_t)(idx ? idx[sidx] : sidx) * kOut + k] - norm[nYm + k]) / norm[nYs + k];
+        if (sidx < n) v = (t[(size_t)sample_row(idx, rows, sidx) * kOut + k] - norm[nYm + k]) / norm[nYs + k];
         S.ty[q][k] = v;
     }
     __syncthreads();
@@ -645,8 +652,8 @@ void launch_mlp_predict(const void* wb, const float* master, const float* norm, 
 }
 
 static cudaError_t grad_launch(const void* wb, const float* master, const float* norm, const float* x, const float* t,
-                               const uint32_t* idx, uint32_t n, float* grad, double* loss_sum, bool adam,
-                               const AdamArgs& A, uint32_t* done, cudaStream_t st) {
+                               const uint32_t* idx, uint32_t rows, uint32_t n, float* grad, double* loss_sum,
+                               bool adam, const AdamArgs& A, uint32_t* done, cudaStream_t st) {
     static std::atomic<uint32_t> attr{0};
     cudaError_t e = cudaSuccess;
     once_per_device(attr, [&] {
@@ -655,23 +662,24 @@ static cudaError_t grad_launch(const void* wb, const float* master, const float*
     if (e != cudaSuccess) return e;
     count_launches(1);
     launch_after(k_mlp_grad, (n + kSamples - 1) / kSamples, kGradThreads, sizeof(GradSmem), st,
-                 static_cast<const __nv_bfloat16*>(wb), master, norm, x, t, idx, n, 1.0f / ((float)n * (float)kOut),
-                 grad, loss_sum, adam ? 1 : 0, A, done);
+                 static_cast<const __nv_bfloat16*>(wb), master, norm, x, t, idx, rows, n,
+                 1.0f / ((float)n * (float)kOut), grad, loss_sum, adam ? 1 : 0, A, done);
     return cudaGetLastError();
 }
 
 cudaError_t launch_mlp_grad(const void* wb, const float* master, const float* norm, const float* x, const float* t,
                             const uint32_t* idx, uint32_t n, float* grad, double* loss_sum, cudaStream_t st) {
     if (!n) return cudaSuccess;
-    return grad_launch(wb, master, norm, x, t, idx, n, grad, loss_sum, false, AdamArgs{}, nullptr, st);
+    return grad_launch(wb, master, norm, x, t, idx, n, n, grad, loss_sum, false, AdamArgs{}, nullptr, st);
 }
 
 cudaError_t launch_mlp_step(void* wb, float* master, const float* norm, const float* x, const float* t,
-                            const uint32_t* idx, uint32_t n, float* grad, double* loss_sum, float* m, float* v, float lr,
-                            float b1, float b2, float eps, float bc1, float bc2, uint32_t* done, cudaStream_t st) {
+                            const uint32_t* idx, uint32_t rows, uint32_t n, float* grad, double* loss_sum, float* m,
+                            float* v, float lr, float b1, float b2, float eps, float bc1, float bc2, uint32_t* done,
+                            cudaStream_t st) {
     if (!n) return cudaSuccess;
     const AdamArgs A{master, m, v, static_cast<__nv_bfloat16*>(wb), lr, b1, b2, eps, bc1, bc2};
-    return grad_launch(wb, master, norm, x, t, idx, n, grad, loss_sum, true, A, done, st);
+    return grad_launch(wb, master, norm, x, t, idx, rows, n, grad, loss_sum, true, A, done, st);
 }
 
 void launch_to_bf16(const float* master, void* wb, cudaStream_t st) {
