@@ -1632,12 +1632,18 @@ static cudaError_t scan_scratch(void** p, size_t bytes, cudaStream_t st) {
             props.location.id = dev;
             cudaMemPool_t made = nullptr;
             uint64_t keep = 32u << 20;
+            // (a process may scan for the first time under a stream capture,
+            // in which making a pool is refused unless the thread is relaxed
+            // about it)
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
             if (cudaMemPoolCreate(&made, &props) == cudaSuccess) {
                 if (cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
                     g_scan_pools[dev] = made;
                 else
                     cudaMemPoolDestroy(made);
             }
+            cudaThreadExchangeStreamCaptureMode(&mode);
             if (!g_scan_pools[dev]) cudaGetLastError();   // not an error of this call
         }
         pool = g_scan_pools[dev];
