@@ -710,7 +710,7 @@ struct Pipeline {
         l.row_px = place(sizeof(unsigned long long) * (size_t)total_rows);
         l.row_count = place(sizeof(uint32_t) * (size_t)total_rows);
         l.row_scan = place(sizeof(uint64_t) * sr::row_scan_words(total_rows));
-        l.row_sort = place(sr::row_sort_one_pass(total_rows)
+        l.row_sort = place(sr::row_sort_one_pass(draw_cap_for(cap, dcap), total_rows)
                                ? sr::row_sort_bytes(draw_cap_for(cap, dcap), total_rows)
                                : sr::sort_scratch_bytes(row_plan(draw_cap_for(cap, dcap), nullptr)));
         l.total = at;
@@ -1022,7 +1022,7 @@ struct Pipeline {
         // the emit counted the records of every row: their exclusive scan is
         // each row's start in the row order, and their digits the sort's
         // histogram
-        const bool one_pass = row_sort_one_pass(total_rows);
+        const bool one_pass = row_sort_one_pass(dcap, total_rows);
         if (one_pass) rp.passes = 0;
         launch_row_starts(rp, wa.row_count, total_rows, row_start.as<int32_t>(), zero + at.row_sort,
                           reinterpret_cast<uint64_t*>(zero + at.row_scan), ctlp + CTL_ROW_SCAN, status, st);

@@ -191,16 +191,17 @@ size_t sort_scratch_bytes(const SortPlan& p);
 void launch_sort_u64(const SortPlan& p, const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out,
                      uint32_t* vals_out, uint64_t* keys_alt, uint32_t* vals_alt, void* scratch,
                      uint32_t* status, cudaStream_t st);
+// The order of n draw records by row in one launch, where the rows and the
+// records are few enough (after launch_row_starts; scratch: row_sort_bytes,
+// zeroed).
+bool row_sort_one_pass(int64_t n, uint32_t rows);
+size_t row_sort_bytes(int64_t n, uint32_t rows);
+void launch_row_sort(const uint32_t* rows_in, int64_t n, const uint32_t* n_dev, uint32_t rows, const int32_t* row_start,
+                     uint32_t* idx_out, void* scratch, uint32_t* status, cudaStream_t st);
 // For a sort by row whose records per row are known: each row's first
 // position row_start[0..rows] (exclusive scan; look-back words and counter
 // zeroed) and every pass's digit counts into the plan's zeroed scratch, so
 // that the sort needs no pass over the keys for them.
-// The order of n draw records by row in one launch, where the rows are few
-// enough (after launch_row_starts; scratch: row_sort_bytes, zeroed).
-bool row_sort_one_pass(uint32_t rows);
-size_t row_sort_bytes(int64_t n, uint32_t rows);
-void launch_row_sort(const uint32_t* rows_in, int64_t n, const uint32_t* n_dev, uint32_t rows, const int32_t* row_start,
-                     uint32_t* idx_out, void* scratch, uint32_t* status, cudaStream_t st);
 size_t row_scan_words(uint32_t rows);
 void launch_row_starts(SortPlan& p, const uint32_t* row_count, uint32_t rows, int32_t* row_start, void* scratch,
                        uint64_t* tile_status, uint32_t* tile_counter, uint32_t* status, cudaStream_t st);

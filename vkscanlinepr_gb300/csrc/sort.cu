@@ -176,9 +176,13 @@ __global__ void __launch_bounds__(kThreads) k_row_starts(const uint32_t* __restr
 // mostly of different rows.  A small frame's row sort is the latency of its
 // launches and of the look-back: two launches instead of three took 18 instead
 // of 21 us for 1,024 rows and 100,000 runs, 14 instead of 21 for 375 rows (a
-// 1000x750 frame of two pixel rows a row).  With 2,048 rows the look-back words
-// and their clearing cost more than a pass: 57 instead of 40 us.
-constexpr uint32_t kRowSortMaxRows = 1024;
+// 1000x750 frame of two pixel rows a row).  The look-back words and their
+// clearing grow with the rows and the draw records: with 1,024 rows the row
+// order of 2.5 M draw records took 30.6 instead of 31.7 us, of 3.3 M 34.7
+// instead of 33.7, of 12.4 M 73.6 instead of 62.4; with 400 rows 42.9 instead of
+// 54.2 for 10.5 M; with 2,048 rows 57 instead of 40 for a small frame.
+constexpr uint32_t kRowSortMaxRows = 1024, kRowSortAnyRows = 512;   // any: whatever the draw records
+constexpr int64_t kRowSortMaxDraws = 3500000;
 constexpr int kRowItems = 8;
 constexpr int kRowWindow = 4;   // look-back words of a row read per step
 constexpr int kRowSortTile = kThreads * kRowItems;
@@ -547,9 +551,11 @@ void launch_sort_u64(const SortPlan& p, const uint64_t* keys_in, const uint32_t*
     sort_dispatch<uint64_t>(p, keys_in, vals_in, keys_out, vals_out, keys_alt, vals_alt, scratch, status, st);
 }
 
-bool row_sort_one_pass(uint32_t rows) { return rows > (uint32_t)kRadix && rows <= kRowSortMaxRows; }
+bool row_sort_one_pass(int64_t n, uint32_t rows) {
+    return rows > (uint32_t)kRadix && rows <= (n <= kRowSortMaxDraws ? kRowSortMaxRows : kRowSortAnyRows);
+}
 
-static int row_sort_bits(uint32_t rows) { return rows <= 512 ? 9 : rows <= 1024 ? 10 : 11; }
+static int row_sort_bits(uint32_t rows) { return rows <= 512 ? 9 : 10; }
 
 size_t row_sort_bytes(int64_t n, uint32_t rows) {
     const size_t tiles = (size_t)((n + kRowSortTile - 1) / kRowSortTile);
@@ -567,11 +573,8 @@ void launch_row_sort(const uint32_t* rows_in, int64_t n, const uint32_t* n_dev, 
     if (bits == 9)
         launch_after(k_row_sort<9>, tiles, kThreads, 0, st, rows_in, n, n_dev, rows, row_start, idx_out, lookback,
                      counter, status, spin_limit());
-    else if (bits == 10)
-        launch_after(k_row_sort<10>, tiles, kThreads, 0, st, rows_in, n, n_dev, rows, row_start, idx_out, lookback,
-                     counter, status, spin_limit());
     else
-        launch_after(k_row_sort<11>, tiles, kThreads, 0, st, rows_in, n, n_dev, rows, row_start, idx_out, lookback,
+        launch_after(k_row_sort<10>, tiles, kThreads, 0, st, rows_in, n, n_dev, rows, row_start, idx_out, lookback,
                      counter, status, spin_limit());
 }
 
