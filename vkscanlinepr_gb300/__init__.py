@@ -462,8 +462,10 @@ def write_image(path, rgba, fmt=None):
 
 
 def scan_status(stream=None):
-    """Waits for `stream`; raises SrError(SR_ERR_TIMEOUT) if a look-back of a
-    standalone scan gave up since the last call (its output is wrong)."""
+    """Waits for `stream`, gives back the memory that exclusive_scan_i32 keeps,
+    and raises SRError (TIMEOUT) if a wait of a standalone scan gave up since
+    the last call.  Only the check of the bounded wait
+    (sr_debug_scan_without_first_tile) has one."""
     _check(lib().sr_scan_status(stream))
 
 
@@ -565,8 +567,9 @@ class ScanlineVGRasterizer:
         return out
 
     def render_device(self, dev_ptr=None, stream=None):
-        """Renders into device memory (dev_ptr or the context's framebuffer)
-        without waiting for the frame."""
+        """Renders into device memory (dev_ptr or the context's framebuffer);
+        returns once the frame is done, as render() does, without the copy to
+        the host."""
         _check(lib().sr_render(self._ctx, dev_ptr, 1, stream))
 
     def stats(self):
