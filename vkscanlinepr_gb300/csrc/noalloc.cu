@@ -5,8 +5,8 @@
 // Some callers cannot allow that: a host that hands all device memory to
 // its own allocator or runs under a hard memory budget forbids third-party
 // allocations, and a frame loop with a fixed latency budget cannot risk an
-// allocation call that may wait on the device.  This variant runs the same
-// kernel with its scratch in a fixed array compiled into the library: every
+// allocation call that may wait on the device.  This variant launches the same
+// kernels with their scratch in a fixed array compiled into the library: every
 // GPU that loads the library holds SR_NOALLOC_SCAN_SCRATCH_BYTES of it until
 // the process exits.
 #include <cstdarg>
@@ -30,13 +30,12 @@ static __device__ __align__(256) uint64_t g_noalloc_scan_scratch[kNoallocWords];
 constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
 uint64_t* g_scratch_addr[kMaxDevices] = {};
-uint32_t* g_status_addr[kMaxDevices] = {};
 
-// Device addresses, on the current device, of the scratch array and of the
-// standalone scans' status word, looked up once per device (the array's
-// name in host code is only a stand-in).  A cudaDeviceReset unloads the
-// library's device code, so these addresses do not survive one.
-sr_status scratch_on_current_device(uint64_t** scratch, uint32_t** status) {
+// Device address, on the current device, of the scratch array, looked up once
+// per device (the array's name in host code is only a stand-in).  A
+// cudaDeviceReset unloads the library's device code, so it does not survive
+// one.
+sr_status scratch_on_current_device(uint64_t** scratch) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return sr::report_error(SR_ERR_CUDA, cudaGetErrorString(e));
@@ -46,14 +45,9 @@ sr_status scratch_on_current_device(uint64_t** scratch, uint32_t** status) {
         void* p = nullptr;
         e = cudaGetSymbolAddress(&p, g_noalloc_scan_scratch);
         if (e != cudaSuccess || !p) return sr::report_error(SR_ERR_CUDA, cudaGetErrorString(e));
-        uint32_t* w = nullptr;
-        e = sr::standalone_scan_status(&w);
-        if (e != cudaSuccess || !w) return sr::report_error(SR_ERR_CUDA, cudaGetErrorString(e));
         g_scratch_addr[dev] = static_cast<uint64_t*>(p);
-        g_status_addr[dev] = w;
     }
     *scratch = g_scratch_addr[dev];
-    *status = g_status_addr[dev];
     return SR_OK;
 }
 
@@ -69,8 +63,7 @@ extern "C" sr_status sr_exclusive_scan_i32_noalloc(const int32_t* d_in, int32_t*
     if (!d_out || (n > 0 && !d_in)) return sr::report_error(SR_ERR_INVALID_ARG, "NULL device pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint64_t* scratch = nullptr;
-    uint32_t* status = nullptr;
-    sr_status s = scratch_on_current_device(&scratch, &status);
+    sr_status s = scratch_on_current_device(&scratch);
     if (s != SR_OK) return s;
     // the sums of the previous call stay in the array; a scan writes what it
     // reads of it

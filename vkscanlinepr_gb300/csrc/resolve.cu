@@ -54,7 +54,7 @@ struct PixRec {
     float sg;           // s*a of green
     uint32_t iau;       // 255 - a
     uint32_t sab;       // (s*a + 128) of red | of blue << 16
-    int32_t row;        // cell row within the CTA
+    uint32_t pad;       // 32 bytes: two 16-byte accesses
     uint32_t idx1;      // 1 + draw index
 };
 
@@ -184,14 +184,14 @@ template <bool GRAD> SR_DEV PixRec pix_rec(const int4 d, uint32_t di) {
         pr.sab = (uint32_t)paint;
         pr.ia = 0.0f;
         pr.sg = 0.0f;
-        pr.row = 0;
+        pr.pad = 0;
         return pr;
     }
     pr.ia = (float)(255u - al);
     pr.sg = (float)(((col >> 8) & 0xFFu) * al);
     pr.iau = 255u - al;
     pr.sab = ((col & 0xFFu) * al + 128u) | ((((col >> 16) & 0xFFu) * al + 128u) << 16);
-    pr.row = 0;
+    pr.pad = 0;
     return pr;
 }
 

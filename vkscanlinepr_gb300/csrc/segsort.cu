@@ -26,9 +26,6 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kRadixBits = 9;   // digits of the 64-bit tile sort
 constexpr int kRadix = 1 << kRadixBits;
-// Lanes with the same digit: __match_any_sync (tiles hold runs of nearly
-// sorted keys, so a warp sees few distinct digits), or one ballot per bit.
-constexpr bool kMatchAny = true;
 
 size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 size_t scan_area(uint32_t P) { return round256(8 * ((size_t)P / kSegThreads + 2)); }
@@ -132,17 +129,6 @@ struct KeyFields {
 
 SR_DEV uint32_t bits_of(uint32_t v) { return v ? 32u - (uint32_t)__clz((int)v) : 0u; }
 SR_DEV uint32_t low_mask(uint32_t b) { return b >= 32 ? 0xFFFFFFFFu : (1u << b) - 1u; }
-
-SR_DEV uint32_t same_digit_lanes(uint32_t d) {
-    if (kMatchAny) return __match_any_sync(0xFFFFFFFFu, d);
-    uint32_t peers = 0xFFFFFFFFu;
-#pragma unroll
-    for (int b = 0; b <= kRadixBits; ++b) {   // 9 bits: digit kRadix marks an empty slot
-        const uint32_t m = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
-        peers &= ((d >> b) & 1u) ? m : ~m;
-    }
-    return peers;
-}
 
 // Shared memory of the pass machinery and the range reduction.
 struct PassSmem {
@@ -399,7 +385,8 @@ SR_DEV uint32_t radix_passes(H* hist, uint32_t* digit_start, uint32_t* scan_tmp,
             const uint32_t j = wfirst + (uint32_t)it * 32u + lane;
             const bool ok = j < len;
             const uint32_t dg = ok ? digit(in[j], shift) : (uint32_t)kRadix;
-            const uint32_t peers = same_digit_lanes(dg);
+            // (tiles hold runs of nearly sorted keys: a warp sees few digits)
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, dg);
             const uint32_t leader = (uint32_t)(__ffs(peers) - 1);
             uint32_t before = 0;
             if (ok && lane == leader) {
@@ -480,9 +467,8 @@ constexpr uint32_t kBins = 4096;
 constexpr uint32_t kHeavyBin = 384;
 constexpr uint32_t kIndexBits = 12;   // a record's index in its tile
 constexpr int kSortBits = 8;          // digits of the radix passes
-constexpr int kBinRounds = (int)kBins / (8 * kSortThreads);   // of eight bins a thread
-static_assert(kTile == 1 << kIndexBits && kBins == 8u * kBinRounds * kSortThreads && kBins <= 1u << 14,
-              "tile geometry");
+static_assert(kTile == 1 << kIndexBits && kBins == 8u * kSortThreads && kBins <= 1u << 14,
+              "tile geometry: eight bins a thread");
 
 struct TileSmem {
     union {
@@ -599,20 +585,11 @@ SR_DEV bool sort_by_bins(TileSmem& S, const TileRanges& R, const BinPlan& B, uin
     }
     if (lane == 0) S.warp_off[warp] = n_off;
     if (__syncthreads_or(heavy)) return false;
-    // ---- the bins' starts over their counts: a warp's bins are `rounds` times
-    // 256, eight a lane
-    const uint32_t rounds = ((R.pmax - R.pmin + 1u) * B.stride + 8u * kSortThreads) / (8u * kSortThreads);
-    const uint32_t word0 = warp * rounds * 32u + lane;
-    uint32_t sums[kBinRounds], wsum = 0;
-#pragma unroll
-    for (int q = 0; q < kBinRounds; ++q) {
-        sums[q] = 0;
-        if ((uint32_t)q >= rounds) break;
-        const uint4 w = S.bins4[word0 + (uint32_t)q * 32u];
-        const uint32_t two = w.x + w.y + w.z + w.w;   // no half carries: a tile's records
-        sums[q] = (two & 0xFFFFu) + (two >> 16);
-        wsum += __reduce_add_sync(0xFFFFFFFFu, sums[q]);
-    }
+    // ---- the bins' starts over their counts, eight bins a thread
+    const uint4 w = S.bins4[tid];
+    const uint32_t two = w.x + w.y + w.z + w.w;   // no half carries: a tile's records
+    const uint32_t sum = (two & 0xFFFFu) + (two >> 16);
+    const uint32_t wsum = __reduce_add_sync(0xFFFFFFFFu, sum);
     if (lane == 0) S.scan_tmp[warp] = wsum;
     if (R.has_off()) {
         // lane v: off-canvas records of the warps before v
@@ -639,27 +616,23 @@ SR_DEV bool sort_by_bins(TileSmem& S, const TileRanges& R, const BinPlan& B, uin
         }
     }
     __syncthreads();
-    uint32_t wstart = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? S.scan_tmp[lane] : 0u);
-#pragma unroll
-    for (int q = 0; q < kBinRounds; ++q) {
-        if ((uint32_t)q >= rounds) break;
-        uint32_t incl = sums[q];
+    {
+        const uint32_t wstart = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? S.scan_tmp[lane] : 0u);
+        uint32_t incl = sum;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
             if ((int)lane >= o) incl += y;
         }
-        const uint4 w = S.bins4[word0 + (uint32_t)q * 32u];
         const uint32_t c4[4] = {w.x, w.y, w.z, w.w};
-        uint32_t s4[4], at0 = wstart + incl - sums[q];
+        uint32_t s4[4], at0 = wstart + incl - sum;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const uint32_t second = at0 + (c4[i] & 0xFFFFu);
             s4[i] = at0 | (second << 16);
             at0 = second + (c4[i] >> 16);
         }
-        S.bins4[word0 + (uint32_t)q * 32u] = make_uint4(s4[0], s4[1], s4[2], s4[3]);
-        wstart += __shfl_sync(0xFFFFFFFFu, incl, 31);
+        S.bins4[tid] = make_uint4(s4[0], s4[1], s4[2], s4[3]);
     }
     __syncthreads();
     // ---- records to their bins
@@ -744,8 +717,7 @@ SR_DEV bool sort_tile(TileSmem& S, uint32_t tile, uint32_t& phase, const uint64_
     if (!tile_span(u, tile, n_cap, a, len, to_alt)) return true;
     uint64_t* out = (to_alt ? keys_alt : keys_out) + a;
     // (the copy's wait publishes these)
-#pragma unroll
-    for (int i = 0; i < kBinRounds; ++i) S.bins4[tid + (uint32_t)i * kSortThreads] = make_uint4(0u, 0u, 0u, 0u);
+    S.bins4[tid] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int i = 0; i < kTile / 4 / kSortThreads; ++i)
         S.slot4[tid + (uint32_t)i * kSortThreads] = make_uint4(~0u, ~0u, ~0u, ~0u);
