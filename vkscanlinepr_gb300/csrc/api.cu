@@ -68,7 +68,7 @@ struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
     uint32_t moves = 0;   // times the memory was replaced
-    bool clear = false;   // new memory starts zeroed
+    bool fresh = false;   // nothing has been written to it yet
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
@@ -89,9 +89,8 @@ cudaError_t ensure(DevBuf& b, size_t bytes, bool slack = true) {
         return e;
     }
     b.cap = want;
-    if (!b.clear) return cudaSuccess;
-    e = cudaMemset(b.p, 0, want);
-    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+    b.fresh = true;
+    return cudaSuccess;
 }
 
 void release(DevBuf& b) {
@@ -459,11 +458,6 @@ struct Pipeline {
         CUDA_TRY(cudaMallocHost(&h_report, sizeof(uint32_t) * CTL_REPORT));
         CUDA_TRY(cudaHostGetDevicePointer(&d_report, h_report, 0));
         CUDA_TRY(ensure(ctl, sizeof(uint32_t) * CTL_WORDS));
-        // The row order's buffers hold indexes of draw records from their first
-        // day on: where a frame fails (keys left unsorted, a wait that gave up),
-        // it has places that nobody wrote in this frame, and the resolve reads
-        // what is there.
-        rvals.clear = rvals_alt.clear = true;
         return SR_OK;
     }
 
@@ -891,6 +885,18 @@ struct Pipeline {
         return t;
     }
 
+    // The row order's buffers hold indexes of draw records from their first
+    // use on: where a frame fails (keys left unsorted, a wait that gave up), it
+    // has places that nobody wrote in this frame, and the resolve reads what is
+    // there.
+    sr_status clear_fresh_order(cudaStream_t st) {
+        for (DevBuf* b : {&rvals, &rvals_alt}) {
+            if (b->fresh) CUDA_TRY(cudaMemsetAsync(b->p, 0, b->cap, st));
+            b->fresh = false;
+        }
+        return SR_OK;
+    }
+
     // Buffers of the stages after the count, for `cap` records and `dcap`
     // draw records.
     sr_status reserve(int64_t cap, int64_t dcap) {
@@ -945,6 +951,7 @@ struct Pipeline {
     // no wait).  The kernels read the actual count from offs[C].
     sr_status enqueue_back(cudaStream_t st, int64_t cap, int64_t dcap_req) {
         using namespace sr;
+        SR_TRY(clear_fresh_order(st));
         uint32_t* ctlp = ctl.as<uint32_t>();
         uint32_t* status = ctlp + CTL_STATUS;
         const bool keep = (flags & SR_FLAG_KEEP_STAGES) != 0;
@@ -1510,6 +1517,7 @@ sr_status sr_render_draw_list(sr_ctx* c, const int32_t* records, int64_t n, void
     CUDA_TRY(ensure(p.rvals, sizeof(uint32_t) * n1));
     CUDA_TRY(ensure(p.rkeys_alt, sizeof(uint32_t) * n1));
     CUDA_TRY(ensure(p.rvals_alt, sizeof(uint32_t) * n1));
+    SR_TRY(p.clear_fresh_order(st));
     CUDA_TRY(ensure(p.row_start, sizeof(int32_t) * ((size_t)rows + 1)));
     CUDA_TRY(cudaMemsetAsync(p.ctl.p, 0, sizeof(uint32_t) * CTL_WORDS, st));
     if (n) {
