@@ -49,7 +49,7 @@ L2_FLUSH_BYTES = 256 << 20
 # "served" (scene index, hash) of served requests
 CHECKS = {"batch": [], "served": []}
 ORACLE_SAMPLE = 64
-# What bounds each stage's main kernel (profiles/ncu_top_kernels_frame4096.md):
+# What bounds each stage's main kernel, from its counters on the 4096^2 frame:
 # the HBM fraction is the roofline only for the stages that move bytes.
 LIMITS = {
     "resolve": "instruction issue: the walk back to each segment's collapse cut, then some 20 a record",

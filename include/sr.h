@@ -38,7 +38,8 @@ typedef enum sr_status {
     SR_OK = 0,
     SR_ERR_INVALID_ARG = 1,   /* bad pointer, size, curve type or fill rule  */
     SR_ERR_OOM = 2,           /* device or host allocation failed             */
-    SR_ERR_OVERFLOW_REFIT = 3,/* a pre-sized buffer overflowed; rerun exact   */
+    SR_ERR_OVERFLOW_REFIT = 3,/* a pre-sized buffer overflowed; rerun exact;
+                               * or more records than a frame takes (2^30)  */
     SR_ERR_TIMEOUT = 4,       /* a bounded device-side wait gave up           */
     SR_ERR_CUDA = 5,          /* a CUDA runtime call failed                   */
     SR_ERR_NO_SCENE = 6,      /* render called before a scene was loaded      */
@@ -244,7 +245,10 @@ typedef enum sr_stage {
 
 /* Copies one stage of the last sr_render (made with SR_FLAG_KEEP_STAGES) to
  * host memory.  If dst is NULL only *bytes is set to the size needed;
- * otherwise *bytes must hold the capacity of dst on entry. */
+ * otherwise *bytes must hold the capacity of dst on entry.  The intersection
+ * records' flags and the draw list are made when they are asked for (with or
+ * without the flag): SR_ERR_INVALID_ARG after a frame that failed before it
+ * had them, SR_ERR_TIMEOUT where a wait of that gives up. */
 sr_status sr_debug_dump(sr_ctx* ctx, int stage, void* dst, size_t* bytes);
 
 /* Replaces the destructor of ScanlineVGRasterizer. */
@@ -294,12 +298,13 @@ sr_status sr_exclusive_scan_i32_noalloc(const int32_t* d_in, int32_t* d_out, int
 sr_status sr_scan_status(void* stream);
 
 /* Sets how many polls every bounded device-side wait (the look-backs of the
- * scans, of the radix sort and of the winding pass) makes before it gives up
- * and the call reports SR_ERR_TIMEOUT; 0 restores the default of 2^22 polls
- * with back-off (a second or more).  Kernels launched after the call use the
- * new limit, in every context of the process; a captured batch graph keeps
- * the limit it was captured with.  No reference counterpart (its waits are
- * host-side queue idles). */
+ * scans, of the radix sort and of the winding pass, and the tile sort's wait
+ * for its copies) makes before it gives up and the call reports
+ * SR_ERR_TIMEOUT (the image of that frame is not painted, or wrong); 0 restores
+ * the default of 2^22 polls with back-off (a second or more).  Kernels launched
+ * after the call use the new limit, in every context of the process; a captured
+ * batch graph keeps the limit it was captured with.  No reference counterpart
+ * (its waits are host-side queue idles). */
 void sr_set_spin_limit(uint32_t polls);
 
 /* Test hook for the bounded waits: the allocating standalone scan with its
@@ -336,7 +341,9 @@ typedef struct sr_synth_params sr_synth_params;
 typedef struct sr_batch_render_opts {
     uint32_t struct_size;
     uint32_t use_graph;          /* capture the frame as a CUDA graph and replay it
-                                    (needs record_capacity >= 0) */
+                                    (needs record_capacity >= 0); captured again
+                                    with other capacities, or once another frame
+                                    has moved one of the batch's buffers */
     int64_t  record_capacity;    /* < 0: size exactly (one host wait for the
                                     record count, as the reference does);
                                     >= 0: pre-sized, no mid-frame wait */

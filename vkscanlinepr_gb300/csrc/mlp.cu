@@ -335,9 +335,9 @@ SR_DEV void red_add4(float* p, float a, float b, float c, float d) {
 // in the order the warps come differs by up to 3e-6 from run to run).  With
 // `adam`, the CTA that finishes last takes the optimiser step (a launch and its
 // gap saved).
-// Shared-memory reads and the latency of its eight phases bound it: a step
-// of 4,096 samples takes 23 us, where 64 CTAs of 64 threads, a sample each,
-// and a separate optimiser launch took 84.
+// Shared-memory reads and the latency of its eight phases bound it: 16 steps
+// of 4,096 samples and the two shuffles before them take 515 us, where 64 CTAs
+// of 64 threads, a sample each, and a separate optimiser launch took 1,740.
 constexpr int kSamples = 32, kGradThreads = 512;
 struct GradSmem {
     Params P;

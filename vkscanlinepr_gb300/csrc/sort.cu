@@ -6,7 +6,8 @@
 // path in its high bits (see pack_key), so one stable sort of the whole
 // array by key gives the reference's per-path order by (signed yx, index).
 //
-// Per pass, each CTA (dynamic tile id) loads a 4096-key tile, ranks keys by
+// Per pass, each CTA takes tile after tile (from a counter; 8, 12 or 16 keys a
+// thread, 3,072 keys by default), ranks keys by
 // digit with warp __match_any_sync / popc, publishes its per-digit counts,
 // and looks back over earlier tiles' per-digit counts to find where its run
 // of each digit starts; the thread of a digit reads the words of 8
@@ -36,8 +37,7 @@ constexpr int kLookWindow = 8;     // look-back words read per step
 // Lanes holding the same digit: one __match_any_sync, or one ballot per
 // digit bit (9 bits: digit 256 marks an empty slot).  The 64-bit fragment
 // keys are ranked by ballots (their low digits vary a lot within a warp);
-// the 32-bit keys (draw rows, chain classes) arrive in runs, where one
-// match is cheaper.
+// the 32-bit keys (draw rows) arrive in runs, where one match is cheaper.
 template <bool kMatchAny> SR_DEV uint32_t same_digit_lanes(uint32_t d) {
     if (kMatchAny) return __match_any_sync(0xFFFFFFFFu, d);
     uint32_t peers = 0xFFFFFFFFu;

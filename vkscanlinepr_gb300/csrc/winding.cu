@@ -16,7 +16,9 @@
 //                         and the paint runs at their output slots (one
 //                         decoupled look-back over the tiles' run counts).
 // k_draw_list writes the reference's draw records, in its order (a record's
-// merged fragment, then the span ending at it), when they are read back.
+// merged fragment, then the span ending at it), when they are read back.  It
+// finds flags and centre sums by itself, from whole 64-bit keys: a change of
+// rule goes into both (the read-back tests hold them together).
 //
 // The reference's winding scan is global over its one scene's records
 // (scanline_rasterizer.cpp:479-506), so a path whose changes do not sum to
