@@ -243,24 +243,20 @@ SR_DEV int32_t axis_range_rd(float a0, float a1, int32_t size, int32_t F, float&
     return n;
 }
 
-// out[from, to) = value, for each lane whose range is not empty, by its warp.
-SR_DEV void fill_ranges(uint32_t* __restrict__ out, uint32_t from, uint32_t to, uint32_t value) {
-    const uint32_t lane = lane_id();
-    for (uint32_t m = __ballot_sync(0xFFFFFFFFu, from < to); m; m &= m - 1) {
-        const int l = __ffs(m) - 1;
-        const uint32_t a = __shfl_sync(0xFFFFFFFFu, from, l), b = __shfl_sync(0xFFFFFFFFu, to, l);
-        const uint32_t v = __shfl_sync(0xFFFFFFFFu, value, l);
-        const uint32_t a4 = min((a + 3u) & ~3u, b), b4 = max(b & ~3u, a4);   // whole 16 bytes between
-        if (a + lane < a4) out[a + lane] = v;
-        for (uint32_t q = a4 + 4 * lane; q < b4; q += 128) *reinterpret_cast<uint4*>(out + q) = make_uint4(v, v, v, v);
-        if (b4 + lane < b) out[b4 + lane] = v;
-    }
+// out[from, to) = value, by the CTA.
+SR_DEV void fill_range(uint32_t* __restrict__ out, uint32_t from, uint32_t to, uint32_t value) {
+    const uint32_t t = threadIdx.x, nt = blockDim.x;
+    const uint32_t a = min((from + 3u) & ~3u, to), b = max(to & ~3u, a);   // whole 16 bytes between
+    if (from + t < a) out[from + t] = value;
+    for (uint32_t q = a + 4 * t; q < b; q += 4 * nt)
+        *reinterpret_cast<uint4*>(out + q) = make_uint4(value, value, value, value);
+    if (b + t < to) out[b + t] = value;
 }
 
 // ---------------------------------------------------------------- K2 ----
 // Paths without curves in a row that a curve's own thread gives their first
-// curve; longer rows take its warp (a thread alone took 10 ms for 2 million
-// such paths, the warp 0.1).
+// curve; longer rows take its CTA (2 million such paths took a thread alone 9
+// ms, a warp 0.17, the CTA 0.12).
 constexpr uint32_t kPathGap = 32;
 // LANES 8: eight lanes a curve, a piece each, for a frame of few curves, whose
 // time is one curve's serial set-up: 9.8 instead of 15 us for 5,000 curves (but
@@ -279,11 +275,13 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const GeomArgs g, float
                                                uint32_t* __restrict__ class_count, uint32_t* __restrict__ status) {
     wait_for_stream();
     __shared__ uint32_t s_hist[kChainClasses], s_total, s_base;
+    __shared__ uint3 s_gap[kCountThreads / LANES + 1];   // paths [x, y) begin at curve z
+    __shared__ uint32_t s_gaps;
     const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) / LANES;
     const uint32_t sub = LANES == 1 ? 0u : threadIdx.x % LANES;   // the piece that this lane sets up
     const bool active = c < g.n_curves;
     if (threadIdx.x < kChainClasses) s_hist[threadIdx.x] = 0;
-    if (threadIdx.x == kChainClasses) s_total = 0;
+    if (threadIdx.x == kChainClasses) s_total = s_gaps = 0;
     __syncthreads();
     constexpr int kMine = LANES == 1 ? kMaxPieces : 1;   // pieces a lane
     uint32_t my_chains[2 * kMine];
@@ -447,33 +445,27 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const GeomArgs g, float
             walk = wadd(walk, __shfl_down_sync(0xFFFFFFFFu, walk, d, LANES));
         }
     }
-    // first curve of every path up to this curve's (curves are grouped by path,
-    // in order; a path without curves starts where the next does)
-    uint32_t gap0 = 0, gap1 = 0, end0 = 0, end1 = 0;
     if (active && sub == 0) {
         const uint32_t path = g.curve_path[c];
         count[c] = pc;
+        // first curve of every path up to this curve's (curves are grouped by
+        // path, in order; a path without curves starts where the next does)
         const uint32_t first = c ? g.curve_path[c - 1] + 1u : 0u;
         if (path + 1u - first > kPathGap) {
-            gap0 = first;
-            gap1 = path + 1u;
+            s_gap[atomicAdd(&s_gaps, 1u)] = make_uint3(first, path + 1u, c);
         } else {
             for (uint32_t q = first; q <= path; ++q) g.path_begin[q] = c;
         }
-        if (c == g.n_curves - 1) {
-            end0 = path + 1u;
-            end1 = g.n_paths + 1u;
-        }
+        if (c == g.n_curves - 1) s_gap[atomicAdd(&s_gaps, 1u)] = make_uint3(path + 1u, g.n_paths + 1u, g.n_curves);
         if (walk != pc) set_error(status, ERR_RECORD_RANGE);
     }
-    fill_ranges(g.path_begin, gap0, gap1, c);
-    fill_ranges(g.path_begin, end0, end1, g.n_curves);
     // append the chains with their classes, and count the classes (one
     // append and at most one add per class for the CTA)
     uint32_t at = 0;
     if (n_chains) at = atomicAdd(&s_total, (uint32_t)n_chains);
     for (int k = 0; k < n_chains; ++k) atomicAdd(&s_hist[my_key[k]], 1u);
     __syncthreads();
+    for (uint32_t i = 0; i < s_gaps; ++i) fill_range(g.path_begin, s_gap[i].x, s_gap[i].y, s_gap[i].z);
     if (threadIdx.x < kChainClasses && s_hist[threadIdx.x]) atomicAdd(&class_count[threadIdx.x], s_hist[threadIdx.x]);
     if (threadIdx.x == kChainClasses && s_total) s_base = atomicAdd(chain_count, s_total);
     __syncthreads();
