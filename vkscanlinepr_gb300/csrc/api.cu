@@ -68,7 +68,6 @@ struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
     uint32_t moves = 0;   // times the memory was replaced
-    bool fresh = false;   // nothing has been written to it yet
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
@@ -89,7 +88,6 @@ cudaError_t ensure(DevBuf& b, size_t bytes, bool slack = true) {
         return e;
     }
     b.cap = want;
-    b.fresh = true;
     return cudaSuccess;
 }
 
@@ -885,18 +883,6 @@ struct Pipeline {
         return t;
     }
 
-    // The row order's buffers hold indexes of draw records from their first
-    // use on: where a frame fails (keys left unsorted, a wait that gave up), it
-    // has places that nobody wrote in this frame, and the resolve reads what is
-    // there.
-    sr_status clear_fresh_order(cudaStream_t st) {
-        for (DevBuf* b : {&rvals, &rvals_alt}) {
-            if (b->fresh) CUDA_TRY(cudaMemsetAsync(b->p, 0, b->cap, st));
-            b->fresh = false;
-        }
-        return SR_OK;
-    }
-
     // Buffers of the stages after the count, for `cap` records and `dcap`
     // draw records.
     sr_status reserve(int64_t cap, int64_t dcap) {
@@ -951,7 +937,6 @@ struct Pipeline {
     // no wait).  The kernels read the actual count from offs[C].
     sr_status enqueue_back(cudaStream_t st, int64_t cap, int64_t dcap_req) {
         using namespace sr;
-        SR_TRY(clear_fresh_order(st));
         uint32_t* ctlp = ctl.as<uint32_t>();
         uint32_t* status = ctlp + CTL_STATUS;
         const bool keep = (flags & SR_FLAG_KEEP_STAGES) != 0;
@@ -1517,7 +1502,6 @@ sr_status sr_render_draw_list(sr_ctx* c, const int32_t* records, int64_t n, void
     CUDA_TRY(ensure(p.rvals, sizeof(uint32_t) * n1));
     CUDA_TRY(ensure(p.rkeys_alt, sizeof(uint32_t) * n1));
     CUDA_TRY(ensure(p.rvals_alt, sizeof(uint32_t) * n1));
-    SR_TRY(p.clear_fresh_order(st));
     CUDA_TRY(ensure(p.row_start, sizeof(int32_t) * ((size_t)rows + 1)));
     CUDA_TRY(cudaMemsetAsync(p.ctl.p, 0, sizeof(uint32_t) * CTL_WORDS, st));
     if (n) {
@@ -1529,7 +1513,7 @@ sr_status sr_render_draw_list(sr_ctx* c, const int32_t* records, int64_t n, void
     uint32_t* status = p.ctl.as<uint32_t>() + CTL_STATUS;
     sr::launch_sort_u32(rp, p.draw_row.as<uint32_t>(), nullptr, p.rkeys.as<uint32_t>(), p.rvals.as<uint32_t>(),
                         p.rkeys_alt.as<uint32_t>(), p.rvals_alt.as<uint32_t>(), p.row_sort_scratch.p, status, st);
-    sr::launch_row_bounds(p.rkeys.as<uint32_t>(), n, nullptr, rows, p.row_start.as<int32_t>(), st);
+    sr::launch_row_bounds(p.rkeys.as<uint32_t>(), n, nullptr, rows, p.row_start.as<int32_t>(), status, st);
     sr::ResolveArgs ra;
     ra.draw = p.draw.as<int4>();
     ra.row_sorted_idx = p.rvals.as<uint32_t>();

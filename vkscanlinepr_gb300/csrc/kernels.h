@@ -180,6 +180,11 @@ struct SortPlan {
     int items;                 // keys per thread of a tile: 8, 12 or 16
     int cleared = 0;           // 1: the caller has zeroed the scratch
     int hist_given = 0;        // 1: the digit counts are in the scratch (launch_row_starts), the rest zeroed
+    // Where a wait of the sort gives up, it has left places of the order
+    // unwritten, and the rows become empty: their starts (set by
+    // launch_row_starts; NULL: none)
+    int32_t* row_start = nullptr;
+    uint32_t rows = 0;
 };
 SortPlan sort_plan(int64_t n, uint32_t key_bits, const uint32_t* n_dev = nullptr, int items = 12);
 // Device scratch needed by a plan (bytes).
@@ -196,7 +201,7 @@ void launch_sort_u64(const SortPlan& p, const uint64_t* keys_in, const uint32_t*
 // zeroed).
 bool row_sort_one_pass(int64_t n, uint32_t rows);
 size_t row_sort_bytes(int64_t n, uint32_t rows);
-void launch_row_sort(const uint32_t* rows_in, int64_t n, const uint32_t* n_dev, uint32_t rows, const int32_t* row_start,
+void launch_row_sort(const uint32_t* rows_in, int64_t n, const uint32_t* n_dev, uint32_t rows, int32_t* row_start,
                      uint32_t* idx_out, void* scratch, uint32_t* status, cudaStream_t st);
 // For a sort by row whose records per row are known: each row's first
 // position row_start[0..rows] (exclusive scan; look-back words and counter
@@ -349,9 +354,10 @@ void launch_aa_accumulate(const uint32_t* img, void* acc, size_t n, bool first, 
 void launch_aa_resolve(const void* acc, uint32_t* img, uint32_t* img2, size_t n, uint32_t k, cudaStream_t st);
 // n pixels from a framebuffer to device memory of this device.
 void launch_copy_image(const uint32_t* src, uint32_t* dst, size_t n, int sm_count, cudaStream_t st);
-// n_dev (optional) holds the record count; n is the capacity.
+// n_dev (optional) holds the record count; n is the capacity.  With a status
+// set by then (the sort gave up) every row is empty.
 void launch_row_bounds(const uint32_t* srows, int64_t n, const uint32_t* n_dev, int32_t rows, int32_t* row_start,
-                       cudaStream_t st);
+                       const uint32_t* status, cudaStream_t st);
 
 // ---- mlp.cu  (learned sizing: 6 features -> 64 -> 64 -> 2, GELU)
 constexpr int kMlpIn = 6, kMlpHidden = 64, kMlpOut = 2;

@@ -20,7 +20,12 @@ namespace sr {
 
 // First index of every cell row in the row-sorted draw list.
 __global__ void k_row_bounds(const uint32_t* __restrict__ srows, int64_t n_cap, const uint32_t* __restrict__ n_dev,
-                             int32_t rows, int32_t* __restrict__ row_start) {
+                             int32_t rows, int32_t* __restrict__ row_start, const uint32_t* __restrict__ status) {
+    if (*status) {   // the order has places that nobody wrote
+        const int32_t step = (int32_t)(gridDim.x * blockDim.x);
+        for (int32_t r = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x); r <= rows; r += step) row_start[r] = 0;
+        return;
+    }
     const int64_t n = n_dev ? (int64_t)min((uint64_t)*n_dev, (uint64_t)n_cap) : n_cap;
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += stride) {
@@ -659,12 +664,12 @@ void launch_copy_image(const uint32_t* src, uint32_t* dst, size_t n, int sm_coun
 }
 
 void launch_row_bounds(const uint32_t* srows, int64_t n, const uint32_t* n_dev, int32_t rows, int32_t* row_start,
-                       cudaStream_t st) {
+                       const uint32_t* status, cudaStream_t st) {
     int64_t work = n + 1;
     int blocks = (int)((work + 255) / 256);
     if (blocks > 1216) blocks = 1216;
     count_launches(1);
-    k_row_bounds<<<blocks, 256, 0, st>>>(srows, n, n_dev, rows, row_start);
+    k_row_bounds<<<blocks, 256, 0, st>>>(srows, n, n_dev, rows, row_start, status);
 }
 
 }  // namespace sr

@@ -166,6 +166,14 @@ __global__ void __launch_bounds__(kThreads) k_row_starts(const uint32_t* __restr
     scan_tile_values<1, kThreads>(v, row_start, rows, tile, tstat, status, spin_limit, s_warp, &total);
 }
 
+// A wait of the row order gave up: some of its places will not be written, and
+// the resolve, which would read what they hold, finds the rows empty.
+SR_DEV void give_up_rows(int32_t* row_start, uint32_t rows, uint32_t* status) {
+    set_error(status, ERR_LOOKBACK_TIMEOUT);
+    if (row_start)
+        for (uint32_t r = 0; r <= rows; ++r) row_start[r] = 0;
+}
+
 // ------------------------------------------------ row sort in one pass ---
 // The order of the paint runs by row, stable, for frames of up to 1,024 rows:
 // one pass with a digit a row.  The rows' starts are known (k_row_starts), so
@@ -190,9 +198,9 @@ constexpr int kRowSortTile = kThreads * kRowItems;
 template <int BITS>
 __global__ void __launch_bounds__(kThreads) k_row_sort(const uint32_t* __restrict__ rows_in, int64_t n_max,
                                                        const uint32_t* __restrict__ n_dev, uint32_t rows,
-                                                       const int32_t* __restrict__ row_start,
-                                                       uint32_t* __restrict__ idx_out, uint32_t* __restrict__ lookback,
-                                                       uint32_t* counter, uint32_t* status, uint32_t spin_limit) {
+                                                       int32_t* row_start, uint32_t* __restrict__ idx_out,
+                                                       uint32_t* __restrict__ lookback, uint32_t* counter,
+                                                       uint32_t* status, uint32_t spin_limit) {
     wait_for_stream();
     constexpr int kR = 1 << BITS, kPer = kR / kThreads;
     __shared__ __align__(16) uint16_t hist[kWarps][kR];
@@ -286,7 +294,7 @@ __global__ void __launch_bounds__(kThreads) k_row_sort(const uint32_t* __restric
         if (!left) break;
         if (!moved) {
             if (++spins > spin_limit) {
-                set_error(status, ERR_LOOKBACK_TIMEOUT);
+                give_up_rows(row_start, rows, status);
                 break;
             }
             __nanosleep(32);
@@ -336,12 +344,17 @@ __global__ void __launch_bounds__(kThreads, onesweep_min_blocks(kVals, ITEMS)) k
                                                        uint32_t shift, uint32_t dmask,
                                                        const uint32_t* __restrict__ digit_count,
                                                        uint32_t* __restrict__ lookback, uint32_t* counter,
-                                                       uint32_t* status, uint32_t spin_limit) {
+                                                       int32_t* row_start, uint32_t rows, uint32_t* status,
+                                                       uint32_t spin_limit) {
     wait_for_stream();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int kItems = ITEMS, kTile = kThreads * ITEMS;
     OnesweepSmem<K, kVals, ITEMS>& S = *reinterpret_cast<OnesweepSmem<K, kVals, ITEMS>*>(smem_raw);
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    // (rows whose counts were left out, as some look-back before had given up,
+    // leave places unwritten too)
+    if (row_start && blockIdx.x == 0 && *status != 0u)
+        for (uint32_t r = threadIdx.x; r <= rows; r += kThreads) row_start[r] = 0;
     const int64_t n = n_dev ? (int64_t)min((uint64_t)*n_dev, (uint64_t)n_max) : n_max;
     // tile after tile until the input's end: the grid follows the GPU, not the
     // capacity, of which a frame's runs are a fraction (a CTA a tile of the
@@ -446,7 +459,7 @@ __global__ void __launch_bounds__(kThreads, onesweep_min_blocks(kVals, ITEMS)) k
                 look -= used;
                 if (used == 0) {
                     if (++spins > spin_limit) {
-                        set_error(status, ERR_LOOKBACK_TIMEOUT);
+                        give_up_rows(row_start, rows, status);
                         break;
                     }
                     __nanosleep(32);
@@ -520,7 +533,8 @@ static void sort_impl(const SortPlan& p, const K* keys_in, const uint32_t* vals_
         count_launches(1);
         launch_after(k_onesweep<K, kVals, ITEMS>, grid, kThreads, smem, st, ksrc, vsrc, kdst, vdst, p.n, p.n_dev,
                      pass * kRadixBits, digit_mask(p.key_bits, pass * kRadixBits), s.hist + pass * kRadix,
-                     s.lookback + (size_t)pass * (p.tiles + 1) * kRadix, s.counters + pass, status, spin_limit());
+                     s.lookback + (size_t)pass * (p.tiles + 1) * kRadix, s.counters + pass, p.row_start, p.rows, status,
+                     spin_limit());
         ksrc = kdst;
         vsrc = vdst;
     }
@@ -562,7 +576,7 @@ size_t row_sort_bytes(int64_t n, uint32_t rows) {
     return 256 + sizeof(uint32_t) * (tiles << row_sort_bits(rows));
 }
 
-void launch_row_sort(const uint32_t* rows_in, int64_t n, const uint32_t* n_dev, uint32_t rows, const int32_t* row_start,
+void launch_row_sort(const uint32_t* rows_in, int64_t n, const uint32_t* n_dev, uint32_t rows, int32_t* row_start,
                      uint32_t* idx_out, void* scratch, uint32_t* status, cudaStream_t st) {
     if (n <= 0) return;
     uint32_t* counter = static_cast<uint32_t*>(scratch);
@@ -584,6 +598,8 @@ void launch_row_starts(SortPlan& p, const uint32_t* row_count, uint32_t rows, in
                        uint64_t* tile_status, uint32_t* tile_counter, uint32_t* status, cudaStream_t st) {
     p.cleared = 1;
     p.hist_given = 1;
+    p.row_start = row_start;
+    p.rows = rows;
     if (rows == 0) {
         cudaMemsetAsync(row_start, 0, sizeof(int32_t), st);
         return;
